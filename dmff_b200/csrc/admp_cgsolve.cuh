@@ -1,5 +1,5 @@
-// The whole induced-dipole CG solve in one persistent cooperative launch (FP32 engines, meshes of
-// at most 64 points per axis).
+// The whole induced-dipole CG solve in one persistent cooperative launch (FP32 engines, meshes that
+// the direct DFT convolution serves).
 //
 // The dipole solve of the reference (pme.py:342-423 solves A U = -E_perm by fixed-point steps;
 // the engine uses preconditioned CG on the same linear system) repeats, per iteration, a chain of
@@ -10,8 +10,8 @@
 // and decides convergence on the device; the passes are separated by a grid barrier:
 //   A  p = z + beta p                                   (beta = rz_k-1 / rz_k-2)
 //   B  matvec warps (fmv = A_real p, p . fmv) and spread warps (p onto the mesh)
-//   C  forward x-plane FFT passes        D  spectrum columns (x FFT, * G, inverse x FFT)
-//   E  inverse x-plane FFT passes        F  field gather (Ap, p . Ap)
+//   C  forward x-plane DFT passes        D  spectrum columns (x DFT, * G, inverse x DFT)
+//   E  inverse x-plane DFT passes        F  field gather (Ap, p . Ap)
 //   G  alpha = rz / pAp, x += alpha p, r -= alpha (Ap + fmv), z = M r, rz and rr reduced
 // (with phase_ns set, block 0 adds the device-clock time of each pass, barrier included)
 // then rr decides: stop when sqrt(rr / 3n) <= tol sqrt(bb / 3n) or at max_iter.
@@ -28,7 +28,7 @@
 #pragma once
 #include <cuda/atomic>
 
-#include "admp_fftconv.cuh"
+#include "admp_dftconv.cuh"
 #include "admp_real.cuh"
 #include "admp_recip.cuh"
 #include "common.cuh"
@@ -75,18 +75,19 @@ __device__ inline bool cg_grid_sync(const CgBarrier& b, unsigned nblocks) {
             cnt.store(0u, cuda::memory_order_relaxed);
             gen.store(g + 1u, cuda::memory_order_release);
         } else {
-            const long long t0 = cg_clock_ns();
-            while (gen.load(cuda::memory_order_acquire) == g) {
-                if (st.load(cuda::memory_order_relaxed) != 0 || cg_clock_ns() - t0 > b.wait_ns) {
+            long long t0 = 0;
+            for (unsigned poll = 1; gen.load(cuda::memory_order_acquire) == g; ++poll) {
+                if (poll & 63u) continue;
+                const long long now = cg_clock_ns();
+                if (t0 == 0) t0 = now;
+                if (st.load(cuda::memory_order_relaxed) != 0 || now - t0 > b.wait_ns) {
                     int expect = 0;
                     st.compare_exchange_strong(expect, DMFFB_CG_TIMEOUT, cuda::memory_order_relaxed);
                     ok = 0;
                     break;
                 }
-                __nanosleep(40);
             }
         }
-        if (st.load(cuda::memory_order_acquire) != 0) ok = 0;
         s_ok = ok;
     }
     __syncthreads();
@@ -110,7 +111,7 @@ struct CgSolveArgs {
     double gscale;  // 2 * DIELECTRIC
     double self1;
     // convolution (grid_in: the spread mesh, grid_out: the convolved mesh)
-    FftConvArgs fc;
+    DftConvArgs<float> fc;
     // scalars
     double* acc;         // [4][4] {p.Ap recip, p.fmv, rz, rr}, zero at launch
     const double* init;  // [0] r.z, [3] r.r, [4] b.b of the initial residual
@@ -121,23 +122,29 @@ struct CgSolveArgs {
     unsigned long long* phase_ns;  // [8] time per pass summed over the iterations (block 0), or null
 };
 
+// elements of the largest working area of the convolution passes
+__host__ __device__ inline size_t cg_work_elems(const DftConvArgs<float>& a) {
+    const size_t f = dft_fwd_elems(a), c = dft_col_elems(a), i = dft_inv_elems(a);
+    const size_t m = f > c ? (f > i ? f : i) : (c > i ? c : i);
+    return (m + 3) & ~(size_t)3;
+}
+
 __global__ void __launch_bounds__(kCgThreads) k_cg_solve(CgSolveArgs a) {
-    extern __shared__ float2 sm[];
+    extern __shared__ __align__(16) unsigned char dft_sm[];
+    float* const sm = (float*)dft_sm;
+    // the DFT matrices stay in shared memory for the whole solve
+    float* const wx = sm + cg_work_elems(a.fc);
+    float* const wy = wx + dft_mat_elems(a.fc.H[0]);
+    float* const wz = wy + dft_mat_elems(a.fc.H[1]);
+    dft_load_mat(a.fc, 0, wx);
+    dft_load_mat(a.fc, 1, wy);
+    dft_load_mat(a.fc, 2, wz);
     const unsigned nb = gridDim.x;
     const int tid = threadIdx.x, nth = blockDim.x;
     const int lane = tid & 31;
     const int warps_cta = nth >> 5;
     const int gwarp = blockIdx.x * warps_cta + (tid >> 5), nwarps = nb * warps_cta;
     const int m3 = 3 * a.n;
-    // stage twiddles of the three line lengths stay in shared memory for the whole solve
-    const size_t work = fc_plane_work(a.fc.K) > fc_col_work(a.fc.K) ? fc_plane_work(a.fc.K) : fc_col_work(a.fc.K);
-    float2* twx = sm + work / sizeof(float2);
-    float2* twy = twx + kFcTw;
-    float2* twz = twy + kFcTw;
-    fc_load_twiddles(twx, a.fc.tw[0], tid, nth);
-    fc_load_twiddles(twy, a.fc.tw[1], tid, nth);
-    fc_load_twiddles(twz, a.fc.tw[2], tid, nth);
-    __syncthreads();
     SpreadArgs<float> sa;
     sa.n = a.n;
     sa.pos = nullptr;
@@ -146,7 +153,7 @@ __global__ void __launch_bounds__(kCgThreads) k_cg_solve(CgSolveArgs a) {
     sa.q1 = nullptr;
     sa.lmax = 1;
     sa.g = a.g;
-    sa.grid = a.fc.grid_in;
+    sa.grid = a.fc.zero_real;
     sa.perm_mul = a.perm_mul;
     FieldCombine cmb;
     cmb.U = a.p;
@@ -157,8 +164,8 @@ __global__ void __launch_bounds__(kCgThreads) k_cg_solve(CgSolveArgs a) {
     double rr = a.init[3];
     int it = 0, conv = 0, status = 0;
     double rz1 = a.init[0], rz2 = 0.0;  // rz of iterations k - 1 and k - 2
-    const int ncol = a.fc.K[1] * a.fc.Kh;
-    const int ncb = (ncol + kFcCols - 1) / kFcCols;
+    const int nfwd = dft_fwd_items(a.fc), ncol = dft_col_items(a.fc), ninv = dft_inv_items(a.fc);
+    const int K3 = a.fc.K[0] * a.fc.K[1] * a.fc.K[2];
     // pass timing on block 0 (device clock at each barrier exit)
     const bool timed = a.phase_ns && blockIdx.x == 0 && tid == 0;
     long long tp = timed ? cg_clock_ns() : 0;
@@ -199,13 +206,26 @@ __global__ void __launch_bounds__(kCgThreads) k_cg_solve(CgSolveArgs a) {
         if (!cg_grid_sync(a.bar, nb)) break;
         mark(1);
         // C, D, E: the convolution
-        for (int x = blockIdx.x; x < a.fc.K[0]; x += nb) fc_fwd_plane(a.fc, x, sm, twy, twz);
+        for (int w = blockIdx.x; w < nfwd; w += nb) {
+            dft_fwd_item<float, 1, 1>(a.fc, w, sm, wy, wz);
+            __syncthreads();
+        }
         if (!cg_grid_sync(a.bar, nb)) break;
         mark(2);
-        for (int c = blockIdx.x; c < ncb; c += nb) fc_column_block(a.fc, c * kFcCols, sm, twx);
+        {
+            double none[7];  // no energy sums in the solve
+            for (int w = blockIdx.x; w < ncol; w += nb) {
+                dft_col_item<float, 1, 1, true>(a.fc, w, sm, wx, none);
+                __syncthreads();
+            }
+            for (int k = blockIdx.x * nth + tid; k < K3; k += nb * nth) a.fc.zero_real[k] = 0.f;
+        }
         if (!cg_grid_sync(a.bar, nb)) break;
         mark(3);
-        for (int x = blockIdx.x; x < a.fc.K[0]; x += nb) fc_inv_plane(a.fc, x, sm, twy, twz);
+        for (int w = blockIdx.x; w < ninv; w += nb) {
+            dft_inv_item<float, 1, 1>(a.fc, w, sm, wy, wz);
+            __syncthreads();
+        }
         if (!cg_grid_sync(a.bar, nb)) break;
         mark(4);
         // F: field gather, Ap = recip field of p + (1/pol + self) p
@@ -252,10 +272,9 @@ __global__ void __launch_bounds__(kCgThreads) k_cg_solve(CgSolveArgs a) {
     }
 }
 
-// dynamic shared memory of k_cg_solve: the larger FFT working area + three twiddle tables
-__host__ inline size_t cg_solve_smem(const int K[3]) {
-    const size_t pw = fc_plane_work(K), cw = fc_col_work(K);
-    return (pw > cw ? pw : cw) + 3 * kFcTw * sizeof(float2);
+// dynamic shared memory of k_cg_solve: the convolution passes' working area and the DFT matrices
+__host__ inline size_t cg_solve_smem(const DftConvArgs<float>& a) {
+    return sizeof(float) * (cg_work_elems(a) + dft_mat_elems(a.H[0]) + dft_mat_elems(a.H[1]) + dft_mat_elems(a.H[2]));
 }
 
 }  // namespace dmffb

@@ -12,6 +12,7 @@
 #include <string>
 #include <array>
 #include <map>
+#include <mutex>
 #include <vector>
 
 #include "../../include/dmffb200.h"
@@ -23,7 +24,7 @@
 #include "disp.cuh"
 #include "classical.cuh"
 #include "nbcells.cuh"
-#include "admp_fftconv.cuh"
+#include "admp_dftconv.cuh"
 #include "admp_cgsolve.cuh"
 #include "pairwise.cuh"
 
@@ -165,10 +166,14 @@ struct dmffb_engine {
     double* d_tdprm[3] = {nullptr, nullptr, nullptr};
     bool want_pgrad = false, charges_set = false;
     bool cell_pass = false;  // dmffb_classical_set_cell_pass: pairs from the cell grid, no list
-    // dipole-solve convolution in one thread-block cluster (FP32, meshes up to 64 per axis)
-    bool fc_enabled = false;  // dmffb_set_fused_fft
-    int fc_ok = -1;          // the engine's FFT convolution serves this mesh (1), not (0), not decided (-1)
-    float2* d_fcW = nullptr;  // [K1][K2][K3/2+1] half spectrum between its passes
+    // mesh convolution by the engine's direct DFT kernels (admp_dftconv.cuh) or cuFFT
+    int dft_mode = -1;        // dmffb_set_fused_fft: 1 DFT kernels (meshes up to 64), 0 cuFFT, -1 the size rule
+    bool dft_used = false;    // the last convolution ran through the DFT kernels
+    void* d_dftW = nullptr;   // DFT matrices of the three axes, (K/2 + 1)^2 (cos, sin) each
+    int64_t dftW_cap = 0;
+    double* d_dftG = nullptr;  // [K1*K2*Kh] influence function of the half spectrum during a dipole solve
+    int64_t dftG_cap = 0;
+    std::array<int, 3> dft_key = {-1, -1, -1};  // the mesh of d_dftW
     int pcg_mode = 2;         // dmffb_set_persistent_cg: 0 off, 1 on, 2 for systems of at most pcg_auto_atoms
     int pcg_auto_atoms = 4096;
     int pcg_max_blocks = -1;  // co-resident k_cg_solve CTAs for the current mesh (0: unavailable, -1: not decided)
@@ -176,8 +181,6 @@ struct dmffb_engine {
     double pcg_wait_s = 2.0;  // limit of one grid-barrier wait
     int pcg_phantom = 0;      // arrivals the next persistent solve's barrier waits for beyond its CTAs (tests)
     double pcg_phase_ms[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // pass times of the persistent solves run while profiling
-    float* d_fcG = nullptr;  // [K1*K2*Kh] influence function of the half spectrum
-    int64_t fcG_cap = 0;
     int32_t* d_covrows = nullptr;  // [n_covrows*3] covalent rows (i < j, nbond)
     int64_t n_covrows = 0;
     int32_t *d_cov_lo = nullptr, *d_cov_hi = nullptr;  // [n] covalent partner index range
@@ -571,93 +574,250 @@ PairArgs<T> pair_args(dmffb_engine* h, const Box& bx, const int32_t* pairs, int6
 
 int lmax_eff(const dmffb_engine* h) { return (h->lmax == 0 && h->lpol) ? 1 : h->lmax; }
 
-// reciprocal pass: spread (Qg and/or U) -> FFT -> convolution -> inverse FFT -> gather
-// per-atom wrapped stencil origins and spline weights at these positions, for the cached dipole
-// spread and field gather of the dipole solve
 // The dynamic shared memory limit of a kernel is a property of the function, shared by every
-// engine of the process (and by the server's slot threads): it is set to what the largest mesh
-// served (64 points per axis) needs, the same value from every caller, never to one engine's own
-// need, which another engine's smaller setting would undercut at its next launch.
-const int kFcMaxMesh[3] = {kFcMaxK, kFcMaxK, kFcMaxK};
+// engine of the process (and by the server's slot threads): every caller sets the same value,
+// which no mesh that the DFT kernels serve exceeds.
+constexpr size_t kDftSmem = 200u << 10;
+constexpr int kDftCtas = 296;  // CTAs aimed at per pass: two per SM
 
-bool fc_grant_smem() {
-    return cudaFuncSetAttribute(k_fc_fwd_planes, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)fc_plane_smem(kFcMaxMesh)) == cudaSuccess &&
-           cudaFuncSetAttribute(k_fc_inv_planes, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)fc_plane_smem(kFcMaxMesh)) == cudaSuccess &&
-           cudaFuncSetAttribute(k_fc_columns, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)fc_col_smem(kFcMaxMesh)) == cudaSuccess &&
-           cudaFuncSetAttribute(k_cg_solve, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)cg_solve_smem(kFcMaxMesh)) == cudaSuccess;
+bool dft_grant_smem() {
+    static std::mutex mtx;
+    static std::map<int, bool> granted;  // per device, asked for once
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    std::lock_guard<std::mutex> lock(mtx);
+    const auto known = granted.find(dev);
+    if (known != granted.end()) return known->second;
+    granted[dev] = false;
+    const void* f[] = {(const void*)k_dft_fwd<float, 2, 2>,            (const void*)k_dft_fwd<float, 1, 1>,
+                       (const void*)k_dft_fwd<double, 2, 2>,           (const void*)k_dft_fwd<double, 1, 1>,
+                       (const void*)k_dft_columns<float, 2, 2, true>,  (const void*)k_dft_columns<float, 1, 1, true>,
+                       (const void*)k_dft_columns<double, 2, 2, true>, (const void*)k_dft_columns<double, 1, 1, true>,
+                       (const void*)k_dft_columns<float, 2, 2, false>, (const void*)k_dft_columns<float, 1, 1, false>,
+                       (const void*)k_dft_columns<double, 2, 2, false>, (const void*)k_dft_columns<double, 1, 1, false>,
+                       (const void*)k_dft_inv<float, 2, 2>,            (const void*)k_dft_inv<float, 1, 1>,
+                       (const void*)k_dft_inv<double, 2, 2>,           (const void*)k_dft_inv<double, 1, 1>,
+                       (const void*)k_cg_solve};
+    for (const void* k : f)
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDftSmem) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+    return granted[dev] = true;
 }
 
-// Whether the engine's FFT convolution serves the current mesh: FP32, extents of at most 64 points
-// and the kernels' shared memory granted; otherwise the cuFFT path runs.
-int fc_decide(dmffb_engine* h) {
-    if (h->fc_ok >= 0) return h->fc_ok;
-    h->fc_ok = 0;
-    if (h->prec != DMFFB_FP32 || !h->lpme) return 0;
-    for (int k = 0; k < 3; ++k) {
-        bool ok = false;
-        fc_plan(h->K[k], &ok);
-        if (!ok) return 0;
-    }
-    if (!fc_grant_smem()) {
-        cudaGetLastError();
-        return 0;
-    }
-    h->fc_ok = 1;
-    return 1;
+// output tile of the DFT passes: 2 x 2 on large meshes, whose shared-memory reads bound them (FP32 at
+// 61^3 40 us against 43 with single outputs, at 85^3 67 against 80), single outputs on small ones,
+// which have too few outputs per CTA to hide the reads' latency otherwise (50^3: 34 us against 40)
+constexpr int kDftWideK = 56;
+bool dft_wide_tile(const dmffb_engine* h) {
+    return std::max(h->K[0], std::max(h->K[1], h->K[2])) > kDftWideK;
 }
 
-// influence-function table and spectrum buffer of the engine's FFT convolution for this box (once
-// per dipole solve)
-int fc_prepare(dmffb_engine* h, cudaStream_t s, const Box& bx) {
-    const int Kh = h->K[2] / 2 + 1;
-    const int64_t m = (int64_t)h->K[0] * h->K[1] * Kh;
-    int st;
-    if (m > h->fcG_cap) {
-        if (h->d_fcG) cudaFree(h->d_fcG);
-        if (h->d_fcW) cudaFree(h->d_fcW);
-        h->d_fcG = nullptr;
-        h->d_fcW = nullptr;
-        h->fcG_cap = m;
-        if ((st = dalloc(h, &h->d_fcG, m * sizeof(float)))) return st;
-        if ((st = dalloc(h, &h->d_fcW, m * sizeof(float2)))) return st;
+// Geometry, matrices and work split of the DFT convolution for about `ctas` CTAs per pass (at most
+// that many when `cap`: a persistent grid then needs one round).
+template <typename T>
+DftConvArgs<T> dft_args(const dmffb_engine* h, int ctas, bool cap) {
+    using T2 = typename Vec2<T>::type;
+    DftConvArgs<T> a = {};
+    const T2* w = (const T2*)h->d_dftW;
+    for (int d = 0; d < 3; ++d) {
+        a.K[d] = h->K[d];
+        a.H[d] = h->K[d] / 2;
+        a.W[d] = w;
+        w += dft_mat_elems(a.H[d]) / 2;
     }
-    LAUNCH(h, s, KC_VEC, k_fc_gtable<<<nblk(m, 256), 256, 0, s>>>(h->K[0], h->K[1], h->K[2], Kh, bx, h->d_bmod,
-                                                                  h->kappa, fabs(det3(bx.h)), h->d_fcG));
-    CK(cudaGetLastError());
-    return DMFFB_OK;
-}
-
-FftConvArgs fc_args(dmffb_engine* h, float* in, float* out) {
-    FftConvArgs a = {};
-    for (int k = 0; k < 3; ++k) a.K[k] = h->K[k];
-    a.Kh = h->K[2] / 2 + 1;
-    a.grid_in = in;
-    a.grid_out = out;
-    a.spec = h->d_fcW;
-    a.G = h->d_fcG;
-    a.px = fc_plan(h->K[0]);
-    a.py = fc_plan(h->K[1]);
-    a.pz = fc_plan(h->K[2]);
-    fc_host_twiddles(a.px, a.tw[0]);
-    fc_host_twiddles(a.py, a.tw[1]);
-    fc_host_twiddles(a.pz, a.tw[2]);
+    const auto split = [&](int m, int per) {  // chunk of m items so that per * (number of chunks) is about ctas
+        const int want = cap ? ctas / per : (ctas + per - 1) / per;
+        const int nc = std::min(std::max(want, 1), m);
+        return (m + nc - 1) / nc;
+    };
+    const int tw = dft_wide_tile(h) ? 2 : 1;
+    a.fwd_chunk = (split(a.H[2] + 1, a.K[0]) + tw - 1) / tw * tw;
+    a.inv_chunk = (split(a.H[1] + 1, a.K[0]) + tw - 1) / tw * tw;
+    a.cols = split(a.K[1] * (a.H[2] + 1), 1);
+    a.spec = (T2*)h->d_cgrid;
+    a.bmod = h->d_bmod;
+    a.kappa = h->kappa;
+    a.kind = CK_COUL;
     return a;
 }
 
-int fc_launch(dmffb_engine* h, cudaStream_t s, float* in, float* out) {
-    static_assert(sizeof(FftConvArgs) <= 4000, "launch arguments of the FFT convolution");
-    FftConvArgs a = fc_args(h, in, out);
-    const size_t sp = fc_plane_smem(h->K), sc = fc_col_smem(h->K);
-    const int ncb = (h->K[1] * a.Kh + kFcCols - 1) / kFcCols;
-    LAUNCH(h, s, KC_FFTCONV, k_fc_fwd_planes<<<h->K[0], kFcPlaneThreads, sp, s>>>(a));
-    LAUNCH(h, s, KC_FFTCONV, k_fc_columns<<<ncb, kFcColThreads, sc, s>>>(a));
-    LAUNCH(h, s, KC_FFTCONV, k_fc_inv_planes<<<h->K[0], kFcPlaneThreads, sp, s>>>(a));
+int largest_prime(int k) {
+    int p = 1;
+    for (int f = 2; k > 1; ++f)
+        for (; k % f == 0; k /= f) p = f;
+    return p;
+}
+
+// Whether the mesh convolution runs through the DFT kernels.  They cost ~K^4 and cuFFT + k_conv ~K^3
+// with steps for large prime factors; forward + multiply + inverse in one evaluation's events (us):
+//   FP32  50: 34 / 42 cuFFT, 61: 40 / 59, 64: 48 / 43, 68: 52 / 56, 80: 65 / 59, 85: 67 / 102, 97: 104 / 131
+//   FP64  40: 31 / 44, 50: 45 / 45, 61: 53 / 72, 64: 65 / 52, 73: 85 / 98, 85: 132 / 120
+template <typename T>
+bool dft_use(const dmffb_engine* h) {
+    if (h->dft_mode == 0) return false;
+    const int kmax = std::max(h->K[0], std::max(h->K[1], h->K[2]));
+    if (std::min(h->K[0], std::min(h->K[1], h->K[2])) < 4) return false;
+    if (h->dft_mode == 1) {
+        if (kmax > 64) return false;
+    } else if (kmax > (sizeof(T) == 4 ? 63 : 49)) {
+        const int p = std::max(largest_prime(h->K[0]), std::max(largest_prime(h->K[1]), largest_prime(h->K[2])));
+        if (kmax > (sizeof(T) == 4 ? 97 : 73) || p <= 16) return false;
+    }
+    const DftConvArgs<T> a = dft_args<T>(h, kDftCtas, false);
+    return std::max(dft_fwd_smem(a), std::max(dft_col_smem(a), dft_inv_smem(a))) <= kDftSmem;
+}
+
+// DFT matrices of the current mesh: rounded from FP64, exact where the angle is a multiple of pi / 2.
+// Made at set-up where the size rule takes the DFT kernels, else when a solve or a switch asks for them.
+template <typename T>
+int dft_setup(dmffb_engine* h) {
+    const std::array<int, 3> key = {h->K[0], h->K[1], h->K[2]};
+    if (h->dft_key == key) return DMFFB_OK;
+    h->dft_key = {-1, -1, -1};
+    if (!dft_grant_smem()) return fail(h, DMFFB_CUDA_ERROR, "shared memory of the DFT kernels");
+    std::vector<T> w;
+    for (int d = 0; d < 3; ++d) {
+        const int K = h->K[d], H = K / 2;
+        std::vector<double> cs(K), sn(K);
+        for (int m = 0; m < K; ++m) {
+            const int q = 4 * m % K == 0 ? 4 * m / K : -1;  // quarter turns
+            cs[m] = q >= 0 ? (q == 0) - (q == 2) : cos(2.0 * M_PI * m / K);
+            sn[m] = q >= 0 ? (q == 1) - (q == 3) : sin(2.0 * M_PI * m / K);
+        }
+        for (int a = 0; a <= H; ++a)
+            for (int b = 0; b < dft_stride(H); ++b) {
+                w.push_back(b <= H ? (T)cs[(int64_t)a * b % K] : T(0));
+                w.push_back(b <= H ? (T)sn[(int64_t)a * b % K] : T(0));
+            }
+    }
+    int st;
+    if ((int64_t)(w.size() * sizeof(T)) > h->dftW_cap) {
+        if (h->d_dftW) cudaFree(h->d_dftW);
+        h->d_dftW = nullptr;
+        h->dftW_cap = (int64_t)(w.size() * sizeof(T));
+        if ((st = dalloc(h, (char**)&h->d_dftW, w.size() * sizeof(T)))) {
+            h->dftW_cap = 0;
+            return st;
+        }
+    }
+    CK(cudaMemcpyAsync(h->d_dftW, w.data(), w.size() * sizeof(T), cudaMemcpyHostToDevice, h->s1));
+    CK(cudaStreamSynchronize(h->s1));  // the host vector goes out of scope
+    h->dft_key = key;
+    return DMFFB_OK;
+}
+
+// the Coulomb influence function of this box for the convolutions of a dipole solve
+int dft_gtable(dmffb_engine* h, cudaStream_t s, const Box& bx) {
+    const int64_t m = (int64_t)h->K[0] * h->K[1] * (h->K[2] / 2 + 1);
+    int st;
+    if (m > h->dftG_cap) {
+        if (h->d_dftG) cudaFree(h->d_dftG);
+        h->d_dftG = nullptr;
+        h->dftG_cap = 0;
+        if ((st = dalloc(h, &h->d_dftG, m * sizeof(double)))) return st;
+        h->dftG_cap = m;
+    }
+    LAUNCH(h, s, KC_VEC, k_dft_gtable<<<nblk(m, 256), 256, 0, s>>>(h->K[0], h->K[1], h->K[2], bx, h->d_bmod, h->kappa,
+                                                                  fabs(det3(bx.h)), h->d_dftG));
     CK(cudaGetLastError());
     return DMFFB_OK;
+}
+
+// threads of a pass: its tiles per CTA and room for the loads of its input
+inline unsigned dft_threads(int tiles) { return (unsigned)std::min(kDftThreads, std::max(256, (tiles + 31) / 32 * 32)); }
+
+template <typename T, int TW, int TV>
+int dft_launch(dmffb_engine* h, cudaStream_t s, const DftConvArgs<T>& a) {
+    const auto tiles = [](int w, int v) { return ((w + TW - 1) / TW) * ((v + TV - 1) / TV); };
+    LAUNCH(h, s, KC_FFTCONV, k_dft_fwd<T, TW, TV><<<dft_fwd_items(a), dft_threads(tiles(a.H[1] + 1, a.fwd_chunk)),
+                                                    dft_fwd_smem(a), s>>>(a));
+    const unsigned nc = dft_col_items(a), tc = dft_threads(tiles(a.H[0] + 1, a.cols));
+    if (a.G && !a.want_energy) LAUNCH(h, s, KC_FFTCONV, k_dft_columns<T, TW, TV, true><<<nc, tc, dft_col_smem(a), s>>>(a));
+    else LAUNCH(h, s, KC_FFTCONV, k_dft_columns<T, TW, TV, false><<<nc, tc, dft_col_smem(a), s>>>(a));
+    LAUNCH(h, s, KC_FFTCONV, k_dft_inv<T, TW, TV><<<dft_inv_items(a), dft_threads(tiles(a.H[2] + 1, a.inv_chunk)),
+                                                    dft_inv_smem(a), s>>>(a));
+    CK(cudaGetLastError());
+    return DMFFB_OK;
+}
+
+// cuFFT plans of the current mesh (cached per mesh shape); made at set-up where the size rule takes
+// cuFFT, else when a switch asks for it
+int fft_plans(dmffb_engine* h) {
+    const std::array<int, 3> key = {h->K[0], h->K[1], h->K[2]};
+    auto it = h->plan_cache.find(key);
+    if (it == h->plan_cache.end()) {
+        cufftHandle pf = 0, pb = 0;
+        cufftType tf = h->prec == DMFFB_FP32 ? CUFFT_R2C : CUFFT_D2Z;
+        cufftType tb = h->prec == DMFFB_FP32 ? CUFFT_C2R : CUFFT_Z2D;
+        if (cufftPlan3d(&pf, h->K[0], h->K[1], h->K[2], tf) != CUFFT_SUCCESS)
+            return fail(h, DMFFB_CUFFT_ERROR, "cufftPlan3d failed");
+        if (cufftPlan3d(&pb, h->K[0], h->K[1], h->K[2], tb) != CUFFT_SUCCESS) {
+            cufftDestroy(pf);
+            return fail(h, DMFFB_CUFFT_ERROR, "cufftPlan3d failed");
+        }
+        it = h->plan_cache.emplace(key, std::make_pair(pf, pb)).first;
+    }
+    h->plan_f = it->second.first;
+    h->plan_b = it->second.second;
+    return DMFFB_OK;
+}
+
+// in -> forward transform -> influence function (ca: kind, scales, energy sums, a mesh to clear) ->
+// inverse transform -> out, by the DFT kernels or by cuFFT and k_conv
+template <typename T>
+int mesh_convolve(dmffb_engine* h, cudaStream_t s, void* in, void* out, ConvArgs<T>& ca) {
+    h->dft_used = dft_use<T>(h);
+    if (h->dft_used) {
+        const int st = dft_setup<T>(h);
+        if (st) return st;
+        DftConvArgs<T> a = dft_args<T>(h, kDftCtas, false);
+        a.grid_in = (const T*)in;
+        a.grid_out = (T*)out;
+        a.G = h->stencils_ready && ca.kind == CK_COUL ? h->d_dftG : nullptr;
+        for (int k = 0; k < 9; ++k) a.hinv[k] = ca.hinv[k];
+        a.V = ca.V;
+        a.escale = ca.escale;
+        a.kind = ca.kind;
+        a.want_energy = ca.want_energy;
+        a.scal = ca.scal;
+        a.zero_real = ca.zero_real;
+        return dft_wide_tile(h) ? dft_launch<T, 2, 2>(h, s, a) : dft_launch<T, 1, 1>(h, s, a);
+    }
+    int st;
+    if (!h->plan_f && (st = fft_plans(h))) return st;
+    CKFFT(cufftSetStream(h->plan_f, s));
+    CKFFT(cufftSetStream(h->plan_b, s));
+    if (sizeof(T) == 4)
+        FFTCALL(h, s, cufftExecR2C(h->plan_f, (cufftReal*)in, (cufftComplex*)h->d_cgrid));
+    else
+        FFTCALL(h, s, cufftExecD2Z(h->plan_f, (cufftDoubleReal*)in, (cufftDoubleComplex*)h->d_cgrid));
+    const int64_t nk = (int64_t)h->K[0] * h->K[1] * ca.Kh;
+    LAUNCH(h, s, KC_CONV, k_conv<T><<<nblk(nk, 256), 256, 0, s>>>(ca));
+    if (sizeof(T) == 4)
+        FFTCALL(h, s, cufftExecC2R(h->plan_b, (cufftComplex*)h->d_cgrid, (cufftReal*)out));
+    else
+        FFTCALL(h, s, cufftExecZ2D(h->plan_b, (cufftDoubleComplex*)h->d_cgrid, (cufftDoubleReal*)out));
+    CK(cudaGetLastError());
+    return DMFFB_OK;
+}
+
+template <typename T>
+ConvArgs<T> conv_args(const dmffb_engine* h, const Box& bx, int kind, double escale, double* scal, bool energy) {
+    ConvArgs<T> ca;
+    for (int k = 0; k < 3; ++k) ca.K[k] = h->K[k];
+    ca.Kh = h->K[2] / 2 + 1;
+    ca.S = (T*)h->d_cgrid;
+    ca.bmod = h->d_bmod;
+    for (int k = 0; k < 9; ++k) ca.hinv[k] = bx.hinv[k];
+    ca.V = fabs(det3(bx.h));
+    ca.kappa = h->kappa;
+    ca.escale = escale;
+    ca.kind = kind;
+    ca.scal = scal;
+    ca.want_energy = energy ? 1 : 0;
+    return ca;
 }
 
 // Co-resident CTAs of the persistent CG solve for the current mesh (0: the graph-replayed solve
@@ -670,7 +830,9 @@ bool pcg_wanted(const dmffb_engine* h) {
 int pcg_decide(dmffb_engine* h) {
     if (h->pcg_max_blocks >= 0) return h->pcg_max_blocks;
     h->pcg_max_blocks = 0;
-    if (fc_decide(h) <= 0) return 0;
+    if (h->prec != DMFFB_FP32 || !h->lpme || std::max(h->K[0], std::max(h->K[1], h->K[2])) > kDftMaxK ||
+        std::min(h->K[0], std::min(h->K[1], h->K[2])) < 4 || dft_setup<float>(h))
+        return 0;
     int dev = 0, coop = 0, nsm = 0, per_sm = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
@@ -678,7 +840,8 @@ int pcg_decide(dmffb_engine* h) {
         cudaGetLastError();
         return 0;
     }
-    const size_t smem = cg_solve_smem(h->K);
+    const size_t smem = cg_solve_smem(dft_args<float>(h, nsm, true));
+    if (smem > kDftSmem) return 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cg_solve, kCgThreads, smem) != cudaSuccess) {
         cudaGetLastError();
         return 0;
@@ -703,9 +866,7 @@ int stencil_prep(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& 
     }
     LAUNCH(h, s, KC_VEC, k_stencil_prep<T><<<nblk(n, 128), 128, 0, s>>>(n, pos, mesh_geom(bx, h->K), h->d_stc_org,
                                                                         (T*)h->d_stc_w));
-    if (sizeof(T) == 4 && (h->fc_enabled || (pcg_wanted(h) && pcg_decide(h) > 0)) && fc_decide(h) > 0 &&
-        (st = fc_prepare(h, s, bx)))
-        return st;
+    if ((dft_use<T>(h) || (sizeof(T) == 4 && pcg_wanted(h) && pcg_decide(h) > 0)) && (st = dft_gtable(h, s, bx))) return st;
     h->stencils_ready = true;
     return DMFFB_OK;
 }
@@ -718,6 +879,8 @@ StencilCache<T> stencil_cache(dmffb_engine* h) {
     return c;
 }
 
+// reciprocal pass: spread (Qg and/or U) -> forward transform -> influence function -> inverse
+// transform -> gather
 template <typename T>
 int recip_pass(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx, bool use_Qg, const double* U,
                int mode, double* field_out, int field_acc, double* const* zero_scal = nullptr) {
@@ -749,36 +912,13 @@ int recip_pass(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx
                 if (zero_scal[k]) CK(cudaMemsetAsync(zero_scal[k], 0, sizeof(double), s));
         LAUNCH(h, s, KC_SPREAD, k_spread<T><<<nblk((int64_t)h->n * 32, 256), 256, 0, s>>>(sa));
     }
-    CKFFT(cufftSetStream(h->plan_f, s));
-    CKFFT(cufftSetStream(h->plan_b, s));
-    if (sizeof(T) == 4) {
-        FFTCALL(h, s, cufftExecR2C(h->plan_f, (cufftReal*)spread_grid, (cufftComplex*)h->d_cgrid));
-    } else {
-        FFTCALL(h, s, cufftExecD2Z(h->plan_f, (cufftDoubleReal*)spread_grid, (cufftDoubleComplex*)h->d_cgrid));
-    }
-    ConvArgs<T> ca;
-    for (int k = 0; k < 3; ++k) ca.K[k] = h->K[k];
-    ca.Kh = h->K[2] / 2 + 1;
-    ca.S = (T*)h->d_cgrid;
-    ca.bmod = h->d_bmod;
-    for (int k = 0; k < 9; ++k) ca.hinv[k] = bx.hinv[k];
-    ca.V = fabs(det3(bx.h));
-    ca.kappa = h->kappa;
-    ca.escale = DMFFB_DIELECTRIC;
-    ca.kind = CK_COUL;
-    ca.scal = h->d_scal + S_RECIP;
-    ca.want_energy = (mode == GATHER_FULL) ? 1 : 0;
+    ConvArgs<T> ca = conv_args<T>(h, bx, CK_COUL, DMFFB_DIELECTRIC, h->d_scal + S_RECIP, mode == GATHER_FULL);
     if (dip) {
         ca.zero_real = (T*)h->d_grid2;
         ca.nzero = K3;
     }
-    const int64_t nk = (int64_t)h->K[0] * h->K[1] * ca.Kh;
-    LAUNCH(h, s, KC_CONV, k_conv<T><<<nblk(nk, 256), 256, 0, s>>>(ca));
-    if (sizeof(T) == 4) {
-        FFTCALL(h, s, cufftExecC2R(h->plan_b, (cufftComplex*)h->d_cgrid, (cufftReal*)h->d_grid));
-    } else {
-        FFTCALL(h, s, cufftExecZ2D(h->plan_b, (cufftDoubleComplex*)h->d_cgrid, (cufftDoubleReal*)h->d_grid));
-    }
+    int st = mesh_convolve<T>(h, s, spread_grid, h->d_grid, ca);
+    if (st) return st;
     GatherArgs<T> ga;
     ga.n = h->n;
     ga.pos = pos;
@@ -856,39 +996,11 @@ int cg_matvec_fused(dmffb_engine* h, cudaStream_t s, const Box& bx, double* sc) 
         if (fork) CK(cudaEventRecord(h->e_join, h->s2));
     }
     LAUNCH(h, s, KC_SPREAD, k_spread_dip_cached<T><<<nblk((int64_t)h->n * 32, 256), 256, 0, s>>>(sa, stencil_cache<T>(h)));
-    if (sizeof(T) == 4 && h->fc_enabled && h->fc_ok > 0) {
-        // forward FFT, influence multiply and inverse FFT in one cluster; it also clears grid2
-        int stc = fc_launch(h, s, (float*)h->d_grid2, (float*)h->d_grid);
-        if (stc) return stc;
-    } else {
-    const int64_t K3 = (int64_t)h->K[0] * h->K[1] * h->K[2];
-    CKFFT(cufftSetStream(h->plan_f, s));
-    CKFFT(cufftSetStream(h->plan_b, s));
-    if (sizeof(T) == 4)
-        FFTCALL(h, s, cufftExecR2C(h->plan_f, (cufftReal*)h->d_grid2, (cufftComplex*)h->d_cgrid));
-    else
-        FFTCALL(h, s, cufftExecD2Z(h->plan_f, (cufftDoubleReal*)h->d_grid2, (cufftDoubleComplex*)h->d_cgrid));
-    ConvArgs<T> ca;
-    for (int k = 0; k < 3; ++k) ca.K[k] = h->K[k];
-    ca.Kh = h->K[2] / 2 + 1;
-    ca.S = (T*)h->d_cgrid;
-    ca.bmod = h->d_bmod;
-    for (int k = 0; k < 9; ++k) ca.hinv[k] = bx.hinv[k];
-    ca.V = fabs(det3(bx.h));
-    ca.kappa = h->kappa;
-    ca.escale = DMFFB_DIELECTRIC;
-    ca.kind = CK_COUL;
-    ca.scal = h->d_scal + S_RECIP;
-    ca.want_energy = 0;
-    ca.zero_real = (T*)h->d_grid2;
-    ca.nzero = K3;
-    const int64_t nk = (int64_t)h->K[0] * h->K[1] * ca.Kh;
-    LAUNCH(h, s, KC_CONV, k_conv<T><<<nblk(nk, 256), 256, 0, s>>>(ca));
-    if (sizeof(T) == 4)
-        FFTCALL(h, s, cufftExecC2R(h->plan_b, (cufftComplex*)h->d_cgrid, (cufftReal*)h->d_grid));
-    else
-        FFTCALL(h, s, cufftExecZ2D(h->plan_b, (cufftDoubleComplex*)h->d_cgrid, (cufftDoubleReal*)h->d_grid));
-    }
+    ConvArgs<T> ca = conv_args<T>(h, bx, CK_COUL, DMFFB_DIELECTRIC, h->d_scal + S_RECIP, false);
+    ca.zero_real = (T*)h->d_grid2;  // cleared for the next spread once it has been transformed
+    ca.nzero = (int64_t)h->K[0] * h->K[1] * h->K[2];
+    int stc = mesh_convolve<T>(h, s, h->d_grid2, h->d_grid, ca);
+    if (stc) return stc;
     FieldCombine cmb;
     const double k = h->kappa;
     cmb.U = h->d_p;
@@ -1066,7 +1178,11 @@ int cg_persistent(dmffb_engine* h, cudaStream_t s, const Box& bx, double* U, con
     a.gscale = 2.0 * DMFFB_DIELECTRIC;
     const double k = h->kappa;
     a.self1 = -2.0 * DMFFB_DIELECTRIC * (k / 1.7724538509055159) * 2.0 * k * k / 3.0;
-    a.fc = fc_args(h, (float*)h->d_grid2, (float*)h->d_grid);
+    a.fc = dft_args<float>(h, h->pcg_max_blocks, true);
+    a.fc.grid_in = (const float*)h->d_grid2;
+    a.fc.zero_real = (float*)h->d_grid2;
+    a.fc.grid_out = (float*)h->d_grid;
+    a.fc.G = h->d_dftG;
     a.acc = (double*)(base + kPcgAcc);
     a.init = sc;
     a.tol = h->cg_tol;
@@ -1080,15 +1196,14 @@ int cg_persistent(dmffb_engine* h, cudaStream_t s, const Box& bx, double* U, con
     h->pcg_phantom = 0;
     a.out = (CgStatus*)(base + kPcgOut);
     a.phase_ns = h->prof ? (unsigned long long*)(base + kPcgPhase) : nullptr;
-    // CTAs: enough warps for the matvec + spread pass (two warps per atom), the x-planes and the
-    // spectrum column blocks, within what the device holds at once
-    const int ncb = (h->K[1] * (h->K[2] / 2 + 1) + kFcCols - 1) / kFcCols;
+    // CTAs: enough warps for the matvec + spread pass (two warps per atom) and the items of the
+    // convolution passes, within what the device holds at once
     int grid = (int)((2 * (int64_t)h->n + kCgThreads / 32 - 1) / (kCgThreads / 32));
-    grid = std::max(grid, std::max(h->K[0], ncb));
+    grid = std::max(grid, std::max(dft_col_items(a.fc), std::max(dft_fwd_items(a.fc), dft_inv_items(a.fc))));
     grid = std::min(grid, h->pcg_max_blocks);
     void* args[] = {&a};
     LAUNCH(h, s, KC_CGSOLVE, CK(cudaLaunchCooperativeKernel((const void*)k_cg_solve, dim3(grid), dim3(kCgThreads),
-                                                            args, cg_solve_smem(h->K), s)));
+                                                            args, cg_solve_smem(a.fc), s)));
     static_assert(sizeof(CgStatus) <= 32, "status block of the persistent solve");
     CK(cudaMemcpyAsync(h->h_scal, a.out, a.phase_ns ? kPcgBytes - kPcgOut : sizeof(CgStatus),
                        cudaMemcpyDeviceToHost, s));
@@ -1175,7 +1290,7 @@ int solve_dipoles(dmffb_engine* h, cudaStream_t s, const double* pos, const Box&
     LAUNCH(h, s, KC_VEC, k_dot2<<<nb3, 256, 0, s>>>(3 * n, h->d_r, h->d_z, h->d_r, h->d_r, sc + 0, sc + 3));
     LAUNCH(h, s, KC_VEC, k_dot2<<<nb3, 256, 0, s>>>(3 * n, h->d_b, h->d_b, nullptr, nullptr, sc + 4, nullptr));
     const bool fused = h->lpme && h->have_plans && h->stencils_ready;
-    if (sizeof(T) == 4 && fused && pcg_wanted(h) && h->d_fcW && pcg_decide(h) > 0)
+    if (sizeof(T) == 4 && fused && pcg_wanted(h) && pcg_decide(h) > 0)
         return cg_persistent(h, s, bx, U, sc, res);
     int it = 0;
     bool conv = false;
@@ -1211,7 +1326,7 @@ int solve_dipoles(dmffb_engine* h, cudaStream_t s, const double* pos, const Box&
         std::vector<double> key = {(double)(uintptr_t)pos, (double)(uintptr_t)pairs, (double)npairs,
                                    (double)(uintptr_t)U, (double)(uintptr_t)h->d_csr_ent, (double)sizeof(T),
                                    (double)(uintptr_t)h->d_mvcoef, (double)(uintptr_t)h->d_csr_off,
-                                   (double)(h->fc_enabled ? h->fc_ok : 0), (double)(uintptr_t)h->d_fcG,
+                                   (double)dft_use<T>(h), (double)(uintptr_t)h->d_dftG, (double)(uintptr_t)h->d_dftW,
                                    (double)fused};
         for (int k = 0; k < 9; ++k) key.push_back(bx.h[k]);
         const bool repeat = key == h->cg_seen_key;
@@ -1538,25 +1653,9 @@ int recip_pass_channel(dmffb_engine* h, cudaStream_t s, const double* pos, const
     sa.grid = (T*)h->d_grid;
     sa.perm_mul = h->perm_mul;
     LAUNCH(h, s, KC_SPREAD, k_spread<T><<<nblk((int64_t)h->n * 32, 256), 256, 0, s>>>(sa));
-    CKFFT(cufftSetStream(h->plan_f, s));
-    CKFFT(cufftSetStream(h->plan_b, s));
-    if (sizeof(T) == 4) FFTCALL(h, s, cufftExecR2C(h->plan_f, (cufftReal*)h->d_grid, (cufftComplex*)h->d_cgrid));
-    else FFTCALL(h, s, cufftExecD2Z(h->plan_f, (cufftDoubleReal*)h->d_grid, (cufftDoubleComplex*)h->d_cgrid));
-    ConvArgs<T> ca;
-    for (int k = 0; k < 3; ++k) ca.K[k] = h->K[k];
-    ca.Kh = h->K[2] / 2 + 1;
-    ca.S = (T*)h->d_cgrid;
-    ca.bmod = h->d_bmod;
-    for (int k = 0; k < 9; ++k) ca.hinv[k] = bx.hinv[k];
-    ca.V = fabs(det3(bx.h));
-    ca.kappa = h->kappa;
-    ca.escale = escale;
-    ca.kind = kind;
-    ca.scal = scal_conv;
-    ca.want_energy = 1;
-    LAUNCH(h, s, KC_CONV, k_conv<T><<<nblk((int64_t)h->K[0] * h->K[1] * ca.Kh, 256), 256, 0, s>>>(ca));
-    if (sizeof(T) == 4) FFTCALL(h, s, cufftExecC2R(h->plan_b, (cufftComplex*)h->d_cgrid, (cufftReal*)h->d_grid));
-    else FFTCALL(h, s, cufftExecZ2D(h->plan_b, (cufftDoubleComplex*)h->d_cgrid, (cufftDoubleReal*)h->d_grid));
+    ConvArgs<T> ca = conv_args<T>(h, bx, kind, escale, scal_conv, true);
+    int st = mesh_convolve<T>(h, s, h->d_grid, h->d_grid, ca);
+    if (st) return st;
     GatherArgs<T> ga;
     ga.n = h->n;
     ga.pos = pos;
@@ -2034,7 +2133,6 @@ int upload_topology(dmffb_engine* h, const dmffb_admp_desc* d) {
 
 // PME mesh of h->K: grids grown to fit, B-spline moduli, cuFFT plans (cached per mesh shape)
 int setup_mesh(dmffb_engine* h) {
-    h->fc_ok = -1;  // whether the engine's FFT convolution serves the mesh is decided again
     h->pcg_max_blocks = -1;
     const size_t ts = h->prec == DMFFB_FP32 ? 4 : 8;
     const int64_t K3 = (int64_t)h->K[0] * h->K[1] * h->K[2];
@@ -2074,22 +2172,12 @@ int setup_mesh(dmffb_engine* h) {
         }
     CK(cudaMemcpyAsync(h->d_bmod, bm.data(), bm.size() * sizeof(double), cudaMemcpyHostToDevice, h->s1));
     CK(cudaStreamSynchronize(h->s1));
-    const std::array<int, 3> key = {h->K[0], h->K[1], h->K[2]};
-    auto it = h->plan_cache.find(key);
-    if (it == h->plan_cache.end()) {
-        cufftHandle pf = 0, pb = 0;
-        cufftType tf = h->prec == DMFFB_FP32 ? CUFFT_R2C : CUFFT_D2Z;
-        cufftType tb = h->prec == DMFFB_FP32 ? CUFFT_C2R : CUFFT_Z2D;
-        if (cufftPlan3d(&pf, h->K[0], h->K[1], h->K[2], tf) != CUFFT_SUCCESS)
-            return fail(h, DMFFB_CUFFT_ERROR, "cufftPlan3d failed");
-        if (cufftPlan3d(&pb, h->K[0], h->K[1], h->K[2], tb) != CUFFT_SUCCESS) {
-            cufftDestroy(pf);
-            return fail(h, DMFFB_CUFFT_ERROR, "cufftPlan3d failed");
-        }
-        it = h->plan_cache.emplace(key, std::make_pair(pf, pb)).first;
-    }
-    h->plan_f = it->second.first;
-    h->plan_b = it->second.second;
+    h->plan_f = h->plan_b = 0;
+    if (h->prec == DMFFB_FP32 ? dft_use<float>(h) : dft_use<double>(h))
+        st = h->prec == DMFFB_FP32 ? dft_setup<float>(h) : dft_setup<double>(h);
+    else
+        st = fft_plans(h);
+    if (st) return st;
     h->have_plans = true;
     return DMFFB_OK;
 }
@@ -2244,7 +2332,7 @@ void dmffb_destroy(dmffb_engine* h) {
                     h->d_q, h->d_qT, h->d_type, h->d_sigtt, h->d_epstt, h->d_dq, h->d_dsig, h->d_deps,
                     h->d_tidx[0], h->d_tidx[1], h->d_tidx[2], h->d_tprm[0], h->d_tprm[1], h->d_tprm[2],
                     h->d_tdprm[0], h->d_tdprm[1], h->d_tdprm[2], h->d_dQloc, h->d_dpa, h->d_dth, h->d_dpol, h->d_dsr, h->d_srows, h->d_nsel, h->d_cubsel,
-                    h->d_cub, h->d_ell_rows, h->d_ell_ent, h->d_maxdeg, h->d_stc_org, h->d_stc_w, h->d_nbmask, h->d_covrows, h->d_cov_lo, h->d_cov_hi, h->d_fcG, h->d_fcW, h->d_pcg, h->d_posc, h->d_srp, h->d_srdp, h->d_srgrad};
+                    h->d_cub, h->d_ell_rows, h->d_ell_ent, h->d_maxdeg, h->d_stc_org, h->d_stc_w, h->d_nbmask, h->d_covrows, h->d_cov_lo, h->d_cov_hi, h->d_dftW, h->d_dftG, h->d_pcg, h->d_posc, h->d_srp, h->d_srdp, h->d_srgrad};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (h->h_scal) cudaFreeHost(h->h_scal);
@@ -3542,7 +3630,7 @@ int dmffb_set_timing(dmffb_engine* h, int32_t enabled) {
 
 int dmffb_set_fused_fft(dmffb_engine* h, int32_t enabled) {
     if (!h) return DMFFB_BAD_ARG;
-    h->fc_enabled = enabled != 0;
+    h->dft_mode = enabled != 0;
     return DMFFB_OK;
 }
 
@@ -3572,7 +3660,7 @@ int dmffb_set_cg_wait_limit(dmffb_engine* h, double seconds, int32_t phantom_arr
 
 int dmffb_fused_fft_active(const dmffb_engine* h) {
     if (!h) return -1;
-    return h->fc_enabled && h->fc_ok > 0 ? 1 : 0;
+    return h->dft_used ? 1 : 0;
 }
 
 int dmffb_set_graphs(dmffb_engine* h, int32_t enabled) {

@@ -319,12 +319,12 @@ class AdmpEngine:
         return buf[: need.value]
 
     def set_fused_fft(self, on=True):
-        """The dipole solve's reciprocal convolution through the engine's own FFT kernels (FP32,
-        meshes up to 64 per axis) or through cuFFT (dmffb_set_fused_fft)."""
+        """The mesh convolution through the engine's direct-DFT kernels (meshes up to 64 per axis) or
+        through cuFFT, instead of the engine's choice by size (dmffb_set_fused_fft)."""
         self._check(self.lib.dmffb_set_fused_fft(self.h, int(bool(on))))
 
     def set_persistent_cg(self, mode=True):
-        """The whole CG dipole solve in one persistent cooperative launch (FP32, meshes up to 64
+        """The whole CG dipole solve in one persistent cooperative launch (FP32, meshes up to 128
         per axis; dmffb_set_persistent_cg): True / 1 always, False / 0 never (the graph-replayed
         per-pass solve), "auto" / 2 (the default) for systems of at most 4096 atoms."""
         m = 2 if mode == "auto" else int(mode)
@@ -349,7 +349,7 @@ class AdmpEngine:
         return {k: arr[i] for i, k in enumerate(self.CG_PHASES)}
 
     def fused_fft_active(self):
-        """Whether the last solve's convolution ran through the engine's FFT (else cuFFT)."""
+        """Whether the last mesh convolution ran through the direct-DFT kernels (else cuFFT)."""
         return bool(self.lib.dmffb_fused_fft_active(self.h))
 
     def set_timing(self, on=True):

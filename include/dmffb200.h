@@ -214,7 +214,7 @@ int dmffb_set_timing(dmffb_engine* h, int32_t enabled);
  * 8 gather FIELD, 9 self+frame forces, 10 vector/CG ops, 11 neighbour build, 12 CG matvec
  * pair-tensor set-up, 13 pair FULL over the topologically scaled rows (FP64), 14 pair FIELD over
  * the scaled rows (FP64), 15 parameter-adjoint pair kernels, 16 bonded terms, 17 the engine-FFT
- * convolution of the dipole solve (dmffb_set_fused_fft), 18 the persistent CG solve
+ * direct-DFT mesh convolution (dmffb_set_fused_fft), 18 the persistent CG solve
  * (dmffb_set_persistent_cg).  Classes 1 and 2
  * hold only the launches over the unscaled rows (kernel precision). */
 int dmffb_set_profiling(dmffb_engine* h, int32_t enabled);
@@ -331,18 +331,18 @@ int dmffb_classical_set_cell_pass(dmffb_engine* h, int32_t enabled);
 int dmffb_classical_param_grads(dmffb_engine* h, void* stream, double* dE_dq, double* dE_dsig, double* dE_deps,
                                 double* dE_dbond, double* dE_dangle, double* dE_dtorsion);
 
-/* The dipole-solve iterations' reciprocal convolution (forward FFT, influence-function multiply,
- * inverse FFT) through the engine's own three-pass FFT (x-planes, spectrum columns with the
- * multiply, x-planes) instead of cuFFT R2C + convolution + C2R, on/off (off by default; FP32
- * engines with meshes of at most 64 points per axis, else cuFFT).
- * dmffb_fused_fft_active returns 1 when the last solve used it, 0 for the cuFFT path. */
+/* The mesh convolution (forward transform, influence-function multiply, inverse transform): by
+ * default the engine's direct-DFT kernels on meshes where they are faster and cuFFT R2C +
+ * convolution + C2R elsewhere (a rule on the extents and the precision).  enabled = 1 asks for the
+ * DFT kernels on meshes of at most 64 points per axis (cuFFT beyond), 0 for cuFFT.
+ * dmffb_fused_fft_active returns 1 when the last convolution ran through the DFT kernels, else 0. */
 int dmffb_set_fused_fft(dmffb_engine* h, int32_t enabled);
 /* The whole CG dipole solve in one persistent cooperative launch (k_cg_solve: direction update,
- * real-space matvec and dipole spread, the engine-FFT convolution, field gather and CG update per
+ * real-space matvec and dipole spread, the direct-DFT convolution, field gather and CG update per
  * iteration, separated by grid barriers; convergence decided on the device, one read-back per
  * solve).  mode 0: off (the graph-replayed per-pass solve), 1: on, 2 (default): on for systems of
  * at most 4096 atoms, where the launch chain of the per-pass solve dominates.  FP32 engines with
- * meshes of at most 64 points per axis on devices with cooperative launch only.
+ * meshes of at most 128 points per axis on devices with cooperative launch only.
  * dmffb_persistent_cg_blocks returns the co-resident CTAs available to it for the current mesh
  * (0: not used).
  * dmffb_set_cg_wait_limit bounds every grid-barrier wait of the kernel (default 2 s): past it the
