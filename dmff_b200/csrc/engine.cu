@@ -76,17 +76,18 @@ struct dmffb_engine {
     double *d_b = nullptr, *d_r = nullptr, *d_z = nullptr, *d_p = nullptr, *d_Ap = nullptr, *d_fr = nullptr;
     double* d_gQ = nullptr;
     double* d_fmv = nullptr;  // CSR matvec output [3n]
-    // slots of the single-pass neighbour build (k_pairs_cell pass 2): capacities per atom from
-    // the largest counts of the last two-pass build (0: no slots yet)
+    // slots of the single-pass neighbour build: capacities per atom, first from the mean density,
+    // then from the largest counts met (0: no slots yet)
     int32_t* d_ell_rows = nullptr;  // [n_cap * ell_cap_h * 3]
     int32_t* d_ell_ent = nullptr;   // [n_cap * ell_cap_f]
     int ell_cap_h = 0, ell_cap_f = 0;
-    int* d_maxdeg = nullptr;        // [2]
+    int32_t* d_nbsum = nullptr;     // NbTotals, then the run sums of the counts [3][runs]
     // a single-pass build whose totals are still on their way to the host: nb_finish waits for
-    // them when the list is first used (and rebuilds with two passes if a slot overflowed)
+    // them when the list is first used (and rebuilds with larger slots if one overflowed)
     bool nb_pending = false, nb_want_csr = false;
+    int nb_cap_h = 0, nb_cap_f = 0;  // the slots it ran with
     cudaEvent_t e_nbtot = nullptr;
-    int64_t* h_nbtot = nullptr;     // pinned [4]: half rows, CSR entries, largest counts (2 x int32)
+    NbTotals* h_nbtot = nullptr;    // pinned
     cudaStream_t nb_stream = nullptr;
     const double* nb_pos = nullptr;
     double nb_box[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
@@ -95,7 +96,6 @@ struct dmffb_engine {
     int64_t csr_cap = 0;
     bool csr_from_build = false;     // CSR built together with the internal pair list
     const int32_t* csr_pairs = nullptr;  // the half list the current CSR belongs to
-    float* d_posf = nullptr;
     void* d_mvcoef = nullptr;  // [csr_cap] MvCoef<T>
     int64_t mv_cap = 0;
     int32_t* d_pcount_f = nullptr;
@@ -111,12 +111,11 @@ struct dmffb_engine {
     int32_t* d_pairs = nullptr;
     int64_t pair_cap = 0, npairs = 0;
     bool have_pairs = false;
-    int32_t *d_atom_cell = nullptr, *d_cell_count = nullptr, *d_cell_start = nullptr, *d_cell_cursor = nullptr,
-            *d_cell_atoms = nullptr, *d_pcount = nullptr;
+    int32_t *d_atom_cell = nullptr, *d_rank = nullptr, *d_cell_count = nullptr, *d_cell_start = nullptr,
+            *d_pcount = nullptr, *d_pcount_s = nullptr, *d_poff_s = nullptr;
+    unsigned* d_bin_done = nullptr;
     int64_t* d_poff = nullptr;
     int ncell_cap = 0;
-    void* d_cub = nullptr;
-    size_t cub_bytes = 0;
     double* h_scal = nullptr;  // pinned
     // ---- timing
     bool timing = false;
@@ -184,7 +183,7 @@ struct dmffb_engine {
     int32_t* d_covrows = nullptr;  // [n_covrows*3] covalent rows (i < j, nbond)
     int64_t n_covrows = 0;
     int32_t *d_cov_lo = nullptr, *d_cov_hi = nullptr;  // [n] covalent partner index range
-    float4* d_posc = nullptr;  // [n] cell-ordered positions of the cell pass
+    float4* d_posc = nullptr;  // [n] cell-ordered positions (pair builds and the cell pass)
     // ---- short-range pairwise terms (engines made by dmffb_pairwise_create, kind 3)
     int sr_kind = 0;
     double sr_sign = 1.0;
@@ -229,7 +228,8 @@ struct dmffb_engine {
     std::map<std::array<int, 3>, std::pair<cufftHandle, cufftHandle>> plan_cache;  // mesh -> (R2C, C2R)
 };
 
-// completion of a single-pass neighbour build (defined after the kernels)
+// start and completion of a single-pass neighbour build (defined after the kernels)
+int nb_start(dmffb_engine* h, cudaStream_t s, const double* pos, const double* box);
 int nb_finish(dmffb_engine* h);
 void nb_discard(dmffb_engine* h);
 
@@ -506,7 +506,8 @@ struct ScaledRow {
 
 // Indices of the rows with nbond != 0 (stable, so still sorted by i), rebuilt when the pair
 // list changes: the FP64 scaled-rows launches run over these (about one row in a hundred)
-// instead of over every row.
+// instead of over every row.  The engine's own builds leave them beside the list (k_nb_place); rows
+// that a caller passes are searched here.
 int scaled_rows(dmffb_engine* h, cudaStream_t s, const int32_t* pairs, int64_t npairs) {
     const bool internal = pairs == h->d_pairs;
     if (internal && h->srows_pairs == pairs && h->srows_npairs == npairs && h->srows_gen == h->pairs_gen)
@@ -1042,22 +1043,27 @@ int matvec_coef_launch(dmffb_engine* h, cudaStream_t s, const Box& bx, const int
     return DMFFB_OK;
 }
 
+// per-atom arrays of the full CSR and of the matvec over it
+int csr_alloc(dmffb_engine* h) {
+    if (h->d_csr_off) return DMFFB_OK;
+    const int nc = h->n_cap;
+    int st;
+    if ((st = dalloc(h, &h->d_csr_off, (nc + 1) * sizeof(int64_t)))) return st;
+    if ((st = dalloc(h, &h->d_csr_deg, nc * sizeof(int32_t)))) return st;
+    if ((st = dalloc(h, &h->d_fmv, 3 * nc * sizeof(double)))) return st;
+    size_t need = 0;
+    cub::DeviceScan::InclusiveSum(nullptr, need, (int32_t*)nullptr, (int64_t*)nullptr, nc);
+    h->cub2_bytes = need;
+    return dalloc(h, &h->d_cub2, need);
+}
+
 // full both-direction CSR of the half-list rows (for the atomics-free CG matvec)
 int build_csr(dmffb_engine* h, cudaStream_t s, const int32_t* pairs, int64_t npairs) {
     const int n = h->n;
     int st;
     if (h->csr_from_build && pairs == h->d_pairs) return DMFFB_OK;  // made by the neighbour build
     h->csr_from_build = false;
-    if (!h->d_csr_off) {
-        const int nc = h->n_cap;
-        if ((st = dalloc(h, &h->d_csr_off, (nc + 1) * sizeof(int64_t)))) return st;
-        if ((st = dalloc(h, &h->d_csr_deg, nc * sizeof(int32_t)))) return st;
-        if ((st = dalloc(h, &h->d_fmv, 3 * nc * sizeof(double)))) return st;
-        size_t need = 0;
-        cub::DeviceScan::InclusiveSum(nullptr, need, (int32_t*)nullptr, (int64_t*)nullptr, nc);
-        h->cub2_bytes = need;
-        if ((st = dalloc(h, &h->d_cub2, need))) return st;
-    }
+    if ((st = csr_alloc(h))) return st;
     if (2 * npairs > h->csr_cap) {
         if (h->d_csr_ent) cudaFree(h->d_csr_ent);
         h->csr_cap = 2 * npairs + 1024;
@@ -1810,59 +1816,280 @@ __global__ void k_self_dq(int n, const double* q, double c, double* dq) {
     if (i < n) dq[i] += c * q[i];
 }
 
-// Half-width cell grid of the cell pass: at least 5 cells of width >= rc/2 per axis (the 5^3
-// stencil then covers every pair within rc), at most 64 per axis.
-bool half_cells(const dmffb_engine* h, const Box& bx, int nc[3]) {
+// Half-width cells (at least rc / 2 wide across each pair of box faces) for the 5^3 stencil; false
+// where an axis holds fewer than five.
+bool half_cells(const Box& bx, double rc, int nc[3]) {
     const double* m = bx.h;
     const double V = fabs(det3(m));
+    bool ok = true;
     for (int k = 0; k < 3; ++k) {
         const double* u = m + 3 * ((k + 1) % 3);
         const double* w = m + 3 * ((k + 2) % 3);
         const double cx = u[1] * w[2] - u[2] * w[1], cy = u[2] * w[0] - u[0] * w[2], cz = u[0] * w[1] - u[1] * w[0];
-        nc[k] = (int)floor(V / sqrt(cx * cx + cy * cy + cz * cz) / (0.5 * h->rc));
-        if (nc[k] > 64) nc[k] = 64;
-        if (nc[k] < 5) return false;
+        const double q = floor(V / sqrt(cx * cx + cy * cy + cz * cz) / (0.5 * rc));
+        nc[k] = q < 64.0 ? (int)q : 64;
+        if (!(nc[k] >= 5)) ok = false;
     }
-    return true;
+    return ok;
 }
 
-// Counting sort of the atoms into the cells nc (the binning of the list build): cell_start /
-// cell_atoms, and the cell-ordered float4 positions of the cell pass.
-int bin_cells(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx, const int nc[3]) {
+// Counting sort of the atoms into the cells nc: cell_start and the cell-ordered float4 positions.
+// With zero, nzero words are cleared on the way.
+int bin_cells(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx, const int nc[3], int32_t* zero = nullptr,
+              int nzero = 0) {
     const int n = h->n;
     int st;
-    if (!h->d_pcount) {
+    if (!h->d_posc) {
         const int cap = h->n_cap;
-        if ((st = dalloc(h, &h->d_pcount, cap * sizeof(int32_t)))) return st;
-        if ((st = dalloc(h, &h->d_poff, (cap + 1) * sizeof(int64_t)))) return st;
-        if ((st = dalloc(h, &h->d_atom_cell, cap * sizeof(int32_t)))) return st;
-        if ((st = dalloc(h, &h->d_cell_atoms, cap * sizeof(int32_t)))) return st;
+        if ((st = dalloc(h, &h->d_atom_cell, cap * sizeof(int32_t))) || (st = dalloc(h, &h->d_rank, cap * sizeof(int32_t))) ||
+            (st = dalloc(h, &h->d_bin_done, sizeof(unsigned))) ||
+            (st = dalloc(h, &h->d_posc, (size_t)cap * sizeof(float4))))
+            return st;
+        CK(cudaMemsetAsync(h->d_bin_done, 0, sizeof(unsigned), s));
     }
     const int ncell = nc[0] * nc[1] * nc[2];
-    if (ncell + 1 > h->ncell_cap) {
-        if (h->d_cell_count) { cudaFree(h->d_cell_count); cudaFree(h->d_cell_start); cudaFree(h->d_cell_cursor); }
-        h->ncell_cap = ncell + 1;
-        if ((st = dalloc(h, &h->d_cell_count, h->ncell_cap * sizeof(int32_t)))) return st;
-        if ((st = dalloc(h, &h->d_cell_start, h->ncell_cap * sizeof(int32_t)))) return st;
-        if ((st = dalloc(h, &h->d_cell_cursor, h->ncell_cap * sizeof(int32_t)))) return st;
+    if (ncell > h->ncell_cap) {
+        if (h->d_cell_count) { cudaFree(h->d_cell_count); cudaFree(h->d_cell_start); }
+        h->d_cell_count = h->d_cell_start = nullptr;
+        h->ncell_cap = (ncell + kBinItems - 1) / kBinItems * kBinItems;
+        if ((st = dalloc(h, &h->d_cell_count, h->ncell_cap * sizeof(int32_t))) ||
+            (st = dalloc(h, &h->d_cell_start, (h->ncell_cap + 1) * sizeof(int32_t)))) {
+            h->ncell_cap = 0;
+            return st;
+        }
+        CK(cudaMemsetAsync(h->d_cell_count, 0, h->ncell_cap * sizeof(int32_t), s));
     }
-    size_t need = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, need, (int32_t*)nullptr, (int32_t*)nullptr, ncell + 1);
-    if (need > h->cub_bytes) {
-        if (h->d_cub) cudaFree(h->d_cub);
-        h->cub_bytes = need;
-        if ((st = dalloc(h, &h->d_cub, need))) return st;
+    BinArgs a;
+    a.n = n;
+    a.pos = pos;
+    a.box = bx;
+    for (int k = 0; k < 3; ++k) a.nc[k] = nc[k];
+    a.atom_cell = h->d_atom_cell;
+    a.rank = h->d_rank;
+    a.cell_count = h->d_cell_count;
+    a.cell_start = h->d_cell_start;
+    a.done = h->d_bin_done;
+    a.zero = zero;
+    a.nzero = nzero;
+    a.posc = h->d_posc;
+    LAUNCH(h, s, KC_NBLIST, k_bin_count<<<nblk(n, kBinThreads), kBinThreads, 0, s>>>(a));
+    LAUNCH(h, s, KC_NBLIST, k_bin_fill<<<nblk(n, 256), 256, 0, s>>>(a));
+    CK(cudaGetLastError());
+    return DMFFB_OK;
+}
+
+// ------------------------------------------------------------------ neighbour builds
+// How a list of (box, rc) is built.  flat: every atom is a candidate (fewer than five half-width cells
+// on an axis).  staged: one CTA per cell with the candidates in shared memory, where 1.5x the mean
+// candidate count fits the 44 KB stage; larger neighbourhoods keep the warp-per-atom kernel, whose
+// L2 gathers run at full occupancy (measured faster there than 100 KB stages), in two passes.
+struct NbPlan {
+    bool flat, staged, ortho;
+    int nc[3], ncell, chmax;
+    int guess;  // neighbours per atom at the mean density, with headroom
+};
+
+NbPlan nb_plan(const dmffb_engine* h, const Box& bx, double rc) {
+    NbPlan p;
+    p.flat = !half_cells(bx, rc, p.nc);
+    p.ncell = p.flat ? 1 : p.nc[0] * p.nc[1] * p.nc[2];
+    const double cand = 125.0 * (double)h->n / (double)p.ncell;
+    p.chmax = (int)std::min(1.5 * cand + 64.0, 1e9);
+    p.staged = !p.flat && (size_t)p.chmax * sizeof(float4) <= kNbStageBytes;
+    const double* m = bx.h;
+    p.ortho = m[1] == 0.0 && m[2] == 0.0 && m[3] == 0.0 && m[5] == 0.0 && m[6] == 0.0 && m[7] == 0.0;
+    const double mean = (double)h->n / fabs(det3(m)) * (4.0 / 3.0) * M_PI * rc * rc * rc;
+    p.guess = (int)std::min(1.35 * mean + 24.0, (double)h->n);
+    return p;
+}
+
+int nb_alloc(dmffb_engine* h, bool want_csr) {
+    int st;
+    const int cap = h->n_cap;
+    if (!h->d_pcount) {
+        if ((st = dalloc(h, &h->d_pcount, cap * sizeof(int32_t))) || (st = dalloc(h, &h->d_pcount_f, cap * sizeof(int32_t))) ||
+            (st = dalloc(h, &h->d_pcount_s, cap * sizeof(int32_t))) ||
+            (st = dalloc(h, &h->d_poff, (cap + 1) * sizeof(int64_t))) ||
+            (st = dalloc(h, &h->d_poff_s, cap * sizeof(int32_t))) ||
+            (st = dalloc(h, &h->d_nbsum, nb_sum_words(cap) * sizeof(int32_t))))
+            return st;
     }
-    CK(cudaMemsetAsync(h->d_cell_count, 0, (ncell + 1) * sizeof(int32_t), s));
-    CK(cudaMemsetAsync(h->d_cell_cursor, 0, (ncell + 1) * sizeof(int32_t), s));
-    LAUNCH(h, s, KC_NBLIST, k_cell_count<<<nblk(n, 256), 256, 0, s>>>(n, pos, bx, nc[0], nc[1], nc[2], h->d_atom_cell,
-                                                                     h->d_cell_count));
-    size_t tb = h->cub_bytes;
-    LAUNCH(h, s, KC_NBLIST, cub::DeviceScan::ExclusiveSum(h->d_cub, tb, h->d_cell_count, h->d_cell_start, ncell + 1, s));
-    LAUNCH(h, s, KC_NBLIST, k_cell_fill<<<nblk(n, 256), 256, 0, s>>>(n, h->d_atom_cell, h->d_cell_start,
-                                                                    h->d_cell_cursor, h->d_cell_atoms));
-    if (!h->d_posc && (st = dalloc(h, &h->d_posc, (size_t)h->n_cap * sizeof(float4)))) return st;
-    LAUNCH(h, s, KC_NBLIST, k_pos_cells<<<nblk(n, 256), 256, 0, s>>>(n, pos, h->d_cell_atoms, h->d_posc));
+    if (!h->h_nbtot && cudaMallocHost((void**)&h->h_nbtot, sizeof(NbTotals)) != cudaSuccess)
+        return fail(h, DMFFB_OOM, "cudaMallocHost failed");
+    return want_csr ? csr_alloc(h) : DMFFB_OK;
+}
+
+// slots for ch half rows and cf CSR entries per atom
+int nb_slots(dmffb_engine* h, int ch, int cf) {
+    int st;
+    if (ch > h->ell_cap_h) {
+        if (h->d_ell_rows) cudaFree(h->d_ell_rows);
+        h->d_ell_rows = nullptr;
+        h->ell_cap_h = 0;
+        if ((st = dalloc(h, &h->d_ell_rows, (size_t)h->n_cap * ch * 3 * sizeof(int32_t)))) return st;
+        h->ell_cap_h = ch;
+    }
+    if (cf > h->ell_cap_f) {
+        if (h->d_ell_ent) cudaFree(h->d_ell_ent);
+        h->d_ell_ent = nullptr;
+        h->ell_cap_f = 0;
+        if ((st = dalloc(h, &h->d_ell_ent, (size_t)h->n_cap * cf * sizeof(int32_t)))) return st;
+        h->ell_cap_f = cf;
+    }
+    return DMFFB_OK;
+}
+
+// the largest counts with an eighth (at least 16) of headroom
+int nb_headroom(int c) { return c + std::max(16, c / 8); }
+
+int nb_pair_cap(dmffb_engine* h, int64_t rows) {
+    if (rows <= h->pair_cap && h->d_pairs) return DMFFB_OK;
+    if (h->d_pairs) cudaFree(h->d_pairs);
+    h->d_pairs = nullptr;
+    h->pair_cap = 0;
+    const int64_t cap = (int64_t)(rows * 1.3) + 64;  // headroom as in nblist.py:37-38
+    const int st = dalloc(h, &h->d_pairs, cap * 3 * sizeof(int32_t));
+    if (!st) h->pair_cap = cap;
+    return st;
+}
+
+int nb_csr_cap(dmffb_engine* h, int64_t entries) {
+    if (entries <= h->csr_cap && h->d_csr_ent) return DMFFB_OK;
+    if (h->d_csr_ent) cudaFree(h->d_csr_ent);
+    h->d_csr_ent = nullptr;
+    h->csr_cap = 0;
+    const int64_t cap = (int64_t)(entries * 1.3) + 1024;
+    const int st = dalloc(h, &h->d_csr_ent, cap * sizeof(int32_t));
+    if (!st) h->csr_cap = cap;
+    return st;
+}
+
+// room for every covalent row in the scaled-row map
+int nb_srows_cap(dmffb_engine* h) {
+    if (h->d_srows && h->cov_cap <= h->srows_cap) return DMFFB_OK;
+    if (h->d_srows) cudaFree(h->d_srows);
+    h->d_srows = nullptr;
+    h->srows_cap = 0;
+    h->srows_pairs = nullptr;
+    const int64_t cap = std::max<int64_t>(h->cov_cap, 64);
+    const int st = dalloc(h, &h->d_srows, cap * sizeof(int32_t));
+    if (!st) h->srows_cap = cap;
+    return st;
+}
+
+Nb2Args nb_args(dmffb_engine* h, const NbPlan& p, const double* pos, const Box& bx, double rc, bool want_csr) {
+    Nb2Args b;
+    b.a.n = h->n;
+    b.a.pos = pos;
+    b.a.box = bx;
+    b.a.rc = rc;
+    for (int k = 0; k < 3; ++k) b.a.nc[k] = p.nc[k];
+    b.a.cell_start = h->d_cell_start;
+    b.a.cell_atoms = nullptr;
+    b.a.cov_ptr = h->d_cov_ptr;
+    b.a.cov_j = h->d_cov_j;
+    b.a.cov_nb = h->d_cov_nb;
+    b.a.cov_lo = h->d_cov_lo;
+    b.a.cov_hi = h->d_cov_hi;
+    b.a.count = h->d_pcount;
+    b.a.offset = h->d_poff;
+    b.a.pairs = nullptr;
+    b.a.cap = 0;
+    b.posc = h->d_posc;
+    b.count_f = want_csr ? h->d_pcount_f : nullptr;
+    b.count_s = h->d_pcount_s;
+    b.sums = h->d_nbsum + sizeof(NbTotals) / 4;
+    b.off_f = want_csr ? h->d_csr_off : nullptr;
+    b.ent = nullptr;
+    b.cap_f = 0;
+    b.srows = nullptr;
+    b.off_s = h->d_poff_s;
+    b.cap_s = 0;
+    return b;
+}
+
+// offsets and totals of the counts in `b`; with slots, the lists too
+int nb_place(dmffb_engine* h, cudaStream_t s, const Nb2Args& b, bool slots, int32_t* rows, int64_t rows_cap, int32_t* ent,
+             int64_t ent_cap, int32_t* srows, int64_t srows_cap) {
+    PlaceArgs a;
+    a.n = h->n;
+    a.count_h = h->d_pcount;
+    a.count_f = b.count_f;
+    a.count_s = h->d_pcount_s;
+    a.sums = b.sums;
+    a.tot = (NbTotals*)h->d_nbsum;
+    a.off_h = h->d_poff;
+    a.off_f = b.count_f ? h->d_csr_off : nullptr;
+    a.off_s = h->d_poff_s;
+    a.ell_rows = slots ? b.ell_rows : nullptr;
+    a.ell_ent = slots ? b.ell_ent : nullptr;
+    a.cap_h = b.ell_cap_h;
+    a.cap_f = b.ell_cap_f;
+    a.rows = rows;
+    a.rows_cap = rows_cap;
+    a.ent = ent;
+    a.ent_cap = ent_cap;
+    a.srows = srows;
+    a.srows_cap = srows_cap;
+    LAUNCH(h, s, KC_NBLIST, k_nb_place<<<nblk(h->n, kPlaceAtoms), kPlaceThreads, 0, s>>>(a));
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(h->h_nbtot, h->d_nbsum, sizeof(NbTotals), cudaMemcpyDeviceToHost, s));
+    return DMFFB_OK;
+}
+
+// binning and distance tests of a single-pass build into the slots
+int nb_single_pass(dmffb_engine* h, cudaStream_t s, const NbPlan& p, const double* pos, const Box& bx, Nb2Args& b) {
+    const int n = h->n, words = nb_sum_words(n);
+    b.ell_rows = h->d_ell_rows;
+    b.ell_cap_h = h->ell_cap_h;
+    b.ell_ent = b.count_f ? h->d_ell_ent : nullptr;
+    b.ell_cap_f = h->ell_cap_f;
+    if (p.flat) {
+        CK(cudaMemsetAsync(h->d_nbsum, 0, words * sizeof(int32_t), s));
+        if (p.ortho) LAUNCH(h, s, KC_NBLIST, k_pairs_flat<true><<<nblk((int64_t)n * 32, 128), 128, 0, s>>>(b));
+        else LAUNCH(h, s, KC_NBLIST, k_pairs_flat<false><<<nblk((int64_t)n * 32, 128), 128, 0, s>>>(b));
+    } else {
+        const int st = bin_cells(h, s, pos, bx, p.nc, h->d_nbsum, words);
+        if (st) return st;
+        b.posc = h->d_posc;
+        b.a.cell_start = h->d_cell_start;
+        const size_t stage = (size_t)p.chmax * sizeof(float4);
+        if (p.ortho) LAUNCH(h, s, KC_NBLIST, k_pairs_cell<2, kNbWarps, true><<<p.ncell, 32 * kNbWarps, stage, s>>>(b, p.chmax));
+        else LAUNCH(h, s, KC_NBLIST, k_pairs_cell<2, kNbWarps, false><<<p.ncell, 32 * kNbWarps, stage, s>>>(b, p.chmax));
+    }
+    CK(cudaGetLastError());
+    return DMFFB_OK;
+}
+
+// count pass of the two-pass build, its totals on the host; the fill pass follows with nb_fill
+int nb_count(dmffb_engine* h, cudaStream_t s, const NbPlan& p, const double* pos, const Box& bx, Nb2Args& b) {
+    const int n = h->n;
+    int st;
+    if ((st = bin_cells(h, s, pos, bx, p.nc, h->d_nbsum, nb_sum_words(n)))) return st;
+    b.posc = h->d_posc;
+    b.a.cell_start = h->d_cell_start;
+    // keep masks for the fill pass: room for 1.5x the mean candidate count (125 cells of the
+    // stencil) per atom, at most 1 GiB; atoms with more candidates repeat the distance tests
+    const double mean_cand = 125.0 * (double)n / (double)p.ncell;
+    int64_t stride = (int64_t)ceil(1.5 * mean_cand / 32.0) + 2;
+    if ((int64_t)n * stride * 4 > ((int64_t)1 << 30)) stride = 0;
+    if (stride > 0 && (int64_t)n * stride > h->nbmask_cap) {
+        if (h->d_nbmask) cudaFree(h->d_nbmask);
+        h->d_nbmask = nullptr;
+        h->nbmask_cap = 0;
+        if ((st = dalloc(h, &h->d_nbmask, (int64_t)n * stride * sizeof(uint32_t)))) return st;
+        h->nbmask_cap = (int64_t)n * stride;
+    }
+    b.mask = stride > 0 ? h->d_nbmask : nullptr;
+    b.mask_stride = (int)stride;
+    LAUNCH(h, s, KC_NBLIST, k_pairs_warp3<0, 2><<<nblk((int64_t)n * 32, 32 * kNbWarps), 32 * kNbWarps, 0, s>>>(b));
+    if ((st = nb_place(h, s, b, false, nullptr, 0, nullptr, 0, nullptr, 0))) return st;
+    CK(cudaStreamSynchronize(s));
+    return DMFFB_OK;
+}
+
+int nb_fill(dmffb_engine* h, cudaStream_t s, const Nb2Args& b) {
+    LAUNCH(h, s, KC_NBLIST, k_pairs_warp3<1, 2><<<nblk((int64_t)h->n * 32, 32 * kNbWarps), 32 * kNbWarps, 0, s>>>(b));
     CK(cudaGetLastError());
     return DMFFB_OK;
 }
@@ -1879,7 +2106,7 @@ int classical_compute_impl(dmffb_engine* h, cudaStream_t s, const double* pos, c
     int st;
     // the cell pass: every pair within rc straight from the cell grid of these positions
     int ncf[3] = {0, 0, 0};
-    const bool cellpass = nonbonded && !pairs && h->cell_pass && h->pbc && !h->want_pgrad && half_cells(h, bx, ncf);
+    const bool cellpass = nonbonded && !pairs && h->cell_pass && h->pbc && !h->want_pgrad && half_cells(bx, h->rc, ncf);
     if (nonbonded && !pairs && !cellpass) {
         if (!h->have_pairs)
             if ((st = dmffb_admp_build_neighbors(h, (void*)s, pos, box))) return st;
@@ -2184,22 +2411,70 @@ int setup_mesh(dmffb_engine* h) {
 
 }  // namespace
 
-// Completes a single-pass build: waits for its totals; if a count or a total outgrew its
-// capacity, the list is rebuilt with the two passes (which resize the slots) from the positions
+// Queues a single-pass build of the engine's list into the slots and capacities at hand; the totals
+// travel to pinned memory behind an event (no host wait here).
+int nb_start(dmffb_engine* h, cudaStream_t s, const double* pos, const double* box) {
+    Box bx;
+    make_box(box, bx);
+    const NbPlan p = nb_plan(h, bx, h->rc);
+    const bool want_csr = h->kind == 0 && h->lpol;
+    Nb2Args b = nb_args(h, p, pos, bx, h->rc, want_csr);
+    int st;
+    if ((st = nb_single_pass(h, s, p, pos, bx, b))) return st;
+    // row indices are 32-bit: lists beyond that keep no map (scaled_rows refuses them)
+    int32_t* const srows = h->pair_cap <= 0x7fffffff ? h->d_srows : nullptr;
+    if ((st = nb_place(h, s, b, true, h->d_pairs, h->pair_cap, want_csr ? h->d_csr_ent : nullptr, h->csr_cap, srows,
+                       h->srows_cap)))
+        return st;
+    if (!h->e_nbtot) CK(cudaEventCreateWithFlags(&h->e_nbtot, cudaEventDisableTiming));
+    CK(cudaEventRecord(h->e_nbtot, s));
+    if (!h->e_build) CK(cudaEventCreateWithFlags(&h->e_build, cudaEventDisableTiming));
+    CK(cudaEventRecord(h->e_build, s));
+    h->nb_pending = true;
+    h->nb_want_csr = want_csr;
+    h->nb_cap_h = b.ell_cap_h;
+    h->nb_cap_f = b.ell_cap_f;
+    h->nb_stream = s;
+    h->nb_pos = pos;
+    for (int k = 0; k < 9; ++k) h->nb_box[k] = box[k];
+    h->npairs = 0;
+    h->have_pairs = true;
+    h->pairs_gen++;
+    h->csr_from_build = want_csr;
+    h->srows_pairs = srows ? h->d_pairs : nullptr;
+    h->srows_npairs = -1;
+    h->srows_gen = h->pairs_gen;
+    return DMFFB_OK;
+}
+
+// Completes a single-pass build: waits for its totals; if a count or a total outgrew its capacity,
+// slots and lists grow to what the counts ask for and the list is built again from the positions
 // the build was given, on its stream.
 int nb_finish(dmffb_engine* h) {
-    if (!h->nb_pending) return DMFFB_OK;
-    h->nb_pending = false;
-    CK(cudaEventSynchronize(h->e_nbtot));
-    const int* md = (const int*)(h->h_nbtot + 2);
-    if (md[0] <= h->ell_cap_h && (!h->nb_want_csr || md[1] <= h->ell_cap_f) && h->h_nbtot[0] <= h->pair_cap &&
-        (!h->nb_want_csr || h->h_nbtot[1] <= h->csr_cap)) {
-        h->npairs = h->h_nbtot[0];
-        return DMFFB_OK;
+    while (h->nb_pending) {
+        h->nb_pending = false;
+        CK(cudaEventSynchronize(h->e_nbtot));
+        const NbTotals t = *h->h_nbtot;
+        const bool csr = h->nb_want_csr;
+        if (t.max_h <= h->nb_cap_h && (!csr || t.max_f <= h->nb_cap_f) && t.rows <= h->pair_cap &&
+            (!csr || t.entries <= h->csr_cap)) {
+            h->npairs = t.rows;
+            // the scaled-row map made with the list, unless other rows have replaced it since
+            if (h->srows_pairs == h->d_pairs && h->srows_gen == h->pairs_gen) {
+                h->n_srows = t.scaled;
+                h->srows_npairs = t.rows;
+            }
+            return DMFFB_OK;
+        }
+        h->have_pairs = false;
+        int st;
+        if ((st = nb_slots(h, t.max_h > h->nb_cap_h ? nb_headroom(t.max_h) : 0,
+                           csr && t.max_f > h->nb_cap_f ? nb_headroom(t.max_f) : 0)))
+            return st;
+        if ((st = nb_pair_cap(h, t.rows)) || (csr && (st = nb_csr_cap(h, t.entries)))) return st;
+        if ((st = nb_start(h, h->nb_stream, h->nb_pos, h->nb_box))) return st;
     }
-    h->have_pairs = false;
-    h->ell_cap_h = h->ell_cap_f = 0;  // the two passes this time
-    return dmffb_admp_build_neighbors(h, (void*)h->nb_stream, h->nb_pos, h->nb_box);
+    return DMFFB_OK;
 }
 
 // Drops a single-pass build whose list will not be used (the engine is reconfigured, staged rows
@@ -2326,13 +2601,13 @@ void dmffb_destroy(dmffb_engine* h) {
     void* ptrs[] = {h->d_axis_type, h->d_axis_idx, h->d_cov_ptr, h->d_cov_j, h->d_cov_nb, h->d_Qloc, h->d_pol,
                     h->d_thole, h->d_polsix, h->d_pos, h->d_U, h->d_forces, h->d_posT, h->d_Qg, h->d_QgT,
                     h->d_gpair, h->d_torque, h->d_fieldT, h->d_grad, h->d_scal, h->d_b, h->d_r, h->d_z, h->d_p,
-                    h->d_Ap, h->d_fr, h->d_gQ, h->d_fmv, h->d_posf, h->d_pcount_f, h->d_mvcoef, h->d_csr_off, h->d_csr_ent, h->d_csr_deg, h->d_cub2, h->d_grid, h->d_grid2, h->d_cgrid, h->d_bmod, h->d_pairs, h->d_atom_cell,
-                    h->d_cell_count, h->d_cell_start, h->d_cell_cursor, h->d_cell_atoms, h->d_pcount, h->d_poff,
+                    h->d_Ap, h->d_fr, h->d_gQ, h->d_fmv, h->d_pcount_f, h->d_pcount_s, h->d_poff_s, h->d_rank, h->d_bin_done, h->d_nbsum, h->d_mvcoef, h->d_csr_off, h->d_csr_ent, h->d_csr_deg, h->d_cub2, h->d_grid, h->d_grid2, h->d_cgrid, h->d_bmod, h->d_pairs, h->d_atom_cell,
+                    h->d_cell_count, h->d_cell_start, h->d_pcount, h->d_poff,
                     h->d_c, h->d_tta, h->d_ttb, h->d_ttq, h->d_glr, h->d_gsr, h->d_dc,
                     h->d_q, h->d_qT, h->d_type, h->d_sigtt, h->d_epstt, h->d_dq, h->d_dsig, h->d_deps,
                     h->d_tidx[0], h->d_tidx[1], h->d_tidx[2], h->d_tprm[0], h->d_tprm[1], h->d_tprm[2],
                     h->d_tdprm[0], h->d_tdprm[1], h->d_tdprm[2], h->d_dQloc, h->d_dpa, h->d_dth, h->d_dpol, h->d_dsr, h->d_srows, h->d_nsel, h->d_cubsel,
-                    h->d_cub, h->d_ell_rows, h->d_ell_ent, h->d_maxdeg, h->d_stc_org, h->d_stc_w, h->d_nbmask, h->d_covrows, h->d_cov_lo, h->d_cov_hi, h->d_dftW, h->d_dftG, h->d_pcg, h->d_posc, h->d_srp, h->d_srdp, h->d_srgrad};
+                    h->d_ell_rows, h->d_ell_ent, h->d_stc_org, h->d_stc_w, h->d_nbmask, h->d_covrows, h->d_cov_lo, h->d_cov_hi, h->d_dftW, h->d_dftG, h->d_pcg, h->d_posc, h->d_srp, h->d_srdp, h->d_srgrad};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (h->h_scal) cudaFreeHost(h->h_scal);
@@ -2811,89 +3086,34 @@ int dmffb_build_neighbors(dmffb_engine* h, void* stream, const double* pos, cons
     const int n = h->n;
     Box bx;
     make_box(box, bx);
-    // cells per axis from the perpendicular widths V / |a_i x a_j|
-    const double* m = bx.h;
-    const double V = fabs(det3(m));
-    int nc[3];
-    bool cells = true;
-    for (int k = 0; k < 3; ++k) {
-        const double* u = m + 3 * ((k + 1) % 3);
-        const double* w = m + 3 * ((k + 2) % 3);
-        const double cx = u[1] * w[2] - u[2] * w[1], cy = u[2] * w[0] - u[0] * w[2], cz = u[0] * w[1] - u[1] * w[0];
-        const double width = V / sqrt(cx * cx + cy * cy + cz * cz);
-        nc[k] = (int)floor(width / rc);
-        if (nc[k] > 64) nc[k] = 64;
-        if (nc[k] < 3) cells = false;
-    }
     int st;
-    if (!h->d_pcount) {
-        const int nc = h->n_cap;
-        if ((st = dalloc(h, &h->d_pcount, nc * sizeof(int32_t)))) return st;
-        if ((st = dalloc(h, &h->d_poff, (nc + 1) * sizeof(int64_t)))) return st;
-        if ((st = dalloc(h, &h->d_atom_cell, nc * sizeof(int32_t)))) return st;
-        if ((st = dalloc(h, &h->d_cell_atoms, nc * sizeof(int32_t)))) return st;
+    if (h->nb_pending && (st = nb_finish(h))) return st;  // the builds of one engine share their scratch
+    const NbPlan p = nb_plan(h, bx, rc);
+    if ((st = nb_alloc(h, false))) return st;
+    Nb2Args b = nb_args(h, p, pos, bx, rc, false);
+    if (p.flat || p.staged) {
+        for (int grow = h->ell_cap_h > 0 ? 0 : p.guess;;) {
+            if ((st = nb_slots(h, grow, 0))) return st;
+            if ((st = nb_single_pass(h, s, p, pos, bx, b))) return st;
+            if ((st = nb_place(h, s, b, true, pairs_out, capacity, nullptr, 0, nullptr, 0))) return st;
+            CK(cudaStreamSynchronize(s));
+            if (h->h_nbtot->max_h <= b.ell_cap_h) break;
+            grow = nb_headroom(h->h_nbtot->max_h);
+        }
+    } else if ((st = nb_count(h, s, p, pos, bx, b))) {
+        return st;
     }
-    const int ncell = cells ? nc[0] * nc[1] * nc[2] : 1;
-    if (ncell + 1 > h->ncell_cap) {
-        if (h->d_cell_count) { cudaFree(h->d_cell_count); cudaFree(h->d_cell_start); cudaFree(h->d_cell_cursor); }
-        h->ncell_cap = ncell + 1;
-        if ((st = dalloc(h, &h->d_cell_count, h->ncell_cap * sizeof(int32_t)))) return st;
-        if ((st = dalloc(h, &h->d_cell_start, h->ncell_cap * sizeof(int32_t)))) return st;
-        if ((st = dalloc(h, &h->d_cell_cursor, h->ncell_cap * sizeof(int32_t)))) return st;
-    }
-    // scan workspace
-    size_t need = 0, need2 = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, need, (int32_t*)nullptr, (int32_t*)nullptr, ncell + 1);
-    cub::DeviceScan::InclusiveSum(nullptr, need2, (int32_t*)nullptr, (int64_t*)nullptr, n);
-    need = std::max(need, need2);
-    if (need > h->cub_bytes) {
-        if (h->d_cub) cudaFree(h->d_cub);
-        h->cub_bytes = need;
-        if ((st = dalloc(h, &h->d_cub, need))) return st;
-    }
-    NbArgs a;
-    a.n = n;
-    a.pos = pos;
-    a.box = bx;
-    a.rc = rc;
-    for (int k = 0; k < 3; ++k) a.nc[k] = cells ? nc[k] : 1;
-    a.cov_ptr = h->d_cov_ptr;
-    a.cov_j = h->d_cov_j;
-    a.cov_nb = h->d_cov_nb;
-    a.count = h->d_pcount;
-    a.offset = h->d_poff;
-    a.pairs = pairs_out;
-    a.cap = capacity;
-    if (cells) {
-        CK(cudaMemsetAsync(h->d_cell_count, 0, (ncell + 1) * sizeof(int32_t), s));
-        CK(cudaMemsetAsync(h->d_cell_cursor, 0, (ncell + 1) * sizeof(int32_t), s));
-        LAUNCH(h, s, KC_NBLIST, k_cell_count<<<nblk(n, 256), 256, 0, s>>>(n, pos, bx, nc[0], nc[1], nc[2], h->d_atom_cell, h->d_cell_count));
-        size_t tb = h->cub_bytes;
-        LAUNCH(h, s, KC_NBLIST, cub::DeviceScan::ExclusiveSum(h->d_cub, tb, h->d_cell_count, h->d_cell_start, ncell + 1, s));
-        LAUNCH(h, s, KC_NBLIST, k_cell_fill<<<nblk(n, 256), 256, 0, s>>>(n, h->d_atom_cell, h->d_cell_start, h->d_cell_cursor, h->d_cell_atoms));
-        a.cell_start = h->d_cell_start;
-        a.cell_atoms = h->d_cell_atoms;
-        LAUNCH(h, s, KC_NBLIST, k_pairs_warp<0><<<nblk((int64_t)n * 32, 256), 256, 0, s>>>(a));
-    } else {
-        LAUNCH(h, s, KC_NBLIST, k_pairs_all<0><<<nblk(n, 128), 128, 0, s>>>(a));
-    }
-    {
-        size_t tb = h->cub_bytes;
-        CK(cudaMemsetAsync(h->d_poff, 0, sizeof(int64_t), s));
-        LAUNCH(h, s, KC_NBLIST, cub::DeviceScan::InclusiveSum(h->d_cub, tb, h->d_pcount, h->d_poff + 1, n, s));
-    }
-    int64_t total = 0;
-    CK(cudaMemcpyAsync(&total, h->d_poff + n, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    *npairs_out = total;
-    if (total > capacity || !pairs_out) {
+    *npairs_out = h->h_nbtot->rows;
+    if (*npairs_out > capacity || !pairs_out) {
         h->err = "neighbour capacity too small";
         return DMFFB_NEIGHBOR_OVERFLOW;
     }
-    if (cells) LAUNCH(h, s, KC_NBLIST, k_pairs_warp<1><<<nblk((int64_t)n * 32, 256), 256, 0, s>>>(a));
-    else LAUNCH(h, s, KC_NBLIST, k_pairs_all<1><<<nblk(n, 128), 128, 0, s>>>(a));
-    CK(cudaGetLastError());
-    CK(cudaStreamSynchronize(s));
+    if (!p.flat && !p.staged) {
+        b.a.pairs = pairs_out;
+        b.a.cap = capacity;
+        if ((st = nb_fill(h, s, b))) return st;
+        CK(cudaStreamSynchronize(s));
+    }
     prof_collect(h);
     return DMFFB_OK;
 }
@@ -2902,248 +3122,40 @@ int dmffb_admp_build_neighbors(dmffb_engine* h, void* stream, const double* pos,
     if (!h || !pos || !box) return DMFFB_BAD_ARG;
     if (h->nb_pending) nb_discard(h);  // this build replaces it
     cudaStream_t s = (cudaStream_t)stream;
-    const int n = h->n;
     Box bx;
     make_box(box, bx);
-    const double* m = bx.h;
-    const double V = fabs(det3(m));
-    int nc[3], nc2[3];
-    bool cells = true, fine = true;  // fine: half-width cells with the 5^3 stencil
-    for (int k = 0; k < 3; ++k) {
-        const double* u = m + 3 * ((k + 1) % 3);
-        const double* w = m + 3 * ((k + 2) % 3);
-        const double cx = u[1] * w[2] - u[2] * w[1], cy = u[2] * w[0] - u[0] * w[2], cz = u[0] * w[1] - u[1] * w[0];
-        const double width = V / sqrt(cx * cx + cy * cy + cz * cz);
-        nc[k] = (int)floor(width / h->rc);
-        if (nc[k] > 64) nc[k] = 64;
-        if (nc[k] < 3) cells = false;
-        nc2[k] = (int)floor(width / (0.5 * h->rc));
-        if (nc2[k] > 64) nc2[k] = 64;
-        if (nc2[k] < 5) fine = false;
-    }
-    if (fine && cells)
-        for (int k = 0; k < 3; ++k) nc[k] = nc2[k];
-    if (!cells) {  // small boxes: the generic builder, CSR later from the rows
-        int64_t need = 0;
-        int st = dmffb_build_neighbors(h, stream, pos, box, h->rc, h->d_pairs, h->pair_cap, &need);
-        if (st == DMFFB_NEIGHBOR_OVERFLOW) {
-            if (h->d_pairs) cudaFree(h->d_pairs);
-            h->pair_cap = (int64_t)(need * 1.3) + 64;
-            if ((st = dalloc(h, &h->d_pairs, h->pair_cap * 3 * sizeof(int32_t)))) return st;
-            st = dmffb_build_neighbors(h, stream, pos, box, h->rc, h->d_pairs, h->pair_cap, &need);
-        }
-        if (st) return st;
-        h->npairs = need;
-        h->have_pairs = true;
-        h->pairs_gen++;
-        h->csr_from_build = false;
-        return DMFFB_OK;
-    }
-    int st;
-    if (!h->d_pcount) {
-        const int nc = h->n_cap;
-        if ((st = dalloc(h, &h->d_pcount, nc * sizeof(int32_t)))) return st;
-        if ((st = dalloc(h, &h->d_poff, (nc + 1) * sizeof(int64_t)))) return st;
-        if ((st = dalloc(h, &h->d_atom_cell, nc * sizeof(int32_t)))) return st;
-        if ((st = dalloc(h, &h->d_cell_atoms, nc * sizeof(int32_t)))) return st;
-    }
-    if (!h->d_posf) {
-        if ((st = dalloc(h, &h->d_posf, 4 * h->n_cap * sizeof(float)))) return st;
-        if ((st = dalloc(h, &h->d_pcount_f, h->n_cap * sizeof(int32_t)))) return st;
-    }
-    if (!h->d_csr_off) {
-        const int nc = h->n_cap;
-        if ((st = dalloc(h, &h->d_csr_off, (nc + 1) * sizeof(int64_t)))) return st;
-        if ((st = dalloc(h, &h->d_csr_deg, nc * sizeof(int32_t)))) return st;
-        if ((st = dalloc(h, &h->d_fmv, 3 * nc * sizeof(double)))) return st;
-        size_t need = 0;
-        cub::DeviceScan::InclusiveSum(nullptr, need, (int32_t*)nullptr, (int64_t*)nullptr, nc);
-        h->cub2_bytes = need;
-        if ((st = dalloc(h, &h->d_cub2, need))) return st;
-    }
-    const int ncell = nc[0] * nc[1] * nc[2];
-    if (ncell + 1 > h->ncell_cap) {
-        if (h->d_cell_count) { cudaFree(h->d_cell_count); cudaFree(h->d_cell_start); cudaFree(h->d_cell_cursor); }
-        h->ncell_cap = ncell + 1;
-        if ((st = dalloc(h, &h->d_cell_count, h->ncell_cap * sizeof(int32_t)))) return st;
-        if ((st = dalloc(h, &h->d_cell_start, h->ncell_cap * sizeof(int32_t)))) return st;
-        if ((st = dalloc(h, &h->d_cell_cursor, h->ncell_cap * sizeof(int32_t)))) return st;
-    }
-    size_t need = 0, need2 = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, need, (int32_t*)nullptr, (int32_t*)nullptr, ncell + 1);
-    cub::DeviceScan::InclusiveSum(nullptr, need2, (int32_t*)nullptr, (int64_t*)nullptr, n);
-    need = std::max(need, need2);
-    if (need > h->cub_bytes) {
-        if (h->d_cub) cudaFree(h->d_cub);
-        h->cub_bytes = need;
-        if ((st = dalloc(h, &h->d_cub, need))) return st;
-    }
-    LAUNCH(h, s, KC_NBLIST, k_pos_f32<<<nblk(n, 256), 256, 0, s>>>(n, pos, h->d_posf));
-    CK(cudaMemsetAsync(h->d_cell_count, 0, (ncell + 1) * sizeof(int32_t), s));
-    CK(cudaMemsetAsync(h->d_cell_cursor, 0, (ncell + 1) * sizeof(int32_t), s));
-    LAUNCH(h, s, KC_NBLIST, k_cell_count<<<nblk(n, 256), 256, 0, s>>>(n, pos, bx, nc[0], nc[1], nc[2], h->d_atom_cell,
-                                                                     h->d_cell_count));
-    size_t tb = h->cub_bytes;
-    LAUNCH(h, s, KC_NBLIST, cub::DeviceScan::ExclusiveSum(h->d_cub, tb, h->d_cell_count, h->d_cell_start, ncell + 1, s));
-    LAUNCH(h, s, KC_NBLIST, k_cell_fill<<<nblk(n, 256), 256, 0, s>>>(n, h->d_atom_cell, h->d_cell_start,
-                                                                    h->d_cell_cursor, h->d_cell_atoms));
-    Nb2Args b;
-    b.a.n = n;
-    b.a.pos = pos;
-    b.a.box = bx;
-    b.a.rc = h->rc;
-    for (int k = 0; k < 3; ++k) b.a.nc[k] = nc[k];
-    b.a.cell_start = h->d_cell_start;
-    b.a.cell_atoms = h->d_cell_atoms;
-    b.a.cov_ptr = h->d_cov_ptr;
-    b.a.cov_j = h->d_cov_j;
-    b.a.cov_nb = h->d_cov_nb;
-    b.a.cov_lo = h->d_cov_lo;
-    b.a.cov_hi = h->d_cov_hi;
-    b.a.count = h->d_pcount;
-    b.a.offset = h->d_poff;
-    b.posf = h->d_posf;
-    // the full CSR feeds only the polarizable dipole solve; other engines take the half rows alone
+    const NbPlan p = nb_plan(h, bx, h->rc);
     const bool want_csr = h->kind == 0 && h->lpol;
-    b.count_f = want_csr ? h->d_pcount_f : nullptr;
-    b.off_f = want_csr ? h->d_csr_off : nullptr;
-    b.ent = nullptr;
-    b.cap_f = 0;
-    if (fine) {
-        // keep masks for the fill pass: room for 1.5x the mean candidate count (125 cells of the
-        // stencil) per atom, at most 1 GiB; atoms with more candidates repeat the distance tests
-        const double mean_cand = 125.0 * (double)n / (double)ncell;
-        int64_t stride = (int64_t)ceil(1.5 * mean_cand / 32.0) + 2;
-        if ((int64_t)n * stride * 4 > ((int64_t)1 << 30)) stride = 0;
-        if (stride > 0 && (int64_t)n * stride > h->nbmask_cap) {
-            if (h->d_nbmask) cudaFree(h->d_nbmask);
-            h->d_nbmask = nullptr;
-            h->nbmask_cap = (int64_t)n * stride;
-            if ((st = dalloc(h, &h->d_nbmask, h->nbmask_cap * sizeof(uint32_t)))) return st;
+    int st;
+    if ((st = nb_alloc(h, want_csr)) || (st = nb_srows_cap(h))) return st;
+    if (p.flat || p.staged) {
+        // a first build sizes slots and lists from the mean density and waits for its totals (the
+        // caller may change the positions when it returns); later ones leave that to nb_finish
+        const bool first = !h->ell_cap_h || (want_csr && !h->ell_cap_f) || !h->d_pairs || (want_csr && !h->d_csr_ent);
+        if (first) {
+            const int64_t rows = (int64_t)h->n * p.guess / 2 + 1;
+            if ((st = nb_slots(h, h->ell_cap_h ? 0 : p.guess, want_csr && !h->ell_cap_f ? p.guess : 0))) return st;
+            if (!h->d_pairs && (st = nb_pair_cap(h, rows))) return st;
+            if (want_csr && !h->d_csr_ent && (st = nb_csr_cap(h, 2 * rows))) return st;
         }
-        b.mask = stride > 0 ? h->d_nbmask : nullptr;
-        b.mask_stride = (int)stride;
-    }
-    // small neighbourhoods (staging room for 1.5x the mean candidate count within 44 KB): one CTA
-    // per cell with the candidates staged in shared memory; larger ones keep the warp-per-atom
-    // kernel, whose L2 gathers run at full occupancy (measured faster there than 100 KB stages)
-    const int chmax = (int)(1.5 * 125.0 * (double)n / (double)ncell + 64.0);
-    const size_t stage_bytes = (size_t)chmax * sizeof(float4);
-    const bool staged = stage_bytes <= kNbStageBytes;
-    const bool ortho = m[1] == 0.0 && m[2] == 0.0 && m[3] == 0.0 && m[5] == 0.0 && m[6] == 0.0 && m[7] == 0.0;
-    if (!h->d_maxdeg && (st = dalloc(h, &h->d_maxdeg, 2 * sizeof(int)))) return st;
-    int maxdeg[2] = {0, 0};
-    // Single pass: the distance tests run once, each atom's rows and CSR entries go to its slots,
-    // the scans of the counts place them and k_ell_compact copies them there (the same row set
-    // and CSR as the two passes below).  Taken when the last two-pass build sized the slots; if a
-    // count or a total outgrows its capacity, the two-pass build runs after all.
-    if (fine && staged && h->ell_cap_h > 0 && (!want_csr || h->ell_cap_f > 0) && h->d_pairs &&
-        (!want_csr || h->d_csr_ent)) {
-        Nb2Args e = b;
-        e.mask = nullptr;
-        e.mask_stride = 0;
-        e.ell_rows = h->d_ell_rows;
-        e.ell_ent = want_csr ? h->d_ell_ent : nullptr;
-        e.ell_cap_h = h->ell_cap_h;
-        e.ell_cap_f = h->ell_cap_f;
-        e.maxdeg = h->d_maxdeg;
-        CK(cudaMemsetAsync(h->d_maxdeg, 0, 2 * sizeof(int), s));
-        if (ortho) LAUNCH(h, s, KC_NBLIST, k_pairs_cell<2, 2, kNbWarps, true><<<ncell, 32 * kNbWarps, stage_bytes, s>>>(e, chmax));
-        else LAUNCH(h, s, KC_NBLIST, k_pairs_cell<2, 2, kNbWarps, false><<<ncell, 32 * kNbWarps, stage_bytes, s>>>(e, chmax));
-        CK(cudaMemsetAsync(h->d_poff, 0, sizeof(int64_t), s));
-        tb = h->cub_bytes;
-        LAUNCH(h, s, KC_NBLIST, cub::DeviceScan::InclusiveSum(h->d_cub, tb, h->d_pcount, h->d_poff + 1, n, s));
-        if (want_csr) {
-            CK(cudaMemsetAsync(h->d_csr_off, 0, sizeof(int64_t), s));
-            tb = h->cub_bytes;
-            LAUNCH(h, s, KC_NBLIST, cub::DeviceScan::InclusiveSum(h->d_cub, tb, h->d_pcount_f, h->d_csr_off + 1, n, s));
-        }
-        LAUNCH(h, s, KC_NBLIST, k_ell_compact<<<nblk((int64_t)n * 32, 256), 256, 0, s>>>(
-                                    n, h->d_pcount, h->d_pcount_f, h->d_poff, h->d_csr_off, h->d_ell_rows, h->ell_cap_h,
-                                    want_csr ? h->d_ell_ent : nullptr, h->ell_cap_f, h->d_pairs, h->pair_cap,
-                                    want_csr ? h->d_csr_ent : nullptr, h->csr_cap));
-        CK(cudaGetLastError());
-        // the totals travel to pinned memory behind an event; no host wait here (nb_finish)
-        if (!h->h_nbtot && cudaMallocHost((void**)&h->h_nbtot, 4 * sizeof(int64_t)) != cudaSuccess)
-            return fail(h, DMFFB_OOM, "cudaMallocHost failed");
-        h->h_nbtot[0] = h->h_nbtot[1] = h->h_nbtot[2] = h->h_nbtot[3] = 0;
-        if (want_csr) CK(cudaMemcpyAsync(h->h_nbtot + 1, h->d_csr_off + n, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-        CK(cudaMemcpyAsync(h->h_nbtot, h->d_poff + n, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-        CK(cudaMemcpyAsync(h->h_nbtot + 2, h->d_maxdeg, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
-        if (!h->e_nbtot) CK(cudaEventCreateWithFlags(&h->e_nbtot, cudaEventDisableTiming));
-        CK(cudaEventRecord(h->e_nbtot, s));
-        if (!h->e_build) CK(cudaEventCreateWithFlags(&h->e_build, cudaEventDisableTiming));
-        CK(cudaEventRecord(h->e_build, s));
-        h->nb_pending = true;
-        h->nb_want_csr = want_csr;
-        h->nb_stream = s;
-        h->nb_pos = pos;
-        for (int k = 0; k < 9; ++k) h->nb_box[k] = box[k];
-        h->npairs = 0;
-        h->have_pairs = true;
-        h->pairs_gen++;
-        h->csr_from_build = want_csr;
-        if (h->prof) {
-            const int stf = nb_finish(h);
-            if (stf) return stf;
+        if ((st = nb_start(h, s, pos, box))) return st;
+        if (first || h->prof) {
+            if ((st = nb_finish(h))) return st;
             prof_collect(h);
         }
         return DMFFB_OK;
     }
-    b.maxdeg = h->d_maxdeg;
-    CK(cudaMemsetAsync(h->d_maxdeg, 0, 2 * sizeof(int), s));
-    if (fine && !staged) LAUNCH(h, s, KC_NBLIST, k_pairs_warp3<0, 2><<<nblk((int64_t)n * 32, 32 * kNbWarps), 32 * kNbWarps, 0, s>>>(b));
-    else if (fine && ortho) LAUNCH(h, s, KC_NBLIST, k_pairs_cell<0, 2, kNbWarps, true><<<ncell, 32 * kNbWarps, stage_bytes, s>>>(b, chmax));
-    else if (fine) LAUNCH(h, s, KC_NBLIST, k_pairs_cell<0, 2, kNbWarps, false><<<ncell, 32 * kNbWarps, stage_bytes, s>>>(b, chmax));
-    else LAUNCH(h, s, KC_NBLIST, k_pairs_warp2<0><<<nblk((int64_t)n * 32, 256), 256, 0, s>>>(b));
-    CK(cudaMemsetAsync(h->d_poff, 0, sizeof(int64_t), s));
-    tb = h->cub_bytes;
-    LAUNCH(h, s, KC_NBLIST, cub::DeviceScan::InclusiveSum(h->d_cub, tb, h->d_pcount, h->d_poff + 1, n, s));
-    int64_t tot[2] = {0, 0};
-    if (want_csr) {
-        CK(cudaMemsetAsync(h->d_csr_off, 0, sizeof(int64_t), s));
-        tb = h->cub_bytes;
-        LAUNCH(h, s, KC_NBLIST, cub::DeviceScan::InclusiveSum(h->d_cub, tb, h->d_pcount_f, h->d_csr_off + 1, n, s));
-        CK(cudaMemcpyAsync(&tot[1], h->d_csr_off + n, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-    }
-    CK(cudaMemcpyAsync(&tot[0], h->d_poff + n, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(maxdeg, h->d_maxdeg, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    // slots for the next build's single pass: the largest counts with an eighth (at least 16) of
-    // headroom, for the cell-staged kernel only (the warp-per-atom kernels leave maxdeg at 0)
-    if (fine && staged && maxdeg[0] > 0) {
-        const int ch = maxdeg[0] + std::max(16, maxdeg[0] / 8), cf = maxdeg[1] + std::max(16, maxdeg[1] / 8);
-        if (ch > h->ell_cap_h || (want_csr && cf > h->ell_cap_f)) {
-            if (h->d_ell_rows) cudaFree(h->d_ell_rows);
-            if (h->d_ell_ent) cudaFree(h->d_ell_ent);
-            h->d_ell_rows = nullptr;
-            h->d_ell_ent = nullptr;
-            h->ell_cap_h = h->ell_cap_f = 0;
-            if ((st = dalloc(h, &h->d_ell_rows, (size_t)h->n_cap * ch * 3 * sizeof(int32_t)))) return st;
-            if (want_csr && (st = dalloc(h, &h->d_ell_ent, (size_t)h->n_cap * cf * sizeof(int32_t)))) return st;
-            h->ell_cap_h = ch;
-            h->ell_cap_f = want_csr ? cf : 0;
-        }
-    }
-    if (tot[0] > h->pair_cap) {
-        if (h->d_pairs) cudaFree(h->d_pairs);
-        h->pair_cap = (int64_t)(tot[0] * 1.3) + 64;  // headroom as in nblist.py:37-38
-        if ((st = dalloc(h, &h->d_pairs, h->pair_cap * 3 * sizeof(int32_t)))) return st;
-    }
-    if (want_csr && tot[1] > h->csr_cap) {
-        if (h->d_csr_ent) cudaFree(h->d_csr_ent);
-        h->csr_cap = (int64_t)(tot[1] * 1.3) + 1024;
-        if ((st = dalloc(h, &h->d_csr_ent, h->csr_cap * sizeof(int32_t)))) return st;
-    }
+    Nb2Args b = nb_args(h, p, pos, bx, h->rc, want_csr);
+    if ((st = nb_count(h, s, p, pos, bx, b))) return st;
+    const NbTotals t = *h->h_nbtot;
+    if ((st = nb_pair_cap(h, t.rows)) || (want_csr && (st = nb_csr_cap(h, t.entries)))) return st;
     b.a.pairs = h->d_pairs;
     b.a.cap = h->pair_cap;
     b.ent = want_csr ? h->d_csr_ent : nullptr;
     b.cap_f = want_csr ? h->csr_cap : 0;
-    if (fine && !staged) LAUNCH(h, s, KC_NBLIST, k_pairs_warp3<1, 2><<<nblk((int64_t)n * 32, 32 * kNbWarps), 32 * kNbWarps, 0, s>>>(b));
-    else if (fine && ortho) LAUNCH(h, s, KC_NBLIST, k_pairs_cell<1, 2, kNbWarps, true><<<ncell, 32 * kNbWarps, stage_bytes, s>>>(b, chmax));
-    else if (fine) LAUNCH(h, s, KC_NBLIST, k_pairs_cell<1, 2, kNbWarps, false><<<ncell, 32 * kNbWarps, stage_bytes, s>>>(b, chmax));
-    else LAUNCH(h, s, KC_NBLIST, k_pairs_warp2<1><<<nblk((int64_t)n * 32, 256), 256, 0, s>>>(b));
-    CK(cudaGetLastError());
+    b.srows = t.rows <= 0x7fffffff ? h->d_srows : nullptr;
+    b.cap_s = h->srows_cap;
+    if ((st = nb_fill(h, s, b))) return st;
     // no host wait for the fill pass: later work on this stream is ordered after it, and compute
     // calls on other streams wait for e_build before they read the engine's list
     if (h->prof) {
@@ -3152,10 +3164,16 @@ int dmffb_admp_build_neighbors(dmffb_engine* h, void* stream, const double* pos,
     }
     if (!h->e_build) CK(cudaEventCreateWithFlags(&h->e_build, cudaEventDisableTiming));
     CK(cudaEventRecord(h->e_build, s));
-    h->npairs = tot[0];
+    h->npairs = t.rows;
     h->have_pairs = true;
     h->pairs_gen++;
     h->csr_from_build = want_csr;
+    if (b.srows) {
+        h->n_srows = t.scaled;
+        h->srows_pairs = h->d_pairs;
+        h->srows_npairs = t.rows;
+        h->srows_gen = h->pairs_gen;
+    }
     return DMFFB_OK;
 }
 

@@ -7,9 +7,11 @@
 // runs in FP64 with every product and sum rounded separately in a fixed order, so the pair set
 // is reproducible bit for bit by an elementwise float64 computation on the host.
 //
-// Atoms are binned by fractional coordinates into nc_k >= 3 cells per axis (cell width >=
-// rc measured perpendicular to the other two lattice vectors), counting-sorted by cell,
-// and each atom scans the 27 surrounding cells twice (count, then write).
+// The engine's builds: k_bin_count + k_bin_fill sort the atoms into half-width cells, one pass of
+// k_pairs_cell (k_pairs_flat in boxes below five such cells) runs the distance tests and leaves each
+// atom's rows in its slots, and k_nb_place scans the counts and copies the slots to their final
+// places.  The kernels before those (k_cell_count .. k_pairs_warp: cells at least rc wide, 27-cell
+// scan, count and write passes) serve the build that allocates no memory.
 #pragma once
 #include "common.cuh"
 
@@ -91,45 +93,8 @@ __device__ __forceinline__ int lookup_nbond(const NbArgs& a, int i, int j) {
     return 0;
 }
 
-// pass 0: count pairs per atom; pass 1: write rows at offset[i]
-template <int PASS>
-__global__ void __launch_bounds__(128) k_pairs(NbArgs a) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.n) return;
-    const double* pi = a.pos + 3 * i;
-    int c3[3];
-    cell_of(a.box, a.nc, pi, c3);
-    int cnt = 0;
-    int64_t out = (PASS == 1) ? a.offset[i] : 0;
-    for (int dx = -1; dx <= 1; ++dx) {
-        const int cx = (c3[0] + dx + a.nc[0]) % a.nc[0];
-        for (int dy = -1; dy <= 1; ++dy) {
-            const int cy = (c3[1] + dy + a.nc[1]) % a.nc[1];
-            for (int dz = -1; dz <= 1; ++dz) {
-                const int cz = (c3[2] + dz + a.nc[2]) % a.nc[2];
-                const int c = (cx * a.nc[1] + cy) * a.nc[2] + cz;
-                for (int k = a.cell_start[c]; k < a.cell_start[c + 1]; ++k) {
-                    const int j = a.cell_atoms[k];
-                    if (j <= i) continue;
-                    if (!within_rc(a.box, pi, a.pos + 3 * j, a.rc)) continue;
-                    if (PASS == 1) {
-                        if (out < a.cap) {
-                            a.pairs[3 * out] = i;
-                            a.pairs[3 * out + 1] = j;
-                            a.pairs[3 * out + 2] = lookup_nbond(a, i, j);
-                        }
-                        ++out;
-                    } else {
-                        ++cnt;
-                    }
-                }
-            }
-        }
-    }
-    if (PASS == 0) a.count[i] = cnt;
-}
-
-// small boxes (fewer than 3 cells on an axis): every j > i is a candidate
+// small boxes (fewer than 3 cells on an axis): every j > i is a candidate.  Pass 0 counts the pairs
+// of each atom, pass 1 writes the rows at offset[i]
 template <int PASS>
 __global__ void __launch_bounds__(128) k_pairs_all(NbArgs a) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -232,128 +197,293 @@ __global__ void __launch_bounds__(256) k_pairs_warp(NbArgs a) {
 }
 
 
-// Same cell scan emitting both layouts the engine uses: half rows (i, j, nbond), j > i, sorted
-// by i (pair kernels), and the full neighbour CSR (j != i, packed j | scale index << 28) for the
-// atomics-free CG matvec.  Positions for the FP32 prefilter come from the FP32 copy (posf);
-// borderline candidates fall back to the exact FP64 test on pos.
+// ------------------------------------------------------------------ the engine's builds
+//
+// Counting sort of the atoms into the cells, in two launches.  k_bin_count takes each atom's cell
+// and its arrival rank there; the last CTA to finish scans the counts into cell_start and clears
+// them for the next call (they are zero between calls), so no memset, no library scan and no
+// cursor array.  k_bin_fill writes the cell-ordered float4 positions (x, y, z, atom index as int
+// bits), all that the pair passes read.  `zero` is cleared on the way (the build's sums and totals).
+// Launch-bound at liquid sizes: the seven launches this replaces (FP32 copy, two memsets, count,
+// two-kernel scan, fill) took 13.5 us of device time at 12288 atoms, these two 7.
+constexpr int kBinThreads = 512;
+constexpr int kBinItems = 8;  // counts per thread and tile of the last CTA's scan
+
+struct BinArgs {
+    int n;
+    const double* pos;
+    Box box;
+    int nc[3];
+    int32_t* atom_cell;   // [n]
+    int32_t* rank;        // [n]
+    int32_t* cell_count;  // [ncell rounded up to kBinItems], zero between calls
+    int32_t* cell_start;  // [ncell + 1]
+    unsigned* done;       // CTAs that have finished, zero between calls
+    int32_t* zero;        // words to clear, or null
+    int nzero;
+    float4* posc;         // [n]
+};
+
+static __global__ void __launch_bounds__(kBinThreads) k_bin_count(BinArgs a) {
+    __shared__ bool s_last;
+    __shared__ int s_warp[kBinThreads / 32];
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < a.n) {
+        int c3[3];
+        const int c = cell_of(a.box, a.nc, a.pos + 3 * i, c3);
+        a.atom_cell[i] = c;
+        a.rank[i] = atomicAdd(a.cell_count + c, 1);
+    }
+    for (int k = i; k < a.nzero; k += gridDim.x * blockDim.x) a.zero[k] = 0;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(a.done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    const int ncell = a.nc[0] * a.nc[1] * a.nc[2];
+    const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+    int carry = 0;
+    for (int t0 = 0; t0 < ncell; t0 += kBinThreads * kBinItems) {
+        const int c0 = t0 + kBinItems * threadIdx.x;
+        int v[kBinItems];
+#pragma unroll
+        for (int k = 0; k < kBinItems; ++k) v[k] = 0;
+        if (c0 < ncell) {
+            int4* src = (int4*)(a.cell_count + c0);
+            *(int4*)v = __ldcg(src);
+            *(int4*)(v + 4) = __ldcg(src + 1);
+            src[0] = make_int4(0, 0, 0, 0);
+            src[1] = make_int4(0, 0, 0, 0);
+        }
+        int sum = 0;
+#pragma unroll
+        for (int k = 0; k < kBinItems; ++k) sum += v[k];
+        int incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += u;
+        }
+        if (lane == 31) s_warp[wl] = incl;
+        __syncthreads();
+        int before = carry, total = 0;
+        for (int w = 0; w < kBinThreads / 32; ++w) {
+            if (w < wl) before += s_warp[w];
+            total += s_warp[w];
+        }
+        int at = before + incl - sum;
+#pragma unroll
+        for (int k = 0; k < kBinItems; ++k) {
+            if (c0 + k < ncell) a.cell_start[c0 + k] = at;
+            at += v[k];
+        }
+        carry += total;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        a.cell_start[ncell] = a.n;
+        *a.done = 0u;
+    }
+}
+
+static __global__ void k_bin_fill(BinArgs a) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= a.n) return;
+    // the image inside the box: FP32 then resolves a distance to about 1e-7 of the box, however far
+    // the caller's coordinates have drifted
+    const double* p = a.pos + 3 * i;
+    double s[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        s[k] = p[0] * a.box.hinv[k] + p[1] * a.box.hinv[3 + k] + p[2] * a.box.hinv[6 + k];
+        s[k] -= floor(s[k]);
+    }
+    float w[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) w[c] = (float)(s[0] * a.box.h[c] + s[1] * a.box.h[3 + c] + s[2] * a.box.h[6 + c]);
+    a.posc[a.cell_start[a.atom_cell[i]] + a.rank[i]] = make_float4(w[0], w[1], w[2], __int_as_float(i));
+}
+
+// Totals of a build (read back by the host) and, behind them in the same array, the sums of the
+// counts over runs of kNbRun atoms (half rows, full-list entries, scaled rows): the pair passes add
+// into the run sums, k_nb_place turns them into offsets.
+constexpr int kNbRun = 1024;
+struct NbTotals {
+    long long rows, entries, scaled;
+    int max_h, max_f;  // largest half-row and full-list count of an atom
+};
+__host__ __device__ inline int nb_runs(int n) { return (n + kNbRun - 1) / kNbRun; }
+__host__ __device__ inline int nb_sum_words(int n) { return (int)(sizeof(NbTotals) / 4) + 3 * nb_runs(n); }
+
+// Both layouts the engine uses: half rows (i, j, nbond), j > i, sorted by i (pair kernels), and the
+// full neighbour CSR (j != i, packed j | scale index << 28) for the atomics-free CG matvec.  FP32
+// positions prefilter the candidates; those within about 2e-3 A of rc take the exact FP64 test on pos.
 struct Nb2Args {
     NbArgs a;
-    const float* posf;      // [n*4]
-    int32_t* count_f;       // [n] pass 0: full-list counts (null: half rows only, no CSR)
-    const int64_t* off_f;   // [n+1] pass 1
-    int32_t* ent;           // [cap_f]
+    const float4* posc;       // [n] cell order
+    int32_t* count_f;         // [n] full-list counts (null: half rows only, no CSR)
+    int32_t* count_s;         // [n] half rows with nbond != 0
+    int32_t* sums;            // [3][runs]
+    const int64_t* off_f;     // [n+1] pass 1 of k_pairs_warp3
+    int32_t* ent;             // [cap_f]
     int64_t cap_f;
+    int32_t* srows;           // [cap_s] pass 1: indices of the half rows with nbond != 0
+    const int32_t* off_s;     // [n]
+    int64_t cap_s;
     // keep masks of the candidate batches (k_pairs_warp3): pass 0 stores one word per batch of 32
     // candidates at mask[i * mask_stride + batch] when the atom's batches fit the stride; pass 1
     // reads them instead of repeating the distance tests (null: no masks)
     uint32_t* mask = nullptr;
     int mask_stride = 0;
-    // single-pass build (k_pairs_cell pass 2): the distance tests run once and each atom's full-
-    // list entries and half rows go to fixed slots, ell_ent[i * ell_cap_f + k] and
-    // ell_rows[3 (i * ell_cap_h + k)], which k_ell_compact then copies to the offsets the scans
-    // of the true counts give; slots past a capacity are dropped (the counts and maxdeg tell)
+    // slots of the single-pass kernels: each atom's full-list entries and half rows go to
+    // ell_ent[i * ell_cap_f + k] and ell_rows[3 (i * ell_cap_h + k)], which k_nb_place copies to the
+    // offsets of the true counts; slots past a capacity are dropped (the totals' maxima tell)
     int32_t* ell_ent = nullptr;
     int32_t* ell_rows = nullptr;
     int ell_cap_f = 0, ell_cap_h = 0;
-    int* maxdeg = nullptr;  // [2] largest half-row and full-list count over the atoms (passes 0 and 2)
 };
 
-template <int PASS>
-__global__ void __launch_bounds__(256) k_pairs_warp2(Nb2Args b) {
+// the FP32 box and prefilter bounds of a pair pass
+struct NbFilter {
+    float h[9], hi[9], rlo2, rhi2;
+    __device__ __forceinline__ explicit NbFilter(const NbArgs& a) {
+#pragma unroll
+        for (int k = 0; k < 9; ++k) { h[k] = (float)a.box.h[k]; hi[k] = (float)a.box.hinv[k]; }
+        // the band around rc covers the FP32 rounding of in-box positions and their images
+        double size = 0.0;
+#pragma unroll
+        for (int k = 0; k < 9; ++k) size += fabs(a.box.h[k]);
+        const double band = 2e-3 + 1e-6 * size;
+        const float rlo = (float)fmax(a.rc - band, 0.0), rhi = (float)(a.rc + band);
+        rlo2 = rlo * rlo;
+        rhi2 = rhi * rhi;
+    }
+};
+
+// Is the pair (i, j), j != i, within rc?  d0, d1, d2: the FP32 difference r_j - r_i.  ORTHO: the box
+// is orthorhombic and the prefilter's minimum image is three multiplies per axis.
+template <bool ORTHO>
+__device__ __forceinline__ bool nb_keep(const NbArgs& a, const NbFilter& f, int i, int j, float d0, float d1, float d2) {
+    bool amb = false;
+    float r2;
+    if (ORTHO) {
+        const float dd[3] = {d0, d1, d2};
+        r2 = 0.f;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            const float tt = dd[q] * f.hi[4 * q];
+            const float sq = tt - floorf(tt + 0.5f);
+            amb |= fabsf(sq) > 0.4999f;
+            const float e = sq * f.h[4 * q];
+            r2 = fmaf(e, e, r2);
+        }
+    } else {
+        float sf[3];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            const float tt = d0 * f.hi[q] + d1 * f.hi[3 + q] + d2 * f.hi[6 + q];
+            sf[q] = tt - floorf(tt + 0.5f);
+            amb |= fabsf(sf[q]) > 0.4999f;
+        }
+        const float e0 = sf[0] * f.h[0] + sf[1] * f.h[3] + sf[2] * f.h[6];
+        const float e1 = sf[0] * f.h[1] + sf[1] * f.h[4] + sf[2] * f.h[7];
+        const float e2 = sf[0] * f.h[2] + sf[1] * f.h[5] + sf[2] * f.h[8];
+        r2 = e0 * e0 + e1 * e1 + e2 * e2;
+    }
+    if (!amb && r2 < f.rlo2) return true;
+    if (!amb && r2 > f.rhi2) return false;
+    return j > i ? within_rc(a.box, a.pos + 3 * i, a.pos + 3 * j, a.rc)
+                 : within_rc(a.box, a.pos + 3 * j, a.pos + 3 * i, a.rc);
+}
+
+// nbond of a pair; the covalent map is read only for partners inside the atom's range [plo, phi]
+__device__ __forceinline__ int nb_bond(const NbArgs& a, int i, int j, int plo, int phi) {
+    return (j < plo || j > phi) ? 0 : (j > i ? lookup_nbond(a, i, j) : lookup_nbond(a, j, i));
+}
+
+// the counts of one atom (lane 0 of its warp)
+__device__ __forceinline__ void nb_counts(const Nb2Args& b, int i, int nh, int nf, int ns) {
+    const int runs = nb_runs(b.a.n), run = i / kNbRun;
+    b.a.count[i] = nh;
+    b.count_s[i] = ns;
+    if (nh) atomicAdd(b.sums + run, nh);
+    if (ns) atomicAdd(b.sums + 2 * runs + run, ns);
+    if (b.count_f) {
+        b.count_f[i] = nf;
+        if (nf) atomicAdd(b.sums + runs + run, nf);
+    }
+}
+
+// One atom's slots: the warp appends a batch of candidates (keep: within rc) to the rows and the
+// CSR entries of atom i and advances its counts.
+struct NbSlots {
+    int32_t *rows, *ent;
+    int cap_h, cap_f, nh = 0, nf = 0, ns = 0;
+    int i, plo, phi;
+    __device__ __forceinline__ NbSlots(const Nb2Args& b, int i_)
+        : rows(b.ell_rows + 3 * (int64_t)i_ * b.ell_cap_h), ent(b.ell_ent ? b.ell_ent + (int64_t)i_ * b.ell_cap_f : nullptr),
+          cap_h(b.ell_cap_h), cap_f(b.ell_cap_f), i(i_), plo(b.a.cov_lo ? b.a.cov_lo[i_] : 0),
+          phi(b.a.cov_hi ? b.a.cov_hi[i_] : b.a.n) {}
+    __device__ __forceinline__ void add(const Nb2Args& b, bool keep, int j, unsigned lt) {
+        const unsigned mf = __ballot_sync(0xffffffffu, keep);
+        if (mf == 0u) return;
+        const unsigned mh = __ballot_sync(0xffffffffu, keep && j > i);
+        bool scaled = false;
+        if (keep) {
+            const int nbd = nb_bond(b.a, i, j, plo, phi);
+            int sidx = nbd - 1;
+            if (sidx < 0) sidx += 6;
+            const int kf = nf + __popc(mf & lt);
+            if (ent && kf < cap_f) ent[kf] = j | (sidx << 28);
+            if (j > i) {
+                scaled = nbd != 0;
+                const int kh = nh + __popc(mh & lt);
+                if (kh < cap_h) {
+                    rows[3 * kh] = i;
+                    rows[3 * kh + 1] = j;
+                    rows[3 * kh + 2] = nbd;
+                }
+            }
+        }
+        nf += __popc(mf);
+        nh += __popc(mh);
+        ns += __popc(__ballot_sync(0xffffffffu, scaled));
+    }
+};
+
+// Boxes of fewer than five half-width cells on an axis: one warp per atom, every other atom is a
+// candidate.  Latency-bound (450 atoms: 14 batches per warp, 450 warps): 10 us at 450 atoms, where
+// the thread-per-atom count and write passes it replaces took 95 + 201 us and the CSR needed two
+// more kernels over the rows.
+template <bool ORTHO>
+__global__ void __launch_bounds__(128) k_pairs_flat(Nb2Args b) {
     const NbArgs& a = b.a;
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (i >= a.n) return;
-    const double* pi = a.pos + 3 * i;
-    const float pix = b.posf[4 * i], piy = b.posf[4 * i + 1], piz = b.posf[4 * i + 2];
-    float hf[9], hif[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) { hf[k] = (float)a.box.h[k]; hif[k] = (float)a.box.hinv[k]; }
-    // FP32 positions carry ~1e-5 A rounding at 100 A: the 2e-3 A band around rc goes to FP64
-    const float rlo = (float)(a.rc - 2e-3), rhi = (float)(a.rc + 2e-3);
-    const float rlo2 = rlo * rlo, rhi2 = rhi * rhi;
-    int c3[3];
-    cell_of(a.box, a.nc, pi, c3);
-    int64_t out_h = (PASS == 1) ? a.offset[i] : 0, out_f = (PASS == 1 && b.off_f) ? b.off_f[i] : 0;
-    int cnt_h = 0, cnt_f = 0;
+    const NbFilter f(a);
     const unsigned lt = (1u << lane) - 1u;
-    for (int dx = -1; dx <= 1; ++dx) {
-        const int cx = (c3[0] + dx + a.nc[0]) % a.nc[0];
-        for (int dy = -1; dy <= 1; ++dy) {
-            const int cy = (c3[1] + dy + a.nc[1]) % a.nc[1];
-            for (int dz = -1; dz <= 1; ++dz) {
-                const int cz = (c3[2] + dz + a.nc[2]) % a.nc[2];
-                const int c = (cx * a.nc[1] + cy) * a.nc[2] + cz;
-                const int cs = a.cell_start[c], ce = a.cell_start[c + 1];
-                for (int base = cs; base < ce; base += 32) {
-                    const int k = base + lane;
-                    bool keep = false;
-                    int j = -1;
-                    if (k < ce) {
-                        j = a.cell_atoms[k];
-                        if (j != i) {
-                            const float d0 = b.posf[4 * j] - pix, d1 = b.posf[4 * j + 1] - piy, d2 = b.posf[4 * j + 2] - piz;
-                            bool amb = false;
-                            float sf[3];
-#pragma unroll
-                            for (int q = 0; q < 3; ++q) {
-                                float t = d0 * hif[q] + d1 * hif[3 + q] + d2 * hif[6 + q];
-                                float nn = floorf(t + 0.5f);
-                                sf[q] = t - nn;
-                                amb |= fabsf(sf[q]) > 0.4999f;
-                            }
-                            const float e0 = sf[0] * hf[0] + sf[1] * hf[3] + sf[2] * hf[6];
-                            const float e1 = sf[0] * hf[1] + sf[1] * hf[4] + sf[2] * hf[7];
-                            const float e2 = sf[0] * hf[2] + sf[1] * hf[5] + sf[2] * hf[8];
-                            const float r2 = e0 * e0 + e1 * e1 + e2 * e2;
-                            if (!amb && r2 < rlo2) keep = true;
-                            else if (!amb && r2 > rhi2) keep = false;
-                            // exact test on the (lower, higher) orientation, as the half list defines it
-                            else keep = j > i ? within_rc(a.box, pi, a.pos + 3 * j, a.rc)
-                                              : within_rc(a.box, a.pos + 3 * j, pi, a.rc);
-                        }
-                    }
-                    const bool up = keep && j > i;
-                    const unsigned mf = __ballot_sync(0xffffffffu, keep);
-                    const unsigned mh = __ballot_sync(0xffffffffu, up);
-                    if (PASS == 1) {
-                        if (keep) {
-                            const int nbd = j > i ? lookup_nbond(a, i, j) : lookup_nbond(a, j, i);
-                            int sidx = nbd - 1;
-                            if (sidx < 0) sidx += 6;
-                            const int64_t sf_ = out_f + __popc(mf & lt);
-                            if (b.ent && sf_ < b.cap_f) b.ent[sf_] = j | (sidx << 28);
-                            if (up) {
-                                const int64_t sh = out_h + __popc(mh & lt);
-                                if (sh < a.cap) {
-                                    a.pairs[3 * sh] = i;
-                                    a.pairs[3 * sh + 1] = j;
-                                    a.pairs[3 * sh + 2] = nbd;
-                                }
-                            }
-                        }
-                        out_f += __popc(mf);
-                        out_h += __popc(mh);
-                    } else {
-                        cnt_f += __popc(mf);
-                        cnt_h += __popc(mh);
-                    }
-                }
-            }
-        }
+    const double pix = a.pos[3 * i], piy = a.pos[3 * i + 1], piz = a.pos[3 * i + 2];
+    NbSlots out(b, i);
+#pragma unroll 4
+    for (int j0 = 0; j0 < a.n; j0 += 32) {
+        const int j = j0 + lane;
+        bool keep = false;
+        if (j < a.n && j != i)
+            keep = nb_keep<ORTHO>(a, f, i, j, (float)(a.pos[3 * j] - pix), (float)(a.pos[3 * j + 1] - piy),
+                                  (float)(a.pos[3 * j + 2] - piz));
+        out.add(b, keep, j, lt);
     }
-    if (PASS == 0 && lane == 0) {
-        a.count[i] = cnt_h;
-        if (b.count_f) b.count_f[i] = cnt_f;
-    }
+    if (lane == 0) nb_counts(b, i, out.nh, out.nf, out.ns);
 }
 
-// k_pairs_warp2 over a finer cell grid: cells at least rc / S wide and a (2S + 1)^3 stencil
-// (S = 2: 125 cells of half width, about 0.58 of the 27-cell search volume).  The warp first
+// Cells at least rc / S wide and a (2S + 1)^3 stencil (S = 2: 125 cells of half width, about 0.58 of
+// the 27-cell search volume), one warp per atom in cell order.  The warp first
 // lays the stencil's cells out as one concatenated candidate list (cell starts and a prefix sum of
 // their counts in shared memory, in the dx, dy, dz order of the 27-cell scan), then walks it in
 // full 32-lane batches; each lane finds its candidate's cell by advancing a cursor (lanes move
-// forward monotonically).  Rows come out grouped by i like the coarse scan's.
+// forward monotonically).  Count pass and fill pass: it serves neighbourhoods too large to stage.
 constexpr int kNbWarps = 8;  // warps per block of k_pairs_warp3
 constexpr size_t kNbStageBytes = 44u << 10;  // largest candidate stage of k_pairs_cell: with its static
                                               // shared arrays it stays under the 48 KB default
@@ -365,18 +495,14 @@ __global__ void __launch_bounds__(32 * kNbWarps) k_pairs_warp3(Nb2Args b) {
     __shared__ int s_off[kNbWarps][NQ + 1];
     const NbArgs& a = b.a;
     const int wl = threadIdx.x >> 5;
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int ks = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
-    if (i >= a.n) return;  // whole warps leave together
-    const double* pi = a.pos + 3 * i;
-    const float pix = b.posf[4 * i], piy = b.posf[4 * i + 1], piz = b.posf[4 * i + 2];
-    float hf[9], hif[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) { hf[k] = (float)a.box.h[k]; hif[k] = (float)a.box.hinv[k]; }
-    const float rlo = (float)(a.rc - 2e-3), rhi = (float)(a.rc + 2e-3);
-    const float rlo2 = rlo * rlo, rhi2 = rhi * rhi;
+    if (ks >= a.n) return;  // whole warps leave together
+    const float4 p4 = b.posc[ks];
+    const int i = __float_as_int(p4.w);
+    const NbFilter f(a);
     int c3[3];
-    cell_of(a.box, a.nc, pi, c3);
+    cell_of(a.box, a.nc, a.pos + 3 * i, c3);
     // stencil cells -> (start, count), prefix-summed in q order
     int carry = 0;
     if (lane == 0) s_off[wl][0] = 0;
@@ -405,7 +531,9 @@ __global__ void __launch_bounds__(32 * kNbWarps) k_pairs_warp3(Nb2Args b) {
     __syncwarp();
     const int total = carry;
     int64_t out_h = (PASS == 1) ? a.offset[i] : 0, out_f = (PASS == 1 && b.off_f) ? b.off_f[i] : 0;
-    int cnt_h = 0, cnt_f = 0;
+    int64_t out_s = (PASS == 1 && b.srows) ? b.off_s[i] : 0;
+    int cnt_h = 0, cnt_f = 0, cnt_s = 0;
+    const int plo = a.cov_lo ? a.cov_lo[i] : 0, phi = a.cov_hi ? a.cov_hi[i] : a.n;
     const unsigned lt = (1u << lane) - 1u;
     int qc = 0;
     // both passes see the same candidate list, so the masks are complete exactly when it fits
@@ -420,40 +548,23 @@ __global__ void __launch_bounds__(32 * kNbWarps) k_pairs_warp3(Nb2Args b) {
             if (mk == 0u) continue;  // warp-uniform: no candidate of this batch is kept
             if ((mk >> lane) & 1u) {
                 while (t >= s_off[wl][qc + 1]) ++qc;
-                j = a.cell_atoms[s_beg[wl][qc] + (t - s_off[wl][qc])];
+                j = __float_as_int(b.posc[s_beg[wl][qc] + (t - s_off[wl][qc])].w);
                 keep = true;
             }
         } else if (t < total) {
             while (t >= s_off[wl][qc + 1]) ++qc;
-            j = a.cell_atoms[s_beg[wl][qc] + (t - s_off[wl][qc])];
-            if (j != i) {
-                const float d0 = b.posf[4 * j] - pix, d1 = b.posf[4 * j + 1] - piy, d2 = b.posf[4 * j + 2] - piz;
-                bool amb = false;
-                float sf[3];
-#pragma unroll
-                for (int q = 0; q < 3; ++q) {
-                    float tt = d0 * hif[q] + d1 * hif[3 + q] + d2 * hif[6 + q];
-                    float nn = floorf(tt + 0.5f);
-                    sf[q] = tt - nn;
-                    amb |= fabsf(sf[q]) > 0.4999f;
-                }
-                const float e0 = sf[0] * hf[0] + sf[1] * hf[3] + sf[2] * hf[6];
-                const float e1 = sf[0] * hf[1] + sf[1] * hf[4] + sf[2] * hf[7];
-                const float e2 = sf[0] * hf[2] + sf[1] * hf[5] + sf[2] * hf[8];
-                const float r2 = e0 * e0 + e1 * e1 + e2 * e2;
-                if (!amb && r2 < rlo2) keep = true;
-                else if (!amb && r2 > rhi2) keep = false;
-                else keep = j > i ? within_rc(a.box, pi, a.pos + 3 * j, a.rc)
-                                  : within_rc(a.box, a.pos + 3 * j, pi, a.rc);
-            }
+            const float4 pj = b.posc[s_beg[wl][qc] + (t - s_off[wl][qc])];
+            j = __float_as_int(pj.w);
+            if (j != i) keep = nb_keep<false>(a, f, i, j, pj.x - p4.x, pj.y - p4.y, pj.z - p4.z);
         }
         const bool up = keep && j > i;
         const unsigned mf = __ballot_sync(0xffffffffu, keep);
         const unsigned mh = __ballot_sync(0xffffffffu, up);
         if (PASS == 0 && use_mask && lane == 0) mrow[base >> 5] = mf;
+        const int nbd = keep ? nb_bond(a, i, j, plo, phi) : 0;
+        const unsigned ms = __ballot_sync(0xffffffffu, up && nbd != 0);
         if (PASS == 1) {
             if (keep) {
-                const int nbd = j > i ? lookup_nbond(a, i, j) : lookup_nbond(a, j, i);
                 int sidx = nbd - 1;
                 if (sidx < 0) sidx += 6;
                 const int64_t sf_ = out_f + __popc(mf & lt);
@@ -465,29 +576,29 @@ __global__ void __launch_bounds__(32 * kNbWarps) k_pairs_warp3(Nb2Args b) {
                         a.pairs[3 * sh + 1] = j;
                         a.pairs[3 * sh + 2] = nbd;
                     }
+                    const int64_t ss = out_s + __popc(ms & lt);
+                    if (nbd != 0 && b.srows && ss < b.cap_s) b.srows[ss] = (int32_t)sh;
                 }
             }
             out_f += __popc(mf);
             out_h += __popc(mh);
+            out_s += __popc(ms);
         } else {
             cnt_f += __popc(mf);
             cnt_h += __popc(mh);
+            cnt_s += __popc(ms);
         }
     }
-    if (PASS == 0 && lane == 0) {
-        a.count[i] = cnt_h;
-        if (b.count_f) b.count_f[i] = cnt_f;
-    }
+    if (PASS == 0 && lane == 0) nb_counts(b, i, cnt_h, cnt_f, cnt_s);
 }
 
-// Block-per-cell form of k_pairs_warp3 (same stencil, candidate order, tests and outputs): one
+// Block-per-cell single pass (same stencil, candidate order and tests as k_pairs_warp3): one
 // CTA takes every atom of one cell.  The cell's (2S + 1)^3 neighbourhood is laid out once per CTA
 // and, when it fits in `chmax` entries, staged in shared memory as (x, y, z, j) float4s, so the
 // cell's atoms read their candidates from shared memory instead of each gathering them from L2;
 // neighbourhoods larger than the stage fall back to the global gathers.  The NW warps of the CTA
-// take the cell's atoms in turn.  ORTHO: the box is orthorhombic and the FP32 prefilter's minimum
-// image is three multiplies per axis (candidates near rc still take the exact FP64 test).
-template <int PASS, int S, int NW, bool ORTHO>
+// take the cell's atoms in turn.
+template <int S, int NW, bool ORTHO>
 __global__ void __launch_bounds__(32 * NW) k_pairs_cell(Nb2Args b, int chmax) {
     constexpr int W = 2 * S + 1, NQ = W * W * W;
     __shared__ int s_beg[NQ];
@@ -532,185 +643,159 @@ __global__ void __launch_bounds__(32 * NW) k_pairs_cell(Nb2Args b, int chmax) {
         int qc = 0;
         for (int t = threadIdx.x; t < total; t += blockDim.x) {
             while (t >= s_off[qc + 1]) ++qc;
-            const int j = a.cell_atoms[s_beg[qc] + (t - s_off[qc])];
-            s_cand[t] = make_float4(b.posf[4 * j], b.posf[4 * j + 1], b.posf[4 * j + 2], __int_as_float(j));
+            s_cand[t] = b.posc[s_beg[qc] + (t - s_off[qc])];
         }
     }
     __syncthreads();
-    float hf[9], hif[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) { hf[k] = (float)a.box.h[k]; hif[k] = (float)a.box.hinv[k]; }
-    const float rlo = (float)(a.rc - 2e-3), rhi = (float)(a.rc + 2e-3);
-    const float rlo2 = rlo * rlo, rhi2 = rhi * rhi;
+    const NbFilter f(a);
     const unsigned lt = (1u << lane) - 1u;
     for (int ai = wl; ai < m; ai += NW) {
-        const int i = a.cell_atoms[cs0 + ai];
-        const double* pi = a.pos + 3 * i;
-        const float pix = b.posf[4 * i], piy = b.posf[4 * i + 1], piz = b.posf[4 * i + 2];
-        const int64_t base_h = PASS == 2 ? (int64_t)i * b.ell_cap_h : 0, base_f = PASS == 2 ? (int64_t)i * b.ell_cap_f : 0;
-        int64_t out_h = (PASS == 1) ? a.offset[i] : base_h, out_f = (PASS == 1 && b.off_f) ? b.off_f[i] : base_f;
-        // where this pass writes: the final rows / CSR (pass 1) or the atom's slots (pass 2)
-        int32_t* const rows_out = PASS == 2 ? b.ell_rows : a.pairs;
-        int32_t* const ent_out = PASS == 2 ? b.ell_ent : b.ent;
-        const int64_t lim_h = PASS == 2 ? base_h + b.ell_cap_h : a.cap;
-        const int64_t lim_f = PASS == 2 ? base_f + b.ell_cap_f : b.cap_f;
-        int cnt_h = 0, cnt_f = 0;
+        const float4 p4 = b.posc[cs0 + ai];
+        const int i = __float_as_int(p4.w);
+        NbSlots out(b, i);
         int qc = 0;
-        // covalent partners of i lie in [plo, phi]: the map is read only for those
-        const int plo = a.cov_lo ? a.cov_lo[i] : 0, phi = a.cov_hi ? a.cov_hi[i] : a.n;
-        const bool use_mask = b.mask && (total + 31) / 32 <= b.mask_stride;
-        uint32_t* mrow = use_mask ? b.mask + (size_t)i * b.mask_stride : nullptr;
         for (int base = 0; base < total; base += 32) {
             const int t = base + lane;
             bool keep = false;
             int j = -1;
-            if (PASS == 1 && use_mask) {
-                const uint32_t mk = mrow[base >> 5];
-                if (mk == 0u) continue;  // warp-uniform: no candidate of this batch is kept
-                if ((mk >> lane) & 1u) {
-                    if (staged) {
-                        j = __float_as_int(s_cand[t].w);
-                    } else {
-                        while (t >= s_off[qc + 1]) ++qc;
-                        j = a.cell_atoms[s_beg[qc] + (t - s_off[qc])];
-                    }
-                    keep = true;
-                }
-            } else if (t < total) {
-                float pjx, pjy, pjz;
+            if (t < total) {
+                float4 pj;
                 if (staged) {
-                    const float4 cv = s_cand[t];
-                    pjx = cv.x;
-                    pjy = cv.y;
-                    pjz = cv.z;
-                    j = __float_as_int(cv.w);
+                    pj = s_cand[t];
                 } else {
                     while (t >= s_off[qc + 1]) ++qc;
-                    j = a.cell_atoms[s_beg[qc] + (t - s_off[qc])];
-                    pjx = b.posf[4 * j];
-                    pjy = b.posf[4 * j + 1];
-                    pjz = b.posf[4 * j + 2];
+                    pj = b.posc[s_beg[qc] + (t - s_off[qc])];
                 }
-                if (j != i) {
-                    const float d0 = pjx - pix, d1 = pjy - piy, d2 = pjz - piz;
-                    bool amb = false;
-                    float r2;
-                    if (ORTHO) {
-                        const float dd[3] = {d0, d1, d2};
-                        r2 = 0.f;
-#pragma unroll
-                        for (int q = 0; q < 3; ++q) {
-                            const float tt = dd[q] * hif[4 * q];
-                            const float sq = tt - floorf(tt + 0.5f);
-                            amb |= fabsf(sq) > 0.4999f;
-                            const float e = sq * hf[4 * q];
-                            r2 = fmaf(e, e, r2);
-                        }
-                    } else {
-                        float sf[3];
-#pragma unroll
-                        for (int q = 0; q < 3; ++q) {
-                            float tt = d0 * hif[q] + d1 * hif[3 + q] + d2 * hif[6 + q];
-                            float nn = floorf(tt + 0.5f);
-                            sf[q] = tt - nn;
-                            amb |= fabsf(sf[q]) > 0.4999f;
-                        }
-                        const float e0 = sf[0] * hf[0] + sf[1] * hf[3] + sf[2] * hf[6];
-                        const float e1 = sf[0] * hf[1] + sf[1] * hf[4] + sf[2] * hf[7];
-                        const float e2 = sf[0] * hf[2] + sf[1] * hf[5] + sf[2] * hf[8];
-                        r2 = e0 * e0 + e1 * e1 + e2 * e2;
-                    }
-                    if (!amb && r2 < rlo2) keep = true;
-                    else if (!amb && r2 > rhi2) keep = false;
-                    else keep = j > i ? within_rc(a.box, pi, a.pos + 3 * j, a.rc)
-                                      : within_rc(a.box, a.pos + 3 * j, pi, a.rc);
-                }
+                j = __float_as_int(pj.w);
+                if (j != i) keep = nb_keep<ORTHO>(a, f, i, j, pj.x - p4.x, pj.y - p4.y, pj.z - p4.z);
             }
-            const bool up = keep && j > i;
-            const unsigned mf = __ballot_sync(0xffffffffu, keep);
-            const unsigned mh = __ballot_sync(0xffffffffu, up);
-            if (PASS == 0 && use_mask && lane == 0) mrow[base >> 5] = mf;
-            if (PASS == 1 || PASS == 2) {
-                if (keep) {
-                    const int nbd = (j < plo || j > phi) ? 0 : (j > i ? lookup_nbond(a, i, j) : lookup_nbond(a, j, i));
-                    int sidx = nbd - 1;
-                    if (sidx < 0) sidx += 6;
-                    const int64_t sf_ = out_f + __popc(mf & lt);
-                    if (ent_out && sf_ < lim_f) ent_out[sf_] = j | (sidx << 28);
-                    if (up) {
-                        const int64_t sh = out_h + __popc(mh & lt);
-                        if (sh < lim_h) {
-                            rows_out[3 * sh] = i;
-                            rows_out[3 * sh + 1] = j;
-                            rows_out[3 * sh + 2] = nbd;
-                        }
-                    }
-                }
-                out_f += __popc(mf);
-                out_h += __popc(mh);
+            out.add(b, keep, j, lt);
+        }
+        if (lane == 0) nb_counts(b, i, out.nh, out.nf, out.ns);
+    }
+}
+
+// Offsets from the counts, and the slots copied there.  A CTA takes kPlaceAtoms atoms: it sums the
+// run sums before their run and the counts of the run's earlier atoms, scans its own, copies each
+// atom's rows and CSR entries (as flat runs of words) and the indices of its rows with nbond != 0,
+// all in atom order; the CTA of the last atom writes the totals.  Nothing is written past a
+// capacity: the caller compares the totals before it uses the lists.  Bound by the copies' latency (42
+// MB moved at 12288 atoms and rc 8 A): 22 us there, one launch for two memsets, two two-kernel
+// scans, a copy kernel and a library selection over all rows that took 47 us and two more host
+// round trips.  A warp per atom: with four atoms per warp in turn it took 38 us at 4000 atoms
+// against 10.
+constexpr int kPlaceAtoms = 8, kPlaceThreads = 32 * kPlaceAtoms;  // a warp per atom
+static_assert(kNbRun % kPlaceAtoms == 0, "a CTA's atoms lie in one run");
+
+// one warp: n words from src to dst, four loads in flight per lane
+__device__ __forceinline__ void nb_copy(int32_t* __restrict__ dst, const int32_t* __restrict__ src, int n, int lane) {
+    int k = lane;
+    for (; k + 96 < n; k += 128) {
+        const int32_t v0 = src[k], v1 = src[k + 32], v2 = src[k + 64], v3 = src[k + 96];
+        dst[k] = v0;
+        dst[k + 32] = v1;
+        dst[k + 64] = v2;
+        dst[k + 96] = v3;
+    }
+    for (; k < n; k += 32) dst[k] = src[k];
+}
+
+struct PlaceArgs {
+    int n;
+    const int32_t *count_h, *count_f, *count_s;  // count_f null: no CSR
+    const int32_t* sums;                         // [3][runs]
+    NbTotals* tot;                               // max_h, max_f zero on entry
+    int64_t *off_h, *off_f;                      // [n+1]; off_f null: no CSR
+    int32_t* off_s;                              // [n]
+    const int32_t *ell_rows, *ell_ent;           // null: offsets and totals only
+    int cap_h, cap_f;
+    int32_t* rows;
+    int64_t rows_cap;
+    int32_t* ent;
+    int64_t ent_cap;
+    int32_t* srows;  // null: not wanted
+    int64_t srows_cap;
+};
+
+static __global__ void __launch_bounds__(kPlaceThreads) k_nb_place(PlaceArgs a) {
+    constexpr int NW = kPlaceThreads / 32;
+    __shared__ long long s_part[NW][3], s_off[3][kPlaceAtoms];
+    const int tid = threadIdx.x, lane = tid & 31, wl = tid >> 5;
+    const int a0 = blockIdx.x * kPlaceAtoms, run = a0 / kNbRun, runs = nb_runs(a.n);
+    const int32_t* const cnt[3] = {a.count_h, a.count_f, a.count_s};
+    long long base[3] = {0, 0, 0};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        if (!cnt[k]) continue;
+        for (int r = tid; r < run; r += kPlaceThreads) base[k] += a.sums[k * runs + r];
+        for (int i = run * kNbRun + tid; i < a0; i += kPlaceThreads) base[k] += cnt[k][i];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) base[k] += __shfl_down_sync(0xffffffffu, base[k], o);
+        if (lane == 0) s_part[wl][k] = base[k];
+    }
+    __syncthreads();
+    if (wl < 3 && cnt[wl]) {  // one warp per count: the atoms of the CTA
+        const int k = wl, i = a0 + lane;
+        const bool mine = lane < kPlaceAtoms && i < a.n;
+        const int c = mine ? cnt[k][i] : 0;
+        long long before = 0;
+        for (int w = 0; w < NW; ++w) before += s_part[w][k];
+        int incl = c, mx = c;
+#pragma unroll
+        for (int o = 1; o < kPlaceAtoms; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+            mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        }
+        const long long off = before + incl - c;
+        if (lane < kPlaceAtoms) s_off[k][lane] = off;
+        if (mine) {
+            if (k == 0 && a.off_h) a.off_h[i] = off;
+            if (k == 1) a.off_f[i] = off;
+            if (k == 2 && a.off_s) a.off_s[i] = (int32_t)off;
+        }
+        if (mine && i == a.n - 1) {
+            const long long total = off + c;
+            if (k == 0) {
+                a.tot->rows = total;
+                if (a.off_h) a.off_h[a.n] = total;
+            } else if (k == 1) {
+                a.tot->entries = total;
+                a.off_f[a.n] = total;
             } else {
-                cnt_f += __popc(mf);
-                cnt_h += __popc(mh);
+                a.tot->scaled = total;
             }
         }
-        if (PASS == 2) {
-            cnt_h = (int)(out_h - base_h);
-            cnt_f = (int)(out_f - base_f);
+        if (lane == 0 && k == 0) atomicMax(&a.tot->max_h, mx);
+        if (lane == 0 && k == 1) atomicMax(&a.tot->max_f, mx);
+    }
+    if (!a.ell_rows) return;  // whole grid
+    __syncthreads();
+    const int i = a0 + wl;
+    if (i >= a.n) return;
+    const int nh = min(a.count_h[i], a.cap_h);
+    const int32_t* const src = a.ell_rows + 3 * (int64_t)i * a.cap_h;
+    const int64_t bh = s_off[0][wl];
+    if (a.rows) {
+        const int64_t room = 3 * (a.rows_cap - bh);
+        nb_copy(a.rows + 3 * bh, src, (int)min((int64_t)(3 * nh), room > 0 ? room : (int64_t)0), lane);
+    }
+    if (a.ent) {
+        const int64_t bf = s_off[1][wl], room = a.ent_cap - bf;
+        nb_copy(a.ent + bf, a.ell_ent + (int64_t)i * a.cap_f,
+                (int)min((int64_t)min(a.count_f[i], a.cap_f), room > 0 ? room : (int64_t)0), lane);
+    }
+    if (a.srows && a.count_s[i] > 0) {
+        int64_t at = s_off[2][wl];
+        for (int k0 = 0; k0 < nh; k0 += 32) {
+            const int k = k0 + lane;
+            const bool sc = k < nh && src[3 * k + 2] != 0;
+            const unsigned ms = __ballot_sync(0xffffffffu, sc);
+            const int64_t p = at + __popc(ms & ((1u << lane) - 1u));
+            if (sc && p < a.srows_cap) a.srows[p] = (int32_t)(bh + k);
+            at += __popc(ms);
         }
-        if (PASS != 1 && lane == 0) {
-            a.count[i] = cnt_h;
-            if (b.count_f) b.count_f[i] = cnt_f;
-            if (b.maxdeg) {
-                atomicMax(b.maxdeg, cnt_h);
-                atomicMax(b.maxdeg + 1, cnt_f);
-            }
-        }
     }
-}
-
-// Copies each atom's slots of the single-pass build to its offsets in the half rows and the CSR
-// (one warp per atom); nothing is written past the capacities, which the caller checks against
-// the totals before it uses the lists.
-static __global__ void k_ell_compact(int n, const int32_t* count_h, const int32_t* count_f, const int64_t* off_h,
-                                     const int64_t* off_f, const int32_t* ell_rows, int cap_h, const int32_t* ell_ent,
-                                     int cap_f, int32_t* rows, int64_t rows_cap, int32_t* ent, int64_t ent_cap) {
-    const int i = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    const int lane = threadIdx.x & 31;
-    if (i >= n) return;
-    const int nh = min(count_h[i], cap_h);
-    const int64_t bh = off_h[i];
-    for (int k = lane; k < nh; k += 32) {
-        if (bh + k >= rows_cap) break;
-        const int32_t* src = ell_rows + 3 * ((int64_t)i * cap_h + k);
-        int32_t* dst = rows + 3 * (bh + k);
-        dst[0] = src[0];
-        dst[1] = src[1];
-        dst[2] = src[2];
-    }
-    if (!ent) return;
-    const int nf = min(count_f[i], cap_f);
-    const int64_t bf = off_f[i];
-    for (int k = lane; k < nf; k += 32) {
-        if (bf + k >= ent_cap) break;
-        ent[bf + k] = ell_ent[(int64_t)i * cap_f + k];
-    }
-}
-
-// cell-ordered float4 copy of the positions (x, y, z, atom index as int bits)
-static __global__ void k_pos_cells(int n, const double* pos, const int32_t* cell_atoms, float4* posc) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    const int a = cell_atoms[k];
-    posc[k] = make_float4((float)pos[3 * a], (float)pos[3 * a + 1], (float)pos[3 * a + 2], __int_as_float(a));
-}
-
-static __global__ void k_pos_f32(int n, const double* pos, float* posf) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    posf[4 * i] = (float)pos[3 * i];
-    posf[4 * i + 1] = (float)pos[3 * i + 1];
-    posf[4 * i + 2] = (float)pos[3 * i + 2];
-    posf[4 * i + 3] = 0.f;
 }
 
 }  // namespace dmffb

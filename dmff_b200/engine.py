@@ -286,7 +286,11 @@ class AdmpEngine:
         b = self._box(box)
         s = torch.cuda.current_stream(self.device)
         need = ctypes.c_int64(0)
-        cap = int(capacity) if capacity else 0
+        # without a capacity: the count at the mean density with headroom, or the last count's
+        n = self.n
+        mean = n / max(abs(float(np.linalg.det(b.reshape(3, 3)))), 1e-300) * (4.0 / 3.0) * np.pi * float(rc) ** 3
+        guess = max(int(min(0.54 * n * mean, 600.0 * n)) + 64, getattr(self, "_rows_hint", 0))
+        cap = int(capacity) if capacity else min(guess, n * (n - 1) // 2)
         buf = torch.empty((max(cap, 1), 3), dtype=torch.int32, device=self.device)
         st = self.lib.dmffb_build_neighbors(self.h, ctypes.c_void_p(s.cuda_stream), _dev(pos),
                                             b.ctypes.data_as(ctypes.c_void_p), float(rc), _dev(buf), cap,
@@ -298,6 +302,7 @@ class AdmpEngine:
                                                 b.ctypes.data_as(ctypes.c_void_p), float(rc), _dev(buf), cap,
                                                 ctypes.byref(need))
         self._check(st)
+        self._rows_hint = need.value + need.value // 16
         return buf[: need.value]
 
     def rebuild_internal_pairs(self, pos, box):
