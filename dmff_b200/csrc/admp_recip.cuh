@@ -7,11 +7,11 @@
 // with B-spline derivatives up to third order (20 sums per atom), giving dE/dpos, dE/dQ,
 // torques and the box gradient in one pass.
 //
-// Layout: each atom's 6x6x6 stencil is split into 36 (x, y) lines of 6 contiguous z points;
-// one warp owns one atom, lanes own lines.  The multipole is first mapped to mesh-derivative
-// coefficients c_abc (mu^u = -B mu, Theta^u = B Theta B^T with B the reference's derivative
-// operator, recip.py:213/251), so the per-point work is a 3-term dot product.  Spreading uses
-// FP32/FP64 atomics on the mesh (it lives in L2); the gather is atomics-free.
+// Layout: each atom's 6x6x6 stencil is 36 (x, y) columns of 6 contiguous z points; one warp owns one
+// atom, its lanes cover whole columns in runs of six consecutive addresses.  The multipole is first
+// mapped to mesh-derivative coefficients c_abc (mu^u = -B mu, Theta^u = B Theta B^T with B the
+// reference's derivative operator, recip.py:213/251), so the per-point work is a 3-term dot product.
+// Spreading uses FP32/FP64 atomics on the mesh (it lives in L2); the gather is atomics-free.
 #pragma once
 #include "common.cuh"
 
@@ -139,54 +139,107 @@ __device__ __forceinline__ void site_multipole(const SpreadArgs<T>& a, int at, T
     }
 }
 
-template <typename T>
-__device__ __forceinline__ void stencil_setup(const MeshGeom& g, const double* pos, int at, int m0[3], T Mx[4][6],
-                                              T My[4][6], T Mz[4][6]) {
-    const double R0 = pos[3 * at], R1 = pos[3 * at + 1], R2 = pos[3 * at + 2];
-    T (*Ms[3])[6] = {Mx, My, Mz};
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        const double x = g.NA[3 * d] * R0 + g.NA[3 * d + 1] * R1 + g.NA[3 * d + 2] * R2;
+// A CTA of the spread and the gather takes `apc` sites (at most kSiteAtoms).  What one site needs once
+// is computed once, by one thread each, into shared memory: the splines of a site and axis (up to
+// derivative ORD, interleaved so that the orders of one point are one vector load), its wrapped first
+// stencil point, and for the spread its coefficients.
+constexpr int kSiteThreads = 256, kSiteAtoms = 32;
+
+// Sites per CTA.  One per warp while that leaves the SMs fewer than eight CTAs (450 sites: 57 CTAs
+// instead of 15), more once the chip is full, where the per-CTA work is shared by more sites.
+inline int sites_per_cta(int n) { return n <= 8 * 8 * 148 ? 8 : (n <= 16 * 8 * 148 ? 16 : kSiteAtoms); }
+
+template <typename T, int ORD>
+struct SiteStencils {
+    static constexpr int NV = ORD <= 1 ? 2 : 4;  // orders stored per point
+    __align__(16) T w[kSiteAtoms][3][6][NV];
+    int org[kSiteAtoms][3];
+
+    __device__ __forceinline__ void set(const MeshGeom& g, const double* pos, int at, int m, int d) {
+        const double x = g.NA[3 * d] * pos[3 * at] + g.NA[3 * d + 1] * pos[3 * at + 1] + g.NA[3 * d + 2] * pos[3 * at + 2];
         const double c = ceil(x);
-        m0[d] = (int)c;
-        bspline6<T>((T)(c - x), Ms[d][0], Ms[d][1], Ms[d][2], Ms[d][3]);
+        org[m][d] = wrapi((int)c - 3, g.K[d]);
+        T M[4][6];
+        bspline6<T>((T)(c - x), M[0], M[1], M[2], M[3]);
+#pragma unroll
+        for (int t = 0; t < 6; ++t)
+#pragma unroll
+            for (int o = 0; o < NV; ++o) w[m][d][t][o] = o <= ORD ? M[o][t] : T(0);
     }
+};
+
+// g + d wrapped into [0, K) for g in [0, K), d >= 0
+__device__ __forceinline__ int wrap_up(int g, int K) {
+    while (g >= K) g -= K;
+    return g;
 }
 
-// one warp per site; lanes cover the 36 (x, y) lines of the 6^3 stencil
-template <typename T>
-__global__ void __launch_bounds__(256) k_spread(SpreadArgs<T> a) {
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (warp >= a.n) return;
+// Spread of the sites' multipoles (CH: charges alone) onto the mesh.  A warp takes a site, first its 36
+// columns' weights (lanes own columns, results through shared memory), then its 216 points 32 at a
+// time: seven atomics per lane whose addresses are runs of six.  Bound by the L2 atomics: 21 M in
+// 36 us for 99000 charges, 23 us for 30000 multipoles.  With lanes owning whole columns and every lane
+// evaluating all splines these took 168 and 56 us.
+template <typename T, bool CH>
+__global__ void __launch_bounds__(kSiteThreads) k_spread(SpreadArgs<T> a, int apc) {
+    constexpr int ORD = CH ? 0 : 2, NW = kSiteThreads / 32;
+    __shared__ SiteStencils<T, ORD> st;
+    __shared__ T s_c[kSiteAtoms][CH ? 1 : 10];
+    __shared__ T s_col[NW][36][CH ? 1 : 3];
+    __shared__ int s_base[NW][36];
+    const int tid = threadIdx.x, lane = tid & 31, wl = tid >> 5;
+    const int first = blockIdx.x * apc, m1 = min(apc, a.n - first);
     // concurrently running warps take atoms far apart in the box, which keeps them off the same
     // mesh addresses (atoms are usually stored in spatial order)
-    const int at = (int)(((int64_t)warp * a.perm_mul) % a.n);
-    int m0[3];
-    T Mx[4][6], My[4][6], Mz[4][6];
-    stencil_setup<T>(a.g, a.pos, at, m0, Mx, My, Mz);
-    T q, mu[3], Th[3][3];
-    site_multipole(a, at, q, mu, Th);
-    T c[10];
-    site_coefs<T>(a.g.B, q, mu, Th, c);
-    const int K0 = a.g.K[0], K1 = a.g.K[1], K2 = a.g.K[2];
-    int gz[6];
+    auto site = [&](int m) { return (int)(((int64_t)(first + m) * a.perm_mul) % a.n); };
+    for (int k = tid; k < 4 * m1; k += kSiteThreads) {
+        const int m = k >> 2, d = k & 3;
+        const int at = site(m);
+        if (d < 3) {
+            st.set(a.g, a.pos, at, m, d);
+        } else if (CH) {
+            s_c[m][0] = a.q1[at];
+        } else {
+            T q, mu[3], Th[3][3], c[10];
+            site_multipole(a, at, q, mu, Th);
+            site_coefs<T>(a.g.B, q, mu, Th, c);
 #pragma unroll
-    for (int t = 0; t < 6; ++t) gz[t] = wrapi(m0[2] - 3 + t, K2);
-    for (int L = lane; L < 36; L += 32) {
-        const int ix = L / 6, iy = L % 6;
-        const T x0 = Mx[0][ix], x1 = Mx[1][ix], x2 = Mx[2][ix];
-        const T y0 = My[0][iy], y1 = My[1][iy], y2 = My[2][iy];
-        const T s0 = c[0] * x0 * y0 + c[1] * x1 * y0 + c[2] * x0 * y1 + c[4] * x2 * y0 + c[5] * x0 * y2 + c[7] * x1 * y1;
-        const T s1 = c[3] * x0 * y0 + c[8] * x1 * y0 + c[9] * x0 * y1;
-        const T s2 = c[6] * x0 * y0;
-        const int gx = wrapi(m0[0] - 3 + ix, K0), gy = wrapi(m0[1] - 3 + iy, K1);
-        T* line = a.grid + ((size_t)gx * K1 + gy) * K2;
-#pragma unroll
-        for (int t = 0; t < 6; ++t) {
-            const T v = s0 * Mz[0][t] + s1 * Mz[1][t] + s2 * Mz[2][t];
-            atomicAdd(line + gz[t], v);
+            for (int j = 0; j < 10; ++j) s_c[m][CH ? 0 : j] = c[j];
         }
+    }
+    __syncthreads();
+    const int K0 = a.g.K[0], K1 = a.g.K[1], K2 = a.g.K[2];
+    for (int m = wl; m < m1; m += NW) {
+        const int ox = st.org[m][0], oy = st.org[m][1], oz = st.org[m][2];
+        for (int L = lane; L < 36; L += 32) {
+            const int ix = L / 6, iy = L - 6 * ix;
+            s_base[wl][L] = wrap_up(ox + ix, K0) * K1 + wrap_up(oy + iy, K1);
+            const T* X = st.w[m][0][ix];
+            const T* Y = st.w[m][1][iy];
+            const T* c = s_c[m];
+            if (CH) {
+                s_col[wl][L][0] = c[0] * (X[0] * Y[0]);
+            } else {
+                constexpr int o1 = CH ? 0 : 1, o2 = CH ? 0 : 2;  // in range for the CH instantiation too
+                const T x0 = X[0], x1 = X[1], x2 = X[o2], y0 = Y[0], y1 = Y[1], y2 = Y[o2];
+                const T xy = x0 * y0, x1y = x1 * y0, xy1 = x0 * y1;
+                s_col[wl][L][0] = c[0] * xy + c[1] * x1y + c[2] * xy1 + c[4] * x2 * y0 + c[5] * x0 * y2 + c[7] * x1 * y1;
+                s_col[wl][L][o1] = c[3] * xy + c[8] * x1y + c[9] * xy1;
+                s_col[wl][L][o2] = c[6] * xy;
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int pass = 0; pass < 7; ++pass) {
+            const int p = lane + 32 * pass;
+            if (p < 216) {
+                const int col = p / 6, iz = p - 6 * col;
+                const T* Z = st.w[m][2][iz];
+                const T* sc = s_col[wl][col];
+                const T v = CH ? sc[0] * Z[0] : sc[0] * Z[0] + sc[CH ? 0 : 1] * Z[1] + sc[CH ? 0 : 2] * Z[CH ? 0 : 2];
+                atomicAdd(a.grid + (size_t)s_base[wl][col] * K2 + wrap_up(oz + iz, K2), v);
+            }
+        }
+        __syncwarp();
     }
 }
 
@@ -247,51 +300,69 @@ __device__ __forceinline__ void influence(int kind, double ksq, double kappa, do
     dlnC = (ksq < 1e-16) ? 0.0 : dfdx / f / (8.0 * kappa * kappa * x);
 }
 
-template <typename T>
+// Influence function, energy and k-space tensor over the half spectrum.  A warp takes rows (k1, k2) in
+// turn, lanes the k3 of a row; the sums stay in registers until the end, so a launch issues seven
+// atomics per CTA of a grid that fills the chip once (kConvCtas).  With one element per thread and
+// a CTA per 256 of them, the atomics of 22 000 CTAs on the same seven words bounded it: 180 us at
+// 225^3, now 57 (FP64 exponentials and quotients, 92 MB moved).
+constexpr int kConvCtas = 8 * 148;
+
+template <typename T, bool COUL>
 __global__ void __launch_bounds__(256) k_conv(ConvArgs<T> a) {
-    const int64_t total = (int64_t)a.K[0] * a.K[1] * a.Kh;
-    const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    const int rows = a.K[0] * a.K[1], Kh = a.Kh;
+    const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+    const double TWO_PI = 6.283185307179586;
+    const double c0 = TWO_PI * a.hinv[2], c1 = TWO_PI * a.hinv[5], c2 = TWO_PI * a.hinv[8];
+    const double ik = 1.0 / (4.0 * a.kappa * a.kappa), pref = TWO_PI / a.V;
     double red[7] = {0, 0, 0, 0, 0, 0, 0};
-    if (idx < total) {
-        const int k3 = (int)(idx % a.Kh);
-        const int k2 = (int)((idx / a.Kh) % a.K[1]);
-        const int k1 = (int)(idx / ((int64_t)a.Kh * a.K[1]));
+    for (int row = gw; row < rows; row += nw) {
+        const int k1 = row / a.K[1], k2 = row - k1 * a.K[1];
         const int m1 = k1 < (a.K[0] + 1) / 2 ? k1 : k1 - a.K[0];
         const int m2 = k2 < (a.K[1] + 1) / 2 ? k2 : k2 - a.K[1];
-        const int m3 = k3 < (a.K[2] + 1) / 2 ? k3 : k3 - a.K[2];
-        const double TWO_PI = 6.283185307179586;
-        double kv[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) kv[c] = TWO_PI * (a.hinv[3 * c] * m1 + a.hinv[3 * c + 1] * m2 + a.hinv[3 * c + 2] * m3);
-        const double ksq = kv[0] * kv[0] + kv[1] * kv[1] + kv[2] * kv[2];
-        const double th = a.bmod[k1] * a.bmod[a.K[0] + k2] * a.bmod[a.K[0] + a.K[1] + k3];
-        double G = 0.0, dlnC = 0.0;
-        const bool zero = (m1 == 0 && m2 == 0 && m3 == 0);
-        if (!(zero && a.kind == CK_COUL)) {
-            double C;
-            influence(a.kind, ksq, a.kappa, a.V, C, dlnC);
-            G = C / (th * th);
+        const double b0 = TWO_PI * (a.hinv[0] * m1 + a.hinv[1] * m2), b1 = TWO_PI * (a.hinv[3] * m1 + a.hinv[4] * m2),
+                     b2 = TWO_PI * (a.hinv[6] * m1 + a.hinv[7] * m2);
+        const double th12 = a.bmod[k1] * a.bmod[a.K[0] + k2];
+        for (int k3 = lane; k3 < Kh; k3 += 32) {
+            const int m3 = k3 < (a.K[2] + 1) / 2 ? k3 : k3 - a.K[2];
+            const double kv[3] = {b0 + c0 * m3, b1 + c1 * m3, b2 + c2 * m3};
+            const double ksq = kv[0] * kv[0] + kv[1] * kv[1] + kv[2] * kv[2];
+            const double th = th12 * a.bmod[a.K[0] + a.K[1] + k3], th2 = th * th;
+            double G = 0.0, dlnC = 0.0;
+            const bool zero = m1 == 0 && m2 == 0 && m3 == 0;
+            if (COUL) {
+                if (!zero) {  // influence() with its quotients brought over one denominator
+                    const double d = 1.0 / (ksq * th2);
+                    G = pref * exp(-ksq * ik) * d;
+                    dlnC = -d * th2 - ik;
+                }
+            } else {
+                double C;
+                influence(a.kind, ksq, a.kappa, a.V, C, dlnC);
+                G = C / th2;
+            }
+            T* s = a.S + 2 * ((size_t)row * Kh + k3);
+            const double re = (double)s[0], im = (double)s[1];
+            if (a.want_energy) {
+                const bool self_conj = (k3 == 0) || ((a.K[2] % 2 == 0) && k3 == a.K[2] / 2);
+                const double w = self_conj ? 1.0 : 2.0;
+                const double Ek = a.escale * w * G * (re * re + im * im);
+                red[0] += Ek;
+                const double f = Ek * dlnC, fx = f * kv[0], fy = f * kv[1];
+                red[1] += fx * kv[0];
+                red[2] += fy * kv[1];
+                red[3] += f * kv[2] * kv[2];
+                red[4] += fx * kv[1];
+                red[5] += fx * kv[2];
+                red[6] += fy * kv[2];
+            }
+            s[0] = (T)(re * G);
+            s[1] = (T)(im * G);
         }
-        T* s = a.S + 2 * idx;
-        const double re = (double)s[0], im = (double)s[1];
-        if (a.want_energy) {
-            const bool self_conj = (k3 == 0) || ((a.K[2] % 2 == 0) && k3 == a.K[2] / 2);
-            const double w = self_conj ? 1.0 : 2.0;
-            const double Ek = a.escale * w * G * (re * re + im * im);
-            red[0] = Ek;
-            const double f = Ek * dlnC;
-            red[1] = f * kv[0] * kv[0];
-            red[2] = f * kv[1] * kv[1];
-            red[3] = f * kv[2] * kv[2];
-            red[4] = f * kv[0] * kv[1];
-            red[5] = f * kv[0] * kv[2];
-            red[6] = f * kv[1] * kv[2];
-        }
-        s[0] = (T)(re * G);
-        s[1] = (T)(im * G);
     }
     // the spread input of this pass has been transformed: clear it for the next spread
-    for (int64_t i = idx; i < a.nzero; i += (int64_t)gridDim.x * blockDim.x) a.zero_real[i] = T(0);
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.nzero; i += (int64_t)gridDim.x * blockDim.x)
+        a.zero_real[i] = T(0);
     if (a.want_energy) block_reduce_add<7>(red, a.scal);
 }
 
@@ -310,92 +381,162 @@ struct GatherArgs {
     double scale;         // dE/dmesh = scale * phi   (2*DIELECTRIC or 2)
     double* grad;         // [n*3] += dE/dpos
     T* torque;            // [n*3] += torque of permanent multipoles (may be null)
-    double* field;        // [n*3] dE/dU (Cartesian); written (FIELD) or accumulated
-    int field_accumulate;
     double* gQ;           // [n*9] += dE/dQ_global (may be null)
     double* dq1;          // [n] += dE/dq for the charge channel (may be null)
     double* scal;         // [0] energy (1/2 sum c P), [1..9] X_NA
-    int want_box;
-    int mode;
 };
 
-template <typename T>
-__global__ void __launch_bounds__(256) k_gather(GatherArgs<T> a) {
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    const bool active = warp < a.n;
-    const int at = active ? warp : 0;
-    int m0[3];
-    T Mx[4][6], My[4][6], Mz[4][6];
-    stencil_setup<T>(a.g, a.pos, at, m0, Mx, My, Mz);
-    const int K0 = a.g.K[0], K1 = a.g.K[1], K2 = a.g.K[2];
-    int gz[6];
+// Sums NS values over the warp by recursive halving: at each of the five steps a lane hands one half
+// of what it holds to its partner and keeps the other, so 20 values take 21 exchanges where a
+// butterfly per value takes 100.  The lanes that end up holding a sum write it to out[0 .. NS).
+template <typename T, int NS>
+__device__ __forceinline__ void warp_sums(T (&v)[NS], T* out, int lane) {
+    int idx = 0, sz = NS;
+    constexpr int H[5] = {(NS + 1) / 2, ((NS + 1) / 2 + 1) / 2, (((NS + 1) / 2 + 1) / 2 + 1) / 2,
+                          ((((NS + 1) / 2 + 1) / 2 + 1) / 2 + 1) / 2,
+                          (((((NS + 1) / 2 + 1) / 2 + 1) / 2 + 1) / 2 + 1) / 2};
 #pragma unroll
-    for (int t = 0; t < 6; ++t) gz[t] = wrapi(m0[2] - 3 + t, K2);
-    // partial sums P_abc, a+b+c <= 3, order: index via table below
-    // 0:000 1:100 2:010 3:001 4:200 5:020 6:002 7:110 8:101 9:011
-    // 10:300 11:030 12:003 13:210 14:201 15:120 16:021 17:102 18:012 19:111
-    T P[20];
+    for (int step = 0; step < 5; ++step) {
+        const int n = step == 0 ? NS : H[step - 1], h = H[step], o = 16 >> step;
+        const bool up = (lane & o) != 0;
 #pragma unroll
-    for (int k = 0; k < 20; ++k) P[k] = T(0);
-    const int maxo = (a.mode == GATHER_FIELD) ? 2 : 3;
-    if (active) {
-        for (int L = lane; L < 36; L += 32) {
-            const int ix = L / 6, iy = L % 6;
-            const int gx = wrapi(m0[0] - 3 + ix, K0), gy = wrapi(m0[1] - 3 + iy, K1);
-            const T* line = a.phi + ((size_t)gx * K1 + gy) * K2;
-            T s[4] = {T(0), T(0), T(0), T(0)};
-#pragma unroll
-            for (int t = 0; t < 6; ++t) {
-                const T v = line[gz[t]];
-                s[0] += v * Mz[0][t];
-                s[1] += v * Mz[1][t];
-                s[2] += v * Mz[2][t];
-                s[3] += v * Mz[3][t];
-            }
-            const T x0 = Mx[0][ix], x1 = Mx[1][ix], x2 = Mx[2][ix], x3 = Mx[3][ix];
-            const T y0 = My[0][iy], y1 = My[1][iy], y2 = My[2][iy], y3 = My[3][iy];
-            P[0] += x0 * y0 * s[0];
-            P[1] += x1 * y0 * s[0];
-            P[2] += x0 * y1 * s[0];
-            P[3] += x0 * y0 * s[1];
-            P[4] += x2 * y0 * s[0];
-            P[5] += x0 * y2 * s[0];
-            P[6] += x0 * y0 * s[2];
-            P[7] += x1 * y1 * s[0];
-            P[8] += x1 * y0 * s[1];
-            P[9] += x0 * y1 * s[1];
-            if (maxo == 3) {
-                P[10] += x3 * y0 * s[0];
-                P[11] += x0 * y3 * s[0];
-                P[12] += x0 * y0 * s[3];
-                P[13] += x2 * y1 * s[0];
-                P[14] += x2 * y0 * s[1];
-                P[15] += x1 * y2 * s[0];
-                P[16] += x0 * y2 * s[1];
-                P[17] += x1 * y0 * s[2];
-                P[18] += x0 * y1 * s[2];
-                P[19] += x1 * y1 * s[1];
-            }
+        for (int k = 0; k < NS; ++k) {
+            if (k >= h) break;
+            const T lo = v[k], hi = k + h < n ? v[k + h < NS ? k + h : 0] : T(0);
+            v[k] = (up ? hi : lo) + __shfl_xor_sync(0xffffffffu, up ? lo : hi, o);
+        }
+        if (up) {
+            idx += h;
+            sz = max(sz - h, 0);
+        } else {
+            sz = min(sz, h);
         }
     }
-    // reduce only the sums this mode uses (field: first derivatives; full: all 20)
-    if (maxo == 2) {
-#pragma unroll
-        for (int k = 1; k < 4; ++k) P[k] = warp_sum(P[k]);
-    } else {
-#pragma unroll
-        for (int k = 0; k < 20; ++k) P[k] = warp_sum(P[k]);
-    }
+    if (sz >= 1) out[idx] = v[0];
+}
 
+// Interpolation of the convolved mesh and its derivatives at the sites (CH: charges alone, value and
+// first derivatives), then dE/dpos, dE/dQ, torques and the box term.  A warp takes a site: lanes
+// 0..29 read five columns' six points per pass (runs of six addresses) and keep the sums over the columns
+// at their own z, contract them with the z splines and add them over the warp.  The rest, a few
+// hundred FP64 operations per site, runs with one thread per site.  Latency-bound (L2 reads): 55 us
+// for 99000 charges, 44 us for 30000 multipoles.  With lane 0 of each warp doing that rest for its one
+// site, ten atomics per eight sites and all 20 sums also for charges these took 336 and 110 us.
+template <typename T, bool CH>
+__global__ void __launch_bounds__(kSiteThreads) k_gather(GatherArgs<T> a, int apc) {
+    constexpr int ORD = CH ? 1 : 3, NS = CH ? 4 : 20, NW = kSiteThreads / 32;
+    __shared__ SiteStencils<T, ORD> st;
+    __shared__ T s_P[kSiteAtoms][NS + 1];  // odd stride: the sites' threads read it side by side
+    const int tid = threadIdx.x, lane = tid & 31, wl = tid >> 5;
+    const int first = blockIdx.x * apc, m1 = min(apc, a.n - first);
+    for (int k = tid; k < 3 * m1; k += kSiteThreads) st.set(a.g, a.pos, first + k / 3, k / 3, k % 3);
+    __syncthreads();
+    const int K0 = a.g.K[0], K1 = a.g.K[1], K2 = a.g.K[2];
+    const int grp = lane / 6, iz = lane - 6 * grp;
+    for (int m = wl; m < m1; m += NW) {
+        const int ox = st.org[m][0], oy = st.org[m][1], gz = wrap_up(st.org[m][2] + iz, K2);
+        T v[8];
+#pragma unroll
+        for (int pass = 0; pass < 8; ++pass) {
+            const int col = grp + 5 * pass, ix = col / 6, iy = col - 6 * ix;
+            v[pass] = grp < 5 && col < 36
+                          ? a.phi[((size_t)wrap_up(ox + ix, K0) * K1 + wrap_up(oy + iy, K1)) * K2 + gz]
+                          : T(0);
+        }
+        // partial sums P_abc, a+b+c <= 3, order:
+        // 0:000 1:100 2:010 3:001 4:200 5:020 6:002 7:110 8:101 9:011
+        // 10:300 11:030 12:003 13:210 14:201 15:120 16:021 17:102 18:012 19:111
+        T P[NS];
+        const T* Z = st.w[m][2][iz];
+        if constexpr (CH) {
+            T A00 = T(0), A10 = T(0), A01 = T(0);
+#pragma unroll
+            for (int pass = 0; pass < 8; ++pass) {
+                const int col = min(grp + 5 * pass, 35), ix = col / 6, iy = col - 6 * ix;
+                const T* X = st.w[m][0][ix];
+                const T* Y = st.w[m][1][iy];
+                const T t0 = v[pass] * Y[0], t1 = v[pass] * Y[1];
+                A00 += X[0] * t0;
+                A10 += X[1] * t0;
+                A01 += X[0] * t1;
+            }
+            P[0] = A00 * Z[0];
+            P[1] = A10 * Z[0];
+            P[2] = A01 * Z[0];
+            P[3] = A00 * Z[1];
+        } else {
+            T A00 = T(0), A10 = T(0), A01 = T(0), A20 = T(0), A11 = T(0), A02 = T(0), A30 = T(0), A21 = T(0),
+              A12 = T(0), A03 = T(0);
+#pragma unroll
+            for (int pass = 0; pass < 8; ++pass) {
+                const int col = min(grp + 5 * pass, 35), ix = col / 6, iy = col - 6 * ix;
+                const T* X = st.w[m][0][ix];
+                const T* Y = st.w[m][1][iy];
+                const T t0 = v[pass] * Y[0], t1 = v[pass] * Y[1], t2 = v[pass] * Y[2], t3 = v[pass] * Y[3];
+                A00 += X[0] * t0;
+                A10 += X[1] * t0;
+                A20 += X[2] * t0;
+                A30 += X[3] * t0;
+                A01 += X[0] * t1;
+                A11 += X[1] * t1;
+                A21 += X[2] * t1;
+                A02 += X[0] * t2;
+                A12 += X[1] * t2;
+                A03 += X[0] * t3;
+            }
+            const T z0 = Z[0], z1 = Z[1], z2 = Z[2], z3 = Z[3];
+            P[0] = A00 * z0;
+            P[1] = A10 * z0;
+            P[2] = A01 * z0;
+            P[3] = A00 * z1;
+            P[4] = A20 * z0;
+            P[5] = A02 * z0;
+            P[6] = A00 * z2;
+            P[7] = A11 * z0;
+            P[8] = A10 * z1;
+            P[9] = A01 * z1;
+            P[10] = A30 * z0;
+            P[11] = A03 * z0;
+            P[12] = A00 * z3;
+            P[13] = A21 * z0;
+            P[14] = A20 * z1;
+            P[15] = A12 * z0;
+            P[16] = A02 * z1;
+            P[17] = A10 * z2;
+            P[18] = A01 * z2;
+            P[19] = A11 * z1;
+        }
+        warp_sums<T, NS>(P, s_P[m], lane);
+    }
+    __syncthreads();
+    if (wl) return;  // one thread per site from here on
     double red[10];
 #pragma unroll
     for (int k = 0; k < 10; ++k) red[k] = 0.0;
-    if (active && lane == 0) {
+    if (CH && lane < m1) {
+        // c = {q}: energy q P_000 / 2, dE/dx = -q (P_100, P_010, P_001)
+        const int at = first + lane;
+        const double q = (double)a.q1[at], P0 = a.scale * (double)s_P[lane][0];
+        double Y[3];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) Y[j] = -q * (a.scale * (double)s_P[lane][1 + j]);
+        const double* NA = a.g.NA;
+        double* gr = a.grad + 3 * at;
+#pragma unroll
+        for (int cc = 0; cc < 3; ++cc) gr[cc] += NA[cc] * Y[0] + NA[3 + cc] * Y[1] + NA[6 + cc] * Y[2];
+        red[0] = 0.5 * (q * P0);
+        if (a.dq1) a.dq1[at] += P0;
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+#pragma unroll
+            for (int cc = 0; cc < 3; ++cc) red[1 + 3 * j + cc] = Y[j] * a.pos[3 * at + cc];
+    }
+    if (!CH && lane < m1) {
+        const int at = first + lane;
         const double sc = a.scale;
         double Pd[20];
 #pragma unroll
-        for (int k = 0; k < 20; ++k) Pd[k] = sc * (double)P[k];
+        for (int k = 0; k < 20; ++k) Pd[k] = sc * (double)s_P[lane][k < NS ? k : 0];
         // site multipole (the one that was spread)
         SpreadArgs<T> sa;
         sa.Qg = a.Qg; sa.U = a.U; sa.q1 = a.q1; sa.lmax = a.lmax;
@@ -413,11 +554,7 @@ __global__ void __launch_bounds__(256) k_gather(GatherArgs<T> a) {
         double dmu[3];
 #pragma unroll
         for (int cc = 0; cc < 3; ++cc) dmu[cc] = -(Pu[0] * B[cc] + Pu[1] * B[3 + cc] + Pu[2] * B[6 + cc]);
-        if (a.mode == GATHER_FIELD) {
-            double* f = a.field + 3 * at;
-            if (a.field_accumulate) { f[0] += dmu[0]; f[1] += dmu[1]; f[2] += dmu[2]; }
-            else { f[0] = dmu[0]; f[1] = dmu[1]; f[2] = dmu[2]; }
-        } else {
+        {
             // dE/dx_j = -sum_abc c_abc P_{abc + e_j}
             // coefficient -> (a,b,c) exponents; index of abc+e_j in P
             const int up[10][3] = {{1, 2, 3},   {4, 7, 8},   {7, 5, 9},   {8, 9, 6},    {10, 13, 14},
@@ -457,11 +594,6 @@ __global__ void __launch_bounds__(256) k_gather(GatherArgs<T> a) {
             g[6] = (dTh[1][2] + dTh[2][1]) * s6;
             g[7] = (dTh[0][0] - dTh[1][1]) * s6;
             g[8] = (dTh[0][1] + dTh[1][0]) * s6;
-            if (a.field) {
-                double* f = a.field + 3 * at;
-                if (a.field_accumulate) { f[0] += dmu[0]; f[1] += dmu[1]; f[2] += dmu[2]; }
-                else { f[0] = dmu[0]; f[1] = dmu[1]; f[2] = dmu[2]; }
-            }
             if (a.gQ) {
 #pragma unroll
                 for (int k = 0; k < 9; ++k) a.gQ[9 * at + k] += g[k];
@@ -479,7 +611,7 @@ __global__ void __launch_bounds__(256) k_gather(GatherArgs<T> a) {
                 atomicAdd(a.torque + 3 * at + 1, t[1]);
                 atomicAdd(a.torque + 3 * at + 2, t[2]);
             }
-            if (a.want_box) {
+            {
                 // X_NA = Y (x) R + (dE/dB)^T,  dE/dB = -Pu (x) mu + 2 P2 B Theta
                 const double R[3] = {a.pos[3 * at], a.pos[3 * at + 1], a.pos[3 * at + 2]};
                 double PB[3][3];
@@ -500,7 +632,11 @@ __global__ void __launch_bounds__(256) k_gather(GatherArgs<T> a) {
             }
         }
     }
-    if (a.mode == GATHER_FULL) block_reduce_add<10>(red, a.scal);
+#pragma unroll
+    for (int k = 0; k < 10; ++k) {
+        const double v = warp_sum(red[k]);
+        if (lane == 0 && v != 0.0) atomicAdd(a.scal + k, v);
+    }
 }
 
 
@@ -613,12 +749,6 @@ struct StencilCache {
     const int4* org;  // wrapped first stencil point per dimension (w unused)
     const T* w;       // [n * 36]
 };
-
-// g + d wrapped into [0, K) for g in [0, K), d >= 0
-__device__ __forceinline__ int wrap_up(int g, int K) {
-    while (g >= K) g -= K;
-    return g;
-}
 
 template <typename T>
 __global__ void __launch_bounds__(256) k_stencil_prep(int n, const double* pos, MeshGeom g, int4* org, T* w) {

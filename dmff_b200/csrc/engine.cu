@@ -795,7 +795,9 @@ int mesh_convolve(dmffb_engine* h, cudaStream_t s, void* in, void* out, ConvArgs
     else
         FFTCALL(h, s, cufftExecD2Z(h->plan_f, (cufftDoubleReal*)in, (cufftDoubleComplex*)h->d_cgrid));
     const int64_t nk = (int64_t)h->K[0] * h->K[1] * ca.Kh;
-    LAUNCH(h, s, KC_CONV, k_conv<T><<<nblk(nk, 256), 256, 0, s>>>(ca));
+    const unsigned ctas = std::min(nblk(nk, 256), (unsigned)kConvCtas);
+    if (ca.kind == CK_COUL) LAUNCH(h, s, KC_CONV, k_conv<T, true><<<ctas, 256, 0, s>>>(ca));
+    else LAUNCH(h, s, KC_CONV, k_conv<T, false><<<ctas, 256, 0, s>>>(ca));
     if (sizeof(T) == 4)
         FFTCALL(h, s, cufftExecC2R(h->plan_b, (cufftComplex*)h->d_cgrid, (cufftReal*)out));
     else
@@ -884,7 +886,7 @@ StencilCache<T> stencil_cache(dmffb_engine* h) {
 // transform -> gather
 template <typename T>
 int recip_pass(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx, bool use_Qg, const double* U,
-               int mode, double* field_out, int field_acc, double* const* zero_scal = nullptr) {
+               int mode, double* field_out, double* const* zero_scal = nullptr) {
     const MeshGeom g = mesh_geom(bx, h->K);
     const int64_t K3 = (int64_t)h->K[0] * h->K[1] * h->K[2];
     // the dipole-only field pass (the CG matvec) spreads into d_grid2, which the convolution
@@ -911,7 +913,8 @@ int recip_pass(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx
         if (zero_scal)
             for (int k = 0; k < 3; ++k)
                 if (zero_scal[k]) CK(cudaMemsetAsync(zero_scal[k], 0, sizeof(double), s));
-        LAUNCH(h, s, KC_SPREAD, k_spread<T><<<nblk((int64_t)h->n * 32, 256), 256, 0, s>>>(sa));
+        const int apc = sites_per_cta(h->n);
+        LAUNCH(h, s, KC_SPREAD, k_spread<T, false><<<nblk(h->n, apc), kSiteThreads, 0, s>>>(sa, apc));
     }
     ConvArgs<T> ca = conv_args<T>(h, bx, CK_COUL, DMFFB_DIELECTRIC, h->d_scal + S_RECIP, mode == GATHER_FULL);
     if (dip) {
@@ -920,6 +923,17 @@ int recip_pass(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx
     }
     int st = mesh_convolve<T>(h, s, spread_grid, h->d_grid, ca);
     if (st) return st;
+    if (mode == GATHER_FIELD) {
+        if (h->stencils_ready)
+            LAUNCH(h, s, KC_GATHER_FIELD, k_gather_field_cached<T><<<nblk((int64_t)h->n * 32, 256), 256, 0, s>>>(
+                                              h->n, stencil_cache<T>(h), g, (const T*)h->d_grid, 2.0 * DMFFB_DIELECTRIC,
+                                              field_out, FieldCombine()));
+        else
+            LAUNCH(h, s, KC_GATHER_FIELD, k_gather_field<T><<<nblk((int64_t)h->n * 32, 256), 256, 0, s>>>(
+                                              h->n, pos, g, (const T*)h->d_grid, 2.0 * DMFFB_DIELECTRIC, field_out));
+        CK(cudaGetLastError());
+        return DMFFB_OK;
+    }
     GatherArgs<T> ga;
     ga.n = h->n;
     ga.pos = pos;
@@ -932,22 +946,11 @@ int recip_pass(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx
     ga.scale = 2.0 * DMFFB_DIELECTRIC;
     ga.grad = h->d_grad;
     ga.torque = (T*)h->d_torque;
-    ga.field = field_out;
-    ga.field_accumulate = field_acc;
-    ga.gQ = (mode == GATHER_FULL) ? h->d_gQ : nullptr;
+    ga.gQ = h->d_gQ;
     ga.dq1 = nullptr;
     ga.scal = h->d_scal + S_GATHER;
-    ga.want_box = 1;
-    ga.mode = mode;
-    if (mode == GATHER_FIELD && !field_acc && h->stencils_ready)
-        LAUNCH(h, s, KC_GATHER_FIELD, k_gather_field_cached<T><<<nblk((int64_t)h->n * 32, 256), 256, 0, s>>>(
-                                          h->n, stencil_cache<T>(h), g, (const T*)h->d_grid, 2.0 * DMFFB_DIELECTRIC, field_out,
-                                          FieldCombine()));
-    else if (mode == GATHER_FIELD && !field_acc)
-        LAUNCH(h, s, KC_GATHER_FIELD, k_gather_field<T><<<nblk((int64_t)h->n * 32, 256), 256, 0, s>>>(
-                                          h->n, pos, g, (const T*)h->d_grid, 2.0 * DMFFB_DIELECTRIC, field_out));
-    else
-        LAUNCH(h, s, (mode == GATHER_FULL ? KC_GATHER_FULL : KC_GATHER_FIELD), k_gather<T><<<nblk((int64_t)h->n * 32, 256), 256, 0, s>>>(ga));
+    const int apc = sites_per_cta(h->n);
+    LAUNCH(h, s, KC_GATHER_FULL, k_gather<T, false><<<nblk(h->n, apc), kSiteThreads, 0, s>>>(ga, apc));
     CK(cudaGetLastError());
     return DMFFB_OK;
 }
@@ -1134,7 +1137,7 @@ int field_eval(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx
     if (fork) CK(cudaEventRecord(h->e_join, h->s2));
     const double* recip = nullptr;
     if (recip_on) {
-        int st = recip_pass<T>(h, s, pos, bx, include_perm, U, GATHER_FIELD, h->d_fr, 0, zero_scal);
+        int st = recip_pass<T>(h, s, pos, bx, include_perm, U, GATHER_FIELD, h->d_fr, zero_scal);
         if (st) return st;
         recip = h->d_fr;
     }
@@ -1520,7 +1523,7 @@ int compute_impl(dmffb_engine* h, cudaStream_t s, const double* pos, const doubl
     if (fork_full) CK(cudaEventRecord(h->e_join, h->s2));
     if (h->timing) CK(cudaEventRecord(h->ev[3], s));
     if (h->lpme && h->have_plans) {
-        if ((st = recip_pass<T>(h, s, pos, bx, true, h->lpol ? U : nullptr, GATHER_FULL, nullptr, 0))) return st;
+        if ((st = recip_pass<T>(h, s, pos, bx, true, h->lpol ? U : nullptr, GATHER_FULL, nullptr))) return st;
     }
     if (fork_full) CK(cudaStreamWaitEvent(s, h->e_join, 0));
     if (h->timing) CK(cudaEventRecord(h->ev[4], s));
@@ -1658,7 +1661,8 @@ int recip_pass_channel(dmffb_engine* h, cudaStream_t s, const double* pos, const
     sa.g = g;
     sa.grid = (T*)h->d_grid;
     sa.perm_mul = h->perm_mul;
-    LAUNCH(h, s, KC_SPREAD, k_spread<T><<<nblk((int64_t)h->n * 32, 256), 256, 0, s>>>(sa));
+    const int apc = sites_per_cta(h->n);
+    LAUNCH(h, s, KC_SPREAD, k_spread<T, true><<<nblk(h->n, apc), kSiteThreads, 0, s>>>(sa, apc));
     ConvArgs<T> ca = conv_args<T>(h, bx, kind, escale, scal_conv, true);
     int st = mesh_convolve<T>(h, s, h->d_grid, h->d_grid, ca);
     if (st) return st;
@@ -1674,14 +1678,10 @@ int recip_pass_channel(dmffb_engine* h, cudaStream_t s, const double* pos, const
     ga.scale = 2.0 * escale;
     ga.grad = grad;
     ga.torque = nullptr;
-    ga.field = nullptr;
-    ga.field_accumulate = 0;
     ga.gQ = nullptr;
     ga.dq1 = dq;
     ga.scal = scal_gather;
-    ga.want_box = 1;
-    ga.mode = GATHER_FULL;
-    LAUNCH(h, s, KC_GATHER_FULL, k_gather<T><<<nblk((int64_t)h->n * 32, 256), 256, 0, s>>>(ga));
+    LAUNCH(h, s, KC_GATHER_FULL, k_gather<T, true><<<nblk(h->n, apc), kSiteThreads, 0, s>>>(ga, apc));
     CK(cudaGetLastError());
     return DMFFB_OK;
 }
