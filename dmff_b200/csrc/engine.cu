@@ -184,6 +184,8 @@ struct dmffb_engine {
     int64_t n_covrows = 0;
     int32_t *d_cov_lo = nullptr, *d_cov_hi = nullptr;  // [n] covalent partner index range
     float4* d_posc = nullptr;  // [n] cell-ordered positions (pair builds and the cell pass)
+    NbRec* d_nbrec = nullptr;  // [n] cell-ordered records of the cell pass
+    void* d_gcell = nullptr;   // [n][4] its gradients in cell order, kernel precision
     // ---- short-range pairwise terms (engines made by dmffb_pairwise_create, kind 3)
     int sr_kind = 0;
     double sr_sign = 1.0;
@@ -2138,12 +2140,18 @@ int classical_compute_impl(dmffb_engine* h, cudaStream_t s, const double* pos, c
         c.rc = h->rc;
         for (int k = 0; k < 3; ++k) c.nc[k] = ncf[k];
         c.cell_start = h->d_cell_start;
+        c.atom_cell = h->d_atom_cell;
         c.cov.cov_ptr = h->d_cov_ptr;
         c.cov.cov_j = h->d_cov_j;
         c.cov.cov_nb = h->d_cov_nb;
         c.cov_lo = h->d_cov_lo;
         c.cov_hi = h->d_cov_hi;
-        c.qT = (const T*)h->d_qT;
+        if (!h->d_nbrec) {
+            if ((st = dalloc(h, &h->d_nbrec, (size_t)h->n_cap * sizeof(NbRec))) ||
+                (st = dalloc(h, &h->d_gcell, (size_t)h->n_cap * 4 * sizeof(T))))
+                return st;
+        }
+        c.rec = h->d_nbrec;
         c.type = h->ntypes > 0 ? h->d_type : nullptr;
         c.ntypes = h->ntypes;
         c.sig_tt = (const T*)h->d_sigtt;
@@ -2154,7 +2162,7 @@ int classical_compute_impl(dmffb_engine* h, cudaStream_t s, const double* pos, c
         c.krf = (T)h->krf;
         c.crf = (T)h->crf;
         c.coul = h->coul;
-        c.grad = (T*)h->d_glr;
+        c.gcell = (T*)h->d_gcell;
         c.scal = h->d_scal;
         {
             const double* m = bx.h;
@@ -2166,7 +2174,13 @@ int classical_compute_impl(dmffb_engine* h, cudaStream_t s, const double* pos, c
                 c.width[k] = V / sqrt(cx * cx + cy * cy + cz * cz);
             }
         }
-        LAUNCH(h, s, KC_PAIR_FULL, k_nb_cells<T><<<nblk((int64_t)n * 32, 32 * kNbWarps), 32 * kNbWarps, 0, s>>>(c));
+        LAUNCH(h, s, KC_NBLIST, k_nb_records<T><<<nblk(n, 256), 256, 0, s>>>(n, c.posc, pos, (const T*)h->d_qT, c.type,
+                                                                             h->d_nbrec, (T*)h->d_gcell));
+        const double* m = bx.h;
+        const bool ortho = m[1] == 0.0 && m[2] == 0.0 && m[3] == 0.0 && m[5] == 0.0 && m[6] == 0.0 && m[7] == 0.0;
+        const unsigned ctas = nblk((int64_t)n * 32, 32 * kNbWarps);
+        if (ortho) LAUNCH(h, s, KC_PAIR_FULL, k_nb_cells<T, true><<<ctas, 32 * kNbWarps, 0, s>>>(c));
+        else LAUNCH(h, s, KC_PAIR_FULL, k_nb_cells<T, false><<<ctas, 32 * kNbWarps, 0, s>>>(c));
         CK(cudaGetLastError());
         // rows with a topological scale: the covalent rows within rc, FP64 for FP32 engines
         pairs = h->d_covrows;
@@ -2240,7 +2254,11 @@ int classical_compute_impl(dmffb_engine* h, cudaStream_t s, const double* pos, c
         else LAUNCH(h, s, KC_BONDED, k_torsions<<<nbk, 128, 0, s>>>(b));
         CK(cudaGetLastError());
     }
-    if (forces)
+    if (forces && cellpass)
+        LAUNCH(h, s, KC_VEC, k_nb_forces<T><<<nblk(n, 256), 256, 0, s>>>(
+                                 n, (const T*)h->d_glr, h->d_grad, (const T*)h->d_gcell, h->d_cell_start, h->d_atom_cell,
+                                 h->d_rank, forces));
+    else if (forces)
         LAUNCH(h, s, KC_VEC, k_disp_finalize<T><<<nblk(3 * n, 256), 256, 0, s>>>(
                                  n, (const T*)h->d_glr, (const T*)nullptr, h->d_grad, forces, (double*)nullptr));
     CK(cudaMemcpyAsync(h->h_scal, h->d_scal, N_SCAL * sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -2607,7 +2625,7 @@ void dmffb_destroy(dmffb_engine* h) {
                     h->d_q, h->d_qT, h->d_type, h->d_sigtt, h->d_epstt, h->d_dq, h->d_dsig, h->d_deps,
                     h->d_tidx[0], h->d_tidx[1], h->d_tidx[2], h->d_tprm[0], h->d_tprm[1], h->d_tprm[2],
                     h->d_tdprm[0], h->d_tdprm[1], h->d_tdprm[2], h->d_dQloc, h->d_dpa, h->d_dth, h->d_dpol, h->d_dsr, h->d_srows, h->d_nsel, h->d_cubsel,
-                    h->d_ell_rows, h->d_ell_ent, h->d_stc_org, h->d_stc_w, h->d_nbmask, h->d_covrows, h->d_cov_lo, h->d_cov_hi, h->d_dftW, h->d_dftG, h->d_pcg, h->d_posc, h->d_srp, h->d_srdp, h->d_srgrad};
+                    h->d_ell_rows, h->d_ell_ent, h->d_stc_org, h->d_stc_w, h->d_nbmask, h->d_covrows, h->d_cov_lo, h->d_cov_hi, h->d_dftW, h->d_dftG, h->d_pcg, h->d_posc, h->d_nbrec, h->d_gcell, h->d_srp, h->d_srdp, h->d_srgrad};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (h->h_scal) cudaFreeHost(h->h_scal);

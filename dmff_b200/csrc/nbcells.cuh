@@ -22,8 +22,8 @@
 //     within rc evaluates them (k_nb_pair with a cut-off test);
 //   * every other kept pair is queued in shared memory and evaluated 32 at a time (every lane
 //     busy): nb_eval in kernel precision on the FP64 minimum-image vector and distance of
-//     k_nb_pair; the force on i accumulates in lane registers (one warp sum and one atomic per
-//     atom), the force on j goes out as an atomic;
+//     k_nb_pair; the force on i accumulates in lane registers (one warp sum and one reduction per
+//     atom), the force on the partner goes out as one 16-byte reduction into its cell slot;
 //   * the count of kept pairs (scaled ones included) is the list's row count.
 // Energies and the box gradient accumulate per lane (about 20 pairs each) and meet in an FP64 block
 // reduction.
@@ -33,21 +33,28 @@
 
 namespace dmffb {
 
+// What a pair reads of a partner, one 32-byte load: the position as the caller gave it and, in w, the
+// charge (FP32 engines: the float charge and the LJ type; FP64 engines: the charge).
+struct __align__(32) NbRec {
+    double x, y, z, w;
+};
+
 template <typename T>
 struct NbCellArgs {
     int n;
-    const double* pos;        // [3n] FP64
-    const float4* posc;       // [n] FP32 x, y, z and the atom index (as int bits), in cell order
+    const double* pos;        // [3n] FP64 (borderline distance tests)
+    const float4* posc;       // [n] FP32 x, y, z inside the box and the atom index (int bits), cell order
     Box boxd;
     double rc;
     int nc[3];                // half-width cells per axis (>= 5)
     double width[3];          // perpendicular widths of the box (the distance between the faces
                               // of constant fractional coordinate k)
     const int32_t* cell_start;
+    const int32_t* atom_cell;  // [n]
     NbArgs cov;               // covalent-map lookup (cov_ptr / cov_j / cov_nb over i < j)
     const int32_t* cov_lo;    // [n] smallest / largest covalent partner index (lo > hi: none)
     const int32_t* cov_hi;
-    const T* qT;              // [n] charges in kernel precision
+    const NbRec* rec;         // [n] in cell order: FP64 position, charge and (FP32) LJ type
     const int32_t* type;      // [n] LJ type or null
     int ntypes;
     const T* sig_tt;
@@ -55,53 +62,132 @@ struct NbCellArgs {
     T mc, ml;                 // scales of nbond 0 (the trailing 1.0 entries)
     T kappa, krf, crf;
     int coul;
-    T* grad;                  // [3n] dE/dpos, written once per atom
+    T* gcell;                 // [n][4] dE/dpos in cell order
     double* scal;             // [0] E_coul, [1] E_lj, [2..10] box gradient, [11] pairs i < j within rc
 };
 
-// One kept pair (i, j), met once: energy, box gradient, the force on i (registers) and on j (atomics).
+__device__ __forceinline__ void nb_rec_get(const NbRec& r, float& q, int& type) {
+    const long long b = __double_as_longlong(r.w);
+    q = __int_as_float((int)b);
+    type = (int)(b >> 32);
+}
+__device__ __forceinline__ void nb_rec_get(const NbRec& r, double& q, int&) { q = r.w; }
+
+// the records of the cell order, and the cell-ordered gradients cleared
 template <typename T>
-__device__ __forceinline__ void nb_cell_pair(const NbCellArgs<T>& a, int i, int j, const double* pi,
-                                             const BoxT<double>& bxd, bool lj, int ti, T qi, T& g0, T& g1, T& g2,
-                                             T (&acc)[11]) {
-    // the pair geometry of k_nb_pair: FP64 minimum image, then kernel precision
-    T e[3], r;
-    T nn[3];
-    {
-        double dr[3] = {a.pos[3 * j] - pi[0], a.pos[3 * j + 1] - pi[1], a.pos[3 * j + 2] - pi[2]};
-        double nd[3];
-        pbc_shift(bxd, dr[0], dr[1], dr[2], nd);
+__global__ void k_nb_records(int n, const float4* posc, const double* pos, const T* qT, const int32_t* type, NbRec* rec,
+                             T* gcell) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    const int i = __float_as_int(posc[k].w);
+    NbRec r;
+    r.x = pos[3 * i];
+    r.y = pos[3 * i + 1];
+    r.z = pos[3 * i + 2];
+    if (sizeof(T) == 4)
+        r.w = __longlong_as_double((long long)(unsigned)__float_as_int((float)qT[i]) |
+                                   ((long long)(type ? type[i] : 0) << 32));
+    else
+        r.w = (double)qT[i];
+    rec[k] = r;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) { e[c] = (T)dr[c]; nn[c] = (T)nd[c]; }
-        r = (T)sqrt(dr[0] * dr[0] + dr[1] * dr[1] + dr[2] * dr[2]);
-    }
-    int tp = 0;
-    if (lj) tp = ti * a.ntypes + a.type[j];
-    T ec, dec, phi, el, del, ds, dp;
-    nb_eval<T>(r, qi * a.qT[j], a.mc, a.ml, lj ? a.sig_tt[tp] : T(0), lj ? a.eps_tt[tp] : T(0), lj, a.coul, a.kappa,
-               a.krf, a.crf, ec, dec, phi, el, del, ds, dp);
-    // e = r_j - r_i (minimum image); dE/dr_i = -(dE/dr / r) e; image counts of r_i - r_j are -nn
-    const T s = (dec + del) / r;
-    g0 -= s * e[0];
-    g1 -= s * e[1];
-    g2 -= s * e[2];
-    atomicAdd(a.grad + 3 * j, s * e[0]);
-    atomicAdd(a.grad + 3 * j + 1, s * e[1]);
-    atomicAdd(a.grad + 3 * j + 2, s * e[2]);
-    acc[0] += ec;
-    acc[1] += el;
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) acc[2 + 3 * k + c] -= nn[k] * s * e[c];
+    for (int c = 0; c < 4; ++c) gcell[4 * (int64_t)k + c] = T(0);
 }
 
+// forces of the cell pass: -(reciprocal and bonded + scaled rows + cell order)
 template <typename T>
+__global__ void k_nb_forces(int n, const T* glr, const double* gd, const T* gcell, const int32_t* cell_start,
+                            const int32_t* atom_cell, const int32_t* rank, double* forces) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const T* g = gcell + 4 * (int64_t)(cell_start[atom_cell[i]] + rank[i]);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) forces[3 * i + c] = -((double)glr[3 * i + c] + (double)g[c] + gd[3 * i + c]);
+}
+
+__device__ __forceinline__ void nb_add(float* g, float x, float y, float z) {
+    atomicAdd((float4*)g, make_float4(x, y, z, 0.f));  // one 16-byte reduction
+}
+__device__ __forceinline__ void nb_add(double* g, double x, double y, double z) {
+    atomicAdd(g, x);
+    atomicAdd(g + 1, y);
+    atomicAdd(g + 2, z);
+}
+
+// distance of an FP64 square in kernel precision: FP32 from the hardware's reciprocal square root and
+// one FP64 Newton step (error 1e-14, so it rounds to the same float as the FP64 root all but always)
+__device__ __forceinline__ void nb_root(double r2, double& r) { r = sqrt(r2); }
+__device__ __forceinline__ void nb_root(double r2, float& r) {
+    const double y = (double)rsqrtf((float)r2);
+    const double q = r2 * y;
+    r = (float)fma(0.5 * y, fma(-q, q, r2), q);
+}
+
+// One kept pair (i, the atom in cell slot k), met once: energy, box gradient, the force on i
+// (registers) and on the partner (a reduction into its slot).
+template <typename T, bool ORTHO>
+__device__ __forceinline__ void nb_cell_pair(const NbCellArgs<T>& a, int k, double xi, double yi, double zi, bool lj,
+                                             int ti, T qi, T& g0, T& g1, T& g2, T (&acc)[11]) {
+    const NbRec rj = a.rec[k];
+    // the pair geometry of k_nb_pair: FP64 minimum image, then kernel precision
+    T e[3], r;
+    double dr[3] = {rj.x - xi, rj.y - yi, rj.z - zi}, nd[3];
+    if (ORTHO) {  // pbc_shift without the products with zero
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            double t = dr[c] * a.boxd.hinv[4 * c];
+            nd[c] = floor(t + 0.5);
+            dr[c] = (t - nd[c]) * a.boxd.h[4 * c];
+        }
+    } else {
+        BoxT<double> bx;
+#pragma unroll
+        for (int c = 0; c < 9; ++c) { bx.h[c] = a.boxd.h[c]; bx.hinv[c] = a.boxd.hinv[c]; }
+        pbc_shift(bx, dr[0], dr[1], dr[2], nd);
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) e[c] = (T)dr[c];
+    nb_root(dr[0] * dr[0] + dr[1] * dr[1] + dr[2] * dr[2], r);
+    T qj;
+    int tj = 0;
+    nb_rec_get(rj, qj, tj);
+    int tp = 0;
+    if (lj) {
+        if (sizeof(T) == 8) tj = a.type[__float_as_int(a.posc[k].w)];
+        tp = ti * a.ntypes + tj;
+    }
+    T ec, dec, phi, el, del, ds, dp;
+    nb_eval<T>(r, qi * qj, a.mc, a.ml, lj ? a.sig_tt[tp] : T(0), lj ? a.eps_tt[tp] : T(0), lj, a.coul, a.kappa,
+               a.krf, a.crf, ec, dec, phi, el, del, ds, dp);
+    // e = r_j - r_i (minimum image); dE/dr_i = -(dE/dr / r) e; image counts of r_i - r_j are -nd
+    const T s = (dec + del) / r;
+    const T f0 = s * e[0], f1 = s * e[1], f2 = s * e[2];
+    g0 -= f0;
+    g1 -= f1;
+    g2 -= f2;
+    nb_add(a.gcell + 4 * (int64_t)k, f0, f1, f2);
+    acc[0] += ec;
+    acc[1] += el;
+    if (nd[0] != 0.0 || nd[1] != 0.0 || nd[2] != 0.0) {  // most pairs meet inside the box
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            const T nn = (T)nd[q];
+            acc[2 + 3 * q] -= nn * f0;
+            acc[3 + 3 * q] -= nn * f1;
+            acc[4 + 3 * q] -= nn * f2;
+        }
+    }
+}
+
+// Bound by instruction issue (FP64 minimum image, erfc / exp, the candidate test): 607 us for the 20.8 M
+// pairs of 99000 atoms at rc 10 A.  Scalar reductions into [3n], three FP64 gathers plus charge
+// and type per partner, FP64 division in the cell pruning and a full FP64 root took it to 822 us.
+template <typename T, bool ORTHO>
 __global__ void __launch_bounds__(32 * kNbWarps, sizeof(T) == 4 ? 4 : 0) k_nb_cells(NbCellArgs<T> a) {
     constexpr int S = 2, W = 2 * S + 1, NQ = (W * W * W + 1) / 2;  // offsets q0 = 62 .. 124 of the 5^3 stencil
     __shared__ int s_beg[kNbWarps][NQ];
     __shared__ int s_off[kNbWarps][NQ + 1];
-    __shared__ int s_q[kNbWarps][64];  // kept candidates waiting for a full 32-lane batch
+    __shared__ int s_q[kNbWarps][64];  // kept candidates (cell slots) waiting for a full 32-lane batch
     const int wl = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     // warps take the atoms in cell order: the warps of a block share one stencil, so their
@@ -114,33 +200,29 @@ __global__ void __launch_bounds__(32 * kNbWarps, sizeof(T) == 4 ? 4 : 0) k_nb_ce
     if (live) {
         const float4 p4 = a.posc[ks];
         const int i = __float_as_int(p4.w);
-        const double* pi = a.pos + 3 * i;
-        const float pix = p4.x, piy = p4.y, piz = p4.z;
+        const NbRec ri = a.rec[ks];
         float hf[9], hif[9];
 #pragma unroll
         for (int k = 0; k < 9; ++k) { hf[k] = (float)a.boxd.h[k]; hif[k] = (float)a.boxd.hinv[k]; }
-        BoxT<double> bxd;
-#pragma unroll
-        for (int k = 0; k < 9; ++k) { bxd.h[k] = a.boxd.h[k]; bxd.hinv[k] = a.boxd.hinv[k]; }
         const float rlo = (float)(a.rc - 2e-3), rhi = (float)(a.rc + 2e-3);
         const float rlo2 = rlo * rlo, rhi2 = rhi * rhi;
-        int c3[3];
-        cell_of(a.boxd, a.nc, pi, c3);
-        // the atom's fractional coordinates (as cell_of takes them): a stencil cell none of whose
-        // points lies within rc + 0.01 A of the atom is skipped (about a third of the forward half
-        // for half-width cells).  Orthorhombic boxes: the exact distance to the cell's box; others
-        // the lower bound max_k gap_k width_k (gap_k the fractional gap along k).  The margin
-        // covers the FP32 prefilter band (rc +- 2e-3 A) and the rounding of the binning, so the
-        // kept pairs are unchanged.
-        double sfr[3];
+        // The atom's cell (from the binning) and its position in it, in cell units.  A stencil cell none of
+        // whose points lies within rc + 0.01 A of the atom is skipped (about a third of the forward
+        // half for half-width cells).  Orthorhombic boxes: the exact distance to the cell's box;
+        // others the lower bound max_k gap_k width_k (gap_k the fractional gap along k).  The margin
+        // covers the FP32 prefilter band (rc +- 2e-3 A) and the rounding of the binning and of
+        // the FP32 gaps, so the kept pairs are unchanged.
+        const int ac = a.atom_cell[i];
+        const int c3[3] = {ac / (a.nc[2] * a.nc[1]), (ac / a.nc[2]) % a.nc[1], ac % a.nc[2]};
+        float u[3], cw[3];
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            const double v = pi[0] * a.boxd.hinv[k] + pi[1] * a.boxd.hinv[3 + k] + pi[2] * a.boxd.hinv[6 + k];
-            sfr[k] = v - floor(v);
+            double v = ri.x * a.boxd.hinv[k] + ri.y * a.boxd.hinv[3 + k] + ri.z * a.boxd.hinv[6 + k];
+            v = (v - floor(v)) * a.nc[k];
+            u[k] = (float)(v - c3[k]);
+            cw[k] = (float)(a.width[k] / a.nc[k]);
         }
-        const bool ortho = a.boxd.h[1] == 0.0 && a.boxd.h[2] == 0.0 && a.boxd.h[3] == 0.0 && a.boxd.h[5] == 0.0 &&
-                           a.boxd.h[6] == 0.0 && a.boxd.h[7] == 0.0;
-        const double rprune = a.rc + 0.01;
+        const float rprune = (float)(a.rc + 0.01);
         int carry = 0;
         if (lane == 0) s_off[wl][0] = 0;
         for (int q0 = 0; q0 < NQ; q0 += 32) {
@@ -148,27 +230,23 @@ __global__ void __launch_bounds__(32 * kNbWarps, sizeof(T) == 4 ? 4 : 0) k_nb_ce
             int cnt = 0;
             if (q < NQ) {
                 const int qq = q + NQ - 1;  // (0, 0, 0) and the offsets after it
-                const int dx = qq / (W * W) - S, dy = (qq / W) % W - S, dz = qq % W - S;
-                const int cx = (c3[0] + dx + a.nc[0]) % a.nc[0];
-                const int cy = (c3[1] + dy + a.nc[1]) % a.nc[1];
-                const int cz = (c3[2] + dz + a.nc[2]) % a.nc[2];
-                const int cc = (cx * a.nc[1] + cy) * a.nc[2] + cz;
+                const int dd[3] = {qq / (W * W) - S, (qq / W) % W - S, qq % W - S};
+                int cc = 0;
+                float d2 = 0.f, dmax = 0.f;
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    int ck = c3[k] + dd[k];
+                    ck += ck < 0 ? a.nc[k] : (ck >= a.nc[k] ? -a.nc[k] : 0);
+                    cc = cc * a.nc[k] + ck;
+                    const float gap = fmaxf(0.f, fmaxf(dd[k] - u[k], u[k] - (dd[k] + 1))) * cw[k];
+                    d2 += gap * gap;
+                    dmax = fmaxf(dmax, gap);
+                }
                 int cs = a.cell_start[cc];
                 const int ce = a.cell_start[cc + 1];
                 if (q == 0) cs = max(cs, ks + 1);  // own cell: the atoms after i in cell order
                 cnt = max(ce - cs, 0);
-                if (q > 0) {
-                    const int dd[3] = {dx, dy, dz};
-                    double d2 = 0.0, dmax = 0.0;
-#pragma unroll
-                    for (int k = 0; k < 3; ++k) {
-                        const double lo = (double)(c3[k] + dd[k]) / a.nc[k], hi = (double)(c3[k] + dd[k] + 1) / a.nc[k];
-                        const double gap = fmax(0.0, fmax(lo - sfr[k], sfr[k] - hi)) * a.width[k];
-                        d2 += gap * gap;
-                        dmax = fmax(dmax, gap);
-                    }
-                    if (ortho ? d2 > rprune * rprune : dmax > rprune) cnt = 0;
-                }
+                if (q > 0 && (ORTHO ? d2 > rprune * rprune : dmax > rprune)) cnt = 0;
                 s_beg[wl][q] = cs;
             }
             int incl = cnt;
@@ -184,26 +262,42 @@ __global__ void __launch_bounds__(32 * kNbWarps, sizeof(T) == 4 ? 4 : 0) k_nb_ce
         const int total = carry;
         const int lo = a.cov_lo[i], hi = a.cov_hi[i];
         const bool lj = a.type != nullptr;
-        const int ti = lj ? a.type[i] : 0;
-        const T qi = a.qT[i];
+        T qi;
+        int ti = 0;
+        nb_rec_get(ri, qi, ti);
+        if (sizeof(T) == 8 && lj) ti = a.type[i];
         T g0 = T(0), g1 = T(0), g2 = T(0);
         T acc[11];  // per-lane sums of about 40 pairs, in kernel precision
 #pragma unroll
         for (int k = 0; k < 11; ++k) acc[k] = T(0);
+        int npair = 0;
         const unsigned lt = (1u << lane) - 1u;
         int qn = 0;  // queued kept candidates (warp-uniform)
         int qc = 0;
         for (int base = 0; base < total; base += 32) {
             const int t = base + lane;
             bool keep = false;
-            int j = -1;
+            int slot = 0, j = -1;
             if (t < total) {
                 while (t >= s_off[wl][qc + 1]) ++qc;
-                const float4 pj = a.posc[s_beg[wl][qc] + (t - s_off[wl][qc])];
+                slot = s_beg[wl][qc] + (t - s_off[wl][qc]);
+                const float4 pj = a.posc[slot];
                 j = __float_as_int(pj.w);
-                if (j != i) {
-                    const float d0 = pj.x - pix, d1 = pj.y - piy, d2 = pj.z - piz;
-                    bool amb = false;
+                const float d0 = pj.x - p4.x, d1 = pj.y - p4.y, d2 = pj.z - p4.z;
+                bool amb = false;
+                float r2;
+                if (ORTHO) {
+                    const float dd[3] = {d0, d1, d2};
+                    r2 = 0.f;
+#pragma unroll
+                    for (int q = 0; q < 3; ++q) {
+                        const float tt = dd[q] * hif[4 * q];
+                        const float sq = tt - floorf(tt + 0.5f);
+                        amb |= fabsf(sq) > 0.4999f;
+                        const float ev = sq * hf[4 * q];
+                        r2 = fmaf(ev, ev, r2);
+                    }
+                } else {
                     float sf[3];
 #pragma unroll
                     for (int q = 0; q < 3; ++q) {
@@ -214,14 +308,14 @@ __global__ void __launch_bounds__(32 * kNbWarps, sizeof(T) == 4 ? 4 : 0) k_nb_ce
                     const float e0 = sf[0] * hf[0] + sf[1] * hf[3] + sf[2] * hf[6];
                     const float e1 = sf[0] * hf[1] + sf[1] * hf[4] + sf[2] * hf[7];
                     const float e2 = sf[0] * hf[2] + sf[1] * hf[5] + sf[2] * hf[8];
-                    const float r2 = e0 * e0 + e1 * e1 + e2 * e2;
-                    if (!amb && r2 < rlo2) keep = true;
-                    else if (!amb && r2 > rhi2) keep = false;
-                    else keep = j > i ? within_rc(a.boxd, pi, a.pos + 3 * j, a.rc)
-                                      : within_rc(a.boxd, a.pos + 3 * j, pi, a.rc);
+                    r2 = e0 * e0 + e1 * e1 + e2 * e2;
                 }
+                if (!amb && r2 < rlo2) keep = true;
+                else if (!amb && r2 > rhi2) keep = false;
+                else keep = j > i ? within_rc(a.boxd, a.pos + 3 * i, a.pos + 3 * j, a.rc)
+                                  : within_rc(a.boxd, a.pos + 3 * j, a.pos + 3 * i, a.rc);
             }
-            if (keep) red[11] += 1.0;
+            if (keep) ++npair;
             // topologically scaled pairs belong to the FP64 covalent pass
             if (keep && j >= lo && j <= hi) {
                 const int nbd = j > i ? lookup_nbond(a.cov, i, j) : lookup_nbond(a.cov, j, i);
@@ -229,11 +323,11 @@ __global__ void __launch_bounds__(32 * kNbWarps, sizeof(T) == 4 ? 4 : 0) k_nb_ce
             }
             // queue the kept candidates; evaluate them 32 at a time with every lane busy
             const unsigned mk = __ballot_sync(0xffffffffu, keep);
-            if (keep) s_q[wl][qn + __popc(mk & lt)] = j;
+            if (keep) s_q[wl][qn + __popc(mk & lt)] = slot;
             qn += __popc(mk);
             __syncwarp();
             if (qn >= 32) {
-                nb_cell_pair<T>(a, i, s_q[wl][lane], pi, bxd, lj, ti, qi, g0, g1, g2, acc);
+                nb_cell_pair<T, ORTHO>(a, s_q[wl][lane], ri.x, ri.y, ri.z, lj, ti, qi, g0, g1, g2, acc);
                 __syncwarp();
                 if (lane < qn - 32) s_q[wl][lane] = s_q[wl][32 + lane];
                 qn -= 32;
@@ -241,17 +335,15 @@ __global__ void __launch_bounds__(32 * kNbWarps, sizeof(T) == 4 ? 4 : 0) k_nb_ce
             }
         }
         if (lane < qn)
-            nb_cell_pair<T>(a, i, s_q[wl][lane], pi, bxd, lj, ti, qi, g0, g1, g2, acc);
+            nb_cell_pair<T, ORTHO>(a, s_q[wl][lane], ri.x, ri.y, ri.z, lj, ti, qi, g0, g1, g2, acc);
 #pragma unroll
         for (int k = 0; k < 11; ++k) red[k] = (double)acc[k];
+        red[11] = (double)npair;
+        __syncwarp();
         g0 = warp_sum(g0);
         g1 = warp_sum(g1);
         g2 = warp_sum(g2);
-        if (lane == 0) {
-            atomicAdd(a.grad + 3 * i, g0);
-            atomicAdd(a.grad + 3 * i + 1, g1);
-            atomicAdd(a.grad + 3 * i + 2, g2);
-        }
+        if (lane == 0) nb_add(a.gcell + 4 * (int64_t)ks, g0, g1, g2);
     }
     block_reduce_add<12>(red, a.scal);
 }
