@@ -102,8 +102,7 @@ struct CgSolveArgs {
     // real-space matvec
     CsrArgs csr;
     const MvCoef<float>* coef;
-    const float* pos4;
-    BoxT<float> bxT;
+    Vec4<float>* p4;  // [n] the direction in FP32
     // spread / gather
     StencilCache<float> st;
     MeshGeom g;
@@ -190,7 +189,12 @@ __global__ void __launch_bounds__(kCgThreads) k_cg_solve(CgSolveArgs a) {
         double* acc = a.acc + 4 * (it & 3);
         // A: direction; clear the next iteration's scalars
         const double beta = rz2 != 0.0 ? rz1 / rz2 : 0.0;
-        for (int k = blockIdx.x * nth + tid; k < m3; k += nb * nth) a.p[k] = a.z[k] + beta * a.p[k];
+        for (int k = blockIdx.x * nth + tid; k < m3; k += nb * nth) {
+            const double pv = a.z[k] + beta * a.p[k];
+            a.p[k] = pv;
+            const int i = k / 3;
+            ((float*)(a.p4 + i))[k - 3 * i] = (float)pv;
+        }
         if (blockIdx.x == 0 && tid < 4) a.acc[4 * ((it + 1) & 3) + tid] = 0.0;
         if (!cg_grid_sync(a.bar, nb)) break;
         mark(0);
@@ -198,7 +202,7 @@ __global__ void __launch_bounds__(kCgThreads) k_cg_solve(CgSolveArgs a) {
         {
             double d[1] = {0.0};
             for (int w = gwarp; w < 2 * a.n; w += nwarps) {
-                if (w < a.n) d[0] += matvec_atom<float>(a.csr, a.coef, a.pos4, a.bxT, a.p, a.fmv, w, lane);
+                if (w < a.n) d[0] += matvec_atom<float>(a.csr, a.coef, a.p4, a.p, a.fmv, w, lane);
                 else spread_dip_atom<float>(sa, a.st, w - a.n, lane);
             }
             block_reduce_add<1>(d, acc + 1);

@@ -720,7 +720,7 @@ __global__ void __launch_bounds__(128) k_admp_pgrad(PgradArgs<T> g) {
 struct CsrArgs {
     int n;
     const int64_t* off;   // [n+1]
-    const int32_t* ent;   // packed (j, scale index)
+    int32_t* ent;         // packed (j, scale index); bit 31: see k_matvec_coef
 };
 
 __device__ __forceinline__ int scale_index(int nb) {
@@ -751,78 +751,16 @@ __global__ void k_csr_fill(int64_t npairs, const int32_t* pairs, int n, const in
     ent[off[j] + kj] = i | (s << 28);
 }
 
+// Matvec split in two: the pair tensors of every CSR entry are fixed during one dipole solve, so they
+// are evaluated once (k_matvec_coef) and each CG iteration only streams them (k_matvec_apply).  A pair
+// tensor is c0 1 + c1 e e^T (c0 = udud1, c1 = udud0 - udud1, e the pair direction); it is kept as c0 and
+// f = sqrt(|c1|) e, one vector load, with the sign of c1 in bit 31 of the entry.
 template <typename T>
-__global__ void __launch_bounds__(256) k_matvec_csr(PairArgs<T> a, CsrArgs c, double* out) {
-    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (w >= c.n) return;
-    const int i = w;
-    const T D = T(DMFFB_DIELECTRIC);
-    BoxT<T> bx;
-#pragma unroll
-    for (int k = 0; k < 9; ++k) { bx.h[k] = (T)a.boxd.h[k]; bx.hinv[k] = (T)a.boxd.hinv[k]; }
-    const T xi = a.pos[4 * i], yi = a.pos[4 * i + 1], zi = a.pos[4 * i + 2];
-    const T thi = a.thole[i], psi = a.polsix[i];
-    const T kap = a.kappa;
-    double acc0 = 0.0, acc1 = 0.0, acc2 = 0.0;
-    const int64_t beg = c.off[i], end = c.off[i + 1];
-    for (int64_t k = beg + lane; k < end; k += 32) {
-        const int e = c.ent[k];
-        const int j = e & 0x0FFFFFFF;
-        const int sidx = (e >> 28) & 7;
-        T dx = xi - a.pos[4 * j], dy = yi - a.pos[4 * j + 1], dz = zi - a.pos[4 * j + 2];
-        pbc_shift(bx, dx, dy, dz, (T*)nullptr);
-        const T r2 = dx * dx + dy * dy + dz * dz;
-        const T rinv = d_rsqrt(r2);
-        const T r = r2 * rinv;
-        const T ez0 = dx * rinv, ez1 = dy * rinv, ez2 = dz * rinv;
-        const T av = kap * r;
-        const T a2 = av * av;
-        const T X = T(DMFFB_TWO_OVER_SQRTPI) * d_exp(-a2);
-        const T t2 = av * X;
-        const T a3X = a2 * t2;
-        const T base = d_erfc(av) + t2 + T(2.0 / 3.0) * a3X;
-        const T pp = a.ps[sidx], dsv = a.dsc[sidx];
-        const T Ath = pp > T(0) ? T(5.0) : thi + a.thole[j];
-        T dmp = psi * a.polsix[j];
-        dmp = dmp < T(1e-8) ? T(1e-8) : dmp;
-        T u = r / dmp;
-        u = u < T(1e8) ? u : T(1e8);
-        const T au = Ath * u;
-        const T ev = au < T(50) ? d_exp(-au) : T(0);
-        const T Pc = T(1) + au + T(0.5) * au * au;
-        const T Pd0 = Pc + au * au * au * T(0.25);
-        const T bd0 = (dsv - T(1)) - dsv * ev * Pd0 + base;
-        const T bd1 = (dsv - T(1)) - dsv * ev * Pc + base;
-        const T r3 = rinv * rinv * rinv;
-        const T udud0 = T(-2.0 / 3.0) * D * r3 * (T(3) * bd0 + a3X);
-        const T udud1 = D * r3 * (bd1 - T(2.0 / 3.0) * a3X);
-        const double* U = a.U + 3 * j;
-        const T u0 = (T)U[0], u1 = (T)U[1], u2 = (T)U[2];
-        const T zu = ez0 * u0 + ez1 * u1 + ez2 * u2;
-        const T dd = (udud0 - udud1) * zu;
-        acc0 += (double)(udud1 * u0 + dd * ez0);
-        acc1 += (double)(udud1 * u1 + dd * ez1);
-        acc2 += (double)(udud1 * u2 + dd * ez2);
-    }
-    acc0 = warp_sum(acc0);
-    acc1 = warp_sum(acc1);
-    acc2 = warp_sum(acc2);
-    if (lane == 0) {
-        out[3 * i] = acc0;
-        out[3 * i + 1] = acc1;
-        out[3 * i + 2] = acc2;
-    }
-}
-
-
-// Matvec split in two: the pair tensors [udud1, udud0 - udud1, z] of every CSR entry are fixed
-// during one dipole solve, so they are evaluated once (k_matvec_coef) and each CG iteration only
-// streams them (k_matvec_apply).
-template <typename T>
-struct MvCoef {
-    T c[2];  // udud1, udud0 - udud1 (the pair direction is recomputed from the positions)
+struct __align__(4 * sizeof(T)) Vec4 {
+    T x, y, z, w;
 };
+template <typename T>
+using MvCoef = Vec4<T>;  // f.x, f.y, f.z, c0
 
 template <typename T>
 __global__ void __launch_bounds__(256) k_matvec_coef(PairArgs<T> a, CsrArgs c, MvCoef<T>* coef) {
@@ -868,35 +806,38 @@ __global__ void __launch_bounds__(256) k_matvec_coef(PairArgs<T> a, CsrArgs c, M
         const T r3 = rinv * rinv * rinv;
         const T udud0 = T(-2.0 / 3.0) * D * r3 * (T(3) * bd0 + a3X);
         const T udud1 = D * r3 * (bd1 - T(2.0 / 3.0) * a3X);
-        MvCoef<T> cf;
-        cf.c[0] = udud1;
-        cf.c[1] = udud0 - udud1;
-        coef[k] = cf;
+        const T c1 = udud0 - udud1, q = d_sqrt(c1 < T(0) ? -c1 : c1) * rinv;
+        coef[k] = MvCoef<T>{q * dx, q * dy, q * dz, udud1};
+        c.ent[k] = c1 < T(0) ? (e | (int)0x80000000) : (e & 0x7FFFFFFF);
     }
 }
 
-// The CG matvec streams 12 bytes per CSR entry (packed j + two coefficients); the pair
-// direction z is recomputed from the positions, which like U stay cache-resident.  One warp per
-// atom i: out_i = sum_j A_ij U_j; returns U_i . out_i in lane 0 (0 elsewhere).
+// The CG matvec streams 20 bytes per CSR entry (FP64 engines 36) and gathers the partners' dipoles as
+// one vector each from a copy in kernel precision (`p4`, ordinary loads: the persistent solve rewrites
+// it between grid barriers), which stays cache-resident.  One warp per
+// atom i: out_i = sum_j A_ij U_j, added up in FP64; returns U_i . out_i in lane 0 (0 elsewhere).
+// Bound by L2 (HBM once the entries outgrow it, at about 30000 atoms): 14 us at 12288 atoms and 2.6 M
+// entries, 39 us at 30000 and 6.4 M.  With 12 bytes per entry, the direction recomputed from gathered
+// positions and three FP64 dipole loads it took 24 and 54 us.
 template <typename T>
-__device__ __forceinline__ double matvec_atom(const CsrArgs& c, const MvCoef<T>* coef, const T* pos4,
-                                              const BoxT<T>& bx, const double* U, double* out, int i, int lane) {
-    const T xi = pos4[4 * i], yi = pos4[4 * i + 1], zi = pos4[4 * i + 2];
+__device__ __forceinline__ double matvec_atom(const CsrArgs& c, const MvCoef<T>* __restrict__ coef,
+                                              const Vec4<T>* p4, const double* U, double* out, int i,
+                                              int lane) {
     double acc0 = 0.0, acc1 = 0.0, acc2 = 0.0;
-    const int64_t beg = c.off[i], end = c.off[i + 1];
-    for (int64_t k = beg + lane; k < end; k += 32) {
-        const int j = c.ent[k] & 0x0FFFFFFF;
-        const MvCoef<T> cf = coef[k];
-        T dx = xi - pos4[4 * j], dy = yi - pos4[4 * j + 1], dz = zi - pos4[4 * j + 2];
-        pbc_shift(bx, dx, dy, dz, (T*)nullptr);
-        const T rinv = d_rsqrt(dx * dx + dy * dy + dz * dz);
-        const T ex = dx * rinv, ey = dy * rinv, ez = dz * rinv;
-        const double* Uj = U + 3 * j;
-        const T u0 = (T)Uj[0], u1 = (T)Uj[1], u2 = (T)Uj[2];
-        const T dd = cf.c[1] * (ex * u0 + ey * u1 + ez * u2);
-        acc0 += (double)(cf.c[0] * u0 + dd * ex);
-        acc1 += (double)(cf.c[0] * u1 + dd * ey);
-        acc2 += (double)(cf.c[0] * u2 + dd * ez);
+    const int64_t beg = c.off[i];
+    const int m = (int)(c.off[i + 1] - beg);
+    const int32_t* __restrict__ ent = c.ent + beg;
+    coef += beg;
+#pragma unroll 4
+    for (int k = lane; k < m; k += 32) {
+        const int e = ent[k];
+        const MvCoef<T> f = coef[k];
+        const Vec4<T> u = p4[e & 0x0FFFFFFF];
+        T dd = f.x * u.x + f.y * u.y + f.z * u.z;
+        dd = e < 0 ? -dd : dd;
+        acc0 += (double)(f.w * u.x + dd * f.x);
+        acc1 += (double)(f.w * u.y + dd * f.y);
+        acc2 += (double)(f.w * u.z + dd * f.z);
     }
     acc0 = warp_sum(acc0);
     acc1 = warp_sum(acc1);
@@ -910,15 +851,22 @@ __device__ __forceinline__ double matvec_atom(const CsrArgs& c, const MvCoef<T>*
 
 // With dot_out, sum_i U_i . out_i is reduced into *dot_out.
 template <typename T>
-__global__ void __launch_bounds__(256) k_matvec_apply(CsrArgs c, const MvCoef<T>* coef, const T* pos4, BoxT<T> bx,
+__global__ void __launch_bounds__(256) k_matvec_apply(CsrArgs c, const MvCoef<T>* coef, const Vec4<T>* p4,
                                                       const double* U, double* out, double* dot_out = nullptr) {
     const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     const bool active = w < c.n;
     if (!active && !dot_out) return;
     double d[1] = {0.0};
-    if (active) d[0] = matvec_atom<T>(c, coef, pos4, bx, U, out, w, lane);
+    if (active) d[0] = matvec_atom<T>(c, coef, p4, U, out, w, lane);
     if (dot_out) block_reduce_add<1>(d, dot_out);
+}
+
+// the dipoles in kernel precision, one vector per atom
+template <typename T>
+__global__ void k_pack_dipoles(int n, const double* U, Vec4<T>* p4) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) p4[i] = Vec4<T>{(T)U[3 * i], (T)U[3 * i + 1], (T)U[3 * i + 2], T(0)};
 }
 
 }  // namespace dmffb

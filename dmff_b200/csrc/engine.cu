@@ -97,6 +97,7 @@ struct dmffb_engine {
     bool csr_from_build = false;     // CSR built together with the internal pair list
     const int32_t* csr_pairs = nullptr;  // the half list the current CSR belongs to
     void* d_mvcoef = nullptr;  // [csr_cap] MvCoef<T>
+    void* d_p4 = nullptr;      // [n_cap] Vec4<T>: the matvec's dipoles in kernel precision
     int64_t mv_cap = 0;
     int32_t* d_pcount_f = nullptr;
     void* d_cub2 = nullptr;
@@ -458,8 +459,10 @@ __global__ void k_cg_update(int n, const double* s, int slot, double* x, double*
     block_reduce_add<1>(w, rr);
 }
 
-// with ctr (the CG step counter, not yet advanced for this step), slot_new = *ctr mod 2
-__global__ void k_cg_p(int n, const double* s, int slot_old, int slot_new, const double* z, double* p,
+// with ctr (the CG step counter, not yet advanced for this step), slot_new = *ctr mod 2; p4: the
+// direction in kernel precision for the matvec
+template <typename T>
+__global__ void k_cg_p(int n, const double* s, int slot_old, int slot_new, const double* z, double* p, Vec4<T>* p4,
                        double* zero = nullptr, const unsigned long long* ctr = nullptr) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (ctr) {
@@ -469,7 +472,10 @@ __global__ void k_cg_p(int n, const double* s, int slot_old, int slot_new, const
     if (k == 0 && zero) *zero = 0.0;
     if (k >= 3 * n) return;
     const double beta = s[slot_old] != 0.0 ? s[slot_new] / s[slot_old] : 0.0;
-    p[k] = z[k] + beta * p[k];
+    const double pv = z[k] + beta * p[k];
+    p[k] = pv;
+    const int i = k / 3;
+    ((T*)(p4 + i))[k - 3 * i] = (T)pv;
 }
 
 __global__ void k_ref_step(int n, const double* f, const double* pol, double* U, double* maxf) {
@@ -983,7 +989,7 @@ int cg_matvec_fused(dmffb_engine* h, cudaStream_t s, const Box& bx, double* sc) 
     sa.zero_scal[0] = sc + 2;
     sa.zero_scal[1] = sc + 3;
     sa.ctr_inc = ctr;
-    LAUNCH(h, s, KC_VEC, k_cg_p<<<nblk(3 * h->n, 256), 256, 0, s>>>(h->n, sc, 1, 0, h->d_z, h->d_p, sc + 5, ctr));
+    LAUNCH(h, s, KC_VEC, k_cg_p<T><<<nblk(3 * h->n, 256), 256, 0, s>>>(h->n, sc, 1, 0, h->d_z, h->d_p, (Vec4<T>*)h->d_p4, sc + 5, ctr));
     const bool fork = h->s2 && !h->prof;
     {
         CsrArgs c;
@@ -997,7 +1003,7 @@ int cg_matvec_fused(dmffb_engine* h, cudaStream_t s, const Box& bx, double* sc) 
             sm = h->s2;
         }
         LAUNCH(h, sm, KC_PAIR_MATVEC, k_matvec_apply<T><<<nblk((int64_t)h->n * 32, 256), 256, 0, sm>>>(
-                                          c, (const MvCoef<T>*)h->d_mvcoef, (const T*)h->d_posT, boxT<T>(bx), h->d_p, h->d_fmv,
+                                          c, (const MvCoef<T>*)h->d_mvcoef, (const Vec4<T>*)h->d_p4, h->d_p, h->d_fmv,
                                           sc + 5));
         if (fork) CK(cudaEventRecord(h->e_join, h->s2));
     }
@@ -1031,6 +1037,7 @@ int matvec_alloc(dmffb_engine* h) {
         h->mv_cap = h->csr_cap;
         if ((st = dalloc(h, &h->d_mvcoef, h->mv_cap * sizeof(MvCoef<T>)))) return st;
     }
+    if (!h->d_p4 && (st = dalloc(h, &h->d_p4, (size_t)h->n_cap * sizeof(Vec4<T>)))) return st;
     return DMFFB_OK;
 }
 
@@ -1133,8 +1140,9 @@ int field_eval(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx
         c.off = h->d_csr_off;
         c.ent = h->d_csr_ent;
         cudaStream_t sm = sr;
+        LAUNCH(h, sm, KC_VEC, k_pack_dipoles<T><<<nblk(h->n, 256), 256, 0, sm>>>(h->n, U, (Vec4<T>*)h->d_p4));
         LAUNCH(h, sm, KC_PAIR_MATVEC, k_matvec_apply<T><<<nblk((int64_t)h->n * 32, 256), 256, 0, sm>>>(
-                                          c, (const MvCoef<T>*)h->d_mvcoef, (const T*)h->d_posT, boxT<T>(bx), U, h->d_fmv));
+                                          c, (const MvCoef<T>*)h->d_mvcoef, (const Vec4<T>*)h->d_p4, U, h->d_fmv));
     }
     if (fork) CK(cudaEventRecord(h->e_join, h->s2));
     const double* recip = nullptr;
@@ -1181,8 +1189,7 @@ int cg_persistent(dmffb_engine* h, cudaStream_t s, const Box& bx, double* U, con
     a.csr.off = h->d_csr_off;
     a.csr.ent = h->d_csr_ent;
     a.coef = (const MvCoef<float>*)h->d_mvcoef;
-    a.pos4 = (const float*)h->d_posT;
-    a.bxT = boxT<float>(bx);
+    a.p4 = (Vec4<float>*)h->d_p4;
     a.st = stencil_cache<float>(h);
     a.g = mesh_geom(bx, h->K);
     a.perm_mul = h->perm_mul;
@@ -1323,7 +1330,7 @@ int solve_dipoles(dmffb_engine* h, cudaStream_t s, const double* pos, const Box&
         if ((st2 = field_eval<T>(h, s, pos, bx, pairs, npairs, h->d_p, false, h->d_Ap, h->d_p, sc + 2, zs))) return st2;
         LAUNCH(h, s, KC_VEC, k_cg_update<<<nb3, 256, 0, s>>>(n, sc, slot, U, h->d_r, h->d_z, h->d_p, h->d_Ap,
                                                            h->d_pol, sc + (1 - slot), sc + 3));
-        LAUNCH(h, s, KC_VEC, k_cg_p<<<nb3, 256, 0, s>>>(n, sc, slot, 1 - slot, h->d_z, h->d_p));
+        LAUNCH(h, s, KC_VEC, k_cg_p<T><<<nb3, 256, 0, s>>>(n, sc, slot, 1 - slot, h->d_z, h->d_p, (Vec4<T>*)h->d_p4));
         return DMFFB_OK;
     };
     // two iterations (slot 0 then 1) are captured once into a CUDA graph and replayed; the graph
@@ -2619,7 +2626,7 @@ void dmffb_destroy(dmffb_engine* h) {
     void* ptrs[] = {h->d_axis_type, h->d_axis_idx, h->d_cov_ptr, h->d_cov_j, h->d_cov_nb, h->d_Qloc, h->d_pol,
                     h->d_thole, h->d_polsix, h->d_pos, h->d_U, h->d_forces, h->d_posT, h->d_Qg, h->d_QgT,
                     h->d_gpair, h->d_torque, h->d_fieldT, h->d_grad, h->d_scal, h->d_b, h->d_r, h->d_z, h->d_p,
-                    h->d_Ap, h->d_fr, h->d_gQ, h->d_fmv, h->d_pcount_f, h->d_pcount_s, h->d_poff_s, h->d_rank, h->d_bin_done, h->d_nbsum, h->d_mvcoef, h->d_csr_off, h->d_csr_ent, h->d_csr_deg, h->d_cub2, h->d_grid, h->d_grid2, h->d_cgrid, h->d_bmod, h->d_pairs, h->d_atom_cell,
+                    h->d_Ap, h->d_fr, h->d_gQ, h->d_fmv, h->d_pcount_f, h->d_pcount_s, h->d_poff_s, h->d_rank, h->d_bin_done, h->d_nbsum, h->d_mvcoef, h->d_p4, h->d_csr_off, h->d_csr_ent, h->d_csr_deg, h->d_cub2, h->d_grid, h->d_grid2, h->d_cgrid, h->d_bmod, h->d_pairs, h->d_atom_cell,
                     h->d_cell_count, h->d_cell_start, h->d_pcount, h->d_poff,
                     h->d_c, h->d_tta, h->d_ttb, h->d_ttq, h->d_glr, h->d_gsr, h->d_dc,
                     h->d_q, h->d_qT, h->d_type, h->d_sigtt, h->d_epstt, h->d_dq, h->d_dsig, h->d_deps,
