@@ -3,23 +3,25 @@
 //
 // The dipole solve of the reference (pme.py:342-423 solves A U = -E_perm by fixed-point steps;
 // the engine uses preconditioned CG on the same linear system) repeats, per iteration, a chain of
-// dependent passes on data that sits in L2: direction update, real-space matvec and dipole spread,
-// 3-D FFT, influence multiply, inverse FFT, field gather, CG update.  Launched one kernel per pass
-// (and the convergence test on the host every few iterations), a small box spends ~60 us per
-// iteration in launch gaps and host round trips.  Here one cooperative grid runs every iteration
-// and decides convergence on the device; the passes are separated by a grid barrier:
-//   A  p = z + beta p                                   (beta = rz_k-1 / rz_k-2)
-//   B  matvec warps (fmv = A_real p, p . fmv) and spread warps (p onto the mesh)
+// dependent passes on data that sits in L2: vector update and dipole spread, 3-D transform, influence
+// multiply, inverse transform, field gather, with the real-space matvec beside them.  CG is taken in
+// its form with one synchronisation per iteration (Chronopoulos and Gear 1989: w = A u of the
+// preconditioned residual u gives gamma = r.u and delta = u.w, from which alpha and beta follow, and
+// s = A p is carried along as s = w + beta s), so that the update of an atom's vectors is local to the
+// warp that spreads it and the real-space matvec can share the pass of the gather.  Launched one
+// kernel per pass, a small box spends most of an iteration in launch gaps and host round trips.
+// Here one cooperative grid runs every iteration and decides convergence on the device; the passes
+// are separated by a grid barrier:
+//   B  p = u + beta p, s = w + beta s, x += alpha p, r -= alpha s, u = M r, u onto the mesh; r.u, r.r
 //   C  forward x-plane DFT passes        D  spectrum columns (x DFT, * G, inverse x DFT)
-//   E  inverse x-plane DFT passes        F  field gather (Ap, p . Ap)
-//   G  alpha = rz / pAp, x += alpha p, r -= alpha (Ap + fmv), z = M r, rz and rr reduced
+//   E  inverse x-plane DFT passes        F  real-space matvec, field gather and diagonal (w = A u), u.w
 // (with phase_ns set, block 0 adds the device-clock time of each pass, barrier included)
-// then rr decides: stop when sqrt(rr / 3n) <= tol sqrt(bb / 3n) or at max_iter.
+// Measured per iteration at 450 / 3999 / 12288 atoms, seven passes and classic CG before: 26 / 35 / 62 us,
+// these five passes 22 / 32 / 61.
 //
-// The four reduced scalars of iteration k accumulate in slot k mod 4 of acc[4][4] and are read
-// after the barriers of iteration k (each CTA keeps the rz of the two previous iterations in
-// registers); slot k + 1 is cleared in pass A of iteration k, three iterations after its last
-// reads.
+// The three sums of iteration k (u.w, r.u, r.r) accumulate in slot k mod 4 of acc[4][4] and are read
+// after the barriers of iteration k; slot k + 1 is cleared in pass C of iteration k, three
+// iterations after its last reads.
 //
 // The grid barrier is an arrival counter and a generation word (release on arrival, acquire on
 // the wait).  Every wait is bounded by the device clock: past `wait_ns` the CTA records
@@ -35,7 +37,7 @@
 
 namespace dmffb {
 
-constexpr int kCgThreads = 512;
+constexpr int kCgThreads = 512;  // 1024 (64 registers, spills) takes 28 us per iteration at 450 atoms against 22
 constexpr int DMFFB_CG_TIMEOUT = 1;    // a grid barrier wait ran out
 constexpr int DMFFB_CG_NONFINITE = 2;  // non-finite residual
 
@@ -94,15 +96,70 @@ __device__ inline bool cg_grid_sync(const CgBarrier& b, unsigned nblocks) {
     return s_ok != 0;
 }
 
+// The vectors of the single-synchronisation CG, FP64 [3n]: solution, residual, u = M r, direction p and
+// s = A p; w = A u, in two parts (reciprocal + diagonal, real space) or whole in Ap (fmv null).
+struct CgVectors {
+    double *x, *r, *u, *p, *s;
+    const double *Ap, *fmv;
+    const double* pol;  // [n]
+};
+
+// alpha and beta of an iteration from its sums and the previous ones (0: first iteration)
+__device__ __forceinline__ void cg_coefs(double gamma, double gamma_prev, double delta, double alpha_prev, double& alpha,
+                                         double& beta) {
+    beta = gamma_prev != 0.0 ? gamma / gamma_prev : 0.0;
+    const double den = delta - (alpha_prev != 0.0 ? beta * gamma / alpha_prev : 0.0);
+    alpha = den != 0.0 ? gamma / den : 0.0;
+}
+
+// The vector update of component c of atom `at`: leaves u and its copy in kernel precision, adds to the
+// sums r.u and r.r, returns u.  The first iteration (beta 0) does not read p and s.
+template <typename T>
+__device__ __forceinline__ double cg_update(const CgVectors& v, Vec4<T>* p4, double alpha, double beta, int at, int c,
+                                            double& ru, double& rr) {
+    const int k = 3 * at + c;
+    double pp = v.pol[at];
+    pp = pp < 1e-8 ? 1e-8 : pp;
+    const double w = v.fmv ? v.Ap[k] + v.fmv[k] : v.Ap[k];
+    const double p = beta != 0.0 ? v.u[k] + beta * v.p[k] : v.u[k];
+    const double s = beta != 0.0 ? w + beta * v.s[k] : w;
+    const double r = v.r[k] - alpha * s, u = r * pp / DMFFB_DIELECTRIC;
+    v.p[k] = p;
+    v.s[k] = s;
+    v.x[k] += alpha * p;
+    v.r[k] = r;
+    v.u[k] = u;
+    ((T*)(p4 + at))[c] = (T)u;
+    ru += r * u;
+    rr += r * r;
+    return u;
+}
+
+// The per-pass solve's vector update, one thread per component.  Folding the next spread into it, a warp
+// per atom, took 16 us at 12288 atoms and 30 at 30000 against 3 + 7.5 and 3.5 + 15.5 for the two
+// launches: three lanes of a warp wait for the vectors where here all threads do.
+template <typename T>
+__global__ void __launch_bounds__(256) k_cg_update1(int n, CgVectors v, Vec4<T>* p4, double* sc) {
+    double alpha, beta;
+    cg_coefs(sc[CGS_RU], sc[CGS_RU_PREV], sc[CGS_UW], sc[CGS_ALPHA_PREV], alpha, beta);
+    double sum[2] = {0.0, 0.0}, rr[1];
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < 3 * n) cg_update<T>(v, p4, alpha, beta, k / 3, k % 3, sum[0], sum[1]);
+    if (k == 0) sc[CGS_ALPHA] = alpha;
+    rr[0] = sum[1];
+    double ru[1] = {sum[0]};
+    block_reduce_add<1>(ru, sc + CGS_RU_NEW);
+    block_reduce_add<1>(rr, sc + CGS_RR);
+}
+
 struct CgSolveArgs {
     int n;
-    // CG vectors [3n] (double) and the polarizabilities [n]
-    double *x, *r, *z, *p, *Ap, *fmv;
-    const double* pol;
+    CgVectors v;
+    double *Ap, *fmv;  // the two parts of w
     // real-space matvec
     CsrArgs csr;
     const MvCoef<float>* coef;
-    Vec4<float>* p4;  // [n] the direction in FP32
+    Vec4<float>* p4;  // [n] u in FP32
     // spread / gather
     StencilCache<float> st;
     MeshGeom g;
@@ -112,8 +169,8 @@ struct CgSolveArgs {
     // convolution (grid_in: the spread mesh, grid_out: the convolved mesh)
     DftConvArgs<float> fc;
     // scalars
-    double* acc;         // [4][4] {p.Ap recip, p.fmv, rz, rr}, zero at launch
-    const double* init;  // [0] r.z, [3] r.r, [4] b.b of the initial residual
+    double* acc;         // [4][4] {u.w, r.u, r.r, -}, zero at launch
+    const double* init;  // CGS_RU_NEW, CGS_RR and CGS_BB of the initial residual
     double tol;
     int max_iter;
     CgBarrier bar;
@@ -144,25 +201,14 @@ __global__ void __launch_bounds__(kCgThreads) k_cg_solve(CgSolveArgs a) {
     const int warps_cta = nth >> 5;
     const int gwarp = blockIdx.x * warps_cta + (tid >> 5), nwarps = nb * warps_cta;
     const int m3 = 3 * a.n;
-    SpreadArgs<float> sa;
-    sa.n = a.n;
-    sa.pos = nullptr;
-    sa.Qg = nullptr;
-    sa.U = a.p;
-    sa.q1 = nullptr;
-    sa.lmax = 1;
-    sa.g = a.g;
-    sa.grid = a.fc.zero_real;
-    sa.perm_mul = a.perm_mul;
     FieldCombine cmb;
-    cmb.U = a.p;
-    cmb.pol = a.pol;
+    cmb.U = a.v.u;
+    cmb.pol = a.v.pol;
     cmb.self1 = a.self1;
-    cmb.dot_out = a.acc;  // only tested for non-null; the sum goes through block_reduce_add
-    const double rms_b = sqrt(a.init[4] / (double)m3);
-    double rr = a.init[3];
+    const double rms_b = sqrt(a.init[CGS_BB] / (double)m3);
+    double rr = a.init[CGS_RR];
     int it = 0, conv = 0, status = 0;
-    double rz1 = a.init[0], rz2 = 0.0;  // rz of iterations k - 1 and k - 2
+    double ru = a.init[CGS_RU_NEW], ru_prev = 0.0, alpha_prev = 0.0;
     const int nfwd = dft_fwd_items(a.fc), ncol = dft_col_items(a.fc), ninv = dft_inv_items(a.fc);
     const int K3 = a.fc.K[0] * a.fc.K[1] * a.fc.K[2];
     // pass timing on block 0 (device clock at each barrier exit)
@@ -175,7 +221,15 @@ __global__ void __launch_bounds__(kCgThreads) k_cg_solve(CgSolveArgs a) {
             tp = t;
         }
     };
-    while (true) {
+    // the initial u onto the mesh
+    for (int w = gwarp; w < a.n; w += nwarps) {
+        const int at = (int)(((int64_t)w * a.perm_mul) % a.n);
+        spread_dip_atom<float>(a.g, a.fc.zero_real, a.st, at, lane, (float)a.v.u[3 * at], (float)a.v.u[3 * at + 1],
+                               (float)a.v.u[3 * at + 2]);
+    }
+    bool ok = cg_grid_sync(a.bar, nb);
+    mark(1);
+    while (ok) {
         const double rms = sqrt(rr / (double)m3);
         if (!isfinite(rms)) {
             status = DMFFB_CG_NONFINITE;
@@ -187,28 +241,7 @@ __global__ void __launch_bounds__(kCgThreads) k_cg_solve(CgSolveArgs a) {
         }
         if (it >= a.max_iter) break;
         double* acc = a.acc + 4 * (it & 3);
-        // A: direction; clear the next iteration's scalars
-        const double beta = rz2 != 0.0 ? rz1 / rz2 : 0.0;
-        for (int k = blockIdx.x * nth + tid; k < m3; k += nb * nth) {
-            const double pv = a.z[k] + beta * a.p[k];
-            a.p[k] = pv;
-            const int i = k / 3;
-            ((float*)(a.p4 + i))[k - 3 * i] = (float)pv;
-        }
         if (blockIdx.x == 0 && tid < 4) a.acc[4 * ((it + 1) & 3) + tid] = 0.0;
-        if (!cg_grid_sync(a.bar, nb)) break;
-        mark(0);
-        // B: real-space matvec warps [0, n), spread warps [n, 2n)
-        {
-            double d[1] = {0.0};
-            for (int w = gwarp; w < 2 * a.n; w += nwarps) {
-                if (w < a.n) d[0] += matvec_atom<float>(a.csr, a.coef, a.p4, a.p, a.fmv, w, lane);
-                else spread_dip_atom<float>(sa, a.st, w - a.n, lane);
-            }
-            block_reduce_add<1>(d, acc + 1);
-        }
-        if (!cg_grid_sync(a.bar, nb)) break;
-        mark(1);
         // C, D, E: the convolution
         for (int w = blockIdx.x; w < nfwd; w += nb) {
             dft_fwd_item<float, 1, 1>(a.fc, w, sm, wy, wz);
@@ -232,38 +265,36 @@ __global__ void __launch_bounds__(kCgThreads) k_cg_solve(CgSolveArgs a) {
         }
         if (!cg_grid_sync(a.bar, nb)) break;
         mark(4);
-        // F: field gather, Ap = recip field of p + (1/pol + self) p
+        // F: real-space matvec and field gather, Ap = recip field of u + (1/pol + self) u
         {
-            double d[1] = {0.0};
-            for (int w = gwarp; w < a.n; w += nwarps)
-                d[0] += gather_field_atom<float>(a.st, a.g, a.fc.grid_out, a.gscale, a.Ap, cmb, w, lane);
-            block_reduce_add<1>(d, acc + 0);
+            double uw[1] = {0.0};
+            for (int w = gwarp; w < 2 * a.n; w += nwarps)
+                uw[0] += w < a.n ? matvec_atom<float>(a.csr, a.coef, a.p4, a.v.u, a.fmv, w, lane)
+                                 : gather_field_atom<float>(a.st, a.g, a.fc.grid_out, a.gscale, a.Ap, cmb, w - a.n, lane);
+            block_reduce_add<1>(uw, acc);
         }
         if (!cg_grid_sync(a.bar, nb)) break;
         mark(5);
-        // G: update
+        // B: update and spread
+        double alpha, beta;
+        cg_coefs(ru, ru_prev, acc[0], alpha_prev, alpha, beta);
         {
-            const double pAp = acc[0] + acc[1];
-            const double alpha = pAp != 0.0 ? rz1 / pAp : 0.0;
-            double v[2] = {0.0, 0.0};
-            for (int k = blockIdx.x * nth + tid; k < m3; k += nb * nth) {
-                double pp = a.pol[k / 3];
-                pp = pp < 1e-8 ? 1e-8 : pp;
-                a.x[k] += alpha * a.p[k];
-                const double rv = a.r[k] - alpha * (a.Ap[k] + a.fmv[k]);
-                a.r[k] = rv;
-                const double zv = rv * pp / DMFFB_DIELECTRIC;
-                a.z[k] = zv;
-                v[0] += rv * zv;
-                v[1] += rv * rv;
+            double sum[2] = {0.0, 0.0};
+            for (int w = gwarp; w < a.n; w += nwarps) {
+                const int at = (int)(((int64_t)w * a.perm_mul) % a.n);
+                const float u =
+                    lane < 3 ? (float)cg_update<float>(a.v, a.p4, alpha, beta, at, lane, sum[0], sum[1]) : 0.f;
+                spread_dip_atom<float>(a.g, a.fc.zero_real, a.st, at, lane, __shfl_sync(0xffffffffu, u, 0),
+                                       __shfl_sync(0xffffffffu, u, 1), __shfl_sync(0xffffffffu, u, 2));
             }
-            block_reduce_add<2>(v, acc + 2);
+            block_reduce_add<2>(sum, acc + 1);
         }
         if (!cg_grid_sync(a.bar, nb)) break;
-        mark(6);
-        rz2 = rz1;
-        rz1 = acc[2];
-        rr = acc[3];
+        mark(1);
+        ru_prev = ru;
+        alpha_prev = alpha;
+        ru = acc[1];
+        rr = acc[2];
         ++it;
     }
     if (blockIdx.x == 0 && tid == 0) {

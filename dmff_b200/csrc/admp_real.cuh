@@ -849,17 +849,11 @@ __device__ __forceinline__ double matvec_atom(const CsrArgs& c, const MvCoef<T>*
     return U[3 * i] * acc0 + U[3 * i + 1] * acc1 + U[3 * i + 2] * acc2;
 }
 
-// With dot_out, sum_i U_i . out_i is reduced into *dot_out.
 template <typename T>
 __global__ void __launch_bounds__(256) k_matvec_apply(CsrArgs c, const MvCoef<T>* coef, const Vec4<T>* p4,
-                                                      const double* U, double* out, double* dot_out = nullptr) {
+                                                      const double* U, double* out) {
     const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    const bool active = w < c.n;
-    if (!active && !dot_out) return;
-    double d[1] = {0.0};
-    if (active) d[0] = matvec_atom<T>(c, coef, p4, U, out, w, lane);
-    if (dot_out) block_reduce_add<1>(d, dot_out);
+    if (w < c.n) matvec_atom<T>(c, coef, p4, U, out, w, threadIdx.x & 31);
 }
 
 // the dipoles in kernel precision, one vector per atom

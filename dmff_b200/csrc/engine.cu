@@ -37,8 +37,8 @@ enum {
     S_RECIP = 16,   // [0] energy, [1..6] k-space tensor (conv kernel)
     S_GATHER = 24,  // [0] energy check, [1..9] X_NA
     S_SELF = 40,    // [0] E_self, [1] E_pol, [2..10] frame box grad
-    S_CG = 56,      // CG scalars
-    N_SCAL = 80
+    S_CG = 56,      // CG scalars, the step count and the last residuals
+    N_SCAL = 56 + 8 + 1 + 32 + 7
 };
 
 }  // namespace
@@ -73,7 +73,7 @@ struct dmffb_engine {
     void* d_fieldT = nullptr;
     double* d_grad = nullptr;
     double* d_scal = nullptr;
-    double *d_b = nullptr, *d_r = nullptr, *d_z = nullptr, *d_p = nullptr, *d_Ap = nullptr, *d_fr = nullptr;
+    double *d_b = nullptr, *d_r = nullptr, *d_z = nullptr, *d_p = nullptr, *d_Ap = nullptr, *d_fr = nullptr, *d_s = nullptr;
     double* d_gQ = nullptr;
     double* d_fmv = nullptr;  // CSR matvec output [3n]
     // slots of the single-pass neighbour build: capacities per atom, first from the mean density,
@@ -104,6 +104,8 @@ struct dmffb_engine {
     size_t cub2_bytes = 0;
     void* d_grid = nullptr;
     void* d_grid2 = nullptr;  // spread target of the dipole-only field pass, kept zero between passes
+    int cg_hint = 0;           // steps that the next dipole solve from U = 0 takes before its first read
+    bool grid2_dirty = false;  // the persistent solve has left its last spread there
     void* d_cgrid = nullptr;
     double* d_bmod = nullptr;
     cufftHandle plan_f = 0, plan_b = 0;
@@ -404,51 +406,39 @@ __global__ void k_field_combine(int n, const double* recip, const T* fT, const d
     if (dot_out) block_reduce_add<1>(d, dot_out);
 }
 
-// CG helpers; scalars live in s[]: [0] rz(even) [1] rz(odd) [2] pAp [3] rr
-__global__ void k_dot2(int m, const double* a, const double* b, const double* c, const double* d, double* s0,
-                       double* s1) {
+// r = -(b + A x), z = M r, p = z and z in kernel precision; r.z, r.r and b.b into their scalars
+template <typename T>
+__global__ void k_cg_init(int n, const double* b, const double* Ax, const double* pol, double* r, double* z, double* p,
+                          Vec4<T>* p4, double* sc) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    double v0[1] = {0.0}, v1[1] = {0.0};
-    if (k < m) {
-        v0[0] = a[k] * b[k];
-        if (c) v1[0] = c[k] * d[k];
+    double v[CGS_COUNT] = {0, 0, 0, 0, 0, 0, 0, 0};
+    if (k < 3 * n) {
+        const int i = k / 3;
+        double pp = pol[i];
+        pp = pp < 1e-8 ? 1e-8 : pp;
+        const double rv = -(b[k] + (Ax ? Ax[k] : 0.0)), zv = rv * pp / DMFFB_DIELECTRIC;
+        r[k] = rv;
+        z[k] = zv;
+        p[k] = zv;
+        ((T*)(p4 + i))[k - 3 * i] = (T)zv;
+        v[CGS_RU_NEW] = rv * zv;
+        v[CGS_RR] = rv * rv;
+        v[CGS_BB] = b[k] * b[k];
     }
-    block_reduce_add<1>(v0, s0);
-    if (s1) block_reduce_add<1>(v1, s1);
+    block_reduce_add<CGS_COUNT>(v, sc);
 }
 
-__global__ void k_cg_init(int n, const double* b, const double* Ax, const double* pol, double* r, double* z,
-                          double* p) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= 3 * n) return;
-    double pp = pol[k / 3];
-    pp = pp < 1e-8 ? 1e-8 : pp;
-    const double rv = -(b[k] + (Ax ? Ax[k] : 0.0));
-    r[k] = rv;
-    z[k] = rv * pp / DMFFB_DIELECTRIC;
-    p[k] = z[k];
-}
-
-// Ap may come in two parts (Ap + Ap2, p.Ap = s[2] + s[5]); s[5] stays 0 when Ap2 is null.
-// With ctr (the CG step counter, already advanced for this step), slot = (*ctr - 1) mod 2 and
-// rz_new points at the slot pair s[0..1], this step's r.z going to rz_new[1 - slot].
+// Classic CG without a reciprocal part; scalars s[]: [0] rz(even) [1] rz(odd) [2] pAp [3] rr
 __global__ void k_cg_update(int n, const double* s, int slot, double* x, double* r, double* z, const double* p,
-                            const double* Ap, const double* pol, double* rz_new, double* rr,
-                            const double* Ap2 = nullptr, const unsigned long long* ctr = nullptr) {
+                            const double* Ap, const double* pol, double* rz_new, double* rr) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (ctr) {
-        slot = (int)((*ctr - 1ull) & 1ull);
-        rz_new += 1 - slot;
-    }
-    const double pAp = s[2] + s[5];
-    const double alpha = pAp != 0.0 ? s[slot] / pAp : 0.0;
+    const double alpha = s[2] != 0.0 ? s[slot] / s[2] : 0.0;
     double v[1] = {0.0}, w[1] = {0.0};
     if (k < 3 * n) {
         double pp = pol[k / 3];
         pp = pp < 1e-8 ? 1e-8 : pp;
         x[k] += alpha * p[k];
-        const double ap = Ap2 ? Ap[k] + Ap2[k] : Ap[k];
-        const double rv = r[k] - alpha * ap;
+        const double rv = r[k] - alpha * Ap[k];
         r[k] = rv;
         const double zv = rv * pp / DMFFB_DIELECTRIC;
         z[k] = zv;
@@ -459,23 +449,11 @@ __global__ void k_cg_update(int n, const double* s, int slot, double* x, double*
     block_reduce_add<1>(w, rr);
 }
 
-// with ctr (the CG step counter, not yet advanced for this step), slot_new = *ctr mod 2; p4: the
-// direction in kernel precision for the matvec
-template <typename T>
-__global__ void k_cg_p(int n, const double* s, int slot_old, int slot_new, const double* z, double* p, Vec4<T>* p4,
-                       double* zero = nullptr, const unsigned long long* ctr = nullptr) {
+__global__ void k_cg_p(int n, const double* s, int slot_old, int slot_new, const double* z, double* p) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (ctr) {
-        slot_new = (int)(*ctr & 1ull);
-        slot_old = 1 - slot_new;
-    }
-    if (k == 0 && zero) *zero = 0.0;
     if (k >= 3 * n) return;
     const double beta = s[slot_old] != 0.0 ? s[slot_new] / s[slot_old] : 0.0;
-    const double pv = z[k] + beta * p[k];
-    p[k] = pv;
-    const int i = k / 3;
-    ((T*)(p4 + i))[k - 3 * i] = (T)pv;
+    p[k] = z[k] + beta * p[k];
 }
 
 __global__ void k_ref_step(int n, const double* f, const double* pol, double* U, double* maxf) {
@@ -882,6 +860,19 @@ int stencil_prep(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& 
     return DMFFB_OK;
 }
 
+CgVectors cg_vectors(const dmffb_engine* h, double* U, bool parts) {
+    CgVectors v;
+    v.x = U;
+    v.r = h->d_r;
+    v.u = h->d_z;
+    v.p = h->d_p;
+    v.s = h->d_s;
+    v.Ap = h->d_Ap;
+    v.fmv = parts ? h->d_fmv : nullptr;
+    v.pol = h->d_pol;
+    return v;
+}
+
 template <typename T>
 StencilCache<T> stencil_cache(dmffb_engine* h) {
     StencilCache<T> c;
@@ -894,7 +885,7 @@ StencilCache<T> stencil_cache(dmffb_engine* h) {
 // transform -> gather
 template <typename T>
 int recip_pass(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx, bool use_Qg, const double* U,
-               int mode, double* field_out, double* const* zero_scal = nullptr) {
+               int mode, double* field_out) {
     const MeshGeom g = mesh_geom(bx, h->K);
     const int64_t K3 = (int64_t)h->K[0] * h->K[1] * h->K[2];
     // the dipole-only field pass (the CG matvec) spreads into d_grid2, which the convolution
@@ -902,6 +893,10 @@ int recip_pass(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx
     const bool dip = mode == GATHER_FIELD && !use_Qg && U;
     void* spread_grid = dip ? h->d_grid2 : h->d_grid;
     if (!dip) CK(cudaMemsetAsync(h->d_grid, 0, K3 * sizeof(T), s));
+    if (dip && h->grid2_dirty) {
+        CK(cudaMemsetAsync(h->d_grid2, 0, K3 * sizeof(T), s));
+        h->grid2_dirty = false;
+    }
     SpreadArgs<T> sa;
     sa.n = h->n;
     sa.pos = pos;
@@ -912,15 +907,9 @@ int recip_pass(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx
     sa.g = g;
     sa.grid = (T*)spread_grid;
     sa.perm_mul = h->perm_mul;
-    if (zero_scal)
-        for (int k = 0; k < 3; ++k) sa.zero_scal[k] = zero_scal[k];
     if (dip && h->stencils_ready) {
-        LAUNCH(h, s, KC_SPREAD, k_spread_dip_cached<T><<<nblk((int64_t)h->n * 32, 256), 256, 0, s>>>(sa, stencil_cache<T>(h)));
+        LAUNCH(h, s, KC_SPREAD, k_spread_dip_cached<T><<<nblk((int64_t)h->n * 32, 256), 256, 0, s>>>(sa, stencil_cache<T>(h), nullptr));
     } else {
-        // the general spread (dipoles alone when Qg is null) clears no scalars itself
-        if (zero_scal)
-            for (int k = 0; k < 3; ++k)
-                if (zero_scal[k]) CK(cudaMemsetAsync(zero_scal[k], 0, sizeof(double), s));
         const int apc = sites_per_cta(h->n);
         LAUNCH(h, s, KC_SPREAD, k_spread<T, false><<<nblk(h->n, apc), kSiteThreads, 0, s>>>(sa, apc));
     }
@@ -933,7 +922,7 @@ int recip_pass(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx
     if (st) return st;
     if (mode == GATHER_FIELD) {
         if (h->stencils_ready)
-            LAUNCH(h, s, KC_GATHER_FIELD, k_gather_field_cached<T><<<nblk((int64_t)h->n * 32, 256), 256, 0, s>>>(
+            LAUNCH(h, s, KC_GATHER_FIELD, k_gather_field_cached<T><<<atom_ctas(h->n, 4), 256, 0, s>>>(
                                               h->n, stencil_cache<T>(h), g, (const T*)h->d_grid, 2.0 * DMFFB_DIELECTRIC,
                                               field_out, FieldCombine()));
         else
@@ -963,67 +952,54 @@ int recip_pass(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx
     return DMFFB_OK;
 }
 
-// One CG step's direction update and matvec A p on the PME path with the stencil cache.  The
-// step's r.z slot comes from the step counter in sc[7] (zero at the start of the solve), so a
-// captured step runs right whatever the parity of the step it is replayed as: k_cg_p reads the
-// counter (slot = count mod 2), forms p = z + beta p (beta from the previous step's r.z) and
-// clears sc[5]; the real-space matvec forks onto the side stream, writes d_fmv and reduces p.fmv
-// into sc[5], overlapping the whole reciprocal pass; the dipole spread clears sc[2] and sc[3]
-// (rr) and advances the counter; the gather writes d_Ap = recip + diagonal p, reduces p.d_Ap into
-// sc[2] and clears sc[1 - slot], the r.z slot this step's update writes.  A p = d_Ap + d_fmv; the
-// caller joins the side stream (h->e_join) before the update reads them.
+// One step of the per-pass solve on the PME path: w = A u into d_Ap, u . w into the scalars, then the
+// vector update (k_cg_update1).  The real-space matvec runs on the side stream beside the spread and
+// the convolution; the gather adds it.
 template <typename T>
-int cg_matvec_fused(dmffb_engine* h, cudaStream_t s, const Box& bx, double* sc) {
-    unsigned long long* ctr = (unsigned long long*)(sc + 7);
+int cg_step(dmffb_engine* h, cudaStream_t s, const Box& bx, double* U, double* sc) {
     const MeshGeom g = mesh_geom(bx, h->K);
+    const bool fork = h->s2 && !h->prof;
+    CsrArgs c;
+    c.n = h->n;
+    c.off = h->d_csr_off;
+    c.ent = h->d_csr_ent;
+    cudaStream_t sm = s;
+    if (fork) {
+        CK(cudaEventRecord(h->e_fork, s));
+        CK(cudaStreamWaitEvent(h->s2, h->e_fork, 0));
+        sm = h->s2;
+    }
+    LAUNCH(h, sm, KC_PAIR_MATVEC, k_matvec_apply<T><<<nblk((int64_t)h->n * 32, 256), 256, 0, sm>>>(
+                                      c, (const MvCoef<T>*)h->d_mvcoef, (const Vec4<T>*)h->d_p4, h->d_z, h->d_fmv));
+    if (fork) CK(cudaEventRecord(h->e_join, h->s2));
     SpreadArgs<T> sa;
     sa.n = h->n;
     sa.pos = nullptr;
     sa.Qg = nullptr;
-    sa.U = h->d_p;
+    sa.U = h->d_z;
     sa.q1 = nullptr;
     sa.lmax = 1;
     sa.g = g;
     sa.grid = (T*)h->d_grid2;
     sa.perm_mul = h->perm_mul;
-    sa.zero_scal[0] = sc + 2;
-    sa.zero_scal[1] = sc + 3;
-    sa.ctr_inc = ctr;
-    LAUNCH(h, s, KC_VEC, k_cg_p<T><<<nblk(3 * h->n, 256), 256, 0, s>>>(h->n, sc, 1, 0, h->d_z, h->d_p, (Vec4<T>*)h->d_p4, sc + 5, ctr));
-    const bool fork = h->s2 && !h->prof;
-    {
-        CsrArgs c;
-        c.n = h->n;
-        c.off = h->d_csr_off;
-        c.ent = h->d_csr_ent;
-        cudaStream_t sm = s;
-        if (fork) {
-            CK(cudaEventRecord(h->e_fork, s));
-            CK(cudaStreamWaitEvent(h->s2, h->e_fork, 0));
-            sm = h->s2;
-        }
-        LAUNCH(h, sm, KC_PAIR_MATVEC, k_matvec_apply<T><<<nblk((int64_t)h->n * 32, 256), 256, 0, sm>>>(
-                                          c, (const MvCoef<T>*)h->d_mvcoef, (const Vec4<T>*)h->d_p4, h->d_p, h->d_fmv,
-                                          sc + 5));
-        if (fork) CK(cudaEventRecord(h->e_join, h->s2));
-    }
-    LAUNCH(h, s, KC_SPREAD, k_spread_dip_cached<T><<<nblk((int64_t)h->n * 32, 256), 256, 0, s>>>(sa, stencil_cache<T>(h)));
+    LAUNCH(h, s, KC_SPREAD, k_spread_dip_cached<T><<<nblk((int64_t)h->n * 32, 256), 256, 0, s>>>(sa, stencil_cache<T>(h), sc));
     ConvArgs<T> ca = conv_args<T>(h, bx, CK_COUL, DMFFB_DIELECTRIC, h->d_scal + S_RECIP, false);
     ca.zero_real = (T*)h->d_grid2;  // cleared for the next spread once it has been transformed
     ca.nzero = (int64_t)h->K[0] * h->K[1] * h->K[2];
-    int stc = mesh_convolve<T>(h, s, h->d_grid2, h->d_grid, ca);
-    if (stc) return stc;
+    const int st = mesh_convolve<T>(h, s, h->d_grid2, h->d_grid, ca);
+    if (st) return st;
     FieldCombine cmb;
     const double k = h->kappa;
-    cmb.U = h->d_p;
+    cmb.U = h->d_z;
     cmb.pol = h->d_pol;
     cmb.self1 = -2.0 * DMFFB_DIELECTRIC * (k / 1.7724538509055159) * 2.0 * k * k / 3.0;
-    cmb.dot_out = sc + 2;
-    cmb.zero_pair = sc;
-    cmb.ctr = ctr;
-    LAUNCH(h, s, KC_GATHER_FIELD, k_gather_field_cached<T><<<nblk((int64_t)h->n * 32, 256), 256, 0, s>>>(
+    cmb.dot_out = sc + CGS_UW;
+    cmb.mv = h->d_fmv;
+    if (fork) CK(cudaStreamWaitEvent(s, h->e_join, 0));
+    LAUNCH(h, s, KC_GATHER_FIELD, k_gather_field_cached<T><<<atom_ctas(h->n, 4), 256, 0, s>>>(
                                       h->n, stencil_cache<T>(h), g, (const T*)h->d_grid, 2.0 * DMFFB_DIELECTRIC, h->d_Ap,
                                       cmb));
+    LAUNCH(h, s, KC_VEC, k_cg_update1<T><<<nblk(3 * h->n, 256), 256, 0, s>>>(h->n, cg_vectors(h, U, false), (Vec4<T>*)h->d_p4, sc));
     CK(cudaGetLastError());
     return DMFFB_OK;
 }
@@ -1096,16 +1072,12 @@ int build_csr(dmffb_engine* h, cudaStream_t s, const int32_t* pairs, int64_t npa
 }
 
 // dE/dU at U (include_perm) or its linear part A U (!include_perm), into out.  With dot_out,
-// dot(dotv, out) is accumulated into *dot_out; zero_scal names three scalars set to 0 before
-// the combine (by the first kernel of the reciprocal pass when there is one)
+// dot(dotv, out) is accumulated into *dot_out
 template <typename T>
 int field_eval(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx, const int32_t* pairs,
                int64_t npairs, const double* U, bool include_perm, double* out, const double* dotv = nullptr,
-               double* dot_out = nullptr, double* const* zero_scal = nullptr, bool with_mvcoef = false) {
+               double* dot_out = nullptr, bool with_mvcoef = false) {
     const bool recip_on = h->lpme && h->have_plans;
-    if (zero_scal && !recip_on)
-        for (int k = 0; k < 3; ++k)
-            if (zero_scal[k]) CK(cudaMemsetAsync(zero_scal[k], 0, sizeof(double), s));
     if (include_perm) CK(cudaMemsetAsync(h->d_fieldT, 0, (size_t)3 * h->n * sizeof(T), s));
     // the real-space work (permanent pair field, matvec) runs on a side stream, overlapping the
     // reciprocal pass; both write their own arrays and meet in the combine
@@ -1147,7 +1119,7 @@ int field_eval(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx
     if (fork) CK(cudaEventRecord(h->e_join, h->s2));
     const double* recip = nullptr;
     if (recip_on) {
-        int st = recip_pass<T>(h, s, pos, bx, include_perm, U, GATHER_FIELD, h->d_fr, zero_scal);
+        int st = recip_pass<T>(h, s, pos, bx, include_perm, U, GATHER_FIELD, h->d_fr);
         if (st) return st;
         recip = h->d_fr;
     }
@@ -1178,13 +1150,9 @@ int cg_persistent(dmffb_engine* h, cudaStream_t s, const Box& bx, double* U, con
     CK(cudaMemsetAsync(base, 0, kPcgBytes, s));
     CgSolveArgs a = {};
     a.n = h->n;
-    a.x = U;
-    a.r = h->d_r;
-    a.z = h->d_z;
-    a.p = h->d_p;
+    a.v = cg_vectors(h, U, true);
     a.Ap = h->d_Ap;
     a.fmv = h->d_fmv;
-    a.pol = h->d_pol;
     a.csr.n = h->n;
     a.csr.off = h->d_csr_off;
     a.csr.ent = h->d_csr_ent;
@@ -1214,10 +1182,10 @@ int cg_persistent(dmffb_engine* h, cudaStream_t s, const Box& bx, double* U, con
     h->pcg_phantom = 0;
     a.out = (CgStatus*)(base + kPcgOut);
     a.phase_ns = h->prof ? (unsigned long long*)(base + kPcgPhase) : nullptr;
-    // CTAs: enough warps for the matvec + spread pass (two warps per atom) and the items of the
-    // convolution passes, within what the device holds at once
-    int grid = (int)((2 * (int64_t)h->n + kCgThreads / 32 - 1) / (kCgThreads / 32));
-    grid = std::max(grid, std::max(dft_col_items(a.fc), std::max(dft_fwd_items(a.fc), dft_inv_items(a.fc))));
+    // CTAs: a warp per atom in the spread and the gather beside the items of the convolution passes
+    // (the matvec takes what they leave idle), within what the device holds at once
+    const int warp_ctas = (h->n + kCgThreads / 32 - 1) / (kCgThreads / 32);
+    int grid = warp_ctas + std::max(dft_col_items(a.fc), std::max(dft_fwd_items(a.fc), dft_inv_items(a.fc)));
     grid = std::min(grid, h->pcg_max_blocks);
     void* args[] = {&a};
     LAUNCH(h, s, KC_CGSOLVE, CK(cudaLaunchCooperativeKernel((const void*)k_cg_solve, dim3(grid), dim3(kCgThreads),
@@ -1289,56 +1257,31 @@ int solve_dipoles(dmffb_engine* h, cudaStream_t s, const double* pos, const Box&
     } stencil_scope{h};
     if (h->lpme && h->have_plans) {
         CK(cudaMemsetAsync(h->d_grid2, 0, (size_t)h->K[0] * h->K[1] * h->K[2] * sizeof(T), s));
+        h->grid2_dirty = false;
         if ((st = stencil_prep<T>(h, s, pos, bx))) return st;
     }
     if (rhs) {
         if ((st = matvec_coef_launch<T>(h, s, bx, pairs, npairs))) return st;
         CK(cudaMemcpyAsync(h->d_b, rhs, (size_t)3 * n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    } else if ((st = field_eval<T>(h, s, pos, bx, pairs, npairs, nullptr, true, h->d_b, nullptr, nullptr, nullptr,
-                                   true))) {
+    } else if ((st = field_eval<T>(h, s, pos, bx, pairs, npairs, nullptr, true, h->d_b, nullptr, nullptr, true))) {
         return st;
     }
     // from U = 0 the residual is -b: no A U pass
     const bool u0 = h->zero_guess || h->u_zeroed || rhs;
     if (h->zero_guess || rhs) CK(cudaMemsetAsync(U, 0, (size_t)3 * n * sizeof(double), s));
     if (!u0 && (st = field_eval<T>(h, s, pos, bx, pairs, npairs, U, false, h->d_Ap))) return st;
-    LAUNCH(h, s, KC_VEC, k_cg_init<<<nb3, 256, 0, s>>>(n, h->d_b, u0 ? nullptr : h->d_Ap, h->d_pol, h->d_r, h->d_z,
-                                                     h->d_p));
-    CK(cudaMemsetAsync(sc, 0, 8 * sizeof(double), s));
-    LAUNCH(h, s, KC_VEC, k_dot2<<<nb3, 256, 0, s>>>(3 * n, h->d_r, h->d_z, h->d_r, h->d_r, sc + 0, sc + 3));
-    LAUNCH(h, s, KC_VEC, k_dot2<<<nb3, 256, 0, s>>>(3 * n, h->d_b, h->d_b, nullptr, nullptr, sc + 4, nullptr));
+    CK(cudaMemsetAsync(sc, 0, (CGS_COUNT + 1) * sizeof(double), s));
+    LAUNCH(h, s, KC_VEC, k_cg_init<T><<<nb3, 256, 0, s>>>(n, h->d_b, u0 ? nullptr : h->d_Ap, h->d_pol, h->d_r, h->d_z,
+                                                        h->d_p, (Vec4<T>*)h->d_p4, sc));
     const bool fused = h->lpme && h->have_plans && h->stencils_ready;
-    if (sizeof(T) == 4 && fused && pcg_wanted(h) && pcg_decide(h) > 0)
-        return cg_persistent(h, s, bx, U, sc, res);
-    int it = 0;
-    bool conv = false;
-    double rms = 0.0, rms_b = 0.0;
-    // one CG iteration; slot = parity of the r.z scalar it reads
-    auto iteration = [&](int slot) -> int {
-        int st2;
-        if (fused) {
-            if ((st2 = cg_matvec_fused<T>(h, s, bx, sc))) return st2;
-            if (h->s2 && !h->prof) CK(cudaStreamWaitEvent(s, h->e_join, 0));
-            LAUNCH(h, s, KC_VEC, k_cg_update<<<nb3, 256, 0, s>>>(n, sc, 0, U, h->d_r, h->d_z, h->d_p, h->d_Ap,
-                                                               h->d_pol, sc, sc + 3, h->d_fmv,
-                                                               (const unsigned long long*)(sc + 7)));
-            return DMFFB_OK;
-        }
-        // Ap = A p with p.Ap reduced into sc[2]; pAp, rr and the r.z slot this step writes are
-        // cleared at the head of the pass (the previous step has read them by then)
-        double* const zs[3] = {sc + 2, sc + 3, sc + (1 - slot)};
-        if ((st2 = field_eval<T>(h, s, pos, bx, pairs, npairs, h->d_p, false, h->d_Ap, h->d_p, sc + 2, zs))) return st2;
-        LAUNCH(h, s, KC_VEC, k_cg_update<<<nb3, 256, 0, s>>>(n, sc, slot, U, h->d_r, h->d_z, h->d_p, h->d_Ap,
-                                                           h->d_pol, sc + (1 - slot), sc + 3));
-        LAUNCH(h, s, KC_VEC, k_cg_p<T><<<nb3, 256, 0, s>>>(n, sc, slot, 1 - slot, h->d_z, h->d_p, (Vec4<T>*)h->d_p4));
-        return DMFFB_OK;
-    };
+    // the classic form keeps r.z in sc[0] / sc[1]
+    if (!fused) CK(cudaMemcpyAsync(sc, sc + CGS_RU_NEW, sizeof(double), cudaMemcpyDeviceToDevice, s));
     // two iterations (slot 0 then 1) are captured once into a CUDA graph and replayed; the graph
     // bakes in pointers and the box, so it is captured on the second solve in a row with the same
     // ones (a one-off solve, such as a serving request of a new size, runs its launches directly
-    // and pays no capture and instantiation) and replayed while they stay the same.  The fused
-    // step takes its parity from the device step counter, so a one-step graph is captured beside
-    // it for a last segment of odd length.
+    // and pays no capture and instantiation) and replayed while they stay the same.  A fused
+    // step is the same launches whatever its number (its scalars move on on the device), so a
+    // one-step graph is captured beside it for segments of odd length.
     bool graphs = h->use_graphs && !h->prof;
     if (graphs) {
         std::vector<double> key = {(double)(uintptr_t)pos, (double)(uintptr_t)pairs, (double)npairs,
@@ -1351,6 +1294,30 @@ int solve_dipoles(dmffb_engine* h, cudaStream_t s, const double* pos, const Box&
         h->cg_seen_key = key;
         if ((!h->cg_exec || key != h->cg_key) && !repeat) graphs = false;
     }
+    // The persistent solve: always, or (the default) for small systems whose solve no graph can replay,
+    // where the per-pass solve is its launches (450 / 3999 atoms: 577 / 813 us a step, replayed
+    // 554 / 726).
+    if (sizeof(T) == 4 && fused && (h->pcg_mode == 1 || !graphs) && pcg_wanted(h) && pcg_decide(h) > 0) {
+        h->grid2_dirty = true;  // its last iteration leaves a spread there
+        return cg_persistent(h, s, bx, U, sc, res);
+    }
+    int it = 0;
+    bool conv = false;
+    double rms = 0.0, rms_b = 0.0;
+    // one CG iteration; slot = parity of the r.z scalar that the classic form reads
+    auto iteration = [&](int slot) -> int {
+        int st2;
+        if (fused) return cg_step<T>(h, s, bx, U, sc);
+        // Ap = A p with p.Ap reduced into sc[2]; pAp, rr and the r.z slot this step writes are
+        // cleared first (the previous step has read them by then)
+        double* const zs[3] = {sc + 2, sc + 3, sc + (1 - slot)};
+        for (double* z : zs) CK(cudaMemsetAsync(z, 0, sizeof(double), s));
+        if ((st2 = field_eval<T>(h, s, pos, bx, pairs, npairs, h->d_p, false, h->d_Ap, h->d_p, sc + 2))) return st2;
+        LAUNCH(h, s, KC_VEC, k_cg_update<<<nb3, 256, 0, s>>>(n, sc, slot, U, h->d_r, h->d_z, h->d_p, h->d_Ap,
+                                                           h->d_pol, sc + (1 - slot), sc + 3));
+        LAUNCH(h, s, KC_VEC, k_cg_p<<<nb3, 256, 0, s>>>(n, sc, slot, 1 - slot, h->d_z, h->d_p));
+        return DMFFB_OK;
+    };
     auto capture = [&](int steps, cudaGraphExec_t* exec, int64_t* launches, int64_t* ffts) -> int {
         if (*exec) { cudaGraphExecDestroy(*exec); *exec = nullptr; }
         cudaGraph_t g;
@@ -1380,12 +1347,13 @@ int solve_dipoles(dmffb_engine* h, cudaStream_t s, const double* pos, const Box&
             h->cg_key = key;
         }
     }
-    // The host reads the residual every few steps (no per-step sync).  On the fused path, from the
-    // second read on, the residual's decay over the last segment predicts the steps still needed:
-    // a segment shorter than check_every then ends at the first step expected to converge.
+    // The host reads the residual every few steps (no per-step sync; a read costs some 25 us with the
+    // launches it holds up).  On the fused path, from the second read on, the residual's decay over the
+    // last segment predicts the steps still needed: a segment shorter than check_every then ends at the
+    // first step expected to converge.  A solve from U = 0 first runs the steps up to the last read but
+    // one of the engine's last such solve without a read (neighbouring configurations take the same
+    // number or one more); the reads left out are made up from the device's history of residuals.
     const int check_every = 4;
-    double r_prev = -1.0;
-    int it_prev = 0;
     auto run_steps = [&](int k) -> int {
         int st2;
         for (; k >= 2; k -= 2) {
@@ -1409,11 +1377,25 @@ int solve_dipoles(dmffb_engine* h, cudaStream_t s, const double* pos, const Box&
         }
         return DMFFB_OK;
     };
-    while (true) {
-        CK(cudaMemcpyAsync(h->h_scal, sc + 3, 2 * sizeof(double), cudaMemcpyDeviceToHost, s));
+    // residual (and the last kCgHist before it) and b.b on the host
+    auto read_residual = [&]() -> int {
+        CK(cudaMemcpyAsync(h->h_scal, sc, (fused ? CGS_COUNT + 1 + kCgHist : CGS_COUNT) * sizeof(double),
+                           cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
-        rms = sqrt(h->h_scal[0] / (3.0 * n));
-        if (it == 0) rms_b = sqrt(h->h_scal[1] / (3.0 * n));
+        rms = sqrt(h->h_scal[CGS_RR] / (3.0 * n));
+        rms_b = sqrt(h->h_scal[CGS_BB] / (3.0 * n));
+        return DMFFB_OK;
+    };
+    if (fused && u0 && !rhs && h->cg_hint > 0) {
+        it = std::min(h->cg_hint, std::min(kCgHist - 1, h->max_iter));
+        if ((st = run_steps(it))) return st;
+    }
+    if ((st = read_residual())) return st;
+    // e walks the reads' schedule; while it lies behind the steps already run it goes by the history,
+    // so that a solve takes the same steps with and without the head start
+    int e = 0, e_prev = 0;
+    double r_prev = -1.0;
+    while (true) {
         if (!std::isfinite(rms)) return fail(h, DMFFB_NONFINITE, "non-finite residual in the dipole solve");
         // relative criterion: RMS(dE/dU) below cg_tol times the RMS permanent field
         if (rms <= h->cg_tol * rms_b) {
@@ -1421,17 +1403,24 @@ int solve_dipoles(dmffb_engine* h, cudaStream_t s, const double* pos, const Box&
             break;
         }
         if (it >= h->max_iter) break;
+        const double r = e < it ? sqrt(h->h_scal[CGS_COUNT + 1 + (e & (kCgHist - 1))] / (3.0 * n)) : rms;
         int k = check_every;
-        if (fused && r_prev > 0.0 && rms < r_prev && it > it_prev) {
-            const double rate = std::pow(rms / r_prev, 1.0 / (double)(it - it_prev));
-            const double need = std::log(h->cg_tol * rms_b / rms) / std::log(rate);
+        if (fused && r_prev > 0.0 && r < r_prev && e > e_prev) {
+            const double rate = std::pow(r / r_prev, 1.0 / (double)(e - e_prev));
+            const double need = std::log(h->cg_tol * rms_b / r) / std::log(rate);
             if (need > 0.0 && need < (double)check_every) k = std::max(1, (int)std::ceil(need));
         }
-        r_prev = rms;
-        it_prev = it;
-        if ((st = run_steps(k))) return st;
-        it += k;
+        r_prev = r;
+        e_prev = e;
+        e += k;
+        if (e > it) {
+            if ((st = run_steps(e - it))) return st;
+            it = e;
+            if ((st = read_residual())) return st;
+        }
     }
+    if (rms_b == 0.0) it = 0;  // nothing to solve
+    if (fused && u0 && !rhs) h->cg_hint = conv ? (e < it ? it - 1 : e_prev) : 0;
     res->n_iter = it;
     res->converged = conv ? 1 : 0;
     res->residual_rms = rms;
@@ -2526,8 +2515,14 @@ int dmffb_admp_create(const dmffb_admp_desc* d, dmffb_engine** out) {
     *out = h;
     // streams and events first: every upload and zeroing below is ordered on the engine stream
     for (int k = 0; k < 8; ++k) cudaEventCreate(&h->ev[k]);
-    cudaStreamCreateWithFlags(&h->s1, cudaStreamNonBlocking);
-    cudaStreamCreateWithFlags(&h->s2, cudaStreamNonBlocking);
+    // The side stream's kernels (pair tensors, matvec, pair passes) fill the chip with short CTAs, the
+    // engine stream's chain beside them (mesh passes) has few CTAs and is latency-bound: with the chain
+    // at the higher priority its CTAs take the places that come free, where they had queued behind the
+    // whole pair pass (30000 atoms: 2317 us a step against 2484)
+    int prio_low = 0, prio_high = 0;
+    cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high);
+    cudaStreamCreateWithPriority(&h->s1, cudaStreamNonBlocking, prio_high);
+    cudaStreamCreateWithPriority(&h->s2, cudaStreamNonBlocking, prio_low);
     cudaEventCreateWithFlags(&h->e_in, cudaEventDisableTiming);
     cudaEventCreateWithFlags(&h->e_out, cudaEventDisableTiming);
     cudaEventCreateWithFlags(&h->e_fork, cudaEventDisableTiming);
@@ -2572,6 +2567,7 @@ int dmffb_admp_create(const dmffb_admp_desc* d, dmffb_engine** out) {
         AL(h->d_z, 3 * n * sizeof(double));
         AL(h->d_p, 3 * n * sizeof(double));
         AL(h->d_Ap, 3 * n * sizeof(double));
+        AL(h->d_s, 3 * n * sizeof(double));
         AL(h->d_fr, 3 * n * sizeof(double));
     }
 #undef AL
@@ -2613,6 +2609,7 @@ int dmffb_admp_reconfigure(dmffb_engine* h, const dmffb_admp_desc* d) {
     }
     h->cg_key.clear();
     h->cg_seen_key.clear();
+    h->cg_hint = 0;
     h->params_set = false;
     h->have_last = false;
     return DMFFB_OK;
@@ -2626,7 +2623,7 @@ void dmffb_destroy(dmffb_engine* h) {
     void* ptrs[] = {h->d_axis_type, h->d_axis_idx, h->d_cov_ptr, h->d_cov_j, h->d_cov_nb, h->d_Qloc, h->d_pol,
                     h->d_thole, h->d_polsix, h->d_pos, h->d_U, h->d_forces, h->d_posT, h->d_Qg, h->d_QgT,
                     h->d_gpair, h->d_torque, h->d_fieldT, h->d_grad, h->d_scal, h->d_b, h->d_r, h->d_z, h->d_p,
-                    h->d_Ap, h->d_fr, h->d_gQ, h->d_fmv, h->d_pcount_f, h->d_pcount_s, h->d_poff_s, h->d_rank, h->d_bin_done, h->d_nbsum, h->d_mvcoef, h->d_p4, h->d_csr_off, h->d_csr_ent, h->d_csr_deg, h->d_cub2, h->d_grid, h->d_grid2, h->d_cgrid, h->d_bmod, h->d_pairs, h->d_atom_cell,
+                    h->d_Ap, h->d_s, h->d_fr, h->d_gQ, h->d_fmv, h->d_pcount_f, h->d_pcount_s, h->d_poff_s, h->d_rank, h->d_bin_done, h->d_nbsum, h->d_mvcoef, h->d_p4, h->d_csr_off, h->d_csr_ent, h->d_csr_deg, h->d_cub2, h->d_grid, h->d_grid2, h->d_cgrid, h->d_bmod, h->d_pairs, h->d_atom_cell,
                     h->d_cell_count, h->d_cell_start, h->d_pcount, h->d_poff,
                     h->d_c, h->d_tta, h->d_ttb, h->d_ttq, h->d_glr, h->d_gsr, h->d_dc,
                     h->d_q, h->d_qT, h->d_type, h->d_sigtt, h->d_epstt, h->d_dq, h->d_dsig, h->d_deps,
@@ -2773,7 +2770,7 @@ int field_at(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx, 
     // the matvec of U needs this call's CSR and pair tensors (not a previous compute's)
     if ((st = build_csr(h, s, pairs, npairs))) return st;
     if ((st = matvec_alloc<T>(h))) return st;
-    return field_eval<T>(h, s, pos, bx, pairs, npairs, U, true, field_out, nullptr, nullptr, nullptr, true);
+    return field_eval<T>(h, s, pos, bx, pairs, npairs, U, true, field_out, nullptr, nullptr, true);
 }
 
 __global__ void k_lin(int64_t m, double* out, const double* x0, double a, const double* d) {
@@ -3033,7 +3030,7 @@ int dmffb_admp_field(dmffb_engine* h, void* stream, const double* pos, const dou
         // the matvec of U needs this call's CSR and pair tensors (not a previous compute's)
         if ((st = build_csr(h, s, pairs, npairs))) return st;
         if ((st = matvec_alloc<T>(h))) return st;
-        st = field_eval<T>(h, s, pos, bx, pairs, npairs, U, true, field_out, nullptr, nullptr, nullptr, true);
+        st = field_eval<T>(h, s, pos, bx, pairs, npairs, U, true, field_out, nullptr, nullptr, true);
         if (st) return st;
         CK(cudaStreamSynchronize(s));
         return DMFFB_OK;

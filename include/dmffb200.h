@@ -337,11 +337,12 @@ int dmffb_classical_param_grads(dmffb_engine* h, void* stream, double* dE_dq, do
  * DFT kernels on meshes of at most 64 points per axis (cuFFT beyond), 0 for cuFFT.
  * dmffb_fused_fft_active returns 1 when the last convolution ran through the DFT kernels, else 0. */
 int dmffb_set_fused_fft(dmffb_engine* h, int32_t enabled);
-/* The whole CG dipole solve in one persistent cooperative launch (k_cg_solve: direction update,
- * real-space matvec and dipole spread, the direct-DFT convolution, field gather and CG update per
- * iteration, separated by grid barriers; convergence decided on the device, one read-back per
- * solve).  mode 0: off (the graph-replayed per-pass solve), 1: on, 2 (default): on for systems of
- * at most 4096 atoms, where the launch chain of the per-pass solve dominates.  FP32 engines with
+/* The whole CG dipole solve in one persistent cooperative launch (k_cg_solve: vector update and dipole
+ * spread, the direct-DFT convolution, real-space matvec and field gather per iteration, separated by
+ * grid barriers; convergence decided on the device, one read-back per solve).  mode 0: off (the
+ * graph-replayed per-pass solve), 1: on, 2 (default): on for systems of at most 4096 atoms whose solve
+ * no graph of this engine can replay (a first solve with these buffers and box), where the launch
+ * chain of the per-pass solve dominates.  FP32 engines with
  * meshes of at most 128 points per axis on devices with cooperative launch only.
  * dmffb_persistent_cg_blocks returns the co-resident CTAs available to it for the current mesh
  * (0: not used).
@@ -351,8 +352,8 @@ int dmffb_set_fused_fft(dmffb_engine* h, int32_t enabled);
 int dmffb_set_persistent_cg(dmffb_engine* h, int32_t mode);
 int dmffb_persistent_cg_blocks(const dmffb_engine* h);
 int dmffb_set_cg_wait_limit(dmffb_engine* h, double seconds, int32_t phantom_arrivals);
-/* Device-clock time of each pass of the persistent solve (0 direction update, 1 matvec + spread,
- * 2 forward planes, 3 spectrum columns, 4 inverse planes, 5 field gather, 6 CG update; barrier
+/* Device-clock time of each pass of the persistent solve (1 vector update + spread, 2 forward planes,
+ * 3 spectrum columns, 4 inverse planes, 5 matvec + field gather; 0 and 6 are unused and stay 0; barrier
  * waits included, measured on CTA 0), summed over the solves run while profiling was on. */
 int dmffb_get_cg_phase_times(const dmffb_engine* h, double* ms_out, int32_t n);
 int dmffb_fused_fft_active(const dmffb_engine* h);
