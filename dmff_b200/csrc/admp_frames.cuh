@@ -106,12 +106,14 @@ struct PrepArgs {
     T* posT;             // [n*4]
     T* QgT;              // [n*9]
     double* Qg;          // [n*9]
+    ClearList clear;     // what the evaluation starts from zero
 };
 
 // positions in kernel precision, local frames, and Q_global = rot_local2global(Q_local)
 template <typename T>
 __global__ void k_prepare(PrepArgs<T> a) {
     const int at = blockIdx.x * blockDim.x + threadIdx.x;
+    clear_all(a.clear, at, (int64_t)gridDim.x * blockDim.x);
     if (at >= a.f.n) return;
     const double* p = a.f.pos + 3 * at;
     a.posT[4 * at] = (T)p[0];

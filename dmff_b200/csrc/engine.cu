@@ -881,6 +881,16 @@ StencilCache<T> stencil_cache(dmffb_engine* h) {
     return c;
 }
 
+// Every spread goes to d_grid2, which the convolution clears again once the forward transform has read
+// it: it is zero between passes, unless a persistent solve has left its last spread there.
+template <typename T>
+int spread_mesh(dmffb_engine* h, cudaStream_t s) {
+    if (!h->grid2_dirty) return DMFFB_OK;
+    CK(cudaMemsetAsync(h->d_grid2, 0, (size_t)h->grid_cap * sizeof(T), s));
+    h->grid2_dirty = false;
+    return DMFFB_OK;
+}
+
 // reciprocal pass: spread (Qg and/or U) -> forward transform -> influence function -> inverse
 // transform -> gather
 template <typename T>
@@ -888,15 +898,9 @@ int recip_pass(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx
                int mode, double* field_out) {
     const MeshGeom g = mesh_geom(bx, h->K);
     const int64_t K3 = (int64_t)h->K[0] * h->K[1] * h->K[2];
-    // the dipole-only field pass (the CG matvec) spreads into d_grid2, which the convolution
-    // clears again once the forward transform has read it: no memset per pass
     const bool dip = mode == GATHER_FIELD && !use_Qg && U;
-    void* spread_grid = dip ? h->d_grid2 : h->d_grid;
-    if (!dip) CK(cudaMemsetAsync(h->d_grid, 0, K3 * sizeof(T), s));
-    if (dip && h->grid2_dirty) {
-        CK(cudaMemsetAsync(h->d_grid2, 0, K3 * sizeof(T), s));
-        h->grid2_dirty = false;
-    }
+    int st;
+    if ((st = spread_mesh<T>(h, s))) return st;
     SpreadArgs<T> sa;
     sa.n = h->n;
     sa.pos = pos;
@@ -905,7 +909,7 @@ int recip_pass(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx
     sa.q1 = nullptr;
     sa.lmax = lmax_eff(h);
     sa.g = g;
-    sa.grid = (T*)spread_grid;
+    sa.grid = (T*)h->d_grid2;
     sa.perm_mul = h->perm_mul;
     if (dip && h->stencils_ready) {
         LAUNCH(h, s, KC_SPREAD, k_spread_dip_cached<T><<<nblk((int64_t)h->n * 32, 256), 256, 0, s>>>(sa, stencil_cache<T>(h), nullptr));
@@ -914,12 +918,9 @@ int recip_pass(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx
         LAUNCH(h, s, KC_SPREAD, k_spread<T, false><<<nblk(h->n, apc), kSiteThreads, 0, s>>>(sa, apc));
     }
     ConvArgs<T> ca = conv_args<T>(h, bx, CK_COUL, DMFFB_DIELECTRIC, h->d_scal + S_RECIP, mode == GATHER_FULL);
-    if (dip) {
-        ca.zero_real = (T*)h->d_grid2;
-        ca.nzero = K3;
-    }
-    int st = mesh_convolve<T>(h, s, spread_grid, h->d_grid, ca);
-    if (st) return st;
+    ca.zero_real = (T*)h->d_grid2;
+    ca.nzero = K3;
+    if ((st = mesh_convolve<T>(h, s, h->d_grid2, h->d_grid, ca))) return st;
     if (mode == GATHER_FIELD) {
         if (h->stencils_ready)
             LAUNCH(h, s, KC_GATHER_FIELD, k_gather_field_cached<T><<<atom_ctas(h->n, 4), 256, 0, s>>>(
@@ -1072,13 +1073,13 @@ int build_csr(dmffb_engine* h, cudaStream_t s, const int32_t* pairs, int64_t npa
 }
 
 // dE/dU at U (include_perm) or its linear part A U (!include_perm), into out.  With dot_out,
-// dot(dotv, out) is accumulated into *dot_out
+// dot(dotv, out) is accumulated into *dot_out; cleared: the pair field (d_fieldT) is zero already
 template <typename T>
 int field_eval(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx, const int32_t* pairs,
                int64_t npairs, const double* U, bool include_perm, double* out, const double* dotv = nullptr,
-               double* dot_out = nullptr, bool with_mvcoef = false) {
+               double* dot_out = nullptr, bool with_mvcoef = false, bool cleared = false) {
     const bool recip_on = h->lpme && h->have_plans;
-    if (include_perm) CK(cudaMemsetAsync(h->d_fieldT, 0, (size_t)3 * h->n * sizeof(T), s));
+    if (include_perm && !cleared) CK(cudaMemsetAsync(h->d_fieldT, 0, (size_t)3 * h->n * sizeof(T), s));
     // the real-space work (permanent pair field, matvec) runs on a side stream, overlapping the
     // reciprocal pass; both write their own arrays and meet in the combine
     const bool real_work = (include_perm && npairs > 0) || U || with_mvcoef;
@@ -1248,29 +1249,26 @@ int solve_dipoles(dmffb_engine* h, cudaStream_t s, const double* pos, const Box&
         res->residual_rms = conv && h->steps_pol <= 0 ? h->h_scal[0] : -1.0;
         return DMFFB_OK;
     }
-    // CG on A U = -b.  The dipole-only field passes keep d_grid2 zero between passes; clear it
-    // here so that an earlier solve that stopped part-way leaves nothing behind
-    // the stencil cache holds for these positions only: it is dropped when the solve returns
+    // CG on A U = -b.  The caller has cleared the permanent field, the scalars and with a zero guess U
+    // (compute_impl); with rhs that is done here.  The stencil cache holds for these positions only: it is dropped when the solve returns
     struct StencilScope {
         dmffb_engine* h;
         ~StencilScope() { h->stencils_ready = false; }
     } stencil_scope{h};
     if (h->lpme && h->have_plans) {
-        CK(cudaMemsetAsync(h->d_grid2, 0, (size_t)h->K[0] * h->K[1] * h->K[2] * sizeof(T), s));
-        h->grid2_dirty = false;
         if ((st = stencil_prep<T>(h, s, pos, bx))) return st;
     }
     if (rhs) {
+        CK(cudaMemsetAsync(sc, 0, (CGS_COUNT + 1) * sizeof(double), s));
+        CK(cudaMemsetAsync(U, 0, (size_t)3 * n * sizeof(double), s));
         if ((st = matvec_coef_launch<T>(h, s, bx, pairs, npairs))) return st;
         CK(cudaMemcpyAsync(h->d_b, rhs, (size_t)3 * n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    } else if ((st = field_eval<T>(h, s, pos, bx, pairs, npairs, nullptr, true, h->d_b, nullptr, nullptr, true))) {
+    } else if ((st = field_eval<T>(h, s, pos, bx, pairs, npairs, nullptr, true, h->d_b, nullptr, nullptr, true, true))) {
         return st;
     }
     // from U = 0 the residual is -b: no A U pass
     const bool u0 = h->zero_guess || h->u_zeroed || rhs;
-    if (h->zero_guess || rhs) CK(cudaMemsetAsync(U, 0, (size_t)3 * n * sizeof(double), s));
     if (!u0 && (st = field_eval<T>(h, s, pos, bx, pairs, npairs, U, false, h->d_Ap))) return st;
-    CK(cudaMemsetAsync(sc, 0, (CGS_COUNT + 1) * sizeof(double), s));
     LAUNCH(h, s, KC_VEC, k_cg_init<T><<<nb3, 256, 0, s>>>(n, h->d_b, u0 ? nullptr : h->d_Ap, h->d_pol, h->d_r, h->d_z,
                                                         h->d_p, (Vec4<T>*)h->d_p4, sc));
     const bool fused = h->lpme && h->have_plans && h->stencils_ready;
@@ -1448,12 +1446,15 @@ int compute_impl(dmffb_engine* h, cudaStream_t s, const double* pos, const doubl
         if ((st = dmffb_admp_build_neighbors(h, (void*)s, pos, box))) return st;
     if (own_list && h->e_build) CK(cudaStreamWaitEvent(s, h->e_build, 0));
     if (h->timing) CK(cudaEventRecord(h->ev[0], s));
-    CK(cudaMemsetAsync(h->d_scal, 0, N_SCAL * sizeof(double), s));
-    CK(cudaMemsetAsync(h->d_gpair, 0, (size_t)3 * n * sizeof(T), s));
-    CK(cudaMemsetAsync(h->d_torque, 0, (size_t)3 * n * sizeof(T), s));
-    CK(cudaMemsetAsync(h->d_grad, 0, (size_t)3 * n * sizeof(double), s));
-    CK(cudaMemsetAsync(h->d_gQ, 0, (size_t)9 * n * sizeof(double), s));
     PrepArgs<T> pa;
+    pa.clear.add(h->d_scal, N_SCAL * sizeof(double));
+    pa.clear.add(h->d_gpair, (size_t)3 * n * sizeof(T));
+    pa.clear.add(h->d_torque, (size_t)3 * n * sizeof(T));
+    pa.clear.add(h->d_grad, (size_t)3 * n * sizeof(double));
+    pa.clear.add(h->d_gQ, (size_t)9 * n * sizeof(double));
+    const bool cg = h->lpol && !h->fixed_U && h->solver != DMFFB_SOLVER_REFERENCE;
+    if (cg) pa.clear.add(h->d_fieldT, (size_t)3 * n * sizeof(T));
+    if (cg && h->zero_guess) pa.clear.add(U, (size_t)3 * n * sizeof(double));
     pa.f.n = n;
     pa.f.pos = pos;
     pa.f.axis_type = h->d_axis_type;
@@ -1648,7 +1649,8 @@ int recip_pass_channel(dmffb_engine* h, cudaStream_t s, const double* pos, const
                        double escale, double* grad, double* dq, double* scal_conv, double* scal_gather) {
     const MeshGeom g = mesh_geom(bx, h->K);
     const int64_t K3 = (int64_t)h->K[0] * h->K[1] * h->K[2];
-    CK(cudaMemsetAsync(h->d_grid, 0, K3 * sizeof(T), s));
+    int st;
+    if ((st = spread_mesh<T>(h, s))) return st;
     SpreadArgs<T> sa;
     sa.n = h->n;
     sa.pos = pos;
@@ -1657,13 +1659,14 @@ int recip_pass_channel(dmffb_engine* h, cudaStream_t s, const double* pos, const
     sa.q1 = q;
     sa.lmax = 0;
     sa.g = g;
-    sa.grid = (T*)h->d_grid;
+    sa.grid = (T*)h->d_grid2;
     sa.perm_mul = h->perm_mul;
     const int apc = sites_per_cta(h->n);
     LAUNCH(h, s, KC_SPREAD, k_spread<T, true><<<nblk(h->n, apc), kSiteThreads, 0, s>>>(sa, apc));
     ConvArgs<T> ca = conv_args<T>(h, bx, kind, escale, scal_conv, true);
-    int st = mesh_convolve<T>(h, s, h->d_grid, h->d_grid, ca);
-    if (st) return st;
+    ca.zero_real = (T*)h->d_grid2;
+    ca.nzero = K3;
+    if ((st = mesh_convolve<T>(h, s, h->d_grid2, h->d_grid, ca))) return st;
     GatherArgs<T> ga;
     ga.n = h->n;
     ga.pos = pos;
@@ -1728,11 +1731,13 @@ int disp_compute_impl(dmffb_engine* h, cudaStream_t s, const double* pos, const 
         npairs = h->npairs;
     }
     res->n_pairs = npairs;
-    CK(cudaMemsetAsync(h->d_scal, 0, N_SCAL * sizeof(double), s));
-    CK(cudaMemsetAsync(h->d_glr, 0, (size_t)3 * n * sizeof(T), s));
-    CK(cudaMemsetAsync(h->d_gsr, 0, (size_t)3 * n * sizeof(T), s));
-    CK(cudaMemsetAsync(h->d_grad, 0, (size_t)3 * n * sizeof(double), s));
-    CK(cudaMemsetAsync(h->d_dc, 0, (size_t)3 * n * sizeof(double), s));
+    ClearList cl;
+    cl.add(h->d_scal, N_SCAL * sizeof(double));
+    cl.add(h->d_glr, (size_t)3 * n * sizeof(T));
+    cl.add(h->d_gsr, (size_t)3 * n * sizeof(T));
+    cl.add(h->d_grad, (size_t)3 * n * sizeof(double));
+    cl.add(h->d_dc, (size_t)3 * n * sizeof(double));
+    LAUNCH(h, s, KC_VEC, k_clear<<<std::min(nblk(6 * (int64_t)n, 256), 592u), 256, 0, s>>>(cl));
     DispArgs<T> a;
     a.n = n;
     a.npairs = npairs;
@@ -2116,9 +2121,11 @@ int classical_compute_impl(dmffb_engine* h, cudaStream_t s, const double* pos, c
     if (!nonbonded) npairs = 0;
     res->n_pairs = npairs;
     const bool pg = h->want_pgrad;
-    CK(cudaMemsetAsync(h->d_scal, 0, N_SCAL * sizeof(double), s));
-    CK(cudaMemsetAsync(h->d_glr, 0, (size_t)3 * n * sizeof(T), s));
-    CK(cudaMemsetAsync(h->d_grad, 0, (size_t)3 * n * sizeof(double), s));
+    ClearList cl;
+    cl.add(h->d_scal, N_SCAL * sizeof(double));
+    cl.add(h->d_glr, (size_t)3 * n * sizeof(T));
+    cl.add(h->d_grad, (size_t)3 * n * sizeof(double));
+    LAUNCH(h, s, KC_VEC, k_clear<<<std::min(nblk(6 * (int64_t)n, 256), 592u), 256, 0, s>>>(cl));
     if (pg) {
         CK(cudaMemsetAsync(h->d_dq, 0, (size_t)n * sizeof(double), s));
         if (h->ntypes > 0) {
