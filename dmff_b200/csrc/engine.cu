@@ -78,14 +78,13 @@ struct dmffb_engine {
     double* d_fmv = nullptr;  // CSR matvec output [3n]
     // slots of the single-pass neighbour build: capacities per atom, first from the mean density,
     // then from the largest counts met (0: no slots yet)
-    int32_t* d_ell_rows = nullptr;  // [n_cap * ell_cap_h * 3]
-    int32_t* d_ell_ent = nullptr;   // [n_cap * ell_cap_f]
-    int ell_cap_h = 0, ell_cap_f = 0;
+    int32_t* d_slots = nullptr;     // [n_cap * slot_cap]
+    int slot_cap = 0;
     int32_t* d_nbsum = nullptr;     // NbTotals, then the run sums of the counts [3][runs]
     // a single-pass build whose totals are still on their way to the host: nb_finish waits for
     // them when the list is first used (and rebuilds with larger slots if one overflowed)
     bool nb_pending = false, nb_want_csr = false;
-    int nb_cap_h = 0, nb_cap_f = 0;  // the slots it ran with
+    int nb_slot_cap = 0;  // the slots it ran with
     cudaEvent_t e_nbtot = nullptr;
     NbTotals* h_nbtot = nullptr;    // pinned
     cudaStream_t nb_stream = nullptr;
@@ -1922,24 +1921,15 @@ int nb_alloc(dmffb_engine* h, bool want_csr) {
     return want_csr ? csr_alloc(h) : DMFFB_OK;
 }
 
-// slots for ch half rows and cf CSR entries per atom
-int nb_slots(dmffb_engine* h, int ch, int cf) {
-    int st;
-    if (ch > h->ell_cap_h) {
-        if (h->d_ell_rows) cudaFree(h->d_ell_rows);
-        h->d_ell_rows = nullptr;
-        h->ell_cap_h = 0;
-        if ((st = dalloc(h, &h->d_ell_rows, (size_t)h->n_cap * ch * 3 * sizeof(int32_t)))) return st;
-        h->ell_cap_h = ch;
-    }
-    if (cf > h->ell_cap_f) {
-        if (h->d_ell_ent) cudaFree(h->d_ell_ent);
-        h->d_ell_ent = nullptr;
-        h->ell_cap_f = 0;
-        if ((st = dalloc(h, &h->d_ell_ent, (size_t)h->n_cap * cf * sizeof(int32_t)))) return st;
-        h->ell_cap_f = cf;
-    }
-    return DMFFB_OK;
+// slots for cap neighbours per atom
+int nb_slots(dmffb_engine* h, int cap) {
+    if (cap <= h->slot_cap) return DMFFB_OK;
+    if (h->d_slots) cudaFree(h->d_slots);
+    h->d_slots = nullptr;
+    h->slot_cap = 0;
+    const int st = dalloc(h, &h->d_slots, (size_t)h->n_cap * cap * sizeof(int32_t));
+    if (!st) h->slot_cap = cap;
+    return st;
 }
 
 // the largest counts with an eighth (at least 16) of headroom
@@ -2024,10 +2014,9 @@ int nb_place(dmffb_engine* h, cudaStream_t s, const Nb2Args& b, bool slots, int3
     a.off_h = h->d_poff;
     a.off_f = b.count_f ? h->d_csr_off : nullptr;
     a.off_s = h->d_poff_s;
-    a.ell_rows = slots ? b.ell_rows : nullptr;
-    a.ell_ent = slots ? b.ell_ent : nullptr;
-    a.cap_h = b.ell_cap_h;
-    a.cap_f = b.ell_cap_f;
+    a.cov = b.a;
+    a.slots = slots ? b.slots : nullptr;
+    a.slot_cap = b.slot_cap;
     a.rows = rows;
     a.rows_cap = rows_cap;
     a.ent = ent;
@@ -2043,10 +2032,8 @@ int nb_place(dmffb_engine* h, cudaStream_t s, const Nb2Args& b, bool slots, int3
 // binning and distance tests of a single-pass build into the slots
 int nb_single_pass(dmffb_engine* h, cudaStream_t s, const NbPlan& p, const double* pos, const Box& bx, Nb2Args& b) {
     const int n = h->n, words = nb_sum_words(n);
-    b.ell_rows = h->d_ell_rows;
-    b.ell_cap_h = h->ell_cap_h;
-    b.ell_ent = b.count_f ? h->d_ell_ent : nullptr;
-    b.ell_cap_f = h->ell_cap_f;
+    b.slots = h->d_slots;
+    b.slot_cap = h->slot_cap;
     if (p.flat) {
         CK(cudaMemsetAsync(h->d_nbsum, 0, words * sizeof(int32_t), s));
         if (p.ortho) LAUNCH(h, s, KC_NBLIST, k_pairs_flat<true><<<nblk((int64_t)n * 32, 128), 128, 0, s>>>(b));
@@ -2057,8 +2044,7 @@ int nb_single_pass(dmffb_engine* h, cudaStream_t s, const NbPlan& p, const doubl
         b.posc = h->d_posc;
         b.a.cell_start = h->d_cell_start;
         const size_t stage = (size_t)p.chmax * sizeof(float4);
-        if (p.ortho) LAUNCH(h, s, KC_NBLIST, k_pairs_cell<2, kNbWarps, true><<<p.ncell, 32 * kNbWarps, stage, s>>>(b, p.chmax));
-        else LAUNCH(h, s, KC_NBLIST, k_pairs_cell<2, kNbWarps, false><<<p.ncell, 32 * kNbWarps, stage, s>>>(b, p.chmax));
+        LAUNCH(h, s, KC_NBLIST, k_pairs_cell<2, kNbWarps><<<p.ncell, 32 * kNbWarps, stage, s>>>(b, p.chmax));
     }
     CK(cudaGetLastError());
     return DMFFB_OK;
@@ -2453,8 +2439,7 @@ int nb_start(dmffb_engine* h, cudaStream_t s, const double* pos, const double* b
     CK(cudaEventRecord(h->e_build, s));
     h->nb_pending = true;
     h->nb_want_csr = want_csr;
-    h->nb_cap_h = b.ell_cap_h;
-    h->nb_cap_f = b.ell_cap_f;
+    h->nb_slot_cap = b.slot_cap;
     h->nb_stream = s;
     h->nb_pos = pos;
     for (int k = 0; k < 9; ++k) h->nb_box[k] = box[k];
@@ -2477,8 +2462,8 @@ int nb_finish(dmffb_engine* h) {
         CK(cudaEventSynchronize(h->e_nbtot));
         const NbTotals t = *h->h_nbtot;
         const bool csr = h->nb_want_csr;
-        if (t.max_h <= h->nb_cap_h && (!csr || t.max_f <= h->nb_cap_f) && t.rows <= h->pair_cap &&
-            (!csr || t.entries <= h->csr_cap)) {
+        const int most = csr ? t.max_f : t.max_h;
+        if (most <= h->nb_slot_cap && t.rows <= h->pair_cap && (!csr || t.entries <= h->csr_cap)) {
             h->npairs = t.rows;
             // the scaled-row map made with the list, unless other rows have replaced it since
             if (h->srows_pairs == h->d_pairs && h->srows_gen == h->pairs_gen) {
@@ -2489,9 +2474,7 @@ int nb_finish(dmffb_engine* h) {
         }
         h->have_pairs = false;
         int st;
-        if ((st = nb_slots(h, t.max_h > h->nb_cap_h ? nb_headroom(t.max_h) : 0,
-                           csr && t.max_f > h->nb_cap_f ? nb_headroom(t.max_f) : 0)))
-            return st;
+        if (most > h->nb_slot_cap && (st = nb_slots(h, nb_headroom(most)))) return st;
         if ((st = nb_pair_cap(h, t.rows)) || (csr && (st = nb_csr_cap(h, t.entries)))) return st;
         if ((st = nb_start(h, h->nb_stream, h->nb_pos, h->nb_box))) return st;
     }
@@ -2636,7 +2619,7 @@ void dmffb_destroy(dmffb_engine* h) {
                     h->d_q, h->d_qT, h->d_type, h->d_sigtt, h->d_epstt, h->d_dq, h->d_dsig, h->d_deps,
                     h->d_tidx[0], h->d_tidx[1], h->d_tidx[2], h->d_tprm[0], h->d_tprm[1], h->d_tprm[2],
                     h->d_tdprm[0], h->d_tdprm[1], h->d_tdprm[2], h->d_dQloc, h->d_dpa, h->d_dth, h->d_dpol, h->d_dsr, h->d_srows, h->d_nsel, h->d_cubsel,
-                    h->d_ell_rows, h->d_ell_ent, h->d_stc_org, h->d_stc_w, h->d_nbmask, h->d_covrows, h->d_cov_lo, h->d_cov_hi, h->d_dftW, h->d_dftG, h->d_pcg, h->d_posc, h->d_nbrec, h->d_gcell, h->d_srp, h->d_srdp, h->d_srgrad};
+                    h->d_slots, h->d_stc_org, h->d_stc_w, h->d_nbmask, h->d_covrows, h->d_cov_lo, h->d_cov_hi, h->d_dftW, h->d_dftG, h->d_pcg, h->d_posc, h->d_nbrec, h->d_gcell, h->d_srp, h->d_srdp, h->d_srgrad};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (h->h_scal) cudaFreeHost(h->h_scal);
@@ -3121,12 +3104,12 @@ int dmffb_build_neighbors(dmffb_engine* h, void* stream, const double* pos, cons
     if ((st = nb_alloc(h, false))) return st;
     Nb2Args b = nb_args(h, p, pos, bx, rc, false);
     if (p.flat || p.staged) {
-        for (int grow = h->ell_cap_h > 0 ? 0 : p.guess;;) {
-            if ((st = nb_slots(h, grow, 0))) return st;
+        for (int grow = h->slot_cap > 0 ? 0 : p.guess;;) {
+            if ((st = nb_slots(h, grow))) return st;
             if ((st = nb_single_pass(h, s, p, pos, bx, b))) return st;
             if ((st = nb_place(h, s, b, true, pairs_out, capacity, nullptr, 0, nullptr, 0))) return st;
             CK(cudaStreamSynchronize(s));
-            if (h->h_nbtot->max_h <= b.ell_cap_h) break;
+            if (h->h_nbtot->max_h <= b.slot_cap) break;
             grow = nb_headroom(h->h_nbtot->max_h);
         }
     } else if ((st = nb_count(h, s, p, pos, bx, b))) {
@@ -3160,10 +3143,10 @@ int dmffb_admp_build_neighbors(dmffb_engine* h, void* stream, const double* pos,
     if (p.flat || p.staged) {
         // a first build sizes slots and lists from the mean density and waits for its totals (the
         // caller may change the positions when it returns); later ones leave that to nb_finish
-        const bool first = !h->ell_cap_h || (want_csr && !h->ell_cap_f) || !h->d_pairs || (want_csr && !h->d_csr_ent);
+        const bool first = !h->slot_cap || !h->d_pairs || (want_csr && !h->d_csr_ent);
         if (first) {
             const int64_t rows = (int64_t)h->n * p.guess / 2 + 1;
-            if ((st = nb_slots(h, h->ell_cap_h ? 0 : p.guess, want_csr && !h->ell_cap_f ? p.guess : 0))) return st;
+            if (!h->slot_cap && (st = nb_slots(h, p.guess))) return st;
             if (!h->d_pairs && (st = nb_pair_cap(h, rows))) return st;
             if (want_csr && !h->d_csr_ent && (st = nb_csr_cap(h, 2 * rows))) return st;
         }

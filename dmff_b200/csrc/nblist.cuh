@@ -336,12 +336,12 @@ struct Nb2Args {
     // reads them instead of repeating the distance tests (null: no masks)
     uint32_t* mask = nullptr;
     int mask_stride = 0;
-    // slots of the single-pass kernels: each atom's full-list entries and half rows go to
-    // ell_ent[i * ell_cap_f + k] and ell_rows[3 (i * ell_cap_h + k)], which k_nb_place copies to the
-    // offsets of the true counts; slots past a capacity are dropped (the totals' maxima tell)
-    int32_t* ell_ent = nullptr;
-    int32_t* ell_rows = nullptr;
-    int ell_cap_f = 0, ell_cap_h = 0;
+    // slots of the single-pass kernels: each atom's entries (all its neighbours, or those j > i where no
+    // CSR is wanted) go to slots[i * slot_cap + k] as j | min(nbond, 7) << 28, which k_nb_place turns into
+    // rows and CSR entries at the offsets of the counts; slots past the capacity are dropped (the
+    // totals' maxima tell)
+    int32_t* slots = nullptr;
+    int slot_cap = 0;
 };
 
 // the FP32 box and prefilter bounds of a pair pass
@@ -415,40 +415,55 @@ __device__ __forceinline__ void nb_counts(const Nb2Args& b, int i, int nh, int n
     }
 }
 
-// One atom's slots: the warp appends a batch of candidates (keep: within rc) to the rows and the
-// CSR entries of atom i and advances its counts.
+// One atom's slots: the warp appends up to 32 neighbours (keep: the lane holds one) to the slots of
+// atom i and advances its counts.
 struct NbSlots {
-    int32_t *rows, *ent;
-    int cap_h, cap_f, nh = 0, nf = 0, ns = 0;
+    int32_t* slots;
+    int cap, nh = 0, nf = 0, ns = 0;
     int i, plo, phi;
+    bool all;  // both directions (CSR wanted)
     __device__ __forceinline__ NbSlots(const Nb2Args& b, int i_)
-        : rows(b.ell_rows + 3 * (int64_t)i_ * b.ell_cap_h), ent(b.ell_ent ? b.ell_ent + (int64_t)i_ * b.ell_cap_f : nullptr),
-          cap_h(b.ell_cap_h), cap_f(b.ell_cap_f), i(i_), plo(b.a.cov_lo ? b.a.cov_lo[i_] : 0),
-          phi(b.a.cov_hi ? b.a.cov_hi[i_] : b.a.n) {}
+        : slots(b.slots + (int64_t)i_ * b.slot_cap), cap(b.slot_cap), i(i_), plo(b.a.cov_lo ? b.a.cov_lo[i_] : 0),
+          phi(b.a.cov_hi ? b.a.cov_hi[i_] : b.a.n), all(b.count_f != nullptr) {}
     __device__ __forceinline__ void add(const Nb2Args& b, bool keep, int j, unsigned lt) {
-        const unsigned mf = __ballot_sync(0xffffffffu, keep);
-        if (mf == 0u) return;
-        const unsigned mh = __ballot_sync(0xffffffffu, keep && j > i);
-        bool scaled = false;
-        if (keep) {
-            const int nbd = nb_bond(b.a, i, j, plo, phi);
-            int sidx = nbd - 1;
-            if (sidx < 0) sidx += 6;
-            const int kf = nf + __popc(mf & lt);
-            if (ent && kf < cap_f) ent[kf] = j | (sidx << 28);
-            if (j > i) {
-                scaled = nbd != 0;
-                const int kh = nh + __popc(mh & lt);
-                if (kh < cap_h) {
-                    rows[3 * kh] = i;
-                    rows[3 * kh + 1] = j;
-                    rows[3 * kh + 2] = nbd;
-                }
-            }
+        const bool up = keep && j > i;
+        const unsigned mf = __ballot_sync(0xffffffffu, keep), mh = __ballot_sync(0xffffffffu, up);
+        int nbd = 0;
+        if (all ? keep : up) {
+            nbd = nb_bond(b.a, i, j, plo, phi);
+            const int k = all ? nf + __popc(mf & lt) : nh + __popc(mh & lt);
+            if (k < cap) slots[k] = j | (min(nbd, 7) << 28);
         }
         nf += __popc(mf);
         nh += __popc(mh);
-        ns += __popc(__ballot_sync(0xffffffffu, scaled));
+        ns += __popc(__ballot_sync(0xffffffffu, up && nbd != 0));
+    }
+};
+
+// Kept candidates wait in shared memory until 32 of them fill the lanes: about a quarter of a batch of
+// candidates is kept, and everything past the distance test runs once per 32 neighbours.
+struct NbQueue {
+    int* q;  // [64] of the warp
+    int n = 0;
+    __device__ __forceinline__ explicit NbQueue(int* q_) : q(q_) {}
+    __device__ __forceinline__ void push(NbSlots& out, const Nb2Args& b, bool keep, int j, int lane, unsigned lt) {
+        const unsigned m = __ballot_sync(0xffffffffu, keep);
+        if (keep) q[n + __popc(m & lt)] = j;
+        n += __popc(m);
+        if (n < 32) return;
+        __syncwarp();
+        out.add(b, true, q[lane], lt);
+        const int tail = q[32 + lane];
+        __syncwarp();
+        n -= 32;
+        if (lane < n) q[lane] = tail;
+        __syncwarp();
+    }
+    __device__ __forceinline__ void flush(NbSlots& out, const Nb2Args& b, int lane, unsigned lt) {
+        __syncwarp();
+        if (n) out.add(b, lane < n, q[lane], lt);
+        __syncwarp();
+        n = 0;
     }
 };
 
@@ -458,6 +473,7 @@ struct NbSlots {
 // more kernels over the rows.
 template <bool ORTHO>
 __global__ void __launch_bounds__(128) k_pairs_flat(Nb2Args b) {
+    __shared__ int s_q[4][64];
     const NbArgs& a = b.a;
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -466,15 +482,16 @@ __global__ void __launch_bounds__(128) k_pairs_flat(Nb2Args b) {
     const unsigned lt = (1u << lane) - 1u;
     const double pix = a.pos[3 * i], piy = a.pos[3 * i + 1], piz = a.pos[3 * i + 2];
     NbSlots out(b, i);
-#pragma unroll 4
+    NbQueue queue(s_q[threadIdx.x >> 5]);
     for (int j0 = 0; j0 < a.n; j0 += 32) {
         const int j = j0 + lane;
         bool keep = false;
         if (j < a.n && j != i)
             keep = nb_keep<ORTHO>(a, f, i, j, (float)(a.pos[3 * j] - pix), (float)(a.pos[3 * j + 1] - piy),
                                   (float)(a.pos[3 * j + 2] - piz));
-        out.add(b, keep, j, lt);
+        queue.push(out, b, keep, j, lane, lt);
     }
+    queue.flush(out, b, lane, lt);
     if (lane == 0) nb_counts(b, i, out.nh, out.nf, out.ns);
 }
 
@@ -592,60 +609,81 @@ __global__ void __launch_bounds__(32 * kNbWarps) k_pairs_warp3(Nb2Args b) {
     if (PASS == 0 && lane == 0) nb_counts(b, i, cnt_h, cnt_f, cnt_s);
 }
 
-// Block-per-cell single pass (same stencil, candidate order and tests as k_pairs_warp3): one
-// CTA takes every atom of one cell.  The cell's (2S + 1)^3 neighbourhood is laid out once per CTA
-// and, when it fits in `chmax` entries, staged in shared memory as (x, y, z, j) float4s, so the
-// cell's atoms read their candidates from shared memory instead of each gathering them from L2;
-// neighbourhoods larger than the stage fall back to the global gathers.  The NW warps of the CTA
-// take the cell's atoms in turn.
-template <int S, int NW, bool ORTHO>
+// Block-per-cell single pass over the (2S + 1)^3 stencil: one CTA takes every atom of one cell.  Cells of
+// a z column are contiguous in cell order, so the stencil is (2S + 1)^2 columns of one run of atoms, two
+// where the column wraps.  The runs are staged in shared memory as (x, y, z, j) float4s, shifted by the
+// lattice vectors their column wraps by: with in-box positions that is the image nearest to the cell's
+// atoms for every pair within rc (the box holds at least 2S + 1 cells of rc / S per axis), so a
+// candidate's test is one difference and one comparison for any box, candidates near rc taking the
+// exact FP64 test.  The NW warps of the CTA take the cell's atoms in turn.  Neighbourhoods larger than
+// `chmax` entries are read from global memory instead.
+// Bound by instruction issue: 49 us at 12288 atoms and rc 8 A, 101 at 30000.  With a minimum image per
+// candidate, the emission run once per batch of candidates, a cell search per staged entry and rows
+// and CSR entries in slots of their own it took 81 and 170.
+template <int S, int NW>
 __global__ void __launch_bounds__(32 * NW) k_pairs_cell(Nb2Args b, int chmax) {
-    constexpr int W = 2 * S + 1, NQ = W * W * W;
-    __shared__ int s_beg[NQ];
-    __shared__ int s_off[NQ + 1];
+    constexpr int W = 2 * S + 1, NC = W * W;
+    static_assert(NC <= 32, "a lane per column");
+    __shared__ int s_beg[2 * NC], s_off[2 * NC + 1];
+    __shared__ float s_sh[2 * NC][3];
+    __shared__ int s_q[NW][64];
     extern __shared__ __align__(16) float4 s_cand[];
     const NbArgs& a = b.a;
     const int c = blockIdx.x;
     const int cs0 = a.cell_start[c], m = a.cell_start[c + 1] - cs0;
     if (m == 0) return;  // whole CTA
     const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int c3[3] = {c / (a.nc[2] * a.nc[1]), (c / a.nc[2]) % a.nc[1], c % a.nc[2]};
     if (wl == 0) {
-        int carry = 0;
-        if (lane == 0) s_off[0] = 0;
-        for (int q0 = 0; q0 < NQ; q0 += 32) {
-            const int q = q0 + lane;
-            int cnt = 0;
-            if (q < NQ) {
-                const int dx = q / (W * W) - S, dy = (q / W) % W - S, dz = q % W - S;
-                const int cx = (c3[0] + dx + a.nc[0]) % a.nc[0];
-                const int cy = (c3[1] + dy + a.nc[1]) % a.nc[1];
-                const int cz = (c3[2] + dz + a.nc[2]) % a.nc[2];
-                const int cc = (cx * a.nc[1] + cy) * a.nc[2] + cz;
-                const int cs = a.cell_start[cc];
-                cnt = a.cell_start[cc + 1] - cs;
-                s_beg[q] = cs;
-            }
-            int incl = cnt;
+        const int c2 = c % a.nc[2], c1 = (c / a.nc[2]) % a.nc[1], c0 = c / (a.nc[2] * a.nc[1]);
+        int cnt[2] = {0, 0};
+        if (lane < NC) {
+            int x = c0 + lane / W - S, y = c1 + lane % W - S;
+            const int nx = x < 0 ? -1 : (x >= a.nc[0] ? 1 : 0), ny = y < 0 ? -1 : (y >= a.nc[1] ? 1 : 0);
+            x -= nx * a.nc[0];
+            y -= ny * a.nc[1];
+            const int* col = a.cell_start + (x * a.nc[1] + y) * a.nc[2];
+            // [z0, z1] inside the box and, wrapped by nz, the rest
+            const int z0 = max(c2 - S, 0), z1 = min(c2 + S, a.nc[2] - 1);
+            const int nz = c2 - S < 0 ? -1 : (c2 + S >= a.nc[2] ? 1 : 0);
+            const int w0 = nz < 0 ? c2 - S + a.nc[2] : 0, w1 = nz < 0 ? a.nc[2] - 1 : c2 + S - a.nc[2];
+            s_beg[2 * lane] = col[z0];
+            cnt[0] = col[z1 + 1] - col[z0];
+            s_beg[2 * lane + 1] = nz ? col[w0] : 0;
+            cnt[1] = nz ? col[w1 + 1] - col[w0] : 0;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int v = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += v;
+            for (int k = 0; k < 3; ++k) {
+                const double sh = nx * a.box.h[k] + ny * a.box.h[3 + k];
+                s_sh[2 * lane][k] = (float)sh;
+                s_sh[2 * lane + 1][k] = (float)(sh + nz * a.box.h[6 + k]);
             }
-            if (q < NQ) s_off[q + 1] = carry + incl;
-            carry += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        int incl = cnt[0] + cnt[1];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        if (lane < NC) {
+            s_off[2 * lane] = incl - cnt[0] - cnt[1];
+            s_off[2 * lane + 1] = incl - cnt[1];
+            if (lane == NC - 1) s_off[2 * NC] = incl;
         }
     }
     __syncthreads();
-    const int total = s_off[NQ];
+    const int total = s_off[2 * NC];
     const bool staged = total <= chmax;
-    if (staged) {
-        int qc = 0;
-        for (int t = threadIdx.x; t < total; t += blockDim.x) {
-            while (t >= s_off[qc + 1]) ++qc;
-            s_cand[t] = b.posc[s_beg[qc] + (t - s_off[qc])];
+    auto candidate = [&](int run, int k) {
+        float4 p = b.posc[s_beg[run] + k];
+        p.x += s_sh[run][0];
+        p.y += s_sh[run][1];
+        p.z += s_sh[run][2];
+        return p;
+    };
+    if (staged)
+        for (int run = wl; run < 2 * NC; run += NW) {
+            const int off = s_off[run], cnt = s_off[run + 1] - off;
+            for (int k = lane; k < cnt; k += 32) s_cand[off + k] = candidate(run, k);
         }
-    }
     __syncthreads();
     const NbFilter f(a);
     const unsigned lt = (1u << lane) - 1u;
@@ -653,62 +691,69 @@ __global__ void __launch_bounds__(32 * NW) k_pairs_cell(Nb2Args b, int chmax) {
         const float4 p4 = b.posc[cs0 + ai];
         const int i = __float_as_int(p4.w);
         NbSlots out(b, i);
-        int qc = 0;
-        for (int base = 0; base < total; base += 32) {
-            const int t = base + lane;
-            bool keep = false;
-            int j = -1;
-            if (t < total) {
-                float4 pj;
-                if (staged) {
-                    pj = s_cand[t];
-                } else {
-                    while (t >= s_off[qc + 1]) ++qc;
-                    pj = b.posc[s_beg[qc] + (t - s_off[qc])];
+        NbQueue queue(s_q[wl]);
+        auto test = [&](const float4& pj) {
+            const float dx = pj.x - p4.x, dy = pj.y - p4.y, dz = pj.z - p4.z;
+            const float r2 = dx * dx + dy * dy + dz * dz;
+            const int j = __float_as_int(pj.w);
+            if (r2 > f.rhi2 || j == i) return false;
+            if (r2 < f.rlo2) return true;
+            return j > i ? within_rc(a.box, a.pos + 3 * i, a.pos + 3 * j, a.rc)
+                         : within_rc(a.box, a.pos + 3 * j, a.pos + 3 * i, a.rc);
+        };
+        if (staged) {
+            for (int base = 0; base < total; base += 32) {
+                const int t = base + lane;
+                bool keep = false;
+                int j = -1;
+                if (t < total) {
+                    const float4 pj = s_cand[t];
+                    j = __float_as_int(pj.w);
+                    keep = test(pj);
                 }
-                j = __float_as_int(pj.w);
-                if (j != i) keep = nb_keep<ORTHO>(a, f, i, j, pj.x - p4.x, pj.y - p4.y, pj.z - p4.z);
+                queue.push(out, b, keep, j, lane, lt);
             }
-            out.add(b, keep, j, lt);
+        } else {
+            for (int run = 0; run < 2 * NC; ++run) {
+                const int cnt = s_off[run + 1] - s_off[run];
+                for (int base = 0; base < cnt; base += 32) {
+                    const int k = base + lane;
+                    bool keep = false;
+                    int j = -1;
+                    if (k < cnt) {
+                        const float4 pj = candidate(run, k);
+                        j = __float_as_int(pj.w);
+                        keep = test(pj);
+                    }
+                    queue.push(out, b, keep, j, lane, lt);
+                }
+            }
         }
+        queue.flush(out, b, lane, lt);
         if (lane == 0) nb_counts(b, i, out.nh, out.nf, out.ns);
     }
 }
 
-// Offsets from the counts, and the slots copied there.  A CTA takes kPlaceAtoms atoms: it sums the
-// run sums before their run and the counts of the run's earlier atoms, scans its own, copies each
-// atom's rows and CSR entries (as flat runs of words) and the indices of its rows with nbond != 0,
-// all in atom order; the CTA of the last atom writes the totals.  Nothing is written past a
-// capacity: the caller compares the totals before it uses the lists.  Bound by the copies' latency (42
-// MB moved at 12288 atoms and rc 8 A): 22 us there, one launch for two memsets, two two-kernel
-// scans, a copy kernel and a library selection over all rows that took 47 us and two more host
-// round trips.  A warp per atom: with four atoms per warp in turn it took 38 us at 4000 atoms
-// against 10.
-constexpr int kPlaceAtoms = 8, kPlaceThreads = 32 * kPlaceAtoms;  // a warp per atom
+// Offsets from the counts, and the slots turned into rows and CSR entries there.  A CTA takes kPlaceAtoms
+// atoms, a warp each: it sums the run sums before their run and the counts of the run's earlier atoms,
+// scans its own, and writes each atom's rows, CSR entries and the indices of its rows with nbond != 0,
+// all in atom order; the CTA of the last atom writes the totals.  Nothing is written past a capacity: the
+// caller compares the totals before it uses the lists.  Bound by latency and the writes: 18 us at 12288
+// atoms (22 copying rows and entries from slots of their own), for two memsets, two two-kernel scans, a copy kernel and a library selection over all rows that took 47 us and
+// two more host round trips.
+constexpr int kPlaceAtoms = 8, kPlaceThreads = 32 * kPlaceAtoms;
 static_assert(kNbRun % kPlaceAtoms == 0, "a CTA's atoms lie in one run");
-
-// one warp: n words from src to dst, four loads in flight per lane
-__device__ __forceinline__ void nb_copy(int32_t* __restrict__ dst, const int32_t* __restrict__ src, int n, int lane) {
-    int k = lane;
-    for (; k + 96 < n; k += 128) {
-        const int32_t v0 = src[k], v1 = src[k + 32], v2 = src[k + 64], v3 = src[k + 96];
-        dst[k] = v0;
-        dst[k + 32] = v1;
-        dst[k + 64] = v2;
-        dst[k + 96] = v3;
-    }
-    for (; k < n; k += 32) dst[k] = src[k];
-}
 
 struct PlaceArgs {
     int n;
-    const int32_t *count_h, *count_f, *count_s;  // count_f null: no CSR
+    NbArgs cov;                                  // the covalent map (nbond past a slot's three bits)
+    const int32_t *count_h, *count_f, *count_s;  // count_f null: no CSR, the slots hold j > i alone
     const int32_t* sums;                         // [3][runs]
     NbTotals* tot;                               // max_h, max_f zero on entry
     int64_t *off_h, *off_f;                      // [n+1]; off_f null: no CSR
     int32_t* off_s;                              // [n]
-    const int32_t *ell_rows, *ell_ent;           // null: offsets and totals only
-    int cap_h, cap_f;
+    const int32_t* slots;                        // null: offsets and totals only
+    int slot_cap;
     int32_t* rows;
     int64_t rows_cap;
     int32_t* ent;
@@ -769,31 +814,47 @@ static __global__ void __launch_bounds__(kPlaceThreads) k_nb_place(PlaceArgs a) 
         if (lane == 0 && k == 0) atomicMax(&a.tot->max_h, mx);
         if (lane == 0 && k == 1) atomicMax(&a.tot->max_f, mx);
     }
-    if (!a.ell_rows) return;  // whole grid
+    if (!a.slots) return;  // whole grid
     __syncthreads();
     const int i = a0 + wl;
     if (i >= a.n) return;
-    const int nh = min(a.count_h[i], a.cap_h);
-    const int32_t* const src = a.ell_rows + 3 * (int64_t)i * a.cap_h;
-    const int64_t bh = s_off[0][wl];
-    if (a.rows) {
-        const int64_t room = 3 * (a.rows_cap - bh);
-        nb_copy(a.rows + 3 * bh, src, (int)min((int64_t)(3 * nh), room > 0 ? room : (int64_t)0), lane);
-    }
-    if (a.ent) {
-        const int64_t bf = s_off[1][wl], room = a.ent_cap - bf;
-        nb_copy(a.ent + bf, a.ell_ent + (int64_t)i * a.cap_f,
-                (int)min((int64_t)min(a.count_f[i], a.cap_f), room > 0 ? room : (int64_t)0), lane);
-    }
-    if (a.srows && a.count_s[i] > 0) {
-        int64_t at = s_off[2][wl];
-        for (int k0 = 0; k0 < nh; k0 += 32) {
-            const int k = k0 + lane;
-            const bool sc = k < nh && src[3 * k + 2] != 0;
-            const unsigned ms = __ballot_sync(0xffffffffu, sc);
-            const int64_t p = at + __popc(ms & ((1u << lane) - 1u));
-            if (sc && p < a.srows_cap) a.srows[p] = (int32_t)(bh + k);
-            at += __popc(ms);
+    const int32_t* const src = a.slots + (int64_t)i * a.slot_cap;
+    const int ns = min(a.count_f ? a.count_f[i] : a.count_h[i], a.slot_cap);
+    int64_t bh = s_off[0][wl], bs = s_off[2][wl];
+    const int64_t bf = a.count_f ? s_off[1][wl] : 0;
+    const unsigned lt = (1u << lane) - 1u;
+    constexpr int U = 4;  // slot loads in flight per lane
+    for (int k0 = 0; k0 < ns; k0 += 32 * U) {
+        int32_t v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int k = k0 + 32 * u + lane;
+            v[u] = k < ns ? src[k] : -1;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int k = k0 + 32 * u + lane;
+            const bool ok = k < ns;
+            const int j = v[u] & 0x0FFFFFFF;
+            int nbd = (v[u] >> 28) & 7;
+            if (ok && nbd == 7) nbd = j > i ? lookup_nbond(a.cov, i, j) : lookup_nbond(a.cov, j, i);
+            int sidx = nbd - 1;
+            if (sidx < 0) sidx += 6;
+            if (ok && a.ent && bf + k < a.ent_cap) a.ent[bf + k] = j | (sidx << 28);
+            const bool up = ok && j > i;
+            const unsigned mh = __ballot_sync(0xffffffffu, up), ms = __ballot_sync(0xffffffffu, up && nbd != 0);
+            if (up) {
+                const int64_t r = bh + __popc(mh & lt);
+                if (a.rows && r < a.rows_cap) {
+                    a.rows[3 * r] = i;
+                    a.rows[3 * r + 1] = j;
+                    a.rows[3 * r + 2] = nbd;
+                }
+                const int64_t p = bs + __popc(ms & lt);
+                if (nbd != 0 && a.srows && p < a.srows_cap) a.srows[p] = (int32_t)r;
+            }
+            bh += __popc(mh);
+            bs += __popc(ms);
         }
     }
 }
