@@ -106,6 +106,9 @@ struct PrepArgs {
     T* posT;             // [n*4]
     T* QgT;              // [n*9]
     double* Qg;          // [n*9]
+    const T* thole;      // [n] (null without polarizabilities)
+    const T* polsix;     // [n]
+    Vec4<T>* rec;        // [n*4] what the pair passes read of a site (PairArgs)
     ClearList clear;     // what the evaluation starts from zero
 };
 
@@ -153,6 +156,11 @@ __global__ void k_prepare(PrepArgs<T> a) {
         a.Qg[9 * at + k] = q[k];
         a.QgT[9 * at + k] = (T)q[k];
     }
+    const T th = a.thole ? a.thole[at] : T(0), ps = a.polsix ? a.polsix[at] : T(0);
+    a.rec[4 * at] = Vec4<T>{(T)p[0], (T)p[1], (T)p[2], th};
+    a.rec[4 * at + 1] = Vec4<T>{(T)q[0], (T)q[1], (T)q[2], (T)q[3]};
+    a.rec[4 * at + 2] = Vec4<T>{(T)q[4], (T)q[5], (T)q[6], (T)q[7]};
+    a.rec[4 * at + 3] = Vec4<T>{(T)q[8], ps, T(0), T(0)};
 }
 
 template <typename T>
@@ -161,7 +169,7 @@ struct SelfArgs {
     const double* Qg;     // [n*9]
     const double* U;      // [n*3] or null
     const double* pol;    // [n] or null
-    const T* torque;      // [n*3] accumulated torques (real + recip)
+    const T* torque;      // [n*4] accumulated torques (real + recip)
     double kappa;
     int lmax_eff;
     int lpme;
@@ -191,7 +199,7 @@ __global__ void __launch_bounds__(128) k_self_frames(SelfArgs<T> a) {
         const double D = DMFFB_DIELECTRIC;
         double Ux = 0, Uy = 0, Uz = 0;
         if (a.U) { Ux = a.U[3 * at]; Uy = a.U[3 * at + 1]; Uz = a.U[3 * at + 2]; }
-        double tau[3] = {(double)a.torque[3 * at], (double)a.torque[3 * at + 1], (double)a.torque[3 * at + 2]};
+        double tau[3] = {(double)a.torque[4 * at], (double)a.torque[4 * at + 1], (double)a.torque[4 * at + 2]};
         if (a.lpme) {
             const double k = a.kappa;
             const double f0 = k / 1.7724538509055159;
@@ -330,7 +338,7 @@ template <typename T>
 __global__ void k_finalize_forces(int n, const T* gpair, const double* gd, double* forces) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= 3 * n) return;
-    forces[k] = -((double)gpair[k] + gd[k]);
+    forces[k] = -((double)gpair[4 * (k / 3) + k % 3] + gd[k]);
 }
 
 }  // namespace dmffb

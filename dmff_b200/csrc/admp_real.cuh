@@ -27,6 +27,8 @@ struct PairArgs {
     int64_t npairs;
     const int32_t* pairs;  // [npairs*3]
     const T* pos;          // [n*4]
+    const Vec4<T>* rec;    // [n*4] position and Thole width, multipoles 0..3, 4..7, 8 and pol^(1/6)
+    const Vec4<T>* U4;     // [n] U in kernel precision (FULL with induced dipoles, else null)
     const double* posd;    // [n*3] FP64 positions (FP64 rows)
     const T* Qg;           // [n*9] permanent multipoles, global harmonic
     const double* Qgd;     // [n*9] the same in FP64
@@ -36,9 +38,9 @@ struct PairArgs {
     T ms[6], ps[6], dsc[6];
     T kappa;
     Box boxd;
-    T* grad;     // [n*3]  dE/dpos
-    T* torque;   // [n*3]  global torque of the permanent multipoles
-    T* field;    // [n*3]  dE/dU (FIELD, MATVEC)
+    T* grad;     // [n*4]  dE/dpos
+    T* torque;   // [n*4]  global torque of the permanent multipoles
+    T* field;    // [n*4]  dE/dU (FIELD)
     double* scal;  // [0] energy, [1..9] box gradient
     int want_box;
     const int32_t* rowmap = nullptr;  // ROWS_SCALED launches: indices of the rows with nbond != 0
@@ -498,19 +500,48 @@ __device__ __forceinline__ void pair_eval_pgrad(const TC dr[3], const TC* QIg, c
     rot9T(gJ, ex, ey, ez, C, GJ);
 }
 
-// load one row's inputs in arithmetic TC and evaluate it
+// load one row's inputs in arithmetic TC and evaluate it: in kernel precision from the sites' records
+// (five vector loads a site), FP64 rows of FP32 engines from the FP64 arrays
 template <typename TC, typename T, bool POL, int MODE>
 __device__ __forceinline__ void pair_row(const PairArgs<T>& a, int i, int j, int nb, TC oi[6], TC oj[6], double& e,
                                          TC nimg[3]) {
-    TC dr[3];
-    if (sizeof(TC) > sizeof(T)) {
+    TC dr[3], QI[9], QJ[9], thi, thj, psi, psj;
+    TC UI[3] = {TC(0), TC(0), TC(0)}, UJ[3] = {TC(0), TC(0), TC(0)};
+    if constexpr (sizeof(TC) > sizeof(T)) {
         dr[0] = (TC)(a.posd[3 * i] - a.posd[3 * j]);
         dr[1] = (TC)(a.posd[3 * i + 1] - a.posd[3 * j + 1]);
         dr[2] = (TC)(a.posd[3 * i + 2] - a.posd[3 * j + 2]);
+#pragma unroll
+        for (int k = 0; k < 9; ++k) { QI[k] = (TC)a.Qgd[9 * i + k]; QJ[k] = (TC)a.Qgd[9 * j + k]; }
+        if (POL && a.U) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) { UI[c] = (TC)a.U[3 * i + c]; UJ[c] = (TC)a.U[3 * j + c]; }
+        }
+        if (POL) {
+            thi = (TC)a.thole[i];
+            thj = (TC)a.thole[j];
+            psi = (TC)a.polsix[i];
+            psj = (TC)a.polsix[j];
+        }
     } else {
-        dr[0] = (TC)(a.pos[4 * i] - a.pos[4 * j]);
-        dr[1] = (TC)(a.pos[4 * i + 1] - a.pos[4 * j + 1]);
-        dr[2] = (TC)(a.pos[4 * i + 2] - a.pos[4 * j + 2]);
+        const Vec4<T>*ri = a.rec + 4 * (int64_t)i, *rj = a.rec + 4 * (int64_t)j;
+        const Vec4<T> pi = ri[0], pj = rj[0], i1 = ri[1], j1 = rj[1], i2 = ri[2], j2 = rj[2], i3 = ri[3], j3 = rj[3];
+        dr[0] = pi.x - pj.x;
+        dr[1] = pi.y - pj.y;
+        dr[2] = pi.z - pj.z;
+        QI[0] = i1.x; QI[1] = i1.y; QI[2] = i1.z; QI[3] = i1.w;
+        QI[4] = i2.x; QI[5] = i2.y; QI[6] = i2.z; QI[7] = i2.w; QI[8] = i3.x;
+        QJ[0] = j1.x; QJ[1] = j1.y; QJ[2] = j1.z; QJ[3] = j1.w;
+        QJ[4] = j2.x; QJ[5] = j2.y; QJ[6] = j2.z; QJ[7] = j2.w; QJ[8] = j3.x;
+        thi = pi.w;
+        thj = pj.w;
+        psi = i3.y;
+        psj = j3.y;
+        if (POL && a.U4) {
+            const Vec4<T> ui = a.U4[i], uj = a.U4[j];
+            UI[0] = ui.x; UI[1] = ui.y; UI[2] = ui.z;
+            UJ[0] = uj.x; UJ[1] = uj.y; UJ[2] = uj.z;
+        }
     }
     BoxT<TC> bx;
 #pragma unroll
@@ -519,26 +550,11 @@ __device__ __forceinline__ void pair_row(const PairArgs<T>& a, int i, int j, int
     int sidx = nb - 1;  // scale index nbond-1, Python-style wrap (nbond 0 -> trailing 1.0), clamped
     if (sidx < 0) sidx += 6;
     sidx = sidx < 0 ? 0 : (sidx > 5 ? 5 : sidx);
-    TC QI[9], QJ[9];
-    if (MODE != PAIR_MATVEC) {
-        if (sizeof(TC) > sizeof(T)) {
-#pragma unroll
-            for (int k = 0; k < 9; ++k) { QI[k] = (TC)a.Qgd[9 * i + k]; QJ[k] = (TC)a.Qgd[9 * j + k]; }
-        } else {
-#pragma unroll
-            for (int k = 0; k < 9; ++k) { QI[k] = (TC)a.Qg[9 * i + k]; QJ[k] = (TC)a.Qg[9 * j + k]; }
-        }
-    }
-    TC UI[3] = {TC(0), TC(0), TC(0)}, UJ[3] = {TC(0), TC(0), TC(0)};
-    if (POL && a.U) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) { UI[c] = (TC)a.U[3 * i + c]; UJ[c] = (TC)a.U[3 * j + c]; }
-    }
     TC Ath = TC(0), dmp = TC(1);
     const TC pp = (TC)a.ps[sidx], dsv = (TC)a.dsc[sidx];
     if (POL) {
-        Ath = pp > TC(0) ? TC(5.0) : (TC)a.thole[i] + (TC)a.thole[j];
-        dmp = (TC)a.polsix[i] * (TC)a.polsix[j];
+        Ath = pp > TC(0) ? TC(5.0) : thi + thj;
+        dmp = psi * psj;
         dmp = dmp < TC(1e-8) ? TC(1e-8) : dmp;
     }
     pair_eval<TC, POL, MODE>(dr, QI, QJ, UI, UJ, (TC)a.ms[sidx], pp, dsv, Ath, dmp, (TC)a.kappa, oi, oj, e);
@@ -549,6 +565,10 @@ __device__ __forceinline__ void pair_row(const PairArgs<T>& a, int i, int j, int
 // are evaluated in FP64 even in the FP32 instantiation.
 enum { ROWS_ALL = 0, ROWS_UNSCALED = 1, ROWS_SCALED = 2 };
 
+// Issue-bound.  A site is five vector loads (its record and dipole) and a force or torque on it one
+// vector reduction; gathering it in 17 scalar loads, with scalar atomics, run tests per summed value and
+// butterflies per reduced value, the FP32 FULL pass took 61 us at 6144 atoms and 11.6 at 450, FIELD
+// 28 and 9.3; now 49 and 5.3, 19 and 4.2.
 // ROWS selects which rows this launch evaluates: all of them, only nbond == 0 rows (FP32
 // arithmetic) or only nbond != 0 rows (always FP64); the FP32 engine launches the last two so
 // that no warp mixes the two arithmetic paths.
@@ -588,27 +608,19 @@ __global__ void __launch_bounds__(128, (sizeof(T) == 4 && ROWS == ROWS_UNSCALED 
         }
     }
 
-    // ---- accumulate
-    const int nout = (MODE == PAIR_FULL) ? 6 : 3;
+    // ---- accumulate: a vector reduction per site and quantity
     T* outp = (MODE == PAIR_FULL) ? a.grad : a.field;
-    const bool head = seg_head(key);
-    const int run = seg_run_id(key);
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-        if (k >= nout) break;
-        T s = seg_sum(oi[k], run);
-        if (head && key >= 0) {
-            T* dst = (k < 3) ? (outp + 3 * key + k) : (a.torque + 3 * key + (k - 3));
-            atomicAdd(dst, s);
-        }
+    const bool head = seg_head(key) && key >= 0;
+    const unsigned reach = seg_reach(seg_run_id(key));
+    {
+        const T s0 = seg_sum(oi[0], reach), s1 = seg_sum(oi[1], reach), s2 = seg_sum(oi[2], reach);
+        if (head) add3(outp + 4 * (int64_t)key, s0, s1, s2);
+        if (valid) add3(outp + 4 * (int64_t)j, oj[0], oj[1], oj[2]);
     }
-    if (valid) {
-#pragma unroll
-        for (int k = 0; k < 6; ++k) {
-            if (k >= nout) break;
-            T* dst = (k < 3) ? (outp + 3 * j + k) : (a.torque + 3 * j + (k - 3));
-            atomicAdd(dst, oj[k]);
-        }
+    if (MODE == PAIR_FULL) {
+        const T s3 = seg_sum(oi[3], reach), s4 = seg_sum(oi[4], reach), s5 = seg_sum(oi[5], reach);
+        if (head) add3(a.torque + 4 * (int64_t)key, s3, s4, s5);
+        if (valid) add3(a.torque + 4 * (int64_t)j, oj[3], oj[4], oj[5]);
     }
     if (MODE == PAIR_FULL) {
         double red[10];
@@ -696,11 +708,11 @@ __global__ void __launch_bounds__(128) k_admp_pgrad(PgradArgs<T> g) {
         else pgrad_row<T, T, POL>(a, i, j, nb, oi, oj);
     }
     const bool head = seg_head(key);
-    const int run = seg_run_id(key);
+    const unsigned reach = seg_reach(seg_run_id(key));
 #pragma unroll
     for (int k = 0; k < 11; ++k) {
         if (!POL && k >= 9) break;
-        const double s = seg_sum(oi[k], run);
+        const double s = seg_sum(oi[k], reach);
         if (head && key >= 0) {
             double* dst = k < 9 ? g.dQ + 9 * key + k : (k == 9 ? g.dpa + key : g.dth + key);
             atomicAdd(dst, s);
@@ -755,10 +767,6 @@ __global__ void k_csr_fill(int64_t npairs, const int32_t* pairs, int n, const in
 // are evaluated once (k_matvec_coef) and each CG iteration only streams them (k_matvec_apply).  A pair
 // tensor is c0 1 + c1 e e^T (c0 = udud1, c1 = udud0 - udud1, e the pair direction); it is kept as c0 and
 // f = sqrt(|c1|) e, one vector load, with the sign of c1 in bit 31 of the entry.
-template <typename T>
-struct __align__(4 * sizeof(T)) Vec4 {
-    T x, y, z, w;
-};
 template <typename T>
 using MvCoef = Vec4<T>;  // f.x, f.y, f.z, c0
 

@@ -378,40 +378,11 @@ struct GatherArgs {
     const T* phi;         // convolved mesh (real)
     double scale;         // dE/dmesh = scale * phi   (2*DIELECTRIC or 2)
     double* grad;         // [n*3] += dE/dpos
-    T* torque;            // [n*3] += torque of permanent multipoles (may be null)
+    T* torque;            // [n*4] += torque of permanent multipoles (may be null)
     double* gQ;           // [n*9] += dE/dQ_global (may be null)
     double* dq1;          // [n] += dE/dq for the charge channel (may be null)
     double* scal;         // [0] energy (1/2 sum c P), [1..9] X_NA
 };
-
-// Sums NS values over the warp by recursive halving: at each of the five steps a lane hands one half
-// of what it holds to its partner and keeps the other, so 20 values take 21 exchanges where a
-// butterfly per value takes 100.  The lanes that end up holding a sum write it to out[0 .. NS).
-template <typename T, int NS>
-__device__ __forceinline__ void warp_sums(T (&v)[NS], T* out, int lane) {
-    int idx = 0, sz = NS;
-    constexpr int H[5] = {(NS + 1) / 2, ((NS + 1) / 2 + 1) / 2, (((NS + 1) / 2 + 1) / 2 + 1) / 2,
-                          ((((NS + 1) / 2 + 1) / 2 + 1) / 2 + 1) / 2,
-                          (((((NS + 1) / 2 + 1) / 2 + 1) / 2 + 1) / 2 + 1) / 2};
-#pragma unroll
-    for (int step = 0; step < 5; ++step) {
-        const int n = step == 0 ? NS : H[step - 1], h = H[step], o = 16 >> step;
-        const bool up = (lane & o) != 0;
-#pragma unroll
-        for (int k = 0; k < NS; ++k) {
-            if (k >= h) break;
-            const T lo = v[k], hi = k + h < n ? v[k + h < NS ? k + h : 0] : T(0);
-            v[k] = (up ? hi : lo) + __shfl_xor_sync(0xffffffffu, up ? lo : hi, o);
-        }
-        if (up) {
-            idx += h;
-            sz = max(sz - h, 0);
-        } else {
-            sz = min(sz, h);
-        }
-    }
-    if (sz >= 1) out[idx] = v[0];
-}
 
 // Interpolation of the convolved mesh and its derivatives at the sites (CH: charges alone, value and
 // first derivatives), then dE/dpos, dE/dQ, torques and the box term.  A warp takes a site: lanes
@@ -605,9 +576,7 @@ __global__ void __launch_bounds__(kSiteThreads) k_gather(GatherArgs<T> a, int ap
                 if (a.lmax < 1) { qp[1] = qp[2] = qp[3] = T(0); }
                 torque9(qp, gT, t);
                 // atomics: the real-space FULL pass may add to the same torques concurrently
-                atomicAdd(a.torque + 3 * at, t[0]);
-                atomicAdd(a.torque + 3 * at + 1, t[1]);
-                atomicAdd(a.torque + 3 * at + 2, t[2]);
+                add3(a.torque + 4 * at, t[0], t[1], t[2]);
             }
             {
                 // X_NA = Y (x) R + (dE/dB)^T,  dE/dB = -Pu (x) mu + 2 P2 B Theta

@@ -166,15 +166,15 @@ __global__ void __launch_bounds__(128) k_nb_pair(NbPairArgs<T> a) {
         }
     }
     const bool head = seg_head(key);
-    const int run = seg_run_id(key);
+    const unsigned reach = seg_reach(seg_run_id(key));
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        const T s1 = seg_sum(g[c], run);
+        const T s1 = seg_sum(g[c], reach);
         if (head && key >= 0) atomicAdd(a.grad + 3 * key + c, s1);
         if (valid) atomicAdd(a.grad + 3 * j + c, -g[c]);
     }
     if (a.dq) {
-        const double dqi = seg_sum(valid ? phi_ij * a.q[j] : 0.0, run);
+        const double dqi = seg_sum(valid ? phi_ij * a.q[j] : 0.0, reach);
         if (head && key >= 0) atomicAdd(a.dq + key, dqi);
     }
     block_reduce_add<11>(red, a.scal);

@@ -42,6 +42,22 @@ template <typename T> __device__ __forceinline__ Dl<T> operator*(Dl<T> a, T s) {
 template <typename T> __device__ __forceinline__ Dl<T> operator+(Dl<T> a, T s) { return Dl<T>(a.v + s, a.d); }
 template <typename T> __device__ __forceinline__ Dl<T> operator-(Dl<T> a, T s) { return Dl<T>(a.v - s, a.d); }
 
+// ------------------------------------------------------------------ vectors
+template <typename T>
+struct __align__(4 * sizeof(T)) Vec4 {
+    T x, y, z, w;
+};
+
+// g[0..2] += (x, y, z) for a 4-element slot: one 16-byte reduction in FP32
+__device__ __forceinline__ void add3(float* g, float x, float y, float z) {
+    atomicAdd((float4*)g, make_float4(x, y, z, 0.f));
+}
+__device__ __forceinline__ void add3(double* g, double x, double y, double z) {
+    atomicAdd(g, x);
+    atomicAdd(g + 1, y);
+    atomicAdd(g + 2, z);
+}
+
 // ------------------------------------------------------------------ warp helpers
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -68,16 +84,54 @@ __device__ __forceinline__ int seg_run_id(int key) {
     const unsigned heads = __ballot_sync(0xffffffffu, seg_head(key));
     return __popc(heads & (0xffffffffu >> (31 - lane)));
 }
-template <typename T>
-__device__ __forceinline__ T seg_sum(T v, int run) {
+// seg_sum takes the lanes' run relations from seg_reach: bit k set where lane + 2^k belongs to the run
+__device__ __forceinline__ unsigned seg_reach(int run) {
     const int lane = threadIdx.x & 31;
+    unsigned m = 0u;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        T ov = __shfl_down_sync(0xffffffffu, v, o);
-        int orun = __shfl_down_sync(0xffffffffu, run, o);
-        if (lane + o < 32 && orun == run) v += ov;
+    for (int k = 0; k < 5; ++k) {
+        const int o = 1 << k, other = __shfl_down_sync(0xffffffffu, run, o);
+        if (lane + o < 32 && other == run) m |= 1u << k;
+    }
+    return m;
+}
+template <typename T>
+__device__ __forceinline__ T seg_sum(T v, unsigned reach) {
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+        const T ov = __shfl_down_sync(0xffffffffu, v, 1 << k);
+        if ((reach >> k) & 1u) v += ov;
     }
     return v;
+}
+
+// Sums NS values over the warp by recursive halving: at each of the five steps a lane hands one half
+// of what it holds to its partner and keeps the other, so 20 values take 21 exchanges where a
+// butterfly per value takes 100.  The lanes that end up holding a sum write it to out[0 .. NS).
+template <typename T, int NS>
+__device__ __forceinline__ void warp_sums(T (&v)[NS], T* out, int lane) {
+    int idx = 0, sz = NS;
+    constexpr int H[5] = {(NS + 1) / 2, ((NS + 1) / 2 + 1) / 2, (((NS + 1) / 2 + 1) / 2 + 1) / 2,
+                          ((((NS + 1) / 2 + 1) / 2 + 1) / 2 + 1) / 2,
+                          (((((NS + 1) / 2 + 1) / 2 + 1) / 2 + 1) / 2 + 1) / 2};
+#pragma unroll
+    for (int step = 0; step < 5; ++step) {
+        const int n = step == 0 ? NS : H[step - 1], h = H[step], o = 16 >> step;
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int k = 0; k < NS; ++k) {
+            if (k >= h) break;
+            const T lo = v[k], hi = k + h < n ? v[k + h < NS ? k + h : 0] : T(0);
+            v[k] = (up ? hi : lo) + __shfl_xor_sync(0xffffffffu, up ? lo : hi, o);
+        }
+        if (up) {
+            idx += h;
+            sz = max(sz - h, 0);
+        } else {
+            sz = min(sz, h);
+        }
+    }
+    if (sz >= 1) out[idx] = v[0];
 }
 
 // block-wide reduction of NV doubles into dst[] with one atomicAdd per value per block
@@ -85,20 +139,23 @@ template <int NV>
 __device__ __forceinline__ void block_reduce_add(double (&v)[NV], double* dst) {
     __shared__ double sh[32][NV];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-    for (int k = 0; k < NV; ++k) v[k] = warp_sum(v[k]);
-    if (lane == 0) {
-#pragma unroll
-        for (int k = 0; k < NV; ++k) sh[wid][k] = v[k];
+    if (NV == 1) {
+        const double t = warp_sum(v[0]);
+        if (lane == 0) sh[wid][0] = t;
+    } else {
+        warp_sums<double, NV>(v, sh[wid], lane);
     }
     __syncthreads();
     const int nw = (blockDim.x + 31) >> 5;
     if (wid == 0) {
-#pragma unroll
-        for (int k = 0; k < NV; ++k) {
-            double s = lane < nw ? sh[lane][k] : 0.0;
-            s = warp_sum(s);
-            if (lane == 0 && s != 0.0) atomicAdd(dst + k, s);
+        if (NV == 1) {
+            double t = lane < nw ? sh[lane][0] : 0.0;
+            t = warp_sum(t);
+            if (lane == 0 && t != 0.0) atomicAdd(dst, t);
+        } else if (lane < NV) {
+            double t = 0.0;
+            for (int w = 0; w < nw; ++w) t += sh[w][lane];
+            if (t != 0.0) atomicAdd(dst + lane, t);
         }
     }
     __syncthreads();  // the shared buffer may be reused by the next call

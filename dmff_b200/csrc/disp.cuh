@@ -190,11 +190,11 @@ __global__ void __launch_bounds__(128) k_disp_pair(DispArgs<T> a) {
         }
     }
     const bool head = seg_head(key);
-    const int run = seg_run_id(key);
+    const unsigned reach = seg_reach(seg_run_id(key));
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        const T s1 = seg_sum(gl[c], run);
-        const T s2 = TT ? seg_sum(gs[c], run) : T(0);
+        const T s1 = seg_sum(gl[c], reach);
+        const T s2 = TT ? seg_sum(gs[c], reach) : T(0);
         if (head && key >= 0) {
             atomicAdd(a.grad_lr + 3 * key + c, s1);
             if (TT) atomicAdd(a.grad_sr + 3 * key + c, s2);
@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(128) k_disp_pair(DispArgs<T> a) {
 #pragma unroll
         for (int k = 0; k < 7; ++k) {
             if (!TT && k >= 3) break;
-            const double sum = seg_sum(pi_[k], run);
+            const double sum = seg_sum(pi_[k], reach);
             double* base = k < 3 ? a.dlr + (size_t)k * a.n : a.dsr + (size_t)(k - 3) * a.n;
             if (head && key >= 0) atomicAdd(base + key, sum);
             if (valid) atomicAdd(base + j, pj_[k]);

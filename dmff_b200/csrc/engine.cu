@@ -68,6 +68,7 @@ struct dmffb_engine {
     void* d_posT = nullptr;
     double* d_Qg = nullptr;
     void* d_QgT = nullptr;
+    void* d_rec = nullptr;  // [n][4] Vec4: the pair passes' site records
     void* d_gpair = nullptr;
     void* d_torque = nullptr;
     void* d_fieldT = nullptr;
@@ -392,7 +393,7 @@ __global__ void k_field_combine(int n, const double* recip, const T* fT, const d
         double p = pol[a];
         p = p < 1e-8 ? 1e-8 : p;
         double v = recip ? recip[k] : 0.0;
-        if (fT) v += (double)fT[k];
+        if (fT) v += (double)fT[4 * a + c];
         if (mv) v += mv[k];
         if (U) v += (DMFFB_DIELECTRIC / p + self1) * U[k];
         if (include_perm) {
@@ -537,6 +538,8 @@ PairArgs<T> pair_args(dmffb_engine* h, const Box& bx, const int32_t* pairs, int6
     a.npairs = npairs;
     a.pairs = pairs;
     a.pos = (const T*)h->d_posT;
+    a.rec = (const Vec4<T>*)h->d_rec;
+    a.U4 = nullptr;
     a.posd = h->cur_pos;
     a.Qg = (const T*)h->d_QgT;
     a.Qgd = h->d_Qg;
@@ -556,6 +559,25 @@ PairArgs<T> pair_args(dmffb_engine* h, const Box& bx, const int32_t* pairs, int6
     a.scal = h->d_scal + S_EREAL;
     a.want_box = 1;
     return a;
+}
+
+template <typename T>
+PrepArgs<T> prep_args(const dmffb_engine* h, const double* pos, const Box& bx) {
+    PrepArgs<T> pa;
+    pa.f.n = h->n;
+    pa.f.pos = pos;
+    pa.f.axis_type = h->d_axis_type;
+    pa.f.axis_idx = h->d_axis_idx;
+    pa.f.box = bx;
+    pa.Qloc = h->d_Qloc;
+    pa.lmax = h->lmax;
+    pa.posT = (T*)h->d_posT;
+    pa.QgT = (T*)h->d_QgT;
+    pa.Qg = h->d_Qg;
+    pa.thole = h->lpol ? (const T*)h->d_thole : nullptr;
+    pa.polsix = h->lpol ? (const T*)h->d_polsix : nullptr;
+    pa.rec = (Vec4<T>*)h->d_rec;
+    return pa;
 }
 
 int lmax_eff(const dmffb_engine* h) { return (h->lmax == 0 && h->lpol) ? 1 : h->lmax; }
@@ -1078,7 +1100,7 @@ int field_eval(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx
                int64_t npairs, const double* U, bool include_perm, double* out, const double* dotv = nullptr,
                double* dot_out = nullptr, bool with_mvcoef = false, bool cleared = false) {
     const bool recip_on = h->lpme && h->have_plans;
-    if (include_perm && !cleared) CK(cudaMemsetAsync(h->d_fieldT, 0, (size_t)3 * h->n * sizeof(T), s));
+    if (include_perm && !cleared) CK(cudaMemsetAsync(h->d_fieldT, 0, (size_t)4 * h->n * sizeof(T), s));
     // the real-space work (permanent pair field, matvec) runs on a side stream, overlapping the
     // reciprocal pass; both write their own arrays and meet in the combine
     const bool real_work = (include_perm && npairs > 0) || U || with_mvcoef;
@@ -1445,25 +1467,15 @@ int compute_impl(dmffb_engine* h, cudaStream_t s, const double* pos, const doubl
         if ((st = dmffb_admp_build_neighbors(h, (void*)s, pos, box))) return st;
     if (own_list && h->e_build) CK(cudaStreamWaitEvent(s, h->e_build, 0));
     if (h->timing) CK(cudaEventRecord(h->ev[0], s));
-    PrepArgs<T> pa;
+    PrepArgs<T> pa = prep_args<T>(h, pos, bx);
     pa.clear.add(h->d_scal, N_SCAL * sizeof(double));
-    pa.clear.add(h->d_gpair, (size_t)3 * n * sizeof(T));
-    pa.clear.add(h->d_torque, (size_t)3 * n * sizeof(T));
+    pa.clear.add(h->d_gpair, (size_t)4 * n * sizeof(T));
+    pa.clear.add(h->d_torque, (size_t)4 * n * sizeof(T));
     pa.clear.add(h->d_grad, (size_t)3 * n * sizeof(double));
     pa.clear.add(h->d_gQ, (size_t)9 * n * sizeof(double));
     const bool cg = h->lpol && !h->fixed_U && h->solver != DMFFB_SOLVER_REFERENCE;
-    if (cg) pa.clear.add(h->d_fieldT, (size_t)3 * n * sizeof(T));
+    if (cg) pa.clear.add(h->d_fieldT, (size_t)4 * n * sizeof(T));
     if (cg && h->zero_guess) pa.clear.add(U, (size_t)3 * n * sizeof(double));
-    pa.f.n = n;
-    pa.f.pos = pos;
-    pa.f.axis_type = h->d_axis_type;
-    pa.f.axis_idx = h->d_axis_idx;
-    pa.f.box = bx;
-    pa.Qloc = h->d_Qloc;
-    pa.lmax = h->lmax;
-    pa.posT = (T*)h->d_posT;
-    pa.QgT = (T*)h->d_QgT;
-    pa.Qg = h->d_Qg;
     LAUNCH(h, s, KC_PREP, k_prepare<T><<<nblk(n, 128), 128, 0, s>>>(pa));
     CK(cudaGetLastError());
     // the work above needs no pair list: it runs while a single-pass build's totals come back
@@ -1498,6 +1510,11 @@ int compute_impl(dmffb_engine* h, cudaStream_t s, const double* pos, const doubl
     }
     if (npairs > 0) {
         PairArgs<T> a = pair_args<T>(h, bx, pairs, npairs, h->lpol ? U : nullptr);
+        if (h->lpol) {
+            if ((st = matvec_alloc<T>(h))) return st;
+            LAUNCH(h, sp, KC_VEC, k_pack_dipoles<T><<<nblk(n, 256), 256, 0, sp>>>(n, U, (Vec4<T>*)h->d_p4));
+            a.U4 = (const Vec4<T>*)h->d_p4;
+        }
         const unsigned nbk = nblk(npairs, 128);
         if (sizeof(T) == 4) {
             const unsigned nbs = nblk(h->n_srows, 128);
@@ -2545,9 +2562,10 @@ int dmffb_admp_create(const dmffb_admp_desc* d, dmffb_engine** out) {
     AL(h->d_posT, 4 * n * ts);
     AL(h->d_Qg, 9 * n * sizeof(double));
     AL(h->d_QgT, 9 * n * ts);
-    AL(h->d_gpair, 3 * n * ts);
-    AL(h->d_torque, 3 * n * ts);
-    AL(h->d_fieldT, 3 * n * ts);
+    AL(h->d_rec, 16 * n * ts);
+    AL(h->d_gpair, 4 * n * ts);
+    AL(h->d_torque, 4 * n * ts);
+    AL(h->d_fieldT, 4 * n * ts);
     AL(h->d_grad, 3 * n * sizeof(double));
     AL(h->d_scal, N_SCAL * sizeof(double));
     AL(h->d_gQ, 9 * n * sizeof(double));
@@ -2612,7 +2630,7 @@ void dmffb_destroy(dmffb_engine* h) {
     if (h->e_nbtot) cudaEventDestroy(h->e_nbtot);
     void* ptrs[] = {h->d_axis_type, h->d_axis_idx, h->d_cov_ptr, h->d_cov_j, h->d_cov_nb, h->d_Qloc, h->d_pol,
                     h->d_thole, h->d_polsix, h->d_pos, h->d_U, h->d_forces, h->d_posT, h->d_Qg, h->d_QgT,
-                    h->d_gpair, h->d_torque, h->d_fieldT, h->d_grad, h->d_scal, h->d_b, h->d_r, h->d_z, h->d_p,
+                    h->d_rec, h->d_gpair, h->d_torque, h->d_fieldT, h->d_grad, h->d_scal, h->d_b, h->d_r, h->d_z, h->d_p,
                     h->d_Ap, h->d_s, h->d_fr, h->d_gQ, h->d_fmv, h->d_pcount_f, h->d_pcount_s, h->d_poff_s, h->d_rank, h->d_bin_done, h->d_nbsum, h->d_mvcoef, h->d_p4, h->d_csr_off, h->d_csr_ent, h->d_csr_deg, h->d_cub2, h->d_grid, h->d_grid2, h->d_cgrid, h->d_bmod, h->d_pairs, h->d_atom_cell,
                     h->d_cell_count, h->d_cell_start, h->d_pcount, h->d_poff,
                     h->d_c, h->d_tta, h->d_ttb, h->d_ttq, h->d_glr, h->d_gsr, h->d_dc,
@@ -2742,17 +2760,7 @@ template <typename T>
 int field_at(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx, const int32_t* pairs, int64_t npairs,
              const double* U, double* field_out) {
     const int n = h->n;
-    PrepArgs<T> pa;
-    pa.f.n = n;
-    pa.f.pos = pos;
-    pa.f.axis_type = h->d_axis_type;
-    pa.f.axis_idx = h->d_axis_idx;
-    pa.f.box = bx;
-    pa.Qloc = h->d_Qloc;
-    pa.lmax = h->lmax;
-    pa.posT = (T*)h->d_posT;
-    pa.QgT = (T*)h->d_QgT;
-    pa.Qg = h->d_Qg;
+    PrepArgs<T> pa = prep_args<T>(h, pos, bx);
     h->cur_pos = pos;
     LAUNCH(h, s, KC_PREP, k_prepare<T><<<nblk(n, 128), 128, 0, s>>>(pa));
     int st;
@@ -2884,17 +2892,7 @@ int admp_backward_impl(dmffb_engine* h, cudaStream_t s, const dmffb_admp_cotange
             LAUNCH(h, s, KC_VEC, k_cdiff<<<nblk(n3, 256), 256, 0, s>>>(n3, g, Fp, Fm, 0.5 / e));
             // tangent (adjoint) solve at z: A dU = -g, by CG from zero
             if ((st = set_point(0.0))) return st;
-            PrepArgs<T> pa;
-            pa.f.n = n;
-            pa.f.pos = pos0;
-            pa.f.axis_type = h->d_axis_type;
-            pa.f.axis_idx = h->d_axis_idx;
-            pa.f.box = bx0;
-            pa.Qloc = h->d_Qloc;
-            pa.lmax = h->lmax;
-            pa.posT = (T*)h->d_posT;
-            pa.QgT = (T*)h->d_QgT;
-            pa.Qg = h->d_Qg;
+            PrepArgs<T> pa = prep_args<T>(h, pos0, bx0);
             h->cur_pos = pos0;
             LAUNCH(h, s, KC_PREP, k_prepare<T><<<nblk(n, 128), 128, 0, s>>>(pa));
             if (sizeof(T) == 4 && npairs > 0 && (st = scaled_rows(h, s, pairs, npairs))) return st;
@@ -3003,17 +3001,7 @@ int dmffb_admp_field(dmffb_engine* h, void* stream, const double* pos, const dou
     const int n = h->n;
     auto run = [&](auto tag) -> int {
         using T = decltype(tag);
-        PrepArgs<T> pa;
-        pa.f.n = n;
-        pa.f.pos = pos;
-        pa.f.axis_type = h->d_axis_type;
-        pa.f.axis_idx = h->d_axis_idx;
-        pa.f.box = bx;
-        pa.Qloc = h->d_Qloc;
-        pa.lmax = h->lmax;
-        pa.posT = (T*)h->d_posT;
-        pa.QgT = (T*)h->d_QgT;
-        pa.Qg = h->d_Qg;
+        PrepArgs<T> pa = prep_args<T>(h, pos, bx);
         LAUNCH(h, s, KC_PREP, k_prepare<T><<<nblk(n, 128), 128, 0, s>>>(pa));
         int st;
         if (sizeof(T) == 4 && npairs > 0 && (st = scaled_rows(h, s, pairs, npairs))) return st;

@@ -105,15 +105,6 @@ __global__ void k_nb_forces(int n, const T* glr, const double* gd, const T* gcel
     for (int c = 0; c < 3; ++c) forces[3 * i + c] = -((double)glr[3 * i + c] + (double)g[c] + gd[3 * i + c]);
 }
 
-__device__ __forceinline__ void nb_add(float* g, float x, float y, float z) {
-    atomicAdd((float4*)g, make_float4(x, y, z, 0.f));  // one 16-byte reduction
-}
-__device__ __forceinline__ void nb_add(double* g, double x, double y, double z) {
-    atomicAdd(g, x);
-    atomicAdd(g + 1, y);
-    atomicAdd(g + 2, z);
-}
-
 // distance of an FP64 square in kernel precision: FP32 from the hardware's reciprocal square root and
 // one FP64 Newton step (error 1e-14, so it rounds to the same float as the FP64 root all but always)
 __device__ __forceinline__ void nb_root(double r2, double& r) { r = sqrt(r2); }
@@ -165,7 +156,7 @@ __device__ __forceinline__ void nb_cell_pair(const NbCellArgs<T>& a, int k, doub
     g0 -= f0;
     g1 -= f1;
     g2 -= f2;
-    nb_add(a.gcell + 4 * (int64_t)k, f0, f1, f2);
+    add3(a.gcell + 4 * (int64_t)k, f0, f1, f2);
     acc[0] += ec;
     acc[1] += el;
     if (nd[0] != 0.0 || nd[1] != 0.0 || nd[2] != 0.0) {  // most pairs meet inside the box
@@ -343,7 +334,7 @@ __global__ void __launch_bounds__(32 * kNbWarps, sizeof(T) == 4 ? 4 : 0) k_nb_ce
         g0 = warp_sum(g0);
         g1 = warp_sum(g1);
         g2 = warp_sum(g2);
-        if (lane == 0) nb_add(a.gcell + 4 * (int64_t)ks, g0, g1, g2);
+        if (lane == 0) add3(a.gcell + 4 * (int64_t)ks, g0, g1, g2);
     }
     block_reduce_add<12>(red, a.scal);
 }

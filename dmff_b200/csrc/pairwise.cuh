@@ -255,17 +255,17 @@ __global__ void __launch_bounds__(128) k_sr_pair(SrArgs<T> a) {
         }
     }
     const bool head = seg_head(key);
-    const int run = seg_run_id(key);
+    const unsigned reach = seg_reach(seg_run_id(key));
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        const T s1 = seg_sum(g[c], run);
+        const T s1 = seg_sum(g[c], reach);
         if (head && key >= 0) atomicAdd(a.grad + 3 * key + c, s1);
         if (valid) atomicAdd(a.grad + 3 * j + c, -g[c]);
     }
     if (a.dp) {
 #pragma unroll
         for (int k = 0; k < NP; ++k) {
-            const double s1 = seg_sum((double)pi_grad[k], run);
+            const double s1 = seg_sum((double)pi_grad[k], reach);
             if (head && key >= 0) atomicAdd(a.dp + (size_t)k * a.n + key, s1);
         }
     }
