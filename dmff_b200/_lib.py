@@ -29,6 +29,7 @@ DMFFB_SOLVER_REFERENCE = 1
 # every function the header declares (checked by the CPU test suite)
 EXPORTED = [
     "dmffb_admp_create", "dmffb_admp_reconfigure", "dmffb_destroy", "dmffb_last_error", "dmffb_admp_set_params",
+    "dmffb_admp_set_params_device", "dmffb_disp_set_params_device",
     "dmffb_admp_compute", "dmffb_admp_compute_host", "dmffb_admp_field", "dmffb_admp_multipole_grads",
     "dmffb_build_neighbors", "dmffb_admp_build_neighbors", "dmffb_engine_pairs", "dmffb_get_timings", "dmffb_set_timing",
     "dmffb_set_profiling", "dmffb_get_kernel_stats", "dmffb_get_counters", "dmffb_build_neighbors_noalloc",
@@ -292,6 +293,8 @@ def load():
     lib.dmffb_last_error.argtypes = [vp]
     lib.dmffb_last_error.restype = ctypes.c_char_p
     lib.dmffb_admp_set_params.argtypes = [vp, vp, vp, vp]
+    lib.dmffb_admp_set_params_device.argtypes = [vp, vp, vp, vp, vp]
+    lib.dmffb_disp_set_params_device.argtypes = [vp, vp, vp, vp, vp, vp]
     lib.dmffb_admp_compute.argtypes = [vp, vp, vp, vp, vp, i64, vp, vp, P(AdmpResult)]
     lib.dmffb_admp_compute_host.argtypes = [vp, vp, vp, vp, i64, vp, vp, P(AdmpResult)]
     lib.dmffb_admp_field.argtypes = [vp, vp, vp, vp, vp, i64, vp, vp]

@@ -154,15 +154,15 @@ def _disp_first(eng, pos, box, pairs, with_tt, want_p):
     g_lr = torch.tensor(list(res.box_grad), dtype=torch.float64).reshape(3, 3)
     # forces from the engine are -dE_lr/dpos (disp) and -dE_sr/dpos (TT) separately
     Flr, Fsr = F
-    first = [(-(Fsr - Flr)) if with_tt else (-Flr).clone(), (g_sr - g_lr) if with_tt else g_lr, None, None, None, None]
+    first = [Flr - Fsr if with_tt else -Flr, (g_sr - g_lr) if with_tt else g_lr, None, None, None, None]
     if want_p:
         pg = eng.param_grads()
         if with_tt:
-            dc = -pg["c"].clone()
+            dc = -pg["c"]
             dc[:, 0] += pg["c6"]
-            first[2:] = [dc, pg["a"].clone(), pg["b"].clone(), pg["q"].clone()]
+            first[2:] = [dc, pg["a"], pg["b"], pg["q"]]
         else:
-            first[2] = pg["c"].clone()
+            first[2] = pg["c"]
     return res, first
 
 
@@ -183,7 +183,7 @@ class _DispFirstDerivs(torch.autograd.Function):
             elif v is None:
                 out.append(torch.zeros_like(t, dtype=torch.float64))
             else:
-                out.append(v.to(t.device).clone())
+                out.append(v.to(t.device).detach())  # a tensor of its own: the payload's stays without a graph
         return tuple(out)
 
     @staticmethod

@@ -12,7 +12,7 @@ import math
 import numpy as np
 import torch
 
-from ..engine import AdmpEngine
+from ..engine import AdmpEngine, _on_device
 from .settings import MAX_N_POL, POL_CONV
 
 DIELECTRIC = 1389.35455846
@@ -70,21 +70,28 @@ class _AdmpEnergy(torch.autograd.Function):
         want_p = any(ctx.needs_input_grad[2:5]) and any(want)
         eng.set_param_grads(want_p)
         U = None
+        from_zero = force.lpol and U0 is None and force.pol_solver == "cg" and dev.type == "cuda"
         if force.lpol:
             U = (U0.detach().to(device=dev, dtype=torch.float64).contiguous().clone() if U0 is not None
                  else torch.zeros((force.n_atoms, 3), dtype=torch.float64, device=dev))
-        res, forces, U = eng.compute(pos, box, pairs=pairs, U=U)
+        if from_zero:
+            eng.set_zero_guess(True)
+        try:
+            res, forces, U = eng.compute(pos, box, pairs=pairs, U=U)
+        finally:
+            if from_zero:
+                eng.set_zero_guess(False)
         force.last_result = res
         if aux is not None:
             aux["U_ind"] = U * 0.1  # Angstrom -> nm, as pme.py:225
             aux["lconverg"] = bool(res.converged)
             aux["n_cycle"] = int(res.n_iter)
-        pg = eng.param_grads() if want_p else None
-        z = lambda t: None if t is None else torch.zeros_like(t, dtype=torch.float64)
-        first = {"pos": -forces.clone(), "box": torch.tensor(list(res.box_grad), dtype=torch.float64).reshape(3, 3),
+        pg = eng.param_grads(with_global=False) if want_p else None
+        z = lambda t: None if t is None or pg is not None else torch.zeros_like(t, dtype=torch.float64)
+        first = {"pos": -forces, "box": torch.tensor(list(res.box_grad), dtype=torch.float64).reshape(3, 3),
                  "Q_local": pg["Q_local"] if pg is not None else None,
                  "pol": pg["pol"] if pg is not None else None, "thole": pg["thole"] if pg is not None else None}
-        ctx.payload = {"force": force, "pairs": pairs, "U": None if U is None else U.clone(), "first": first,
+        ctx.payload = {"force": force, "pairs": pairs, "U": U, "first": first,
                        "zero": (z(Q_local), z(pol), z(tholes))}
         ctx.save_for_backward(positions, box, Q_local, pol, tholes)
         return torch.tensor(res.energy, dtype=torch.float64, device=positions.device)
@@ -121,9 +128,9 @@ class _AdmpFirstDerivs(torch.autograd.Function):
             if v is None:
                 return zz.clone()
             v = v[:, : like.shape[1]] if like.dim() == 2 and v.dim() == 2 else v
-            return v.to(like.device).clone()
+            return v.to(like.device).detach()  # a tensor of its own: the payload's stays without a graph
 
-        return (f["pos"].to(positions.device).clone(), f["box"].to(box.device).clone(),
+        return (f["pos"].to(positions.device).detach(), f["box"].to(box.device).detach(),
                 out(f["Q_local"], Q_local, zero[0]), out(f["pol"], pol, zero[1]), out(f["thole"], tholes, zero[2]))
 
     @staticmethod
@@ -181,31 +188,35 @@ class ADMPPmeForce:
         return self._engine
 
     def _sync_params(self, Q_local, pol, tholes, mScales, pScales, dScales):
-        # keyed by value: a fresh tensor can reuse a freed one's address, so identity is not enough
-        vals = tuple(None if t is None else torch.as_tensor(t, dtype=torch.float64).detach().cpu().clone()
-                     for t in (Q_local, pol, tholes))
-        scales = tuple(tuple(np.asarray(torch.as_tensor(s).detach().cpu()).tolist()) if s is not None else None
-                       for s in (mScales, pScales, dScales))
-        old = self._param_key
-        if old is not None and old[1] == scales and all(
-                (a is None and b is None) or (a is not None and b is not None and a.shape == b.shape and torch.equal(a, b))
-                for a, b in zip(old[0], vals)):
-            return
-        key = (vals, scales)
+        scales = tuple(None if t is None else tuple(np.asarray(torch.as_tensor(t).detach().cpu(), np.float64).tolist())
+                       for t in (mScales, pScales, dScales))
         # scales are part of the engine description: rebuild when they change
-        ms = np.asarray(torch.as_tensor(mScales).detach().cpu(), np.float64)
-        ps = np.asarray(torch.as_tensor(pScales).detach().cpu(), np.float64) if pScales is not None else None
-        ds = np.asarray(torch.as_tensor(dScales).detach().cpu(), np.float64) if dScales is not None else None
-        scales = (tuple(ms), None if ps is None else tuple(ps), None if ds is None else tuple(ds))
         if getattr(self, "_scales", None) != scales:
             self._engine = AdmpEngine(
                 self.n_atoms, self.lmax, self.lpol, self.lpme, self.rc, self.kappa, (self.K1, self.K2, self.K3),
                 self.axis_type if self.lmax > 0 else None, self.axis_indices if self.lmax > 0 else None,
-                self.cov_rows, ms, ps, ds, precision=self.precision, solver=self.pol_solver, cg_tol=self.cg_tol,
+                self.cov_rows, *scales, precision=self.precision, solver=self.pol_solver, cg_tol=self.cg_tol,
                 max_iter=self.max_iter, steps_pol=self.steps_pol, device=self.device)
             self._scales = scales
-        self.engine.set_params(Q_local, pol if self.lpol else None, tholes if self.lpol else None)
-        self._param_key = key
+            self._param_key = None
+        if not self.lpol:
+            pol = tholes = None
+        if _on_device(self.engine.device, Q_local, pol, tholes):
+            # set each time: three copies on the device, no wait
+            self.engine.set_params(Q_local, pol, tholes)
+            self._param_key = None
+            return
+        # host parameters are keyed by value: a fresh tensor can reuse a freed one's address, so identity is
+        # not enough
+        vals = tuple(None if t is None else torch.as_tensor(t, dtype=torch.float64).detach().cpu().clone()
+                     for t in (Q_local, pol, tholes))
+        old = self._param_key
+        if old is not None and all(
+                (a is None and b is None) or (a is not None and b is not None and a.shape == b.shape and torch.equal(a, b))
+                for a, b in zip(old, vals)):
+            return
+        self.engine.set_params(Q_local, pol, tholes)
+        self._param_key = vals
 
     def second_order(self, positions, box, Q_local, pol, tholes, pairs, U, c_pos, c_box, c_Q, c_pol, c_thole):
         """Vector-Jacobian product through the first derivatives of an evaluation (the backward of
@@ -259,7 +270,9 @@ class ADMPPmeForce:
         U0 = None
         if self.lpol:
             U0 = U_init if U_init is not None else self.U_ind
-            U0 = torch.as_tensor(np.asarray(U0) if not torch.is_tensor(U0) else U0, dtype=torch.float64) * 10.0
+            U0 = torch.as_tensor(np.asarray(U0) if not torch.is_tensor(U0) else U0, dtype=torch.float64)
+            # zeros on the host (the initial U_ind) need not travel: the solve starts from U = 0
+            U0 = None if not U0.is_cuda and not bool(U0.any()) else U0 * 10.0
         Q_local = torch.as_tensor(Q_local, dtype=torch.float64)
         if self.lpol:
             pol = torch.as_tensor(pol, dtype=torch.float64)

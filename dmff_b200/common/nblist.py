@@ -39,7 +39,7 @@ class NeighborList:
         return self._engine
 
     def allocate(self, coords, box=None):
-        pos = _host_f64(coords)
+        pos = _f64(coords)
         self._positions = coords
         n = pos.shape[0]
         eng = self._eng(n)
@@ -64,6 +64,11 @@ class NeighborList:
         return self._positions
 
 
+def _f64(coords):
+    """Coordinates in float64; a CUDA tensor stays on its device."""
+    return coords.detach().to(torch.float64) if torch.is_tensor(coords) and coords.is_cuda else _host_f64(coords)
+
+
 def _host_f64(coords):
     return torch.as_tensor(np.asarray(coords.detach().cpu() if torch.is_tensor(coords) else coords),
                            dtype=torch.float64)
@@ -80,9 +85,11 @@ def _padded(nl, rows, n):
     nl.capacity_multiplier = max(nl.capacity_multiplier, count)
     pad = nl.capacity_multiplier - count
     if pad > 0:
-        padding = torch.full((pad, 3), n, dtype=torch.int32, device=rows.device)
-        padding[:, 2] = 0
-        rows = torch.cat([rows, padding], dim=0)
+        out = torch.empty((nl.capacity_multiplier, 3), dtype=torch.int32, device=rows.device)
+        out[:count] = rows
+        out[count:, :2] = n
+        out[count:, 2] = 0
+        rows = out
     return rows
 
 

@@ -153,6 +153,8 @@ struct dmffb_engine {
     void *d_glr = nullptr, *d_gsr = nullptr;
     double* d_dc = nullptr;  // [3n] dE_lr/dc per channel (reciprocal part)
     double e_self_disp = 0.0;
+    double* d_self_c = nullptr;  // [3] sums of the squared c6, c8, c10 set from device arrays
+    bool self_on_device = false;
     // ---- classical terms (engines made by dmffb_classical_create, kind 2)
     int ntypes = 0, coul = 0, pbc = 1;
     double krf = 0.0, crf = 0.0, e_self_coul = 0.0;
@@ -228,6 +230,8 @@ struct dmffb_engine {
     int64_t last_npairs = 0;
     double* last_U = nullptr;
     std::vector<double> h_Qloc, h_pol, h_thole;  // host copies of the last set_params
+    bool h_params_stale = false;  // set from device arrays since: fetched when the second-order pass needs them
+    double* d_th64 = nullptr;     // [n_cap] the Thole widths of that call
     double* d_bk = nullptr;  // [52 n] scratch of the second-order pass
     int64_t bk_cap = 0;
     std::map<std::array<int, 3>, std::pair<cufftHandle, cufftHandle>> plan_cache;  // mesh -> (R2C, C2R)
@@ -1729,6 +1733,37 @@ void recip_box_grad(const Box& bx, const int K[3], const double* conv, const dou
         }
 }
 
+// Ewald self energy of the dispersion channels from the sums of their squares (disp_pme.py:264-289)
+double disp_self_energy(double kappa, int pmax, double s6, double s8, double s10) {
+    const double k2 = kappa * kappa;
+    double e = -k2 * k2 * k2 / 12.0 * s6;
+    if (pmax >= 8) e -= k2 * k2 * k2 * k2 / 48.0 * s8;
+    if (pmax >= 10) e -= k2 * k2 * k2 * k2 * k2 / 240.0 * s10;
+    return e;
+}
+
+// parameters from device arrays: c [n][3] to channels, the TT parameters, kernel precision; sums of c^2
+template <typename T>
+__global__ void __launch_bounds__(256) k_disp_params(int n, const double* c, const double* a, const double* b,
+                                                     const double* q, T* cT, T* ta, T* tb, T* tq, double* sums) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    double v[3] = {0.0, 0.0, 0.0};
+    if (i < n) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const double x = c[3 * i + k];
+            cT[(size_t)k * n + i] = (T)x;
+            v[k] = x * x;
+        }
+        if (a) {
+            ta[i] = (T)a[i];
+            tb[i] = (T)b[i];
+            tq[i] = (T)q[i];
+        }
+    }
+    block_reduce_add<3>(v, sums);
+}
+
 template <typename T>
 int disp_compute_impl(dmffb_engine* h, cudaStream_t s, const double* pos, const double* box, const int32_t* pairs,
                       int64_t npairs, double* f_lr, double* f_sr, dmffb_disp_result* res) {
@@ -1811,6 +1846,8 @@ int disp_compute_impl(dmffb_engine* h, cudaStream_t s, const double* pos, const 
     h->have_pgrad = pg;
     LAUNCH(h, s, KC_VEC, k_disp_finalize<T><<<nblk(3 * n, 256), 256, 0, s>>>(
                              n, (const T*)h->d_glr, h->tt ? (const T*)h->d_gsr : nullptr, h->d_grad, f_lr, f_sr));
+    if (h->self_on_device)
+        CK(cudaMemcpyAsync(h->h_scal + N_SCAL, h->d_self_c, 3 * sizeof(double), cudaMemcpyDeviceToHost, s));
     CK(cudaMemcpyAsync(h->h_scal, h->d_scal, N_SCAL * sizeof(double), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     prof_collect(h);
@@ -1818,6 +1855,11 @@ int disp_compute_impl(dmffb_engine* h, cudaStream_t s, const double* pos, const 
     res->e_real = sc[0];
     res->e_sr = sc[1];
     res->e_recip = (h->lpme && h->have_plans) ? sc[24] : 0.0;
+    if (h->self_on_device) {
+        const double* s3 = h->h_scal + N_SCAL;
+        h->e_self_disp = disp_self_energy(h->kappa, h->pmax, s3[0], s3[1], s3[2]);
+        h->self_on_device = false;
+    }
     res->e_self = h->lpme ? h->e_self_disp : 0.0;
     res->energy = res->e_real + res->e_recip + res->e_self;
     for (int k = 0; k < 9; ++k) {
@@ -2579,7 +2621,7 @@ int dmffb_admp_create(const dmffb_admp_desc* d, dmffb_engine** out) {
         AL(h->d_fr, 3 * n * sizeof(double));
     }
 #undef AL
-    if (cudaMallocHost((void**)&h->h_scal, N_SCAL * sizeof(double)) != cudaSuccess)
+    if (cudaMallocHost((void**)&h->h_scal, (N_SCAL + 3) * sizeof(double)) != cudaSuccess)
         return fail(h, DMFFB_OOM, "cudaMallocHost failed");
     if (h->lpme && (st = setup_mesh(h))) return st;
     cudaError_t e = cudaStreamSynchronize(h->s1);
@@ -2636,7 +2678,7 @@ void dmffb_destroy(dmffb_engine* h) {
                     h->d_c, h->d_tta, h->d_ttb, h->d_ttq, h->d_glr, h->d_gsr, h->d_dc,
                     h->d_q, h->d_qT, h->d_type, h->d_sigtt, h->d_epstt, h->d_dq, h->d_dsig, h->d_deps,
                     h->d_tidx[0], h->d_tidx[1], h->d_tidx[2], h->d_tprm[0], h->d_tprm[1], h->d_tprm[2],
-                    h->d_tdprm[0], h->d_tdprm[1], h->d_tdprm[2], h->d_dQloc, h->d_dpa, h->d_dth, h->d_dpol, h->d_dsr, h->d_srows, h->d_nsel, h->d_cubsel,
+                    h->d_tdprm[0], h->d_tdprm[1], h->d_tdprm[2], h->d_dQloc, h->d_dpa, h->d_dth, h->d_dpol, h->d_dsr, h->d_th64, h->d_self_c, h->d_srows, h->d_nsel, h->d_cubsel,
                     h->d_slots, h->d_stc_org, h->d_stc_w, h->d_nbmask, h->d_covrows, h->d_cov_lo, h->d_cov_hi, h->d_dftW, h->d_dftG, h->d_pcg, h->d_posc, h->d_nbrec, h->d_gcell, h->d_srp, h->d_srdp, h->d_srgrad};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -2667,6 +2709,7 @@ int dmffb_admp_set_params(dmffb_engine* h, const double* Q_local, const double* 
     const int n = h->n;
     // ordered on the engine stream (no device-wide synchronisation: other engines keep running)
     cudaStream_t s = h->s1;
+    h->h_params_stale = false;
     h->h_Qloc.assign(Q_local, Q_local + 9 * (size_t)n);
     if (pol) h->h_pol.assign(pol, pol + n);
     else h->h_pol.assign(n, 0.0);
@@ -2686,6 +2729,34 @@ int dmffb_admp_set_params(dmffb_engine* h, const double* Q_local, const double* 
         k_set_thole<double><<<nblk(n, 128), 128, 0, s>>>(n, h->d_pol, dth, (double*)h->d_thole, (double*)h->d_polsix);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(s));
+    h->params_set = true;
+    return DMFFB_OK;
+}
+
+int dmffb_admp_set_params_device(dmffb_engine* h, void* stream, const double* Q_local, const double* pol,
+                                 const double* thole) {
+    if (!h || !Q_local) return fail(h, DMFFB_BAD_ARG, "null handle or Q_local");
+    if (h->lpol && (!pol || !thole)) return fail(h, DMFFB_BAD_ARG, "polarizable system needs pol and thole");
+    const int n = h->n;
+    cudaStream_t caller = (cudaStream_t)stream, s = h->s1;
+    int st;
+    if (!h->d_th64 && (st = dalloc(h, &h->d_th64, (size_t)h->n_cap * sizeof(double)))) return st;
+    CK(cudaEventRecord(h->e_in, caller));
+    CK(cudaStreamWaitEvent(s, h->e_in, 0));
+    CK(cudaMemcpyAsync(h->d_Qloc, Q_local, 9 * (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, s));
+    if (pol) CK(cudaMemcpyAsync(h->d_pol, pol, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
+    else CK(cudaMemsetAsync(h->d_pol, 0, n * sizeof(double), s));
+    if (thole) CK(cudaMemcpyAsync(h->d_th64, thole, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
+    else CK(cudaMemsetAsync(h->d_th64, 0, n * sizeof(double), s));
+    const double* th = thole ? h->d_th64 : nullptr;
+    if (h->prec == DMFFB_FP32)
+        k_set_thole<float><<<nblk(n, 128), 128, 0, s>>>(n, h->d_pol, th, (float*)h->d_thole, (float*)h->d_polsix);
+    else
+        k_set_thole<double><<<nblk(n, 128), 128, 0, s>>>(n, h->d_pol, th, (double*)h->d_thole, (double*)h->d_polsix);
+    CK(cudaGetLastError());
+    CK(cudaEventRecord(h->e_out, s));
+    CK(cudaStreamWaitEvent(caller, h->e_out, 0));
+    h->h_params_stale = true;
     h->params_set = true;
     return DMFFB_OK;
 }
@@ -2836,6 +2907,16 @@ int admp_backward_impl(dmffb_engine* h, cudaStream_t s, const dmffb_admp_cotange
         (st = maxabs_dev(h->lpol ? c->pol : nullptr, n, &mpol)) || (st = maxabs_dev(h->lpol ? c->thole : nullptr, n, &mth)))
         return st;
     for (int k = 0; k < 9; ++k) mbox = std::max(mbox, fabs(c->box[k]));
+    if (h->h_params_stale) {
+        h->h_Qloc.resize(n9);
+        h->h_pol.resize(n);
+        h->h_thole.resize(n);
+        CK(cudaMemcpyAsync(h->h_Qloc.data(), h->d_Qloc, n9 * sizeof(double), cudaMemcpyDeviceToHost, s));
+        CK(cudaMemcpyAsync(h->h_pol.data(), h->d_pol, n * sizeof(double), cudaMemcpyDeviceToHost, s));
+        CK(cudaMemcpyAsync(h->h_thole.data(), h->d_th64, n * sizeof(double), cudaMemcpyDeviceToHost, s));
+        CK(cudaStreamSynchronize(s));
+        h->h_params_stale = false;
+    }
     const double sQ = std::max(maxabs_host(h->h_Qloc), 1e-12);
     const double sp = std::max(maxabs_host(h->h_pol), 1e-12), sth = std::max(maxabs_host(h->h_thole), 1e-12);
     const double rate = std::max(std::max(std::max(mpos, mbox), std::max(mQ / sQ, mpol / sp)), mth / sth);
@@ -3243,11 +3324,9 @@ int dmffb_disp_set_params(dmffb_engine* h, const double* c_list, const double* a
         s8 += c_list[3 * i + 1] * c_list[3 * i + 1];
         s10 += c_list[3 * i + 2] * c_list[3 * i + 2];
     }
-    const double k2 = h->kappa * h->kappa;
-    double e = -k2 * k2 * k2 / 12.0 * s6;
-    if (h->pmax >= 8) e -= k2 * k2 * k2 * k2 / 48.0 * s8;
-    if (h->pmax >= 10) e -= k2 * k2 * k2 * k2 * k2 / 240.0 * s10;
+    const double e = disp_self_energy(h->kappa, h->pmax, s6, s8, s10);
     h->e_self_disp = e;
+    h->self_on_device = false;
     // staged through the FP64 gradient scratch ([3n], rewritten by every compute), on the engine stream
     double* tmp = h->d_grad;
     auto up = [&](const double* src, int m, void* dst) -> int {
@@ -3262,6 +3341,32 @@ int dmffb_disp_set_params(dmffb_engine* h, const double* c_list, const double* a
     if (!st && h->tt) st = up(b, n, h->d_ttb);
     if (!st && h->tt) st = up(q, n, h->d_ttq);
     if (st) return st;
+    h->params_set = true;
+    return DMFFB_OK;
+}
+
+int dmffb_disp_set_params_device(dmffb_engine* h, void* stream, const double* c_list, const double* a, const double* b,
+                                 const double* q) {
+    if (!h || h->kind != 1 || !c_list) return fail(h, DMFFB_BAD_ARG, "dispersion engine and c_list required");
+    if (h->tt && (!a || !b || !q)) return fail(h, DMFFB_BAD_ARG, "TT damping needs a, b, q");
+    const int n = h->n;
+    cudaStream_t caller = (cudaStream_t)stream, s = h->s1;
+    int st;
+    if (!h->d_self_c && (st = dalloc(h, &h->d_self_c, 3 * sizeof(double)))) return st;
+    CK(cudaEventRecord(h->e_in, caller));
+    CK(cudaStreamWaitEvent(s, h->e_in, 0));
+    CK(cudaMemsetAsync(h->d_self_c, 0, 3 * sizeof(double), s));
+    const double* ta = h->tt ? a : nullptr;
+    if (h->prec == DMFFB_FP32)
+        k_disp_params<float><<<nblk(n, 256), 256, 0, s>>>(n, c_list, ta, b, q, (float*)h->d_c, (float*)h->d_tta,
+                                                          (float*)h->d_ttb, (float*)h->d_ttq, h->d_self_c);
+    else
+        k_disp_params<double><<<nblk(n, 256), 256, 0, s>>>(n, c_list, ta, b, q, (double*)h->d_c, (double*)h->d_tta,
+                                                           (double*)h->d_ttb, (double*)h->d_ttq, h->d_self_c);
+    CK(cudaGetLastError());
+    CK(cudaEventRecord(h->e_out, s));
+    CK(cudaStreamWaitEvent(caller, h->e_out, 0));
+    h->self_on_device = true;
     h->params_set = true;
     return DMFFB_OK;
 }

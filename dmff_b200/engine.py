@@ -48,6 +48,12 @@ def _pairs_arg(pairs, device):
     return _dev(pairs), pairs.shape[0]
 
 
+def _on_device(device, first, *rest):
+    """Whether every given array is a float64 CUDA tensor on ``device``."""
+    return all(x is None or (torch.is_tensor(x) and x.is_cuda and x.device == device and x.dtype == torch.float64)
+               for x in (first, *rest)) and first is not None
+
+
 class AdmpEngine:
     """One ADMP multipolar PME system on one GPU.
 
@@ -138,6 +144,19 @@ class AdmpEngine:
         return st
 
     def set_params(self, Q_local, pol=None, thole=None):
+        """Per-atom parameters.  CUDA tensors on the engine's device stay there (no host copy, no wait);
+        anything else goes through host arrays."""
+        if _on_device(self.device, Q_local, pol, thole):
+            Q = Q_local.detach()
+            if Q.shape[1] < 9:
+                Q = torch.nn.functional.pad(Q, (0, 9 - Q.shape[1]))
+            Q = Q[:, :9].contiguous()
+            p, t = (None, None) if pol is None else (pol.detach().contiguous(), thole.detach().contiguous())
+            s = torch.cuda.current_stream(self.device)
+            self._check(self.lib.dmffb_admp_set_params_device(
+                self.h, ctypes.c_void_p(s.cuda_stream), _dev(Q), None if p is None else _dev(p),
+                None if t is None else _dev(t)))
+            return
         Q = np.zeros((self.n, 9), dtype=np.float64)
         Qi = np.asarray(Q_local.detach().cpu() if torch.is_tensor(Q_local) else Q_local, dtype=np.float64)
         Q[:, : Qi.shape[1]] = Qi
@@ -227,15 +246,17 @@ class AdmpEngine:
         self._check(self.lib.dmffb_admp_set_zero_guess(self.h, int(bool(on))))
         self._zero_guess = bool(on)
 
-    def param_grads(self):
-        """{'Q_global', 'Q_local': [n, 9], 'pol', 'thole': [n]} of the last compute."""
+    def param_grads(self, with_global=True):
+        """{'Q_global', 'Q_local': [n, 9], 'pol', 'thole': [n]} of the last compute (without Q_global on
+        request)."""
         dev = self.device
-        out = {"Q_global": torch.empty((self.n, 9), dtype=torch.float64, device=dev),
+        out = {"Q_global": torch.empty((self.n, 9), dtype=torch.float64, device=dev) if with_global else None,
                "Q_local": torch.empty((self.n, 9), dtype=torch.float64, device=dev),
                "pol": torch.empty(self.n, dtype=torch.float64, device=dev),
                "thole": torch.empty(self.n, dtype=torch.float64, device=dev)}
         s = torch.cuda.current_stream(dev)
-        self._check(self.lib.dmffb_admp_param_grads(self.h, ctypes.c_void_p(s.cuda_stream), _dev(out["Q_global"]),
+        self._check(self.lib.dmffb_admp_param_grads(self.h, ctypes.c_void_p(s.cuda_stream),
+                                                    _dev(out["Q_global"]) if with_global else None,
                                                     _dev(out["Q_local"]), _dev(out["pol"]), _dev(out["thole"])))
         return out
 
@@ -433,6 +454,12 @@ class DispEngine:
     kernel_stats = AdmpEngine.kernel_stats
 
     def set_params(self, c_list, a=None, b=None, q=None):
+        if _on_device(self.device, c_list, a, b, q):
+            t = [None if x is None else x.detach().contiguous() for x in (c_list, a, b, q)]
+            s = torch.cuda.current_stream(self.device)
+            self._check(self.lib.dmffb_disp_set_params_device(
+                self.h, ctypes.c_void_p(s.cuda_stream), *(None if x is None else _dev(x) for x in t)))
+            return
         host = lambda x: None if x is None else np.ascontiguousarray(
             np.asarray(x.detach().cpu() if torch.is_tensor(x) else x, np.float64))
         c, a, b, q = host(c_list), host(a), host(b), host(q)

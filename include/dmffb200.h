@@ -98,6 +98,10 @@ int dmffb_admp_reconfigure(dmffb_engine* h, const dmffb_admp_desc* desc);
  * reference's units (params["ADMPPmeForce"]["Q_local"][map_atomtype], admp.py:1373),
  * zero-padded to 9 components; pol [n] (A^3) and thole [n] (may be NULL when lpol == 0). */
 int dmffb_admp_set_params(dmffb_engine* h, const double* Q_local, const double* pol, const double* thole);
+/* The same from device arrays, after the work queued on `stream` and before later work there: no copy
+ * through the host and no wait (a parameter fit sets them for every sample). */
+int dmffb_admp_set_params_device(dmffb_engine* h, void* stream, const double* Q_local, const double* pol,
+                                 const double* thole);
 
 /* Energy + forces + box gradient: ADMPPmeForce.get_energy (pme.py:186-232) with
  * jax.value_and_grad over (positions, box).  Device pointers: pos [n*3] A, U_inout [n*3]
@@ -253,6 +257,9 @@ int dmffb_disp_create(const dmffb_disp_desc* desc, dmffb_engine** out);
  * (A/2625.5, B*0.0529177249, Q; admp.py:187-193), NULL without TT.  ADMPDispPmeForce.get_energy
  * argument c_list (disp_pme.py:45-49). */
 int dmffb_disp_set_params(dmffb_engine* h, const double* c_list, const double* a, const double* b, const double* q);
+/* The same from device arrays, ordered on `stream` as dmffb_admp_set_params_device. */
+int dmffb_disp_set_params_device(dmffb_engine* h, void* stream, const double* c_list, const double* a, const double* b,
+                                 const double* q);
 /* forces_lr = -dE_lr/dpos, forces_sr = -dE_sr/dpos (device [n*3], either may be NULL);
  * pairs as in dmffb_admp_compute (NULL: the engine's own neighbour list). */
 int dmffb_disp_compute(dmffb_engine* h, void* stream, const double* pos, const double* box, const int32_t* pairs,
