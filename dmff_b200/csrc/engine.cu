@@ -1098,11 +1098,12 @@ int build_csr(dmffb_engine* h, cudaStream_t s, const int32_t* pairs, int64_t npa
 }
 
 // dE/dU at U (include_perm) or its linear part A U (!include_perm), into out.  With dot_out,
-// dot(dotv, out) is accumulated into *dot_out; cleared: the pair field (d_fieldT) is zero already
+// dot(dotv, out) is accumulated into *dot_out; cleared: the pair field (d_fieldT) is zero already; head:
+// the reciprocal pass has been queued already, from e_fork on (compute_impl)
 template <typename T>
 int field_eval(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx, const int32_t* pairs,
                int64_t npairs, const double* U, bool include_perm, double* out, const double* dotv = nullptr,
-               double* dot_out = nullptr, bool with_mvcoef = false, bool cleared = false) {
+               double* dot_out = nullptr, bool with_mvcoef = false, bool cleared = false, bool head = false) {
     const bool recip_on = h->lpme && h->have_plans;
     if (include_perm && !cleared) CK(cudaMemsetAsync(h->d_fieldT, 0, (size_t)4 * h->n * sizeof(T), s));
     // the real-space work (permanent pair field, matvec) runs on a side stream, overlapping the
@@ -1111,8 +1112,9 @@ int field_eval(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx
     const bool fork = real_work && h->s2 && !h->prof;
     cudaStream_t sr = s;
     if (fork) {
-        CK(cudaEventRecord(h->e_fork, s));
+        if (!head) CK(cudaEventRecord(h->e_fork, s));
         CK(cudaStreamWaitEvent(h->s2, h->e_fork, 0));
+        if (head && h->e_build) CK(cudaStreamWaitEvent(h->s2, h->e_build, 0));
         sr = h->s2;
     }
     // the CG matvec's pair tensors, needed only after this pass: also beside the reciprocal pass
@@ -1145,7 +1147,7 @@ int field_eval(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx
     if (fork) CK(cudaEventRecord(h->e_join, h->s2));
     const double* recip = nullptr;
     if (recip_on) {
-        int st = recip_pass<T>(h, s, pos, bx, include_perm, U, GATHER_FIELD, h->d_fr);
+        int st = head ? DMFFB_OK : recip_pass<T>(h, s, pos, bx, include_perm, U, GATHER_FIELD, h->d_fr);
         if (st) return st;
         recip = h->d_fr;
     }
@@ -1237,9 +1239,14 @@ int cg_persistent(dmffb_engine* h, cudaStream_t s, const Box& bx, double* U, con
     return DMFFB_OK;
 }
 
+struct StencilScope {  // the stencil cache ends with the positions it was made for
+    dmffb_engine* h;
+    ~StencilScope() { h->stencils_ready = false; }
+};
+
 template <typename T>
 int solve_dipoles(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx, const int32_t* pairs,
-                  int64_t npairs, double* U, dmffb_admp_result* res, const double* rhs = nullptr) {
+                  int64_t npairs, double* U, dmffb_admp_result* res, const double* rhs = nullptr, bool head = false) {
     const int n = h->n;
     const unsigned nb3 = nblk(3 * n, 256);
     double* sc = h->d_scal + S_CG;
@@ -1275,12 +1282,11 @@ int solve_dipoles(dmffb_engine* h, cudaStream_t s, const double* pos, const Box&
         return DMFFB_OK;
     }
     // CG on A U = -b.  The caller has cleared the permanent field, the scalars and with a zero guess U
-    // (compute_impl); with rhs that is done here.  The stencil cache holds for these positions only: it is dropped when the solve returns
-    struct StencilScope {
-        dmffb_engine* h;
-        ~StencilScope() { h->stencils_ready = false; }
-    } stencil_scope{h};
-    if (h->lpme && h->have_plans) {
+    // (compute_impl; with head it has also made the stencil cache and queued the permanent field's
+    // reciprocal pass); with rhs that is done here.  The stencil cache holds for these positions only: it is
+    // dropped when the solve returns
+    StencilScope stencil_scope{h};
+    if (h->lpme && h->have_plans && !head) {
         if ((st = stencil_prep<T>(h, s, pos, bx))) return st;
     }
     if (rhs) {
@@ -1288,7 +1294,8 @@ int solve_dipoles(dmffb_engine* h, cudaStream_t s, const double* pos, const Box&
         CK(cudaMemsetAsync(U, 0, (size_t)3 * n * sizeof(double), s));
         if ((st = matvec_coef_launch<T>(h, s, bx, pairs, npairs))) return st;
         CK(cudaMemcpyAsync(h->d_b, rhs, (size_t)3 * n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    } else if ((st = field_eval<T>(h, s, pos, bx, pairs, npairs, nullptr, true, h->d_b, nullptr, nullptr, true, true))) {
+    } else if ((st = field_eval<T>(h, s, pos, bx, pairs, npairs, nullptr, true, h->d_b, nullptr, nullptr, true, true,
+                                   head))) {
         return st;
     }
     // from U = 0 the residual is -b: no A U pass
@@ -1482,7 +1489,21 @@ int compute_impl(dmffb_engine* h, cudaStream_t s, const double* pos, const doubl
     if (cg && h->zero_guess) pa.clear.add(U, (size_t)3 * n * sizeof(double));
     LAUNCH(h, s, KC_PREP, k_prepare<T><<<nblk(n, 128), 128, 0, s>>>(pa));
     CK(cudaGetLastError());
-    // the work above needs no pair list: it runs while a single-pass build's totals come back
+    // Mesh work that needs no pair list is queued before the host waits for a single-pass build's totals:
+    // the permanent field's reciprocal pass of a dipole solve, or the whole reciprocal pass without
+    // polarizabilities.  The pair passes start from e_fork on the side stream, so what comes with the
+    // list must need no kernel on this one: the CSR and scaled-row map of the engine's own build.
+    const bool mesh = own_list && h->lpme && h->have_plans && h->s2 && !h->prof && !h->timing &&
+                      h->srows_pairs == h->d_pairs && h->srows_gen == h->pairs_gen;
+    StencilScope stencil_scope{h};
+    const bool field_head = mesh && cg && h->csr_from_build, full_head = mesh && !h->lpol;
+    if (field_head && (st = stencil_prep<T>(h, s, pos, bx))) return st;
+    if (field_head || full_head) {
+        CK(cudaEventRecord(h->e_fork, s));
+        st = field_head ? recip_pass<T>(h, s, pos, bx, true, nullptr, GATHER_FIELD, h->d_fr)
+                        : recip_pass<T>(h, s, pos, bx, true, nullptr, GATHER_FULL, nullptr);
+        if (st) return st;
+    }
     if (own_list) {
         if ((st = nb_finish(h))) return st;
         if (h->e_build) CK(cudaStreamWaitEvent(s, h->e_build, 0));
@@ -1498,7 +1519,7 @@ int compute_impl(dmffb_engine* h, cudaStream_t s, const double* pos, const doubl
         if ((st = scaled_rows(h, s, pairs, npairs))) return st;
     if (h->timing) CK(cudaEventRecord(h->ev[1], s));
     if (h->lpol && !h->fixed_U) {
-        if ((st = solve_dipoles<T>(h, s, pos, bx, pairs, npairs, U, res))) return st;
+        if ((st = solve_dipoles<T>(h, s, pos, bx, pairs, npairs, U, res, nullptr, field_head))) return st;
     } else {
         res->converged = 1;
     }
@@ -1508,8 +1529,9 @@ int compute_impl(dmffb_engine* h, cudaStream_t s, const double* pos, const doubl
     const bool fork_full = npairs > 0 && h->lpme && h->have_plans && h->s2 && !h->prof && !h->timing;
     cudaStream_t sp = s;
     if (fork_full) {
-        CK(cudaEventRecord(h->e_fork, s));
+        if (!full_head) CK(cudaEventRecord(h->e_fork, s));
         CK(cudaStreamWaitEvent(h->s2, h->e_fork, 0));
+        if (h->e_build && own_list) CK(cudaStreamWaitEvent(h->s2, h->e_build, 0));
         sp = h->s2;
     }
     if (npairs > 0) {
@@ -1541,7 +1563,7 @@ int compute_impl(dmffb_engine* h, cudaStream_t s, const double* pos, const doubl
     }
     if (fork_full) CK(cudaEventRecord(h->e_join, h->s2));
     if (h->timing) CK(cudaEventRecord(h->ev[3], s));
-    if (h->lpme && h->have_plans) {
+    if (h->lpme && h->have_plans && !full_head) {
         if ((st = recip_pass<T>(h, s, pos, bx, true, h->lpol ? U : nullptr, GATHER_FULL, nullptr))) return st;
     }
     if (fork_full) CK(cudaStreamWaitEvent(s, h->e_join, 0));
@@ -2155,16 +2177,10 @@ int classical_compute_impl(dmffb_engine* h, cudaStream_t s, const double* pos, c
     // the cell pass: every pair within rc straight from the cell grid of these positions
     int ncf[3] = {0, 0, 0};
     const bool cellpass = nonbonded && !pairs && h->cell_pass && h->pbc && !h->want_pgrad && half_cells(bx, h->rc, ncf);
-    if (nonbonded && !pairs && !cellpass) {
-        if (!h->have_pairs)
-            if ((st = dmffb_admp_build_neighbors(h, (void*)s, pos, box))) return st;
-        if ((st = nb_finish(h))) return st;
-        if (h->e_build) CK(cudaStreamWaitEvent(s, h->e_build, 0));
-        pairs = h->d_pairs;
-        npairs = h->npairs;
-    }
+    const bool own_list = nonbonded && !pairs && !cellpass;
+    if (own_list && !h->have_pairs)
+        if ((st = dmffb_admp_build_neighbors(h, (void*)s, pos, box))) return st;
     if (!nonbonded) npairs = 0;
-    res->n_pairs = npairs;
     const bool pg = h->want_pgrad;
     ClearList cl;
     cl.add(h->d_scal, N_SCAL * sizeof(double));
@@ -2178,6 +2194,39 @@ int classical_compute_impl(dmffb_engine* h, cudaStream_t s, const double* pos, c
             CK(cudaMemsetAsync(h->d_deps, 0, (size_t)h->ntypes * h->ntypes * sizeof(double), s));
         }
     }
+    const bool recip = h->coul == COUL_PME && h->lpme && h->have_plans;
+    if (recip) {
+        if ((st = recip_pass_channel<T>(h, s, pos, bx, (const T*)h->d_qT, CK_COUL, DMFFB_DIELECTRIC, h->d_grad,
+                                        pg ? h->d_dq : nullptr, h->d_scal + 24, h->d_scal + 32)))
+            return st;
+        if (pg)
+            LAUNCH(h, s, KC_SELF, k_self_dq<<<nblk(n, 256), 256, 0, s>>>(
+                                      n, h->d_q, -2.0 * DMFFB_DIELECTRIC * h->kappa / sqrt(M_PI), h->d_dq));
+    }
+    for (int kind = 0; kind < 3; ++kind) {
+        if (h->nterm[kind] <= 0) continue;
+        BondedArgs b;
+        b.nterm = (int)h->nterm[kind];
+        b.idx = h->d_tidx[kind];
+        b.prm = h->d_tprm[kind];
+        b.pos = pos;
+        b.grad = h->d_grad;
+        b.dprm = pg ? h->d_tdprm[kind] : nullptr;
+        b.scal = h->d_scal + 12 + kind;
+        const unsigned nbk = nblk(h->nterm[kind], 128);
+        if (kind == 0) LAUNCH(h, s, KC_BONDED, k_bonds<<<nbk, 128, 0, s>>>(b));
+        else if (kind == 1) LAUNCH(h, s, KC_BONDED, k_angles<<<nbk, 128, 0, s>>>(b));
+        else LAUNCH(h, s, KC_BONDED, k_torsions<<<nbk, 128, 0, s>>>(b));
+        CK(cudaGetLastError());
+    }
+    // the work above needs no pair list: it runs while a single-pass build's totals come back
+    if (own_list) {
+        if ((st = nb_finish(h))) return st;
+        if (h->e_build) CK(cudaStreamWaitEvent(s, h->e_build, 0));
+        pairs = h->d_pairs;
+        npairs = h->npairs;
+    }
+    res->n_pairs = npairs;
     if (cellpass) {
         if ((st = bin_cells(h, s, pos, bx, ncf))) return st;
         NbCellArgs<T> c;
@@ -2275,31 +2324,6 @@ int classical_compute_impl(dmffb_engine* h, cudaStream_t s, const double* pos, c
         } else {
             LAUNCH(h, s, KC_PAIR_FULL, k_nb_pair<T, 0><<<nbk, 128, 0, s>>>(a));
         }
-        CK(cudaGetLastError());
-    }
-    const bool recip = h->coul == COUL_PME && h->lpme && h->have_plans;
-    if (recip) {
-        if ((st = recip_pass_channel<T>(h, s, pos, bx, (const T*)h->d_qT, CK_COUL, DMFFB_DIELECTRIC, h->d_grad,
-                                        pg ? h->d_dq : nullptr, h->d_scal + 24, h->d_scal + 32)))
-            return st;
-        if (pg)
-            LAUNCH(h, s, KC_SELF, k_self_dq<<<nblk(n, 256), 256, 0, s>>>(
-                                      n, h->d_q, -2.0 * DMFFB_DIELECTRIC * h->kappa / sqrt(M_PI), h->d_dq));
-    }
-    for (int kind = 0; kind < 3; ++kind) {
-        if (h->nterm[kind] <= 0) continue;
-        BondedArgs b;
-        b.nterm = (int)h->nterm[kind];
-        b.idx = h->d_tidx[kind];
-        b.prm = h->d_tprm[kind];
-        b.pos = pos;
-        b.grad = h->d_grad;
-        b.dprm = pg ? h->d_tdprm[kind] : nullptr;
-        b.scal = h->d_scal + 12 + kind;
-        const unsigned nbk = nblk(h->nterm[kind], 128);
-        if (kind == 0) LAUNCH(h, s, KC_BONDED, k_bonds<<<nbk, 128, 0, s>>>(b));
-        else if (kind == 1) LAUNCH(h, s, KC_BONDED, k_angles<<<nbk, 128, 0, s>>>(b));
-        else LAUNCH(h, s, KC_BONDED, k_torsions<<<nbk, 128, 0, s>>>(b));
         CK(cudaGetLastError());
     }
     if (forces && cellpass)
