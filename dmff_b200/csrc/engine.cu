@@ -2238,6 +2238,8 @@ int classical_compute_impl(dmffb_engine* h, cudaStream_t s, const double* pos, c
         for (int k = 0; k < 3; ++k) c.nc[k] = ncf[k];
         c.cell_start = h->d_cell_start;
         c.atom_cell = h->d_atom_cell;
+        c.cov.box = bx;
+        c.cov.rc = h->rc;
         c.cov.cov_ptr = h->d_cov_ptr;
         c.cov.cov_j = h->d_cov_j;
         c.cov.cov_nb = h->d_cov_nb;

@@ -8,8 +8,9 @@
 //   * one warp per atom i walks the forward half of the 5^3 stencil of half-width cells (the 62
 //     offsets after (0, 0, 0) in lexicographic order, and in its own cell the atoms after it in
 //     cell order), so every unordered pair is met once, as one concatenated candidate list, 32
-//     candidates per batch, reading a cell-ordered float4 copy of the positions (contiguous runs
-//     per cell, the atom index in the w slot); atoms are taken in cell order, so the warps of a
+//     candidates per batch, reading a cell-ordered float4 copy of the positions (a contiguous run
+//     per z column of cells, two where it wraps, seen from the image the column wraps to, which is the
+//     nearest one for every pair within rc; the atom index in the w slot); atoms are taken in cell order, so the warps of a
 //     block share their candidates through L1 (with at least 5 cells per axis the 5 offsets of an
 //     axis are distinct cells, and a box of at least 2.5 rc has one image of a pair within rc);
 //   * stencil cells with no point within rc of the atom are skipped (per atom, from its position
@@ -25,8 +26,8 @@
 //     k_nb_pair; the force on i accumulates in lane registers (one warp sum and one reduction per
 //     atom), the force on the partner goes out as one 16-byte reduction into its cell slot;
 //   * the count of kept pairs (scaled ones included) is the list's row count.
-// Energies and the box gradient accumulate per lane (about 20 pairs each) and meet in an FP64 block
-// reduction.
+// Energies accumulate per lane (about seven pairs each), the box gradient per lane in FP64; they meet in
+// an FP64 block reduction.
 #pragma once
 #include "classical.cuh"
 #include "nblist.cuh"
@@ -114,11 +115,11 @@ __device__ __forceinline__ void nb_root(double r2, float& r) {
     r = (float)fma(0.5 * y, fma(-q, q, r2), q);
 }
 
-// One kept pair (i, the atom in cell slot k), met once: energy, box gradient, the force on i
-// (registers) and on the partner (a reduction into its slot).
+// One kept pair (i, the atom in cell slot k), met once: energy, box gradient (the lane's FP64 sums
+// box[0], box[32], ...), the force on i (registers) and on the partner (a reduction into its slot).
 template <typename T, bool ORTHO>
 __device__ __forceinline__ void nb_cell_pair(const NbCellArgs<T>& a, int k, double xi, double yi, double zi, bool lj,
-                                             int ti, T qi, T& g0, T& g1, T& g2, T (&acc)[11]) {
+                                             int ti, T qi, T& g0, T& g1, T& g2, T (&acc)[2], double* box) {
     const NbRec rj = a.rec[k];
     // the pair geometry of k_nb_pair: FP64 minimum image, then kernel precision
     T e[3], r;
@@ -162,22 +163,24 @@ __device__ __forceinline__ void nb_cell_pair(const NbCellArgs<T>& a, int k, doub
     if (nd[0] != 0.0 || nd[1] != 0.0 || nd[2] != 0.0) {  // most pairs meet inside the box
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
-            const T nn = (T)nd[q];
-            acc[2 + 3 * q] -= nn * f0;
-            acc[3 + 3 * q] -= nn * f1;
-            acc[4 + 3 * q] -= nn * f2;
+            box[32 * (3 * q)] -= nd[q] * (double)f0;
+            box[32 * (3 * q + 1)] -= nd[q] * (double)f1;
+            box[32 * (3 * q + 2)] -= nd[q] * (double)f2;
         }
     }
 }
 
-// Bound by instruction issue (FP64 minimum image, erfc / exp, the candidate test): 607 us for the 20.8 M
-// pairs of 99000 atoms at rc 10 A.  Scalar reductions into [3n], three FP64 gathers plus charge
-// and type per partner, FP64 division in the cell pruning and a full FP64 root took it to 822 us.
+// Bound by instruction issue (FP64 minimum image, erf / exp; 71 % of the issue slots): 475 us for
+// the 20.8 M pairs of 99000 atoms at rc 10 A.  Before: with a minimum image per candidate, 63 cells per
+// atom searched and pruned one by one and FP32 box sums in registers 563; with scalar reductions into
+// [3n], three FP64 gathers plus charge and type per partner, FP64 division in the pruning and a full FP64
+// root 822.
 template <typename T, bool ORTHO>
 __global__ void __launch_bounds__(32 * kNbWarps, sizeof(T) == 4 ? 4 : 0) k_nb_cells(NbCellArgs<T> a) {
-    constexpr int S = 2, W = 2 * S + 1, NQ = (W * W * W + 1) / 2;  // offsets q0 = 62 .. 124 of the 5^3 stencil
-    __shared__ int s_beg[kNbWarps][NQ];
-    __shared__ int s_off[kNbWarps][NQ + 1];
+    constexpr int NC = 13, NR = 2 * NC;  // forward columns of the 5^3 stencil, runs
+    __shared__ int s_beg[kNbWarps][NR], s_off[kNbWarps][NR + 1], s_img[kNbWarps][NR];
+    __shared__ float s_shift[18][3];  // lattice vectors a column can wrap by: 9 nx + 3 (ny + 1) + nz + 1
+    __shared__ double s_box[kNbWarps][9][32];  // the lanes' box gradients: in FP64, and few pairs cross the box
     __shared__ int s_q[kNbWarps][64];  // kept candidates (cell slots) waiting for a full 32-lane batch
     const int wl = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -185,6 +188,13 @@ __global__ void __launch_bounds__(32 * kNbWarps, sizeof(T) == 4 ? 4 : 0) k_nb_ce
     // candidate reads (contiguous runs of the cell-ordered copy) hit L1 after the first
     const int ks = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const bool live = ks < a.n;  // warps past the end still take part in the block reduction
+    if (threadIdx.x < 18) {
+        const int t = threadIdx.x, nx = t / 9, ny = (t / 3) % 3 - 1, nz = t % 3 - 1;
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+            s_shift[t][c] = (float)(nx * a.boxd.h[c] + ny * a.boxd.h[3 + c] + nz * a.boxd.h[6 + c]);
+    }
+    __syncthreads();
     double red[12];
 #pragma unroll
     for (int k = 0; k < 12; ++k) red[k] = 0.0;
@@ -192,17 +202,13 @@ __global__ void __launch_bounds__(32 * kNbWarps, sizeof(T) == 4 ? 4 : 0) k_nb_ce
         const float4 p4 = a.posc[ks];
         const int i = __float_as_int(p4.w);
         const NbRec ri = a.rec[ks];
-        float hf[9], hif[9];
-#pragma unroll
-        for (int k = 0; k < 9; ++k) { hf[k] = (float)a.boxd.h[k]; hif[k] = (float)a.boxd.hinv[k]; }
-        const float rlo = (float)(a.rc - 2e-3), rhi = (float)(a.rc + 2e-3);
-        const float rlo2 = rlo * rlo, rhi2 = rhi * rhi;
-        // The atom's cell (from the binning) and its position in it, in cell units.  A stencil cell none of
-        // whose points lies within rc + 0.01 A of the atom is skipped (about a third of the forward
-        // half for half-width cells).  Orthorhombic boxes: the exact distance to the cell's box;
-        // others the lower bound max_k gap_k width_k (gap_k the fractional gap along k).  The margin
-        // covers the FP32 prefilter band (rc +- 2e-3 A) and the rounding of the binning and of
-        // the FP32 gaps, so the kept pairs are unchanged.
+        const NbFilter f(a.cov);
+        // The atom's cell (from the binning) and its position in it, in cell units.  A lane takes one of
+        // the 13 columns (dx, dy) whose cells follow the atom's in lexicographic order and cuts its z range
+        // to the cells with a point within rc + 0.01 A of the atom.  Orthorhombic boxes: by the exact
+        // distance to the cell's box; others by the lower bound max_k gap_k width_k (gap_k the
+        // fractional gap along k).  The margin covers the FP32 prefilter band and the rounding of the
+        // binning and of the FP32 gaps, so the kept pairs are unchanged.
         const int ac = a.atom_cell[i];
         const int c3[3] = {ac / (a.nc[2] * a.nc[1]), (ac / a.nc[2]) % a.nc[1], ac % a.nc[2]};
         float u[3], cw[3];
@@ -214,43 +220,51 @@ __global__ void __launch_bounds__(32 * kNbWarps, sizeof(T) == 4 ? 4 : 0) k_nb_ce
             cw[k] = (float)(a.width[k] / a.nc[k]);
         }
         const float rprune = (float)(a.rc + 0.01);
-        int carry = 0;
-        if (lane == 0) s_off[wl][0] = 0;
-        for (int q0 = 0; q0 < NQ; q0 += 32) {
-            const int q = q0 + lane;
-            int cnt = 0;
-            if (q < NQ) {
-                const int qq = q + NQ - 1;  // (0, 0, 0) and the offsets after it
-                const int dd[3] = {qq / (W * W) - S, (qq / W) % W - S, qq % W - S};
-                int cc = 0;
-                float d2 = 0.f, dmax = 0.f;
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    int ck = c3[k] + dd[k];
-                    ck += ck < 0 ? a.nc[k] : (ck >= a.nc[k] ? -a.nc[k] : 0);
-                    cc = cc * a.nc[k] + ck;
-                    const float gap = fmaxf(0.f, fmaxf(dd[k] - u[k], u[k] - (dd[k] + 1))) * cw[k];
-                    d2 += gap * gap;
-                    dmax = fmaxf(dmax, gap);
+        int cnt[2] = {0, 0}, beg[2] = {0, 0}, img = 0, nz = 0;
+        if (lane < NC) {
+            const int dx = lane < 3 ? 0 : 1 + (lane - 3) / 5, dy = lane < 3 ? lane : (lane - 3) % 5 - 2;
+            const float gx = fmaxf(0.f, dx - u[0]) * cw[0];
+            const float gy = fmaxf(0.f, fmaxf(dy - u[1], u[1] - (dy + 1))) * cw[1];
+            const float rest = ORTHO ? rprune * rprune - gx * gx - gy * gy : rprune - fmaxf(gx, gy);
+            if (rest >= 0.f) {
+                const float reach = (ORTHO ? sqrtf(rest) : rprune) / cw[2];  // in cells
+                const int up = min(2, (int)floorf(u[2] + reach));
+                const int dn = lane == 0 ? 0 : max(-2, (int)ceilf(u[2] - 1.f - reach));
+                int x = c3[0] + dx, y = c3[1] + dy;
+                const int nx = x >= a.nc[0] ? 1 : 0, ny = y < 0 ? -1 : (y >= a.nc[1] ? 1 : 0);
+                x -= nx * a.nc[0];
+                y -= ny * a.nc[1];
+                const int* col = a.cell_start + (x * a.nc[1] + y) * a.nc[2];
+                const int zb = c3[2] + dn, ze = c3[2] + up;
+                const int z0 = max(zb, 0), z1 = min(ze, a.nc[2] - 1);
+                nz = zb < 0 ? -1 : (ze >= a.nc[2] ? 1 : 0);
+                beg[0] = lane == 0 ? ks + 1 : col[z0];  // own column: the atoms after i in cell order
+                cnt[0] = max(col[z1 + 1] - beg[0], 0);
+                if (nz) {
+                    const int w0 = nz < 0 ? zb + a.nc[2] : 0, w1 = nz < 0 ? a.nc[2] - 1 : ze - a.nc[2];
+                    beg[1] = col[w0];
+                    cnt[1] = col[w1 + 1] - beg[1];
                 }
-                int cs = a.cell_start[cc];
-                const int ce = a.cell_start[cc + 1];
-                if (q == 0) cs = max(cs, ks + 1);  // own cell: the atoms after i in cell order
-                cnt = max(ce - cs, 0);
-                if (q > 0 && (ORTHO ? d2 > rprune * rprune : dmax > rprune)) cnt = 0;
-                s_beg[wl][q] = cs;
+                img = 9 * nx + 3 * (ny + 1) + 1;
             }
-            int incl = cnt;
+        }
+        int incl = cnt[0] + cnt[1];
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int v = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += v;
-            }
-            if (q < NQ) s_off[wl][q + 1] = carry + incl;
-            carry += __shfl_sync(0xffffffffu, incl, 31);
+        for (int o = 1; o < 16; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        if (lane < NC) {
+            s_beg[wl][2 * lane] = beg[0];
+            s_beg[wl][2 * lane + 1] = beg[1];
+            s_img[wl][2 * lane] = img;
+            s_img[wl][2 * lane + 1] = img + nz;
+            s_off[wl][2 * lane] = incl - cnt[0] - cnt[1];
+            s_off[wl][2 * lane + 1] = incl - cnt[1];
+            if (lane == NC - 1) s_off[wl][NR] = incl;
         }
         __syncwarp();
-        const int total = carry;
+        const int total = s_off[wl][NR];
         const int lo = a.cov_lo[i], hi = a.cov_hi[i];
         const bool lj = a.type != nullptr;
         T qi;
@@ -258,53 +272,38 @@ __global__ void __launch_bounds__(32 * kNbWarps, sizeof(T) == 4 ? 4 : 0) k_nb_ce
         nb_rec_get(ri, qi, ti);
         if (sizeof(T) == 8 && lj) ti = a.type[i];
         T g0 = T(0), g1 = T(0), g2 = T(0);
-        T acc[11];  // per-lane sums of about 40 pairs, in kernel precision
+        T acc[2] = {T(0), T(0)};  // per-lane energies of about seven pairs, in kernel precision
+        double* const box = &s_box[wl][0][lane];
 #pragma unroll
-        for (int k = 0; k < 11; ++k) acc[k] = T(0);
+        for (int k = 0; k < 9; ++k) box[32 * k] = 0.0;
         int npair = 0;
         const unsigned lt = (1u << lane) - 1u;
         int qn = 0;  // queued kept candidates (warp-uniform)
-        int qc = 0;
+        // the lane's run: its end, the slot of candidate 0 and the atom seen from the run's image
+        int run = -1, end = 0, first = 0;
+        float bx = 0.f, by = 0.f, bz = 0.f;
         for (int base = 0; base < total; base += 32) {
             const int t = base + lane;
             bool keep = false;
             int slot = 0, j = -1;
             if (t < total) {
-                while (t >= s_off[wl][qc + 1]) ++qc;
-                slot = s_beg[wl][qc] + (t - s_off[wl][qc]);
+                if (t >= end) {
+                    do end = s_off[wl][++run + 1];
+                    while (t >= end);
+                    first = s_beg[wl][run] - s_off[wl][run];
+                    const float* sh = s_shift[s_img[wl][run]];
+                    bx = p4.x - sh[0];
+                    by = p4.y - sh[1];
+                    bz = p4.z - sh[2];
+                }
+                slot = first + t;
                 const float4 pj = a.posc[slot];
                 j = __float_as_int(pj.w);
-                const float d0 = pj.x - p4.x, d1 = pj.y - p4.y, d2 = pj.z - p4.z;
-                bool amb = false;
-                float r2;
-                if (ORTHO) {
-                    const float dd[3] = {d0, d1, d2};
-                    r2 = 0.f;
-#pragma unroll
-                    for (int q = 0; q < 3; ++q) {
-                        const float tt = dd[q] * hif[4 * q];
-                        const float sq = tt - floorf(tt + 0.5f);
-                        amb |= fabsf(sq) > 0.4999f;
-                        const float ev = sq * hf[4 * q];
-                        r2 = fmaf(ev, ev, r2);
-                    }
-                } else {
-                    float sf[3];
-#pragma unroll
-                    for (int q = 0; q < 3; ++q) {
-                        const float tt = d0 * hif[q] + d1 * hif[3 + q] + d2 * hif[6 + q];
-                        sf[q] = tt - floorf(tt + 0.5f);
-                        amb |= fabsf(sf[q]) > 0.4999f;
-                    }
-                    const float e0 = sf[0] * hf[0] + sf[1] * hf[3] + sf[2] * hf[6];
-                    const float e1 = sf[0] * hf[1] + sf[1] * hf[4] + sf[2] * hf[7];
-                    const float e2 = sf[0] * hf[2] + sf[1] * hf[5] + sf[2] * hf[8];
-                    r2 = e0 * e0 + e1 * e1 + e2 * e2;
-                }
-                if (!amb && r2 < rlo2) keep = true;
-                else if (!amb && r2 > rhi2) keep = false;
-                else keep = j > i ? within_rc(a.boxd, a.pos + 3 * i, a.pos + 3 * j, a.rc)
-                                  : within_rc(a.boxd, a.pos + 3 * j, a.pos + 3 * i, a.rc);
+                const float dx = pj.x - bx, dy = pj.y - by, dz = pj.z - bz;
+                const float r2 = dx * dx + dy * dy + dz * dz;
+                if (r2 < f.rlo2) keep = true;
+                else if (r2 <= f.rhi2) keep = j > i ? within_rc(a.boxd, a.pos + 3 * i, a.pos + 3 * j, a.rc)
+                                                    : within_rc(a.boxd, a.pos + 3 * j, a.pos + 3 * i, a.rc);
             }
             if (keep) ++npair;
             // topologically scaled pairs belong to the FP64 covalent pass
@@ -318,7 +317,7 @@ __global__ void __launch_bounds__(32 * kNbWarps, sizeof(T) == 4 ? 4 : 0) k_nb_ce
             qn += __popc(mk);
             __syncwarp();
             if (qn >= 32) {
-                nb_cell_pair<T, ORTHO>(a, s_q[wl][lane], ri.x, ri.y, ri.z, lj, ti, qi, g0, g1, g2, acc);
+                nb_cell_pair<T, ORTHO>(a, s_q[wl][lane], ri.x, ri.y, ri.z, lj, ti, qi, g0, g1, g2, acc, box);
                 __syncwarp();
                 if (lane < qn - 32) s_q[wl][lane] = s_q[wl][32 + lane];
                 qn -= 32;
@@ -326,9 +325,11 @@ __global__ void __launch_bounds__(32 * kNbWarps, sizeof(T) == 4 ? 4 : 0) k_nb_ce
             }
         }
         if (lane < qn)
-            nb_cell_pair<T, ORTHO>(a, s_q[wl][lane], ri.x, ri.y, ri.z, lj, ti, qi, g0, g1, g2, acc);
+            nb_cell_pair<T, ORTHO>(a, s_q[wl][lane], ri.x, ri.y, ri.z, lj, ti, qi, g0, g1, g2, acc, box);
 #pragma unroll
-        for (int k = 0; k < 11; ++k) red[k] = (double)acc[k];
+        for (int k = 0; k < 9; ++k) red[2 + k] = box[32 * k];
+        red[0] = (double)acc[0];
+        red[1] = (double)acc[1];
         red[11] = (double)npair;
         __syncwarp();
         g0 = warp_sum(g0);
