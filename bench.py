@@ -185,7 +185,7 @@ def class_rooflines(stats, steps, work, fp32_peak, hbm_peak):
 
 def cg_solve_bytes(s, n_pairs, iters):
     """Algorithmic bytes of one persistent CG solve (k_cg_solve) of ``iters`` iterations, per
-    iteration: the matvec's 12 B per CSR entry (24 B per pair), the dipole spread and field gather
+    iteration: the matvec's 20 B per CSR entry (40 B per pair), the dipole spread and field gather
     (N(12 + 16) + 4K^3 and 4K^3 + N(12 + 16 + 24)), the three FFT passes (mesh read, spectrum
     written, spectrum read and written by the column pass, spectrum read, mesh written: 24 K^3 in
     FP32 complex half-spectrum units counted as 4 B per real mesh point), and the CG vectors (the
@@ -193,14 +193,14 @@ def cg_solve_bytes(s, n_pairs, iters):
     r, z: 24 + 80 B per atom component)."""
     n = s["n_atoms"]
     K3 = float(np.prod(s["K"]))
-    per_iter = 24.0 * n_pairs + n * (12 + 16) + 4 * K3 + 4 * K3 + n * (12 + 16 + 24) + 24 * K3 + 3 * n * (24 + 80)
+    per_iter = 40.0 * n_pairs + n * (12 + 16) + 4 * K3 + 4 * K3 + n * (12 + 16 + 24) + 24 * K3 + 3 * n * (24 + 80)
     return iters * per_iter
 
 
 def admp_work(s, n_pairs, n_scaled, iters=0):
     """Algorithmic work per launch of each class for a polarizable ADMP step (fixed convention:
     FMA = 2 flop, exp / erf / erfc / sqrt / div = 1 flop): pair FULL polarizable 1900 flop/pair,
-    FIELD 600 flop/pair, the CG matvec 12 B per CSR entry (two entries per pair: packed j + two
+    FIELD 600 flop/pair, the CG matvec 20 B per CSR entry (two entries per pair: packed j + four
     FP32 coefficients), its coefficient set-up 200 flop/pair, dipole spread N(12 + 4*4) + 4K^3 B,
     field gather 4K^3 + N(12 + 4*4 + 24) B, convolution 16 K^3 B, neighbour build 12N + 12Np B per
     step (its launches share it).  Pair classes count the rows they run over: the FP32 launches
@@ -210,7 +210,7 @@ def admp_work(s, n_pairs, n_scaled, iters=0):
     un = n_pairs - n_scaled
     return {"pair_full": ("fp32", 1900.0 * un), "pair_field": ("fp32", 600.0 * un),
             "pair_full_scaled": ("fp64", 1900.0 * n_scaled), "pair_field_scaled": ("fp64", 600.0 * n_scaled),
-            "pair_matvec": ("hbm", 12.0 * 2 * n_pairs), "matvec_coef": ("fp32", 200.0 * n_pairs),
+            "pair_matvec": ("hbm", 20.0 * 2 * n_pairs), "matvec_coef": ("fp32", 200.0 * n_pairs),
             "spread": ("hbm", n * (12 + 4 * 4) + 4 * K3), "gather_field": ("hbm", 4 * K3 + n * (12 + 16 + 24)),
             "conv": ("hbm", 16 * K3), "cg_persistent": ("hbm", cg_solve_bytes(s, n_pairs, iters))}
 
@@ -810,8 +810,8 @@ def main():
         roof = headline_roofline(classes, cg_solve_bytes(s, n_pairs, n_iter_med), None, peaks["hbm_gbs"], src,
                                  "k_cg_solve (persistent CG dipole solve)", "cg_persistent")
     else:
-        # the per-pass solve: the CG matvec, 12 B per CSR entry
-        roof = headline_roofline(classes, 12.0 * 2 * n_pairs, None, peaks["hbm_gbs"], src,
+        # the per-pass solve: the CG matvec, 20 B per CSR entry
+        roof = headline_roofline(classes, 20.0 * 2 * n_pairs, None, peaks["hbm_gbs"], src,
                                  "k_matvec_apply (CG matvec)", "pair_matvec")
 
     c4 = None

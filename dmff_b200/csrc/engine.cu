@@ -1450,7 +1450,14 @@ int solve_dipoles(dmffb_engine* h, cudaStream_t s, const double* pos, const Box&
         }
     }
     if (rms_b == 0.0) it = 0;  // nothing to solve
-    if (fused && u0 && !rhs) h->cg_hint = conv ? (e < it ? it - 1 : e_prev) : 0;
+    if (fused && u0 && !rhs) {
+        h->cg_hint = conv ? e_prev : 0;
+        if (conv && e < it && it < kCgHist) {  // the head start was too long: one short of where it converged
+            int k = 0;
+            while (k < it && sqrt(h->h_scal[CGS_COUNT + 1 + k] / (3.0 * n)) > h->cg_tol * rms_b) ++k;
+            h->cg_hint = std::max(k - 1, 0);
+        }
+    }
     res->n_iter = it;
     res->converged = conv ? 1 : 0;
     res->residual_rms = rms;
