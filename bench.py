@@ -23,6 +23,7 @@ import os
 import statistics
 import subprocess
 import sys
+import threading
 import time
 
 import numpy as np
@@ -56,7 +57,7 @@ def parse():
                    help="per-request latency of single serving boxes (150-9000 waters) with the per-pass and "
                         "the persistent dipole solve, one JSON line, then exit")
     p.add_argument("--fused-fft", action="store_true",
-                   help="dipole-solve convolution through the engine's FFT kernels instead of cuFFT")
+                   help="ask for the direct-DFT convolution kernels; default is the engine's size rule")
     return p.parse_args()
 
 
@@ -76,23 +77,43 @@ def workload_config(name, s, world=1):
 class ClockSampler:
     """SM clock, power and clock-event reasons sampled while the timed region runs: one
     ``nvidia-smi --query-gpu ... -lms 20`` process (read-only queries, a sample every 20 ms) from
-    entry to exit, its CSV parsed afterwards."""
+    entry to exit, its CSV read by a thread.  The process takes longer to start than a short timed region
+    lasts, so untimed steps of the same work (``load``) run until its first sample arrives and for three
+    periods after the region: the samples are all taken under that load, around and in the region."""
     FIELDS = ("index,clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,"
               "clocks_event_reasons.hw_slowdown,clocks_event_reasons.hw_thermal_slowdown,"
               "clocks_event_reasons.sw_thermal_slowdown,clocks_event_reasons.sw_power_cap")
     NAMES = ["hw_slowdown", "hw_thermal_slowdown", "sw_thermal_slowdown", "sw_power_cap"]
     PERIOD_MS = 20
 
-    def __init__(self, gpu_index):
+    def __init__(self, gpu_index, load):
         self.gpu = gpu_index
+        self.load = load
         self.rows = []  # (sm_mhz, max_mhz, [reason names])
         self._p = None
+        self._reader = None
+
+    def _read(self):
+        for line in self._p.stdout:
+            r = [x.strip() for x in line.split(",")]
+            if len(r) >= 9 and r[1].replace(".", "").isdigit():
+                self.rows.append((float(r[1]), float(r[2]),
+                                  [n for k, n in enumerate(self.NAMES) if r[5 + k] == "Active"]))
+
+    def _run_load(self, seconds, until_sample=False):
+        end = time.perf_counter() + seconds
+        while time.perf_counter() < end and not (until_sample and self.rows):
+            self.load()
+            torch.cuda.synchronize()
 
     def __enter__(self):
         try:
             self._p = subprocess.Popen(["nvidia-smi", "-i", str(self.gpu), f"--query-gpu={self.FIELDS}",
                                         "--format=csv,noheader,nounits", "-lms", str(self.PERIOD_MS)],
                                        stdout=subprocess.PIPE, stderr=subprocess.DEVNULL, text=True)
+            self._reader = threading.Thread(target=self._read, daemon=True)
+            self._reader.start()
+            self._run_load(3.0, until_sample=True)
         except Exception:
             self._p = None
         return self
@@ -100,18 +121,14 @@ class ClockSampler:
     def __exit__(self, *a):
         if self._p is None:
             return
-        time.sleep(2 * self.PERIOD_MS / 1000.0)  # at least one sample after the timed region
+        self._run_load(3 * self.PERIOD_MS / 1000.0)
         self._p.terminate()
         try:
-            out, _ = self._p.communicate(timeout=10)
+            self._p.wait(timeout=10)
         except Exception:
             self._p.kill()
-            out, _ = self._p.communicate()
-        for line in out.strip().splitlines():
-            r = [x.strip() for x in line.split(",")]
-            if len(r) >= 9 and r[1].replace(".", "").isdigit():
-                self.rows.append((float(r[1]), float(r[2]),
-                                  [n for k, n in enumerate(self.NAMES) if r[5 + k] == "Active"]))
+            self._p.wait()
+        self._reader.join(timeout=10)
 
     def summary(self):
         sm = [r[0] for r in self.rows]
@@ -500,20 +517,20 @@ def measure_c4(args, dev, peaks, fp32_peak, world=1, dist=None):
         res, F = step()
     flush = torch.empty(L2_FLUSH_BYTES // 4, dtype=torch.float32, device=dev)
     torch.cuda.synchronize()
-    l0 = eng.counters()
     evs = [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)) for _ in range(args.steps)]
-    if dist is not None:
-        dist.barrier()
-    torch.cuda.synchronize()
-    with ClockSampler(dev.index or 0) as clk:
+    with ClockSampler(dev.index or 0, step) as clk:
+        if dist is not None:
+            dist.barrier()
+        torch.cuda.synchronize()
+        l0 = eng.counters()
         for k in range(args.steps):
             flush.zero_()
             evs[k][0].record(stream)
             res, F = step()
             evs[k][1].record(stream)
         torch.cuda.synchronize()
+        l1 = eng.counters()
     total = sum(a.elapsed_time(b) for a, b in evs)
-    l1 = eng.counters()
     if dist is not None:
         t = torch.tensor([total], device=dev)
         dist.all_reduce(t, op=dist.ReduceOp.MAX)
@@ -727,7 +744,8 @@ def main():
                      s["axis_indices"], s["cov_rows"], s["mscales"], s["pscales"], s["dscales"], precision="fp32",
                      solver="cg", cg_tol=1e-6, max_iter=1000, device=dev)
     eng.set_params(s["Q_local"], s.get("pol"), s.get("thole"))
-    eng.set_fused_fft(args.fused_fft)
+    if args.fused_fft:
+        eng.set_fused_fft(True)
     eng.set_persistent_cg({"auto": "auto", "persistent": 1, "per-pass": 0}[args.cg])
     if s["lpol"]:
         eng.set_zero_guess(True)  # every step solves from U = 0 (the reference's U_init = None)
@@ -743,13 +761,13 @@ def main():
     for _ in range(args.warmup):
         res, F, U = step()
     torch.cuda.synchronize()
-    launches0 = eng.counters()
     evs = [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)) for _ in range(args.steps)]
     iters = []
-    if world > 1:
-        dist.barrier()
-    torch.cuda.synchronize()
-    with ClockSampler(local) as clk:
+    with ClockSampler(local, step) as clk:
+        if world > 1:
+            dist.barrier()
+        torch.cuda.synchronize()
+        launches0 = eng.counters()
         for k in range(args.steps):
             flush.zero_()
             evs[k][0].record(stream)
@@ -757,11 +775,11 @@ def main():
             evs[k][1].record(stream)
             iters.append(res.n_iter)
         torch.cuda.synchronize()
-    if world > 1:
-        dist.barrier()
+        if world > 1:
+            dist.barrier()
+        launches1 = eng.counters()
     step_ms = [a.elapsed_time(b) for a, b in evs]
     total_ms = sum(step_ms)
-    launches1 = eng.counters()
     if world > 1:
         t = torch.tensor([total_ms], device=dev)
         dist.all_reduce(t, op=dist.ReduceOp.MAX)
@@ -842,8 +860,8 @@ def main():
         pcg = eng.persistent_cg_blocks() > 0
         out["config"]["dipole_solve"] = (f"persistent CG kernel k_cg_solve ({eng.persistent_cg_blocks()} co-resident CTAs)"
                                          if pcg else "graph-replayed per-pass CG")
-        out["config"]["dipole_convolution"] = ("engine FFT passes inside k_cg_solve" if pcg else
-                                               "engine FFT kernels (k_fc_*)" if eng.fused_fft_active()
+        out["config"]["dipole_convolution"] = ("direct-DFT passes inside k_cg_solve" if pcg else
+                                               "direct-DFT kernels (k_dft_*)" if eng.fused_fft_active()
                                                else "cuFFT R2C + k_conv + cuFFT C2R")
         if world == 1 and not args.no_cpu_baseline:
             cs, run, cores = cpu_reference_runner()
