@@ -77,7 +77,8 @@ def workload_config(name, s, world=1):
 class ClockSampler:
     """SM clock, power and clock-event reasons sampled while the timed region runs: one
     ``nvidia-smi --query-gpu ... -lms 20`` process (read-only queries, a sample every 20 ms) from
-    entry to exit, its CSV read by a thread.  The process takes longer to start than a short timed region
+    entry to exit, its CSV read by a thread from a terminal pair (into a pipe nvidia-smi writes blocks of
+    4 KB, some 80 samples late).  The process takes longer to start than a short timed region
     lasts, so untimed steps of the same work (``load``) run until its first sample arrives and for three
     periods after the region: the samples are all taken under that load, around and in the region."""
     FIELDS = ("index,clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,"
@@ -93,14 +94,19 @@ class ClockSampler:
         self._p = None
         self._reader = None
 
-    def _read(self):
-        for line in self._p.stdout:
-            r = [x.strip() for x in line.split(",")]
-            if len(r) >= 9 and r[1].replace(".", "").isdigit():
-                self.rows.append((float(r[1]), float(r[2]),
-                                  [n for k, n in enumerate(self.NAMES) if r[5 + k] == "Active"]))
+    def _read(self, fd):
+        with open(fd, "r", errors="replace") as f:
+            try:
+                for line in f:
+                    r = [x.strip() for x in line.split(",")]
+                    if len(r) >= 9 and r[1].replace(".", "").isdigit():
+                        self.rows.append((float(r[1]), float(r[2]),
+                                          [n for k, n in enumerate(self.NAMES) if r[5 + k] == "Active"]))
+            except OSError:  # the writing end closed
+                pass
 
     def _run_load(self, seconds, until_sample=False):
+        import torch
         end = time.perf_counter() + seconds
         while time.perf_counter() < end and not (until_sample and self.rows):
             self.load()
@@ -108,14 +114,17 @@ class ClockSampler:
 
     def __enter__(self):
         try:
+            master, slave = os.openpty()
             self._p = subprocess.Popen(["nvidia-smi", "-i", str(self.gpu), f"--query-gpu={self.FIELDS}",
                                         "--format=csv,noheader,nounits", "-lms", str(self.PERIOD_MS)],
-                                       stdout=subprocess.PIPE, stderr=subprocess.DEVNULL, text=True)
-            self._reader = threading.Thread(target=self._read, daemon=True)
+                                       stdin=subprocess.DEVNULL, stdout=slave, stderr=subprocess.DEVNULL)
+            os.close(slave)
+            self._reader = threading.Thread(target=self._read, args=(master,), daemon=True)
             self._reader.start()
-            self._run_load(3.0, until_sample=True)
         except Exception:
             self._p = None
+            return self
+        self._run_load(10.0, until_sample=True)
         return self
 
     def __exit__(self, *a):
