@@ -741,26 +741,51 @@ __device__ __forceinline__ int scale_index(int nb) {
     return sidx < 0 ? 0 : (sidx > 5 ? 5 : sidx);
 }
 
+// Full CSR of a caller's rows.  Bound by the atomics on the atoms' counters: rows of a list come grouped
+// by their first atom, so 32 lanes hit the same counter.  Neighbouring lanes with the same first atom make
+// one addition of their number; rows in any other order make shorter runs and the same lists.  At 6144
+// atoms: count 31 -> 8.4, fill 42 -> 13.2 us.
+struct RowRun {
+    int i, j;    // i < 0: no row, or one that counts nothing
+    int start;   // lane of the run's first row
+    int len;     // rows of the run, in that lane
+};
+
+__device__ __forceinline__ RowRun row_run(int64_t r, int64_t npairs, const int32_t* pairs, int n) {
+    const int lane = threadIdx.x & 31;
+    RowRun q = {-1, -1, lane, 0};
+    if (r < npairs) {
+        const int i = pairs[3 * r], j = pairs[3 * r + 1];
+        if (i >= 0 && i < j && j < n) { q.i = i; q.j = j; }
+    }
+    const int before = __shfl_up_sync(~0u, q.i, 1);
+    const unsigned heads = __ballot_sync(~0u, lane == 0 || before != q.i);
+    q.start = 31 - __clz(heads & (~0u >> (31 - lane)));
+    const unsigned later = heads & ~(~0u >> (31 - lane));
+    q.len = (later ? __ffs(later) - 1 : 32) - lane;
+    return q;
+}
+
 __global__ void k_csr_count(int64_t npairs, const int32_t* pairs, int n, int32_t* deg) {
-    const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= npairs) return;
-    const int i = pairs[3 * r], j = pairs[3 * r + 1];
-    if (i < 0 || i >= j || j >= n) return;
-    atomicAdd(deg + i, 1);
-    atomicAdd(deg + j, 1);
+    const RowRun q = row_run((int64_t)blockIdx.x * blockDim.x + threadIdx.x, npairs, pairs, n);
+    if (q.i < 0) return;
+    if (q.start == (threadIdx.x & 31)) atomicAdd(deg + q.i, q.len);
+    atomicAdd(deg + q.j, 1);
 }
 
 __global__ void k_csr_fill(int64_t npairs, const int32_t* pairs, int n, const int64_t* off, int32_t* cursor,
                            int32_t* ent) {
     const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= npairs) return;
-    const int i = pairs[3 * r], j = pairs[3 * r + 1];
-    if (i < 0 || i >= j || j >= n) return;
+    const int lane = threadIdx.x & 31;
+    const RowRun q = row_run(r, npairs, pairs, n);
+    int ki = 0;
+    if (q.i >= 0 && q.start == lane) ki = atomicAdd(cursor + q.i, q.len);
+    ki = __shfl_sync(~0u, ki, q.start) + lane - q.start;
+    if (q.i < 0) return;
     const int s = scale_index(pairs[3 * r + 2]);
-    const int ki = atomicAdd(cursor + i, 1);
-    const int kj = atomicAdd(cursor + j, 1);
-    ent[off[i] + ki] = j | (s << 28);
-    ent[off[j] + kj] = i | (s << 28);
+    const int kj = atomicAdd(cursor + q.j, 1);
+    ent[off[q.i] + ki] = q.j | (s << 28);
+    ent[off[q.j] + kj] = q.i | (s << 28);
 }
 
 // Matvec split in two: the pair tensors of every CSR entry are fixed during one dipole solve, so they
