@@ -54,6 +54,13 @@ def _on_device(device, first, *rest):
                for x in (first, *rest)) and first is not None
 
 
+def _per_site(n, **arrays):
+    """Host arrays of at least n values each (None stays None): the engine reads the first n of them."""
+    for name, x in arrays.items():
+        if x is not None and x.size < n:
+            raise ValueError(f"{name}: {x.size} values for {n} sites")
+
+
 class AdmpEngine:
     """One ADMP multipolar PME system on one GPU.
 
@@ -144,13 +151,13 @@ class AdmpEngine:
         return st
 
     def set_params(self, Q_local, pol=None, thole=None):
-        """Per-atom parameters.  CUDA tensors on the engine's device stay there (no host copy, no wait);
-        anything else goes through host arrays."""
-        if _on_device(self.device, Q_local, pol, thole):
+        """Per-atom parameters.  CUDA tensors on the engine's device with a row or value per atom stay there
+        (no host copy, no wait); anything else goes through host arrays."""
+        if _on_device(self.device, Q_local, pol, thole) and self._per_atom(Q_local, pol, thole):
             Q = Q_local.detach()
             if Q.shape[1] < 9:
                 Q = torch.nn.functional.pad(Q, (0, 9 - Q.shape[1]))
-            Q = Q[:, :9].contiguous()
+            Q = Q.contiguous()
             p, t = (None, None) if pol is None else (pol.detach().contiguous(), thole.detach().contiguous())
             s = torch.cuda.current_stream(self.device)
             self._check(self.lib.dmffb_admp_set_params_device(
@@ -163,12 +170,19 @@ class AdmpEngine:
         Q = np.ascontiguousarray(Q)
         p = t = None
         if pol is not None:
-            p = np.ascontiguousarray(np.asarray(pol.detach().cpu() if torch.is_tensor(pol) else pol, np.float64))
-            t = np.ascontiguousarray(np.asarray(thole.detach().cpu() if torch.is_tensor(thole) else thole, np.float64))
+            p, t = (None if x is None else np.ascontiguousarray(np.asarray(x.detach().cpu() if torch.is_tensor(x) else x, np.float64))
+                    for x in (pol, thole))
+            _per_site(self.n, pol=p, thole=t)
         with torch.cuda.device(self.device):
             self._check(self.lib.dmffb_admp_set_params(
                 self.h, Q.ctypes.data_as(ctypes.c_void_p), None if p is None else p.ctypes.data_as(ctypes.c_void_p),
                 None if t is None else t.ctypes.data_as(ctypes.c_void_p)))
+
+    def _per_atom(self, Q_local, pol, thole):
+        """Whether the arrays hold what the device copies read: [n, c <= 9] and n values each.  The host path
+        broadcasts or refuses the rest."""
+        return (Q_local.dim() == 2 and Q_local.shape[0] == self.n and Q_local.shape[1] <= 9
+                and (pol is None or (thole is not None and pol.numel() == self.n and thole.numel() == self.n)))
 
     @staticmethod
     def _box(box):
