@@ -58,7 +58,7 @@ def _per_site(n, **arrays):
     """Host arrays of at least n values each (None stays None): the engine reads the first n of them."""
     for name, x in arrays.items():
         if x is not None and x.size < n:
-            raise ValueError(f"{name}: {x.size} values for {n} sites")
+            raise ValueError(f"{name}: {x.size} values where {n} are read")
 
 
 class AdmpEngine:
@@ -468,7 +468,7 @@ class DispEngine:
     kernel_stats = AdmpEngine.kernel_stats
 
     def set_params(self, c_list, a=None, b=None, q=None):
-        if _on_device(self.device, c_list, a, b, q):
+        if _on_device(self.device, c_list, a, b, q) and self._per_atom(c_list, a, b, q):
             t = [None if x is None else x.detach().contiguous() for x in (c_list, a, b, q)]
             s = torch.cuda.current_stream(self.device)
             self._check(self.lib.dmffb_disp_set_params_device(
@@ -477,9 +477,15 @@ class DispEngine:
         host = lambda x: None if x is None else np.ascontiguousarray(
             np.asarray(x.detach().cpu() if torch.is_tensor(x) else x, np.float64))
         c, a, b, q = host(c_list), host(a), host(b), host(q)
+        _per_site(3 * self.n, c_list=c)
+        _per_site(self.n, a=a, b=b, q=q)
         ptr = lambda x: None if x is None else x.ctypes.data_as(ctypes.c_void_p)
         with torch.cuda.device(self.device):
             self._check(self.lib.dmffb_disp_set_params(self.h, ptr(c), ptr(a), ptr(b), ptr(q)))
+
+    def _per_atom(self, c_list, a, b, q):
+        """Whether the arrays hold what the device copies read: [n, 3] and n values each."""
+        return tuple(c_list.shape) == (self.n, 3) and all(x is None or x.numel() == self.n for x in (a, b, q))
 
     def compute(self, pos, box, pairs=None):
         """Returns (result, (forces_lr, forces_sr)); forces = -dE/dpos of E_lr and E_sr."""

@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 import torch
 
+from dmff_b200.engine import DispEngine
 from dmff_b200.synthetic import water_box
 from tests.helpers import make_engine
 
@@ -29,3 +30,13 @@ def test_admp_shapes():
         eng.set_params(row, pol, thole)
         E.append(eng.compute(pos, box)[0].energy)
     assert max(E) - min(E) <= 1e-9 * max(abs(E[0]), 1.0)
+
+
+def test_dispersion_shapes():
+    s = water_box(8, 9.3, seed=3, lmax=2, pol=True, rc=4.4)
+    n = len(s["pos"])
+    eng = DispEngine(n, 10, True, 4.4, 0.5, (12, 12, 12), None, (0, 0, 0, 1, 1, 1), tt=True)
+    c, a = torch.ones((n, 3), dtype=torch.float64, device="cuda"), torch.ones(n, dtype=torch.float64, device="cuda")
+    for args in ((c[:, :1], a, a, a), (c[:-1], a, a, a), (c, a[:-1], a, a), (c, a, a, a[:1])):
+        with pytest.raises(ValueError):
+            eng.set_params(*args)

@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 import torch
 
-from dmff_b200.engine import AdmpEngine
+from dmff_b200.engine import AdmpEngine, DispEngine
 
 N = 4
 
@@ -18,6 +18,11 @@ class _Lib:
     def dmffb_admp_set_params(self, h, Q, pol, thole):
         vals = lambda p, m: None if p is None else np.ctypeslib.as_array((ctypes.c_double * m).from_address(p.value)).copy()  # noqa: E731
         self.calls.append((vals(Q, 9 * N).reshape(N, 9), vals(pol, N), vals(thole, N)))
+        return 0
+
+    def dmffb_disp_set_params(self, h, c, a, b, q):
+        vals = lambda p, m: None if p is None else np.ctypeslib.as_array((ctypes.c_double * m).from_address(p.value)).copy()  # noqa: E731
+        self.calls.append((vals(c, 3 * N), vals(a, N), vals(b, N), vals(q, N)))
         return 0
 
 
@@ -59,6 +64,32 @@ def test_host_path_broadcasts_and_refuses():
     eng.set_params(_z(N, 9), _z(N, 1), None)  # the engine answers a missing thole
     assert lib.calls.pop()[2] is None
     for args in ((_z(N - 1, 9),), (_z(N, 10),), (_z(N, 9), _z(N - 1), _z(N)), (_z(N, 9), _z(N), _z(1))):
+        with pytest.raises(ValueError):
+            eng.set_params(*args)
+    assert not lib.calls
+
+
+@pytest.mark.parametrize("c,rest,ok", [
+    (_z(N, 3), (None, None, None), True),
+    (_z(N, 3), (_z(N), _z(N, 1), _z(N)), True),
+    (_z(3, N), (None, None, None), False),
+    (_z(3 * N), (None, None, None), False),
+    (_z(N - 1, 3), (None, None, None), False),
+    (_z(N, 1), (None, None, None), False),
+    (_z(N, 3), (_z(N), _z(N - 1), _z(N)), False),
+    (_z(N, 3), (_z(N), _z(N), _z(1)), False),
+])
+def test_what_the_dispersion_device_copies_may_read(c, rest, ok):
+    assert _engine(DispEngine, None)._per_atom(c, *rest) is ok
+
+
+def test_dispersion_host_path():
+    lib = _Lib()
+    eng = _engine(DispEngine, lib)
+    eng.set_params(np.arange(3.0 * N), *(np.full(N + 1, float(k)) for k in range(3)))  # flat, longer arrays
+    c, a, b, q = lib.calls.pop()
+    assert np.array_equal(c, np.arange(3.0 * N)) and [x[0] for x in (a, b, q)] == [0.0, 1.0, 2.0]
+    for args in ((_z(N, 1),), (_z(N - 1, 3),), (_z(N, 3), _z(N), _z(N - 1), _z(N))):
         with pytest.raises(ValueError):
             eng.set_params(*args)
     assert not lib.calls
