@@ -160,9 +160,9 @@ class AdmpEngine:
             Q = Q.contiguous()
             p, t = (None, None) if pol is None else (pol.detach().contiguous(), thole.detach().contiguous())
             s = torch.cuda.current_stream(self.device)
-            self._check(self.lib.dmffb_admp_set_params_device(
-                self.h, ctypes.c_void_p(s.cuda_stream), _dev(Q), None if p is None else _dev(p),
-                None if t is None else _dev(t)))
+            with torch.cuda.device(self.device):
+                self._check(self.lib.dmffb_admp_set_params_device(
+                    self.h, ctypes.c_void_p(s.cuda_stream), _dev(Q), _dev(p), _dev(t)))
             return
         Q = np.zeros((self.n, 9), dtype=np.float64)
         Qi = np.asarray(Q_local.detach().cpu() if torch.is_tensor(Q_local) else Q_local, dtype=np.float64)
@@ -471,8 +471,9 @@ class DispEngine:
         if _on_device(self.device, c_list, a, b, q) and self._per_atom(c_list, a, b, q):
             t = [None if x is None else x.detach().contiguous() for x in (c_list, a, b, q)]
             s = torch.cuda.current_stream(self.device)
-            self._check(self.lib.dmffb_disp_set_params_device(
-                self.h, ctypes.c_void_p(s.cuda_stream), *(None if x is None else _dev(x) for x in t)))
+            with torch.cuda.device(self.device):
+                self._check(self.lib.dmffb_disp_set_params_device(
+                    self.h, ctypes.c_void_p(s.cuda_stream), *(_dev(x) for x in t)))
             return
         host = lambda x: None if x is None else np.ascontiguousarray(
             np.asarray(x.detach().cpu() if torch.is_tensor(x) else x, np.float64))

@@ -1,11 +1,15 @@
 """Shapes of the per-atom parameters before they reach the engine: what the device copies may read, and
-what the host path broadcasts or refuses.  No GPU: the library is a stand-in that records its calls."""
+what the host path broadcasts or refuses; the device that the copies are queued on.  No GPU: the library is
+a stand-in that records its calls."""
+import contextlib
 import ctypes
+import types
 
 import numpy as np
 import pytest
 import torch
 
+from dmff_b200 import engine
 from dmff_b200.engine import AdmpEngine, DispEngine
 
 N = 4
@@ -93,3 +97,25 @@ def test_dispersion_host_path():
         with pytest.raises(ValueError):
             eng.set_params(*args)
     assert not lib.calls
+
+
+@pytest.mark.parametrize("cls,name,args", [
+    (AdmpEngine, "dmffb_admp_set_params_device", (_z(N, 4), _z(N), _z(N))),
+    (DispEngine, "dmffb_disp_set_params_device", (_z(N, 3), None, None, None)),
+])
+def test_device_path_enters_the_engines_device(monkeypatch, cls, name, args):
+    """Buffers are allocated and kernels launched there: both go by the current device."""
+    current, seen = [], []
+
+    @contextlib.contextmanager
+    def device(d):
+        current.append(d)
+        yield
+        current.pop()
+
+    monkeypatch.setattr(engine, "_on_device", lambda *a: True)
+    monkeypatch.setattr(torch.cuda, "device", device)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda d: types.SimpleNamespace(cuda_stream=0))
+    lib = types.SimpleNamespace(**{name: lambda *a: seen.append(list(current)) or 0})
+    _engine(cls, lib).set_params(*args)
+    assert seen == [[-1]]
