@@ -347,6 +347,7 @@ struct Nb2Args {
 // the FP32 box and prefilter bounds of a pair pass
 struct NbFilter {
     float h[9], hi[9], rlo2, rhi2;
+    float far[3];  // fractional differences (by the sum of their terms' sizes) that FP32 resolves to the band
     __device__ __forceinline__ explicit NbFilter(const NbArgs& a) {
 #pragma unroll
         for (int k = 0; k < 9; ++k) { h[k] = (float)a.box.h[k]; hi[k] = (float)a.box.hinv[k]; }
@@ -358,11 +359,19 @@ struct NbFilter {
         const float rlo = (float)fmax(a.rc - band, 0.0), rhi = (float)(a.rc + band);
         rlo2 = rlo * rlo;
         rhi2 = rhi * rhi;
+        // a fractional difference of size t is rounded by at most 2.4e-7 t (three roundings a term and two
+        // sums), its image vector by that times |h_k| for each axis k: two thirds of the band over the three axes
+        // (the vector's own rounding has the rest), and less than half the margin of the image test
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            far[k] = (float)fmin(band / (1.1e-6 * (fabs(a.box.h[3 * k]) + fabs(a.box.h[3 * k + 1]) + fabs(a.box.h[3 * k + 2]))),
+                                 200.0);
     }
 };
 
 // Is the pair (i, j), j != i, within rc?  d0, d1, d2: the FP32 difference r_j - r_i.  ORTHO: the box
-// is orthorhombic and the prefilter's minimum image is three multiplies per axis.
+// is orthorhombic and the prefilter's minimum image is three multiplies per axis.  Coordinates that have
+// drifted so far apart that FP32 does not resolve the band take the exact test.
 template <bool ORTHO>
 __device__ __forceinline__ bool nb_keep(const NbArgs& a, const NbFilter& f, int i, int j, float d0, float d1, float d2) {
     bool amb = false;
@@ -374,7 +383,7 @@ __device__ __forceinline__ bool nb_keep(const NbArgs& a, const NbFilter& f, int 
         for (int q = 0; q < 3; ++q) {
             const float tt = dd[q] * f.hi[4 * q];
             const float sq = tt - floorf(tt + 0.5f);
-            amb |= fabsf(sq) > 0.4999f;
+            amb |= fabsf(sq) > 0.4999f || !(fabsf(tt) <= f.far[q]);
             const float e = sq * f.h[4 * q];
             r2 = fmaf(e, e, r2);
         }
@@ -382,9 +391,9 @@ __device__ __forceinline__ bool nb_keep(const NbArgs& a, const NbFilter& f, int 
         float sf[3];
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
-            const float tt = d0 * f.hi[q] + d1 * f.hi[3 + q] + d2 * f.hi[6 + q];
+            const float t0 = d0 * f.hi[q], t1 = d1 * f.hi[3 + q], t2 = d2 * f.hi[6 + q], tt = t0 + t1 + t2;
             sf[q] = tt - floorf(tt + 0.5f);
-            amb |= fabsf(sf[q]) > 0.4999f;
+            amb |= fabsf(sf[q]) > 0.4999f || !(fabsf(t0) + fabsf(t1) + fabsf(t2) <= f.far[q]);
         }
         const float e0 = sf[0] * f.h[0] + sf[1] * f.h[3] + sf[2] * f.h[6];
         const float e1 = sf[0] * f.h[1] + sf[1] * f.h[4] + sf[2] * f.h[7];
