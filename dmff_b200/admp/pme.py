@@ -74,12 +74,14 @@ class _AdmpEnergy(torch.autograd.Function):
         if force.lpol:
             U = (U0.detach().to(device=dev, dtype=torch.float64).contiguous().clone() if U0 is not None
                  else torch.zeros((force.n_atoms, 3), dtype=torch.float64, device=dev))
-        if from_zero:
+        # the caller's own switch stays as it is
+        switch = from_zero and not eng.zero_guess
+        if switch:
             eng.set_zero_guess(True)
         try:
             res, forces, U = eng.compute(pos, box, pairs=pairs, U=U)
         finally:
-            if from_zero:
+            if switch:
                 eng.set_zero_guess(False)
         force.last_result = res
         if aux is not None:

@@ -229,7 +229,7 @@ class AdmpEngine:
         Uh = out_array(U_out)
         if U is not None:
             Uh[...] = np.asarray(U, np.float64)
-        elif U_out is not None and not getattr(self, "_zero_guess", False):
+        elif U_out is not None and not self.zero_guess:
             Uh[...] = 0.0  # the default initial guess (ignored by the engine under set_zero_guess)
         F = out_array(forces_out)
         res = L.AdmpResult()
@@ -259,6 +259,11 @@ class AdmpEngine:
         ignored on input and receives the solution); the CG set-up then skips its A U pass."""
         self._check(self.lib.dmffb_admp_set_zero_guess(self.h, int(bool(on))))
         self._zero_guess = bool(on)
+
+    @property
+    def zero_guess(self):
+        """Whether set_zero_guess is on."""
+        return getattr(self, "_zero_guess", False)
 
     def param_grads(self, with_global=True):
         """{'Q_global', 'Q_local': [n, 9], 'pol', 'thole': [n]} of the last compute (without Q_global on
