@@ -802,29 +802,67 @@ __device__ __forceinline__ void spread_dip_atom(const MeshGeom& g, T* grid, cons
 }
 
 // Scalars of the per-pass solve: r.u, its previous value, u.w, r.r, b.b, alpha, its previous value and
-// the r.u that an update is adding up; behind them the number of steps begun and the r.r that each of
-// the last kCgHist steps began with.
+// the r.u that an update is adding up; behind them the solve's schedule: the steps begun, the next step
+// before which the residual is read, the last one and its residual, whether the solve has stopped, and at
+// which step.
 enum { CGS_RU = 0, CGS_RU_PREV = 1, CGS_UW = 2, CGS_RR = 3, CGS_BB = 4, CGS_ALPHA = 5, CGS_ALPHA_PREV = 6, CGS_RU_NEW = 7,
-       CGS_COUNT = 8 };
-constexpr int kCgHist = 32;
+       CGS_COUNT = 8, CGS_STEP = 8, CGS_NEXT = 9, CGS_LAST = 10, CGS_LAST_RMS = 11, CGS_DONE = 12, CGS_STOP = 13,
+       CGS_WORDS = 14 };
+constexpr int kCgCheckEvery = 4;  // steps between two reads of the residual, at most
+constexpr int kCgHead = 31;       // steps queued before a solve's first read, at most
 
-// the sums move on between an update and the next step's reductions (one thread, in the spread)
-__device__ __forceinline__ void cg_next(double* sc) {
-    const int step = (int)sc[CGS_COUNT];
-    sc[CGS_COUNT] = step + 1;
-    sc[CGS_COUNT + 1 + (step & (kCgHist - 1))] = sc[CGS_RR];
+// steps from a read at `step`, with residual rms, to the next: kCgCheckEvery, or fewer where the decay since the
+// last read (rms 0: none yet) says that the solve will have converged by then
+__host__ __device__ inline int cg_segment(int step, double rms, int last, double last_rms, double goal) {
+    if (!(last_rms > 0.0 && rms < last_rms && step > last)) return kCgCheckEvery;
+    const double rate = pow(rms / last_rms, 1.0 / (double)(step - last));
+    const double need = log(goal / rms) / log(rate);
+    if (!(need > 0.0 && need < (double)kCgCheckEvery)) return kCgCheckEvery;
+    const int k = (int)ceil(need);
+    return k > 1 ? k : 1;
+}
+
+// What a step of the per-pass solve goes by: the scalars, the number of components and the relative
+// tolerance.  every: the solve stops at the first step that has converged (as the persistent solve does), else at
+// the first read that finds it converged.
+struct CgSchedule {
+    double* sc;
+    double n3, tol;
+    int every;
+};
+
+// A step begins (one thread, in the spread): the residual the last one left is read where a read is due, and
+// the sums move on.  A solve that has converged stops here: its later steps change nothing (k_cg_update1), so
+// that steps queued without a read in between leave what a solve with every read leaves.
+__device__ __forceinline__ void cg_next(const CgSchedule& g) {
+    double* sc = g.sc;
+    if (sc[CGS_DONE] != 0.0) return;
+    const int step = (int)sc[CGS_STEP];
+    const double rms = sqrt(sc[CGS_RR] / g.n3), goal = g.tol * sqrt(sc[CGS_BB] / g.n3);
+    const bool read = step == (int)sc[CGS_NEXT];
+    if ((read || g.every) && rms <= goal) {
+        sc[CGS_DONE] = 1.0;
+        sc[CGS_STOP] = step;
+        return;
+    }
+    if (read) {
+        sc[CGS_NEXT] = step + cg_segment(step, rms, (int)sc[CGS_LAST], sc[CGS_LAST_RMS], goal);
+        sc[CGS_LAST] = step;
+        sc[CGS_LAST_RMS] = rms;
+    }
+    sc[CGS_STEP] = step + 1;
     sc[CGS_RU_PREV] = sc[CGS_RU];
     sc[CGS_RU] = sc[CGS_RU_NEW];
     sc[CGS_ALPHA_PREV] = sc[CGS_ALPHA];
     sc[CGS_RU_NEW] = sc[CGS_RR] = sc[CGS_UW] = 0.0;
 }
 
-// sc: the scalars of the solve whose step this spread begins, or null
+// sched: the solve whose step this spread begins (sc null: none)
 template <typename T>
-__global__ void __launch_bounds__(256) k_spread_dip_cached(SpreadArgs<T> a, StencilCache<T> st, double* sc) {
+__global__ void __launch_bounds__(256) k_spread_dip_cached(SpreadArgs<T> a, StencilCache<T> st, CgSchedule sched) {
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
-    if (sc && blockIdx.x == 0 && threadIdx.x == 0) cg_next(sc);
+    if (sched.sc && blockIdx.x == 0 && threadIdx.x == 0) cg_next(sched);
     if (warp >= a.n) return;  // whole warps: every lane takes part in the shuffles
     const int at = (int)(((int64_t)warp * a.perm_mul) % a.n);
     spread_dip_atom<T>(a.g, a.grid, st, at, lane, (T)a.U[3 * at], (T)a.U[3 * at + 1], (T)a.U[3 * at + 2]);

@@ -37,8 +37,8 @@ enum {
     S_RECIP = 16,   // [0] energy, [1..6] k-space tensor (conv kernel)
     S_GATHER = 24,  // [0] energy check, [1..9] X_NA
     S_SELF = 40,    // [0] E_self, [1] E_pol, [2..10] frame box grad
-    S_CG = 56,      // CG scalars, the step count and the last residuals
-    N_SCAL = 56 + 8 + 1 + 32 + 7
+    S_CG = 56,      // CG scalars and the solve's schedule
+    N_SCAL = 80
 };
 
 }  // namespace
@@ -939,7 +939,7 @@ int recip_pass(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx
     sa.grid = (T*)h->d_grid2;
     sa.perm_mul = h->perm_mul;
     if (dip && h->stencils_ready) {
-        LAUNCH(h, s, KC_SPREAD, k_spread_dip_cached<T><<<nblk((int64_t)h->n * 32, 256), 256, 0, s>>>(sa, stencil_cache<T>(h), nullptr));
+        LAUNCH(h, s, KC_SPREAD, k_spread_dip_cached<T><<<nblk((int64_t)h->n * 32, 256), 256, 0, s>>>(sa, stencil_cache<T>(h), CgSchedule{}));
     } else {
         const int apc = sites_per_cta(h->n);
         LAUNCH(h, s, KC_SPREAD, k_spread<T, false><<<nblk(h->n, apc), kSiteThreads, 0, s>>>(sa, apc));
@@ -984,7 +984,7 @@ int recip_pass(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx
 // vector update (k_cg_update1).  The real-space matvec runs on the side stream beside the spread and
 // the convolution; the gather adds it.
 template <typename T>
-int cg_step(dmffb_engine* h, cudaStream_t s, const Box& bx, double* U, double* sc) {
+int cg_step(dmffb_engine* h, cudaStream_t s, const Box& bx, double* U, const CgSchedule& sched) {
     const MeshGeom g = mesh_geom(bx, h->K);
     const bool fork = h->s2 && !h->prof;
     CsrArgs c;
@@ -1010,7 +1010,7 @@ int cg_step(dmffb_engine* h, cudaStream_t s, const Box& bx, double* U, double* s
     sa.g = g;
     sa.grid = (T*)h->d_grid2;
     sa.perm_mul = h->perm_mul;
-    LAUNCH(h, s, KC_SPREAD, k_spread_dip_cached<T><<<nblk((int64_t)h->n * 32, 256), 256, 0, s>>>(sa, stencil_cache<T>(h), sc));
+    LAUNCH(h, s, KC_SPREAD, k_spread_dip_cached<T><<<nblk((int64_t)h->n * 32, 256), 256, 0, s>>>(sa, stencil_cache<T>(h), sched));
     ConvArgs<T> ca = conv_args<T>(h, bx, CK_COUL, DMFFB_DIELECTRIC, h->d_scal + S_RECIP, false);
     ca.zero_real = (T*)h->d_grid2;  // cleared for the next spread once it has been transformed
     ca.nzero = (int64_t)h->K[0] * h->K[1] * h->K[2];
@@ -1021,13 +1021,13 @@ int cg_step(dmffb_engine* h, cudaStream_t s, const Box& bx, double* U, double* s
     cmb.U = h->d_z;
     cmb.pol = h->d_pol;
     cmb.self1 = -2.0 * DMFFB_DIELECTRIC * (k / 1.7724538509055159) * 2.0 * k * k / 3.0;
-    cmb.dot_out = sc + CGS_UW;
+    cmb.dot_out = sched.sc + CGS_UW;
     cmb.mv = h->d_fmv;
     if (fork) CK(cudaStreamWaitEvent(s, h->e_join, 0));
     LAUNCH(h, s, KC_GATHER_FIELD, k_gather_field_cached<T><<<atom_ctas(h->n, 4), 256, 0, s>>>(
                                       h->n, stencil_cache<T>(h), g, (const T*)h->d_grid, 2.0 * DMFFB_DIELECTRIC, h->d_Ap,
                                       cmb));
-    LAUNCH(h, s, KC_VEC, k_cg_update1<T><<<nblk(3 * h->n, 256), 256, 0, s>>>(h->n, cg_vectors(h, U, false), (Vec4<T>*)h->d_p4, sc));
+    LAUNCH(h, s, KC_VEC, k_cg_update1<T><<<nblk(3 * h->n, 256), 256, 0, s>>>(h->n, cg_vectors(h, U, false), (Vec4<T>*)h->d_p4, sched.sc));
     CK(cudaGetLastError());
     return DMFFB_OK;
 }
@@ -1292,7 +1292,7 @@ int solve_dipoles(dmffb_engine* h, cudaStream_t s, const double* pos, const Box&
         if ((st = stencil_prep<T>(h, s, pos, bx))) return st;
     }
     if (rhs) {
-        CK(cudaMemsetAsync(sc, 0, (CGS_COUNT + 1) * sizeof(double), s));
+        CK(cudaMemsetAsync(sc, 0, CGS_WORDS * sizeof(double), s));
         CK(cudaMemsetAsync(U, 0, (size_t)3 * n * sizeof(double), s));
         if ((st = matvec_coef_launch<T>(h, s, bx, pairs, npairs))) return st;
         CK(cudaMemcpyAsync(h->d_b, rhs, (size_t)3 * n * sizeof(double), cudaMemcpyDeviceToDevice, s));
@@ -1315,12 +1315,15 @@ int solve_dipoles(dmffb_engine* h, cudaStream_t s, const double* pos, const Box&
     // step is the same launches whatever its number (its scalars move on on the device), so a
     // one-step graph is captured beside it for segments of odd length.
     bool graphs = h->use_graphs && !h->prof;
+    // a system whose solve the persistent kernel may take (below) stops where that one would
+    const bool small = sizeof(T) == 4 && fused && pcg_wanted(h) && pcg_decide(h) > 0;
+    const CgSchedule sched = {sc, 3.0 * n, h->cg_tol, small ? 1 : 0};
     if (graphs) {
         std::vector<double> key = {(double)(uintptr_t)pos, (double)(uintptr_t)pairs, (double)npairs,
                                    (double)(uintptr_t)U, (double)(uintptr_t)h->d_csr_ent, (double)sizeof(T),
                                    (double)(uintptr_t)h->d_mvcoef, (double)(uintptr_t)h->d_csr_off,
                                    (double)dft_use<T>(h), (double)(uintptr_t)h->d_dftG, (double)(uintptr_t)h->d_dftW,
-                                   (double)fused};
+                                   (double)fused, (double)sched.every};
         for (int k = 0; k < 9; ++k) key.push_back(bx.h[k]);
         const bool repeat = key == h->cg_seen_key;
         h->cg_seen_key = key;
@@ -1329,7 +1332,7 @@ int solve_dipoles(dmffb_engine* h, cudaStream_t s, const double* pos, const Box&
     // The persistent solve: always, or (the default) for small systems whose solve no graph can replay,
     // where the per-pass solve is its launches (450 / 3999 atoms: 577 / 813 us a step, replayed
     // 554 / 726).
-    if (sizeof(T) == 4 && fused && (h->pcg_mode == 1 || !graphs) && pcg_wanted(h) && pcg_decide(h) > 0) {
+    if (small && (h->pcg_mode == 1 || !graphs)) {
         h->grid2_dirty = true;  // its last iteration leaves a spread there
         return cg_persistent(h, s, bx, U, sc, res);
     }
@@ -1339,7 +1342,7 @@ int solve_dipoles(dmffb_engine* h, cudaStream_t s, const double* pos, const Box&
     // one CG iteration; slot = parity of the r.z scalar that the classic form reads
     auto iteration = [&](int slot) -> int {
         int st2;
-        if (fused) return cg_step<T>(h, s, bx, U, sc);
+        if (fused) return cg_step<T>(h, s, bx, U, sched);
         // Ap = A p with p.Ap reduced into sc[2]; pAp, rr and the r.z slot this step writes are
         // cleared first (the previous step has read them by then)
         double* const zs[3] = {sc + 2, sc + 3, sc + (1 - slot)};
@@ -1380,12 +1383,10 @@ int solve_dipoles(dmffb_engine* h, cudaStream_t s, const double* pos, const Box&
         }
     }
     // The host reads the residual every few steps (no per-step sync; a read costs some 25 us with the
-    // launches it holds up).  On the fused path, from the second read on, the residual's decay over the
-    // last segment predicts the steps still needed: a segment shorter than check_every then ends at the
-    // first step expected to converge.  A solve from U = 0 first runs the steps up to the last read but
-    // one of the engine's last such solve without a read (neighbouring configurations take the same
-    // number or one more); the reads left out are made up from the device's history of residuals.
-    const int check_every = 4;
+    // launches it holds up): cg_segment.  A solve from U = 0 first runs the steps up to the last read but one of
+    // the engine's last such solve without a read (neighbouring configurations take the same number or one
+    // more); the device makes those reads itself (cg_next), so that the solve stops where it would have, however
+    // many steps were queued, and leaves the same dipoles.
     auto run_steps = [&](int k) -> int {
         int st2;
         for (; k >= 2; k -= 2) {
@@ -1409,57 +1410,48 @@ int solve_dipoles(dmffb_engine* h, cudaStream_t s, const double* pos, const Box&
         }
         return DMFFB_OK;
     };
-    // residual (and the last kCgHist before it) and b.b on the host
+    // residual, b.b and on the fused path the schedule on the host
+    bool done = false;
     auto read_residual = [&]() -> int {
-        CK(cudaMemcpyAsync(h->h_scal, sc, (fused ? CGS_COUNT + 1 + kCgHist : CGS_COUNT) * sizeof(double),
-                           cudaMemcpyDeviceToHost, s));
+        CK(cudaMemcpyAsync(h->h_scal, sc, (fused ? CGS_WORDS : CGS_COUNT) * sizeof(double), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
         rms = sqrt(h->h_scal[CGS_RR] / (3.0 * n));
         rms_b = sqrt(h->h_scal[CGS_BB] / (3.0 * n));
+        done = fused && h->h_scal[CGS_DONE] != 0.0;
         return DMFFB_OK;
     };
+    int last = 0;  // the read before this one and its residual
+    double last_rms = 0.0;
     if (fused && u0 && !rhs && h->cg_hint > 0) {
-        it = std::min(h->cg_hint, std::min(kCgHist - 1, h->max_iter));
-        if ((st = run_steps(it))) return st;
+        it = std::min(std::min(h->cg_hint, kCgHead), h->max_iter);
+        if ((st = run_steps(it)) || (st = read_residual())) return st;
+        last = (int)h->h_scal[CGS_LAST];
+        last_rms = h->h_scal[CGS_LAST_RMS];
+        const int next = (int)h->h_scal[CGS_NEXT];
+        if (!done && next > it) {
+            if ((st = run_steps(next - it)) || (st = read_residual())) return st;
+            it = next;
+        }
+    } else if ((st = read_residual())) {
+        return st;
     }
-    if ((st = read_residual())) return st;
-    // e walks the reads' schedule; while it lies behind the steps already run it goes by the history,
-    // so that a solve takes the same steps with and without the head start
-    int e = 0, e_prev = 0;
-    double r_prev = -1.0;
     while (true) {
         if (!std::isfinite(rms)) return fail(h, DMFFB_NONFINITE, "non-finite residual in the dipole solve");
         // relative criterion: RMS(dE/dU) below cg_tol times the RMS permanent field
-        if (rms <= h->cg_tol * rms_b) {
+        if (done || rms <= h->cg_tol * rms_b) {
             conv = true;
+            if (done) it = (int)h->h_scal[CGS_STOP];
             break;
         }
         if (it >= h->max_iter) break;
-        const double r = e < it ? sqrt(h->h_scal[CGS_COUNT + 1 + (e & (kCgHist - 1))] / (3.0 * n)) : rms;
-        int k = check_every;
-        if (fused && r_prev > 0.0 && r < r_prev && e > e_prev) {
-            const double rate = std::pow(r / r_prev, 1.0 / (double)(e - e_prev));
-            const double need = std::log(h->cg_tol * rms_b / r) / std::log(rate);
-            if (need > 0.0 && need < (double)check_every) k = std::max(1, (int)std::ceil(need));
-        }
-        r_prev = r;
-        e_prev = e;
-        e += k;
-        if (e > it) {
-            if ((st = run_steps(e - it))) return st;
-            it = e;
-            if ((st = read_residual())) return st;
-        }
+        const int k = fused ? cg_segment(it, rms, last, last_rms, h->cg_tol * rms_b) : kCgCheckEvery;
+        last = it;
+        last_rms = rms;
+        if ((st = run_steps(k))) return st;
+        it += k;
+        if ((st = read_residual())) return st;
     }
-    if (rms_b == 0.0) it = 0;  // nothing to solve
-    if (fused && u0 && !rhs) {
-        h->cg_hint = conv ? e_prev : 0;
-        if (conv && e < it && it < kCgHist) {  // the head start was too long: one short of where it converged
-            int k = 0;
-            while (k < it && sqrt(h->h_scal[CGS_COUNT + 1 + k] / (3.0 * n)) > h->cg_tol * rms_b) ++k;
-            h->cg_hint = std::max(k - 1, 0);
-        }
-    }
+    if (fused && u0 && !rhs) h->cg_hint = conv ? last : 0;
     res->n_iter = it;
     res->converged = conv ? 1 : 0;
     res->residual_rms = rms;
