@@ -331,6 +331,24 @@ MeshGeom mesh_geom(const Box& b, const int K[3]) {
 
 inline unsigned nblk(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
+// Evaluations (on the engine's stream) and neighbour builds (on the caller's) share arrays whatever list an
+// evaluation uses: the scaled-row map, the cells and their counters.  An evaluation on s therefore comes after
+// the last build, and a build on s after the last evaluation and the last build, on whichever streams those ran.
+int after_build(dmffb_engine* h, cudaStream_t s) {
+    if (h->e_build) CK(cudaStreamWaitEvent(s, h->e_build, 0));
+    return DMFFB_OK;
+}
+int after_all(dmffb_engine* h, cudaStream_t s) {
+    CK(cudaStreamWaitEvent(s, h->e_out, 0));
+    return after_build(h, s);
+}
+// the engine's stream takes up an evaluation that the caller queued on `caller`
+int enter(dmffb_engine* h, cudaStream_t caller) {
+    CK(cudaEventRecord(h->e_in, caller));
+    CK(cudaStreamWaitEvent(h->s1, h->e_in, 0));
+    return after_build(h, h->s1);
+}
+
 // kernel classes for dmffb_get_kernel_stats
 enum { KC_PREP = 0, KC_PAIR_FULL, KC_PAIR_FIELD, KC_PAIR_MATVEC, KC_SPREAD, KC_FFT, KC_CONV, KC_GATHER_FULL,
        KC_GATHER_FIELD, KC_SELF, KC_VEC, KC_NBLIST, KC_MVCOEF,
@@ -1477,7 +1495,6 @@ int compute_impl(dmffb_engine* h, cudaStream_t s, const double* pos, const doubl
     const bool own_list = !pairs;
     if (own_list && !h->have_pairs)
         if ((st = dmffb_admp_build_neighbors(h, (void*)s, pos, box))) return st;
-    if (own_list && h->e_build) CK(cudaStreamWaitEvent(s, h->e_build, 0));
     if (h->timing) CK(cudaEventRecord(h->ev[0], s));
     PrepArgs<T> pa = prep_args<T>(h, pos, bx);
     pa.clear.add(h->d_scal, N_SCAL * sizeof(double));
@@ -2666,6 +2683,7 @@ int dmffb_admp_reconfigure(dmffb_engine* h, const dmffb_admp_desc* d) {
     if (d->lpme && (d->K[0] <= 0 || d->K[1] <= 0 || d->K[2] <= 0 || !(d->kappa > 0)))
         return fail(h, DMFFB_BAD_ARG, "bad PME mesh or kappa");
     CK(cudaStreamSynchronize(h->s1));
+    if (h->e_build) CK(cudaEventSynchronize(h->e_build));  // a build may still read the topology
     set_scalars(h, d);
     int st;
     if ((st = upload_topology(h, d))) return st;
@@ -2795,9 +2813,9 @@ int dmffb_admp_compute(dmffb_engine* h, void* stream, const double* pos, const d
     // the evaluation runs on the engine's own stream (capturable into CUDA graphs), ordered
     // after the caller's prior work on `stream` and before the caller's later work
     cudaStream_t caller = (cudaStream_t)stream;
-    CK(cudaEventRecord(h->e_in, caller));
-    CK(cudaStreamWaitEvent(h->s1, h->e_in, 0));
-    int st = h->prec == DMFFB_FP32
+    int st = enter(h, caller);
+    if (st) return st;
+    st = h->prec == DMFFB_FP32
                  ? compute_impl<float>(h, h->s1, pos, box, pairs, npairs, U_inout, forces_out, result)
                  : compute_impl<double>(h, h->s1, pos, box, pairs, npairs, U_inout, forces_out, result);
     cudaEventRecord(h->e_out, h->s1);
@@ -2811,6 +2829,8 @@ int dmffb_admp_compute_host(dmffb_engine* h, const double* pos, const double* bo
     if (pairs && npairs < 0) return fail(h, DMFFB_BAD_ARG, "negative npairs");
     const int n = h->n;
     cudaStream_t s = h->s1;  // engine stream: host-buffer calls of different engines overlap on the GPU
+    const int sw = after_build(h, s);
+    if (sw) return sw;
     CK(cudaMemcpyAsync(h->d_pos, pos, 3 * n * sizeof(double), cudaMemcpyHostToDevice, s));
     int32_t* dp = nullptr;
     if (pairs) {  // staged in the engine's pair buffer (grown when short)
@@ -3077,8 +3097,7 @@ int dmffb_admp_backward(dmffb_engine* h, void* stream, const dmffb_admp_cotangen
         h->admp_pgrad = was;
     }
     cudaStream_t caller = (cudaStream_t)stream;
-    CK(cudaEventRecord(h->e_in, caller));
-    CK(cudaStreamWaitEvent(h->s1, h->e_in, 0));
+    if ((st = enter(h, caller))) return st;
     st = h->prec == DMFFB_FP32 ? admp_backward_impl<float>(h, h->s1, c, out) : admp_backward_impl<double>(h, h->s1, c, out);
     cudaEventRecord(h->e_out, h->s1);
     cudaStreamWaitEvent(caller, h->e_out, 0);
@@ -3090,6 +3109,8 @@ int dmffb_admp_field(dmffb_engine* h, void* stream, const double* pos, const dou
     if (!h || !pos || !box || !field_out) return fail(h, DMFFB_BAD_ARG, "null argument");
     if (!h->lpol) return fail(h, DMFFB_BAD_ARG, "field requires a polarizable system");
     cudaStream_t s = (cudaStream_t)stream;
+    int sw = after_all(h, s);
+    if (sw) return sw;
     Box bx;
     make_box(box, bx);
     h->cur_pos = pos;
@@ -3196,6 +3217,7 @@ int dmffb_build_neighbors(dmffb_engine* h, void* stream, const double* pos, cons
     make_box(box, bx);
     int st;
     if (h->nb_pending && (st = nb_finish(h))) return st;  // the builds of one engine share their scratch
+    if ((st = after_all(h, s))) return st;
     const NbPlan p = nb_plan(h, bx, rc);
     if ((st = nb_alloc(h, false))) return st;
     Nb2Args b = nb_args(h, p, pos, bx, rc, false);
@@ -3235,7 +3257,7 @@ int dmffb_admp_build_neighbors(dmffb_engine* h, void* stream, const double* pos,
     const NbPlan p = nb_plan(h, bx, h->rc);
     const bool want_csr = h->kind == 0 && h->lpol;
     int st;
-    if ((st = nb_alloc(h, want_csr)) || (st = nb_srows_cap(h))) return st;
+    if ((st = after_all(h, s)) || (st = nb_alloc(h, want_csr)) || (st = nb_srows_cap(h))) return st;
     if (p.flat || p.staged) {
         // a first build sizes slots and lists from the mean density and waits for its totals (the
         // caller may change the positions when it returns); later ones leave that to nb_finish
@@ -3402,9 +3424,9 @@ int dmffb_disp_compute(dmffb_engine* h, void* stream, const double* pos, const d
                        int64_t npairs, double* forces_lr, double* forces_sr, dmffb_disp_result* result) {
     if (!h || h->kind != 1 || !pos || !box || !result) return fail(h, DMFFB_BAD_ARG, "bad arguments");
     cudaStream_t caller = (cudaStream_t)stream;
-    CK(cudaEventRecord(h->e_in, caller));
-    CK(cudaStreamWaitEvent(h->s1, h->e_in, 0));
-    int st = h->prec == DMFFB_FP32 ? disp_compute_impl<float>(h, h->s1, pos, box, pairs, npairs, forces_lr, forces_sr, result)
+    int st = enter(h, caller);
+    if (st) return st;
+    st = h->prec == DMFFB_FP32 ? disp_compute_impl<float>(h, h->s1, pos, box, pairs, npairs, forces_lr, forces_sr, result)
                                    : disp_compute_impl<double>(h, h->s1, pos, box, pairs, npairs, forces_lr, forces_sr, result);
     cudaEventRecord(h->e_out, h->s1);
     cudaStreamWaitEvent(caller, h->e_out, 0);
@@ -3551,9 +3573,9 @@ int dmffb_pairwise_compute(dmffb_engine* h, void* stream, const double* pos, con
     if (!h || h->kind != 3) return fail(h, DMFFB_BAD_ARG, "pairwise engine required");
     if (pairs && npairs < 0) return fail(h, DMFFB_BAD_ARG, "negative npairs");
     cudaStream_t caller = (cudaStream_t)stream;
-    CK(cudaEventRecord(h->e_in, caller));
-    CK(cudaStreamWaitEvent(h->s1, h->e_in, 0));
-    int st = h->prec == DMFFB_FP32 ? pairwise_compute_impl<float>(h, h->s1, pos, box, pairs, npairs, forces_out, result)
+    int st = enter(h, caller);
+    if (st) return st;
+    st = h->prec == DMFFB_FP32 ? pairwise_compute_impl<float>(h, h->s1, pos, box, pairs, npairs, forces_out, result)
                                    : pairwise_compute_impl<double>(h, h->s1, pos, box, pairs, npairs, forces_out, result);
     cudaEventRecord(h->e_out, h->s1);
     cudaStreamWaitEvent(caller, h->e_out, 0);
@@ -3718,9 +3740,9 @@ int dmffb_classical_compute(dmffb_engine* h, void* stream, const double* pos, co
                             int64_t npairs, double* forces_out, dmffb_classical_result* result) {
     if (!h || h->kind != 2 || !pos || !box || !result) return fail(h, DMFFB_BAD_ARG, "bad arguments");
     cudaStream_t caller = (cudaStream_t)stream;
-    CK(cudaEventRecord(h->e_in, caller));
-    CK(cudaStreamWaitEvent(h->s1, h->e_in, 0));
-    int st = h->prec == DMFFB_FP32 ? classical_compute_impl<float>(h, h->s1, pos, box, pairs, npairs, forces_out, result)
+    int st = enter(h, caller);
+    if (st) return st;
+    st = h->prec == DMFFB_FP32 ? classical_compute_impl<float>(h, h->s1, pos, box, pairs, npairs, forces_out, result)
                                    : classical_compute_impl<double>(h, h->s1, pos, box, pairs, npairs, forces_out, result);
     cudaEventRecord(h->e_out, h->s1);
     cudaStreamWaitEvent(caller, h->e_out, 0);
