@@ -140,7 +140,6 @@ __device__ __forceinline__ double cg_update(const CgVectors& v, Vec4<T>* p4, dou
 // launches: three lanes of a warp wait for the vectors where here all threads do.
 template <typename T>
 __global__ void __launch_bounds__(256) k_cg_update1(int n, CgVectors v, Vec4<T>* p4, double* sc) {
-    if (sc[CGS_DONE] != 0.0) return;  // the solve had converged before this step
     double alpha, beta;
     cg_coefs(sc[CGS_RU], sc[CGS_RU_PREV], sc[CGS_UW], sc[CGS_ALPHA_PREV], alpha, beta);
     double sum[2] = {0.0, 0.0}, rr[1];

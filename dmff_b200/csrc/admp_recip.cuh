@@ -832,37 +832,42 @@ struct CgSchedule {
 };
 
 // A step begins (one thread, in the spread): the residual the last one left is read where a read is due, and
-// the sums move on.  A solve that has converged stops here: its later steps change nothing (k_cg_update1), so
-// that steps queued without a read in between leave what a solve with every read leaves.
-__device__ __forceinline__ void cg_next(const CgSchedule& g) {
+// the sums move on.  A solve that has converged stops here: r.u of 0 makes alpha and beta of its later steps 0
+// (cg_coefs), which leave x, r and u as they are, so that steps queued without a read in between leave what a
+// solve with every read leaves.
+__device__ __noinline__ void cg_next(const CgSchedule& g) {
     double* sc = g.sc;
-    if (sc[CGS_DONE] != 0.0) return;
     const int step = (int)sc[CGS_STEP];
     const double rms = sqrt(sc[CGS_RR] / g.n3), goal = g.tol * sqrt(sc[CGS_BB] / g.n3);
     const bool read = step == (int)sc[CGS_NEXT];
-    if ((read || g.every) && rms <= goal) {
+    if (sc[CGS_DONE] != 0.0 || ((read || g.every) && rms <= goal)) {
+        if (sc[CGS_DONE] == 0.0) sc[CGS_STOP] = step;
         sc[CGS_DONE] = 1.0;
-        sc[CGS_STOP] = step;
-        return;
+        sc[CGS_RU] = 0.0;
+    } else {
+        if (read) {
+            sc[CGS_NEXT] = step + cg_segment(step, rms, (int)sc[CGS_LAST], sc[CGS_LAST_RMS], goal);
+            sc[CGS_LAST] = step;
+            sc[CGS_LAST_RMS] = rms;
+        }
+        sc[CGS_STEP] = step + 1;
+        sc[CGS_RU_PREV] = sc[CGS_RU];
+        sc[CGS_RU] = sc[CGS_RU_NEW];
+        sc[CGS_ALPHA_PREV] = sc[CGS_ALPHA];
     }
-    if (read) {
-        sc[CGS_NEXT] = step + cg_segment(step, rms, (int)sc[CGS_LAST], sc[CGS_LAST_RMS], goal);
-        sc[CGS_LAST] = step;
-        sc[CGS_LAST_RMS] = rms;
-    }
-    sc[CGS_STEP] = step + 1;
-    sc[CGS_RU_PREV] = sc[CGS_RU];
-    sc[CGS_RU] = sc[CGS_RU_NEW];
-    sc[CGS_ALPHA_PREV] = sc[CGS_ALPHA];
     sc[CGS_RU_NEW] = sc[CGS_RR] = sc[CGS_UW] = 0.0;
 }
 
-// sched: the solve whose step this spread begins (sc null: none)
+// sched: the solve whose step this spread begins (sc null: none); a CTA of its own in front does that
 template <typename T>
 __global__ void __launch_bounds__(256) k_spread_dip_cached(SpreadArgs<T> a, StencilCache<T> st, CgSchedule sched) {
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    int cta = blockIdx.x;
+    if (sched.sc && cta-- == 0) {
+        if (threadIdx.x == 0) cg_next(sched);
+        return;
+    }
+    const int warp = (cta * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
-    if (sched.sc && blockIdx.x == 0 && threadIdx.x == 0) cg_next(sched);
     if (warp >= a.n) return;  // whole warps: every lane takes part in the shuffles
     const int at = (int)(((int64_t)warp * a.perm_mul) % a.n);
     spread_dip_atom<T>(a.g, a.grid, st, at, lane, (T)a.U[3 * at], (T)a.U[3 * at + 1], (T)a.U[3 * at + 2]);

@@ -1028,7 +1028,7 @@ int cg_step(dmffb_engine* h, cudaStream_t s, const Box& bx, double* U, const CgS
     sa.g = g;
     sa.grid = (T*)h->d_grid2;
     sa.perm_mul = h->perm_mul;
-    LAUNCH(h, s, KC_SPREAD, k_spread_dip_cached<T><<<nblk((int64_t)h->n * 32, 256), 256, 0, s>>>(sa, stencil_cache<T>(h), sched));
+    LAUNCH(h, s, KC_SPREAD, k_spread_dip_cached<T><<<nblk((int64_t)h->n * 32, 256) + 1, 256, 0, s>>>(sa, stencil_cache<T>(h), sched));
     ConvArgs<T> ca = conv_args<T>(h, bx, CK_COUL, DMFFB_DIELECTRIC, h->d_scal + S_RECIP, false);
     ca.zero_real = (T*)h->d_grid2;  // cleared for the next spread once it has been transformed
     ca.nzero = (int64_t)h->K[0] * h->K[1] * h->K[2];
