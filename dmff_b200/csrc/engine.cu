@@ -105,7 +105,7 @@ struct dmffb_engine {
     void* d_grid = nullptr;
     void* d_grid2 = nullptr;  // spread target of the dipole-only field pass, kept zero between passes
     int cg_hint = 0;           // steps that the next dipole solve from U = 0 takes before its first read
-    bool grid2_dirty = false;  // the persistent solve has left its last spread there
+    bool grid2_dirty = false;  // it holds a spread (clean_mesh)
     void* d_cgrid = nullptr;
     double* d_bmod = nullptr;
     cufftHandle plan_f = 0, plan_b = 0;
@@ -799,7 +799,7 @@ int fft_plans(dmffb_engine* h) {
 // in -> forward transform -> influence function (ca: kind, scales, energy sums, a mesh to clear) ->
 // inverse transform -> out, by the DFT kernels or by cuFFT and k_conv
 template <typename T>
-int mesh_convolve(dmffb_engine* h, cudaStream_t s, void* in, void* out, ConvArgs<T>& ca) {
+int mesh_convolve(dmffb_engine* h, cudaStream_t s, void* in, void* out, const ConvArgs<T>& ca) {
     h->dft_used = dft_use<T>(h);
     if (h->dft_used) {
         const int st = dft_setup<T>(h);
@@ -927,11 +927,26 @@ StencilCache<T> stencil_cache(dmffb_engine* h) {
 }
 
 // Every spread goes to d_grid2, which the convolution clears again once the forward transform has read
-// it: it is zero between passes, unless a persistent solve has left its last spread there.
+// it: it is zero between passes.  A spread left there (by the persistent solve, or where an error came between
+// it and the convolution) is cleared before the next one.
 template <typename T>
-int spread_mesh(dmffb_engine* h, cudaStream_t s) {
+int clean_mesh(dmffb_engine* h, cudaStream_t s) {
     if (!h->grid2_dirty) return DMFFB_OK;
     CK(cudaMemsetAsync(h->d_grid2, 0, (size_t)h->grid_cap * sizeof(T), s));
+    h->grid2_dirty = false;
+    return DMFFB_OK;
+}
+
+// spread() onto d_grid2, its convolution by ca into d_grid
+template <typename T, typename Spread>
+int mesh_pass(dmffb_engine* h, cudaStream_t s, ConvArgs<T> ca, Spread&& spread) {
+    int st;
+    if ((st = clean_mesh<T>(h, s))) return st;
+    h->grid2_dirty = true;
+    spread();
+    ca.zero_real = (T*)h->d_grid2;
+    ca.nzero = (int64_t)h->K[0] * h->K[1] * h->K[2];
+    if ((st = mesh_convolve<T>(h, s, h->d_grid2, h->d_grid, ca))) return st;
     h->grid2_dirty = false;
     return DMFFB_OK;
 }
@@ -942,10 +957,8 @@ template <typename T>
 int recip_pass(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx, bool use_Qg, const double* U,
                int mode, double* field_out) {
     const MeshGeom g = mesh_geom(bx, h->K);
-    const int64_t K3 = (int64_t)h->K[0] * h->K[1] * h->K[2];
     const bool dip = mode == GATHER_FIELD && !use_Qg && U;
     int st;
-    if ((st = spread_mesh<T>(h, s))) return st;
     SpreadArgs<T> sa;
     sa.n = h->n;
     sa.pos = pos;
@@ -956,16 +969,15 @@ int recip_pass(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx
     sa.g = g;
     sa.grid = (T*)h->d_grid2;
     sa.perm_mul = h->perm_mul;
-    if (dip && h->stencils_ready) {
-        LAUNCH(h, s, KC_SPREAD, k_spread_dip_cached<T><<<nblk((int64_t)h->n * 32, 256), 256, 0, s>>>(sa, stencil_cache<T>(h), CgSchedule{}));
-    } else {
+    const auto spread = [&] {
         const int apc = sites_per_cta(h->n);
-        LAUNCH(h, s, KC_SPREAD, k_spread<T, false><<<nblk(h->n, apc), kSiteThreads, 0, s>>>(sa, apc));
-    }
-    ConvArgs<T> ca = conv_args<T>(h, bx, CK_COUL, DMFFB_DIELECTRIC, h->d_scal + S_RECIP, mode == GATHER_FULL);
-    ca.zero_real = (T*)h->d_grid2;
-    ca.nzero = K3;
-    if ((st = mesh_convolve<T>(h, s, h->d_grid2, h->d_grid, ca))) return st;
+        if (dip && h->stencils_ready)
+            LAUNCH(h, s, KC_SPREAD, k_spread_dip_cached<T><<<nblk((int64_t)h->n * 32, 256), 256, 0, s>>>(sa, stencil_cache<T>(h), CgSchedule{}));
+        else
+            LAUNCH(h, s, KC_SPREAD, k_spread<T, false><<<nblk(h->n, apc), kSiteThreads, 0, s>>>(sa, apc));
+    };
+    if ((st = mesh_pass<T>(h, s, conv_args<T>(h, bx, CK_COUL, DMFFB_DIELECTRIC, h->d_scal + S_RECIP, mode == GATHER_FULL), spread)))
+        return st;
     if (mode == GATHER_FIELD) {
         if (h->stencils_ready)
             LAUNCH(h, s, KC_GATHER_FIELD, k_gather_field_cached<T><<<atom_ctas(h->n, 4), 256, 0, s>>>(
@@ -1028,11 +1040,10 @@ int cg_step(dmffb_engine* h, cudaStream_t s, const Box& bx, double* U, const CgS
     sa.g = g;
     sa.grid = (T*)h->d_grid2;
     sa.perm_mul = h->perm_mul;
-    LAUNCH(h, s, KC_SPREAD, k_spread_dip_cached<T><<<nblk((int64_t)h->n * 32, 256) + 1, 256, 0, s>>>(sa, stencil_cache<T>(h), sched));
-    ConvArgs<T> ca = conv_args<T>(h, bx, CK_COUL, DMFFB_DIELECTRIC, h->d_scal + S_RECIP, false);
-    ca.zero_real = (T*)h->d_grid2;  // cleared for the next spread once it has been transformed
-    ca.nzero = (int64_t)h->K[0] * h->K[1] * h->K[2];
-    const int st = mesh_convolve<T>(h, s, h->d_grid2, h->d_grid, ca);
+    const auto spread = [&] {
+        LAUNCH(h, s, KC_SPREAD, k_spread_dip_cached<T><<<nblk((int64_t)h->n * 32, 256) + 1, 256, 0, s>>>(sa, stencil_cache<T>(h), sched));
+    };
+    const int st = mesh_pass<T>(h, s, conv_args<T>(h, bx, CK_COUL, DMFFB_DIELECTRIC, h->d_scal + S_RECIP, false), spread);
     if (st) return st;
     FieldCombine cmb;
     const double k = h->kappa;
@@ -1324,6 +1335,7 @@ int solve_dipoles(dmffb_engine* h, cudaStream_t s, const double* pos, const Box&
     LAUNCH(h, s, KC_VEC, k_cg_init<T><<<nb3, 256, 0, s>>>(n, h->d_b, u0 ? nullptr : h->d_Ap, h->d_pol, h->d_r, h->d_z,
                                                         h->d_p, (Vec4<T>*)h->d_p4, sc));
     const bool fused = h->lpme && h->have_plans && h->stencils_ready;
+    if (fused && (st = clean_mesh<T>(h, s))) return st;  // before a step is captured
     // the classic form keeps r.z in sc[0] / sc[1]
     if (!fused) CK(cudaMemcpyAsync(sc, sc + CGS_RU_NEW, sizeof(double), cudaMemcpyDeviceToDevice, s));
     // two iterations (slot 0 then 1) are captured once into a CUDA graph and replayed; the graph
@@ -1708,9 +1720,7 @@ template <typename T>
 int recip_pass_channel(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx, const T* q, int kind,
                        double escale, double* grad, double* dq, double* scal_conv, double* scal_gather) {
     const MeshGeom g = mesh_geom(bx, h->K);
-    const int64_t K3 = (int64_t)h->K[0] * h->K[1] * h->K[2];
     int st;
-    if ((st = spread_mesh<T>(h, s))) return st;
     SpreadArgs<T> sa;
     sa.n = h->n;
     sa.pos = pos;
@@ -1722,11 +1732,8 @@ int recip_pass_channel(dmffb_engine* h, cudaStream_t s, const double* pos, const
     sa.grid = (T*)h->d_grid2;
     sa.perm_mul = h->perm_mul;
     const int apc = sites_per_cta(h->n);
-    LAUNCH(h, s, KC_SPREAD, k_spread<T, true><<<nblk(h->n, apc), kSiteThreads, 0, s>>>(sa, apc));
-    ConvArgs<T> ca = conv_args<T>(h, bx, kind, escale, scal_conv, true);
-    ca.zero_real = (T*)h->d_grid2;
-    ca.nzero = K3;
-    if ((st = mesh_convolve<T>(h, s, h->d_grid2, h->d_grid, ca))) return st;
+    const auto spread = [&] { LAUNCH(h, s, KC_SPREAD, k_spread<T, true><<<nblk(h->n, apc), kSiteThreads, 0, s>>>(sa, apc)); };
+    if ((st = mesh_pass<T>(h, s, conv_args<T>(h, bx, kind, escale, scal_conv, true), spread))) return st;
     GatherArgs<T> ga;
     ga.n = h->n;
     ga.pos = pos;
