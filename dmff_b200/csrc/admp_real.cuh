@@ -19,7 +19,7 @@
 
 namespace dmffb {
 
-enum { PAIR_FULL = 0, PAIR_FIELD = 1, PAIR_MATVEC = 2 };
+enum { PAIR_FULL = 0, PAIR_FIELD = 1 };
 
 template <typename T>
 struct PairArgs {
@@ -171,29 +171,6 @@ __device__ __forceinline__ void pair_eval(const TC dr[3], const TC* QIg, const T
     const Dl<TC> R2 = R1 * R1;
     const Dl<TC> R3 = R2 * R1;
 
-    if (MODE == PAIR_MATVEC) {
-        // induced-induced only: T_ij = udud1 I + (udud0 - udud1) z z^T  (pme.py:872-878)
-        TC u = r / dmp;
-        u = u < TC(1e8) ? u : TC(1e8);
-        const TC au = Ath * u;
-        const TC ev = au < TC(50) ? d_exp(-au) : TC(0);
-        const TC Pc = TC(1) + au + TC(0.5) * au * au;
-        const TC Pd0 = Pc + au * au * au * TC(0.25);
-        const TC base = ERFC.v + t2.v + t3.v;
-        const TC bd0 = (dsv - TC(1)) - dsv * ev * Pd0 + base;
-        const TC bd1 = (dsv - TC(1)) - dsv * ev * Pc + base;
-        const TC udud0 = TC(-2.0 / 3.0) * D * R3.v * (TC(3) * bd0 + a3X.v);
-        const TC udud1 = D * R3.v * (bd1 - TC(2.0 / 3.0) * a3X.v);
-        const TC zUI = ez[0] * UI[0] + ez[1] * UI[1] + ez[2] * UI[2];
-        const TC zUJ = ez[0] * UJ[0] + ez[1] * UJ[1] + ez[2] * UJ[2];
-        const TC dd = udud0 - udud1;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            oi[c] = udud1 * UJ[c] + dd * zUJ * ez[c];
-            oj[c] = udud1 * UI[c] + dd * zUI * ez[c];
-        }
-        return;
-    }
     TC ex[3], ey[3];
     qi_frame(ez, ex, ey);
     TC C[5][5];

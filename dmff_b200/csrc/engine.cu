@@ -95,7 +95,6 @@ struct dmffb_engine {
     int32_t *d_csr_ent = nullptr, *d_csr_deg = nullptr;
     int64_t csr_cap = 0;
     bool csr_from_build = false;     // CSR built together with the internal pair list
-    const int32_t* csr_pairs = nullptr;  // the half list the current CSR belongs to
     void* d_mvcoef = nullptr;  // [csr_cap] MvCoef<T>
     void* d_p4 = nullptr;      // [n_cap] Vec4<T>: the matvec's dipoles in kernel precision
     int64_t mv_cap = 0;
@@ -2700,7 +2699,6 @@ int dmffb_admp_reconfigure(dmffb_engine* h, const dmffb_admp_desc* d) {
     h->have_pairs = false;
     h->npairs = 0;
     h->csr_from_build = false;
-    h->csr_pairs = nullptr;
     if (h->cg_exec) {
         cudaGraphExecDestroy(h->cg_exec);
         h->cg_exec = nullptr;
