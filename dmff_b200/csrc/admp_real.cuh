@@ -32,7 +32,7 @@ struct PairArgs {
     const double* posd;    // [n*3] FP64 positions (FP64 rows)
     const T* Qg;           // [n*9] permanent multipoles, global harmonic
     const double* Qgd;     // [n*9] the same in FP64
-    const double* U;       // [n*3] Cartesian induced dipoles (FULL/FIELD may be null) or CG vector (MATVEC)
+    const double* U;       // [n*3] Cartesian induced dipoles (may be null)
     const T* thole;        // [n]
     const T* polsix;       // [n]  pol^(1/6)
     T ms[6], ps[6], dsc[6];
@@ -145,7 +145,7 @@ __device__ __forceinline__ void qi_frame(const T ez[3], T ex[3], T ey[3]) {
 // Per-pair physics in arithmetic TC.  dr: minimum-image r_i - r_j; QI/QJ: global harmonic
 // multipoles; UI/UJ: Cartesian induced dipoles (POL); scales for this row; thole width Ath and
 // distance scale dmp.  Outputs: FULL: oi = dE/ddr (3) + torque_i (3), oj = -dE/ddr + torque_j;
-// FIELD/MATVEC: oi/oj = dE/dU_i, dE/dU_j.  e = pair energy (FULL).
+// FIELD: oi/oj = dE/dU_i, dE/dU_j.  e = pair energy (FULL).
 template <typename TC, bool POL, int MODE>
 __device__ __forceinline__ void pair_eval(const TC dr[3], const TC* QIg, const TC* QJg, const TC UI[3], const TC UJ[3],
                                           TC m, TC pp, TC dsv, TC Ath, TC dmp, TC kap, TC oi[6], TC oj[6], double& e) {
@@ -239,7 +239,7 @@ __device__ __forceinline__ void pair_eval(const TC dr[3], const TC* QIg, const T
     }
 
     if (MODE == PAIR_FIELD) {
-        // dE/du of the permanent-induced terms (the P^T q part; U-U is MATVEC)
+        // dE/du of the permanent-induced terms (the P^T q part; U-U is k_matvec_coef)
         const TC guI0 = TC(0.5) * (-cud.v * qJ[0] + dud0.v * qJ[1] - udq0.v * qJ[4]);
         const TC guI1 = TC(0.5) * (dud1.v * qJ[2] - udq1.v * qJ[5]);
         const TC guI2 = TC(0.5) * (dud1.v * qJ[3] - udq1.v * qJ[6]);
@@ -562,7 +562,7 @@ __global__ void __launch_bounds__(128, (sizeof(T) == 4 && ROWS == ROWS_UNSCALED 
                        (ROWS == ROWS_ALL || (ROWS == ROWS_UNSCALED) == (nb == 0));
     const int key = valid ? i : -1;
 
-    T oi[6], oj[6];  // FULL: grad(3) + torque(3); FIELD/MATVEC: field(3)
+    T oi[6], oj[6];  // FULL: grad(3) + torque(3); FIELD: field(3)
 #pragma unroll
     for (int k = 0; k < 6; ++k) { oi[k] = T(0); oj[k] = T(0); }
     double eacc = 0.0;
