@@ -3807,7 +3807,7 @@ int dmffb_set_timing(dmffb_engine* h, int32_t enabled) {
 
 int dmffb_set_fused_fft(dmffb_engine* h, int32_t enabled) {
     if (!h) return DMFFB_BAD_ARG;
-    h->dft_mode = enabled != 0;
+    h->dft_mode = enabled < 0 ? -1 : (enabled != 0);
     return DMFFB_OK;
 }
 

@@ -365,8 +365,9 @@ class AdmpEngine:
 
     def set_fused_fft(self, on=True):
         """The mesh convolution through the engine's direct-DFT kernels (meshes up to 64 per axis) or
-        through cuFFT, instead of the engine's choice by size (dmffb_set_fused_fft)."""
-        self._check(self.lib.dmffb_set_fused_fft(self.h, int(bool(on))))
+        through cuFFT, instead of the engine's choice by size, which "auto" returns to
+        (dmffb_set_fused_fft)."""
+        self._check(self.lib.dmffb_set_fused_fft(self.h, -1 if on == "auto" else int(bool(on))))
 
     def set_persistent_cg(self, mode=True):
         """The whole CG dipole solve in one persistent cooperative launch (FP32, meshes up to 128

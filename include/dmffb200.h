@@ -341,7 +341,7 @@ int dmffb_classical_param_grads(dmffb_engine* h, void* stream, double* dE_dq, do
 /* The mesh convolution (forward transform, influence-function multiply, inverse transform): by
  * default the engine's direct-DFT kernels on meshes where they are faster and cuFFT R2C +
  * convolution + C2R elsewhere (a rule on the extents and the precision).  enabled = 1 asks for the
- * DFT kernels on meshes of at most 64 points per axis (cuFFT beyond), 0 for cuFFT.
+ * DFT kernels on meshes of at most 64 points per axis (cuFFT beyond), 0 for cuFFT, -1 for the rule again.
  * dmffb_fused_fft_active returns 1 when the last convolution ran through the DFT kernels, else 0. */
 int dmffb_set_fused_fft(dmffb_engine* h, int32_t enabled);
 /* The whole CG dipole solve in one persistent cooperative launch (k_cg_solve: vector update and dipole
