@@ -106,15 +106,6 @@ __global__ void k_nb_forces(int n, const T* glr, const double* gd, const T* gcel
     for (int c = 0; c < 3; ++c) forces[3 * i + c] = -((double)glr[3 * i + c] + (double)g[c] + gd[3 * i + c]);
 }
 
-// distance of an FP64 square in kernel precision: FP32 from the hardware's reciprocal square root and
-// one FP64 Newton step (error 1e-14, so it rounds to the same float as the FP64 root all but always)
-__device__ __forceinline__ void nb_root(double r2, double& r) { r = sqrt(r2); }
-__device__ __forceinline__ void nb_root(double r2, float& r) {
-    const double y = (double)rsqrtf((float)r2);
-    const double q = r2 * y;
-    r = (float)fma(0.5 * y, fma(-q, q, r2), q);
-}
-
 // One kept pair (i, the atom in cell slot k), met once: energy, box gradient (the lane's FP64 sums
 // box[0], box[32], ...), the force on i (registers) and on the partner (a reduction into its slot).
 template <typename T, bool ORTHO>
@@ -139,7 +130,7 @@ __device__ __forceinline__ void nb_cell_pair(const NbCellArgs<T>& a, int k, doub
     }
 #pragma unroll
     for (int c = 0; c < 3; ++c) e[c] = (T)dr[c];
-    nb_root(dr[0] * dr[0] + dr[1] * dr[1] + dr[2] * dr[2], r);
+    r = (T)sqrt(dr[0] * dr[0] + dr[1] * dr[1] + dr[2] * dr[2]);
     T qj;
     int tj = 0;
     nb_rec_get(rj, qj, tj);
@@ -170,11 +161,11 @@ __device__ __forceinline__ void nb_cell_pair(const NbCellArgs<T>& a, int k, doub
     }
 }
 
-// Bound by instruction issue (FP64 minimum image, erf / exp; 71 % of the issue slots): 475 us for
-// the 20.8 M pairs of 99000 atoms at rc 10 A.  Before: with a minimum image per candidate, 63 cells per
+// Bound by instruction issue (FP64 minimum image, erf / exp; 73 % of the issue slots): 486 us for
+// the 20.8 M pairs of 99000 atoms at rc 10 A, FP64 root included (479 with a reciprocal root and one Newton
+// step, good to 1e-14, in its place).  Before: with a minimum image per candidate, 63 cells per
 // atom searched and pruned one by one and FP32 box sums in registers 563; with scalar reductions into
-// [3n], three FP64 gathers plus charge and type per partner, FP64 division in the pruning and a full FP64
-// root 822.
+// [3n], three FP64 gathers plus charge and type per partner and FP64 division in the pruning 822.
 template <typename T, bool ORTHO>
 __global__ void __launch_bounds__(32 * kNbWarps, sizeof(T) == 4 ? 4 : 0) k_nb_cells(NbCellArgs<T> a) {
     constexpr int NC = 13, NR = 2 * NC;  // forward columns of the 5^3 stencil, runs
