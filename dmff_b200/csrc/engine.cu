@@ -853,12 +853,19 @@ ConvArgs<T> conv_args(const dmffb_engine* h, const Box& bx, int kind, double esc
     return ca;
 }
 
-// Co-resident CTAs of the persistent CG solve for the current mesh (0: the graph-replayed solve
-// runs instead): needs the engine-FFT convolution for the mesh, the kernel's shared memory and a
-// device that takes cooperative launches.
+// Whether the persistent solve is asked for.  By size: up to 4096 atoms, on meshes whose direct DFTs, one multiply-add
+// chain of K0 + K1 + K2 a point, do not outgrow the launches they replace.  One evaluation of 450 / 1500 / 3999
+// atoms, direct launches against persistent (us): 61^3 743 / 647 / 782 and 609 / 552 / 721, 72^3 942 / 883 / 1014
+// and 743 / 693 / 884, 80^3 988 / 895 / 1052 and 1012 / 910 / 1164, 100^3 1015 / 940 / 1105 and 1485 / 1332 / 1643,
+// 32 x 48 x 96 821 / 783 / 909 and 562 / 520 / 689.
 bool pcg_wanted(const dmffb_engine* h) {
-    return h->pcg_mode == 1 || (h->pcg_mode == 2 && h->n <= h->pcg_auto_atoms);
+    if (h->pcg_mode != 2) return h->pcg_mode == 1;
+    return h->n <= h->pcg_auto_atoms && (double)h->K[0] * h->K[1] * h->K[2] * (h->K[0] + h->K[1] + h->K[2]) <= 9e7;
 }
+
+// Co-resident CTAs of the persistent CG solve for the current mesh (0: the graph-replayed solve
+// runs instead): needs a mesh that the direct DFT can serve, the kernel's shared memory and a
+// device that takes cooperative launches.
 
 int pcg_decide(dmffb_engine* h) {
     if (h->pcg_max_blocks >= 0) return h->pcg_max_blocks;

@@ -372,8 +372,9 @@ class AdmpEngine:
     def set_persistent_cg(self, mode=True):
         """The whole CG dipole solve in one persistent cooperative launch (FP32, meshes up to 128
         per axis; dmffb_set_persistent_cg): True / 1 always, False / 0 never (the graph-replayed
-        per-pass solve), "auto" / 2 (the default) for systems of at most 4096 atoms in solves that
-        no captured graph can replay (new buffers or a new box)."""
+        per-pass solve), "auto" / 2 (the default) for systems of at most 4096 atoms, on meshes of
+        moderate size, in solves that no captured graph can replay (new buffers, a new box or another
+        pair count)."""
         m = 2 if mode == "auto" else int(mode)
         self._check(self.lib.dmffb_set_persistent_cg(self.h, m))
 

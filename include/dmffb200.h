@@ -347,9 +347,10 @@ int dmffb_set_fused_fft(dmffb_engine* h, int32_t enabled);
 /* The whole CG dipole solve in one persistent cooperative launch (k_cg_solve: vector update and dipole
  * spread, the direct-DFT convolution, real-space matvec and field gather per iteration, separated by
  * grid barriers; convergence decided on the device, one read-back per solve).  mode 0: off (the
- * graph-replayed per-pass solve), 1: on, 2 (default): on for systems of at most 4096 atoms whose solve
- * no graph of this engine can replay (a first solve with these buffers and box), where the launch
- * chain of the per-pass solve dominates.  FP32 engines with
+ * graph-replayed per-pass solve), 1: on, 2 (default): on for systems of at most 4096 atoms on meshes with
+ * K0 K1 K2 (K0 + K1 + K2) of at most 9e7 (72^3), whose solve no graph of this engine can replay (a first
+ * solve in a row with these buffers, this box and this pair count), where the launch chain of the per-pass
+ * solve dominates.  FP32 engines with
  * meshes of at most 128 points per axis on devices with cooperative launch only.
  * dmffb_persistent_cg_blocks returns the co-resident CTAs available to it for the current mesh
  * (0: not used).
