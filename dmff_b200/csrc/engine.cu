@@ -2000,7 +2000,8 @@ int bin_cells(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx,
 struct NbPlan {
     bool flat, staged, ortho;
     int nc[3], ncell, chmax;
-    int guess;  // neighbours per atom at the mean density, with headroom
+    double mean;  // neighbours per atom at the mean density
+    int guess;    // the same with headroom, at most n
 };
 
 NbPlan nb_plan(const dmffb_engine* h, const Box& bx, double rc) {
@@ -2012,8 +2013,9 @@ NbPlan nb_plan(const dmffb_engine* h, const Box& bx, double rc) {
     p.staged = !p.flat && (size_t)p.chmax * sizeof(float4) <= kNbStageBytes;
     const double* m = bx.h;
     p.ortho = m[1] == 0.0 && m[2] == 0.0 && m[3] == 0.0 && m[5] == 0.0 && m[6] == 0.0 && m[7] == 0.0;
-    const double mean = (double)h->n / fabs(det3(m)) * (4.0 / 3.0) * M_PI * rc * rc * rc;
-    p.guess = (int)std::min(1.35 * mean + 24.0, (double)h->n);
+    p.mean = std::min((double)h->n / fabs(det3(m)) * (4.0 / 3.0) * M_PI * rc * rc * rc, (double)h->n);
+    if (!(p.mean >= 0.0)) p.mean = h->n;  // no volume
+    p.guess = (int)std::min(1.35 * p.mean + 24.0, (double)h->n);
     return p;
 }
 
@@ -3275,7 +3277,7 @@ int dmffb_admp_build_neighbors(dmffb_engine* h, void* stream, const double* pos,
         // caller may change the positions when it returns); later ones leave that to nb_finish
         const bool first = !h->slot_cap || !h->d_pairs || (want_csr && !h->d_csr_ent);
         if (first) {
-            const int64_t rows = (int64_t)h->n * p.guess / 2 + 1;
+            const int64_t rows = (int64_t)(0.5 * h->n * p.mean) + 1;  // nb_pair_cap and nb_csr_cap add the headroom
             if (!h->slot_cap && (st = nb_slots(h, p.guess))) return st;
             if (!h->d_pairs && (st = nb_pair_cap(h, rows))) return st;
             if (want_csr && !h->d_csr_ent && (st = nb_csr_cap(h, 2 * rows))) return st;
