@@ -69,6 +69,20 @@ dmffb_admp_desc request_desc(const dmffb_server* s, const dmffb_request* r) {
     return a;
 }
 
+// Accounting convention: per-atom engine arrays, neighbour rows, their slots and the both-direction CSR with the
+// matvec pair tensors (a half pair: 12 bytes of rows, 8 of CSR and 32 of tensors, FP64 64, with a headroom of 1.3,
+// and 11 of slots: 79 and 120 bytes), and the mesh with its complex transform, cuFFT work area and (with
+// polarization) the second real grid of the dipole field pass.
+int64_t footprint(int32_t n_atoms, double rc, const int32_t K[3], double box_volume, int32_t lpol, int32_t precision) {
+    const double n = n_atoms;
+    const double dens = box_volume > 0 ? n / box_volume : 0.1;
+    const double half_pairs = n * dens * (4.0 / 3.0) * M_PI * rc * rc * rc / 2.0;
+    const double K3 = (double)K[0] * K[1] * K[2];
+    const double bytes = n * (600.0 + (lpol ? 320.0 : 0.0)) + half_pairs * (precision == DMFFB_FP64 ? 132.0 : 92.0) +
+                         (lpol ? 20.0 : 16.0) * K3;
+    return (int64_t)bytes;
+}
+
 // one request on one slot; returns the evaluation status
 int run_request(dmffb_server* s, int slot, dmffb_request* r) {
     dmffb_engine* h = s->eng[slot];
@@ -126,15 +140,7 @@ void worker(dmffb_server* s, int slot) {
 extern "C" {
 
 int64_t dmffb_request_footprint(int32_t n_atoms, double rc, const int32_t K[3], double box_volume, int32_t lpol) {
-    // accounting convention: per-atom engine arrays, neighbour rows, their slots and the both-direction
-    // CSR with the matvec pair tensors, and the mesh with its complex transform, cuFFT work area and (with
-    // polarization) the second real grid of the dipole field pass
-    const double n = n_atoms;
-    const double dens = box_volume > 0 ? n / box_volume : 0.1;
-    const double half_pairs = n * dens * (4.0 / 3.0) * M_PI * rc * rc * rc / 2.0;
-    const double K3 = (double)K[0] * K[1] * K[2];
-    const double bytes = n * (600.0 + (lpol ? 320.0 : 0.0)) + half_pairs * 132.0 + (lpol ? 20.0 : 16.0) * K3;
-    return (int64_t)bytes;
+    return footprint(n_atoms, rc, K, box_volume, lpol, DMFFB_FP32);
 }
 
 int dmffb_server_create(const dmffb_server_desc* d, dmffb_server** out) {
@@ -194,7 +200,7 @@ int dmffb_server_submit(dmffb_server* s, dmffb_request* r) {
     const double V = fabs(r->box[0] * (r->box[4] * r->box[8] - r->box[5] * r->box[7]) -
                           r->box[1] * (r->box[3] * r->box[8] - r->box[5] * r->box[6]) +
                           r->box[2] * (r->box[3] * r->box[7] - r->box[4] * r->box[6]));
-    r->footprint_bytes = dmffb_request_footprint(r->n_atoms, r->rc, r->K, V, s->d.lpol);
+    r->footprint_bytes = footprint(r->n_atoms, r->rc, r->K, V, s->d.lpol, s->d.precision);
     r->done = 0;
     r->status = -1;
     r->slot = -1;

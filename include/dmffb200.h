@@ -473,7 +473,8 @@ int dmffb_server_submit(dmffb_server* srv, dmffb_request* req);
 int dmffb_server_wait(dmffb_server* srv, double timeout_s);
 /* Seconds since the server was created (the clock of t_arrival / t_start / t_done). */
 double dmffb_server_clock(const dmffb_server* srv);
-/* Device bytes a request of this size is accounted for at admission. */
+/* Device bytes a request of this size is accounted for at admission on an FP32 server (an FP64 server counts 132
+ * instead of 92 bytes for a pair). */
 int64_t dmffb_request_footprint(int32_t n_atoms, double rc, const int32_t K[3], double box_volume, int32_t lpol);
 /* Run each request once on every slot, untimed (grows buffers and caches cuFFT plans). */
 int dmffb_server_prewarm(dmffb_server* srv, dmffb_request* reqs, int32_t n_reqs);
