@@ -328,8 +328,10 @@ class AdmpEngine:
         need = ctypes.c_int64(0)
         # without a capacity: the count at the mean density with headroom, or the last count's
         n = self.n
-        mean = n / max(abs(float(np.linalg.det(b.reshape(3, 3)))), 1e-300) * (4.0 / 3.0) * np.pi * float(rc) ** 3
-        guess = max(int(min(0.54 * n * mean, 600.0 * n)) + 64, getattr(self, "_rows_hint", 0))
+        r = float(rc)
+        mean = n / max(abs(float(np.linalg.det(b.reshape(3, 3)))), 1e-300) * (4.0 / 3.0) * np.pi * (r * r * r)
+        rows = 0.54 * n * mean
+        guess = max(int(rows if rows < 600.0 * n else 600.0 * n) + 64, getattr(self, "_rows_hint", 0))
         cap = int(capacity) if capacity else min(guess, n * (n - 1) // 2)
         buf = torch.empty((max(cap, 1), 3), dtype=torch.int32, device=self.device)
         st = self.lib.dmffb_build_neighbors(self.h, ctypes.c_void_p(s.cuda_stream), _dev(pos),
