@@ -353,7 +353,7 @@ enum { KC_PREP = 0, KC_PAIR_FULL, KC_PAIR_FIELD, KC_PAIR_MATVEC, KC_SPREAD, KC_F
        KC_GATHER_FIELD, KC_SELF, KC_VEC, KC_NBLIST, KC_MVCOEF,
        // FP64 launches over the topologically scaled rows, parameter-adjoint pair kernels, bonded terms
        KC_PAIR_FULL_SCALED, KC_PAIR_FIELD_SCALED, KC_PGRAD, KC_BONDED,
-       KC_FFTCONV,  // the dipole solve's forward FFT + influence multiply + inverse FFT (engine FFT)
+       KC_FFTCONV,  // the mesh convolution by the direct-DFT kernels
        KC_CGSOLVE,  // the whole CG solve in one persistent cooperative launch
        KC_COUNT };
 static_assert(KC_COUNT <= 32, "kernel-class statistics arrays hold 32 classes");
@@ -1355,11 +1355,14 @@ int solve_dipoles(dmffb_engine* h, cudaStream_t s, const double* pos, const Box&
     const bool small = sizeof(T) == 4 && fused && pcg_wanted(h) && pcg_decide(h) > 0;
     const CgSchedule sched = {sc, 3.0 * n, h->cg_tol, small ? 1 : 0};
     if (graphs) {
-        std::vector<double> key = {(double)(uintptr_t)pos, (double)(uintptr_t)pairs, (double)npairs,
-                                   (double)(uintptr_t)U, (double)(uintptr_t)h->d_csr_ent, (double)sizeof(T),
+        std::vector<double> key = {(double)(uintptr_t)U, (double)(uintptr_t)h->d_csr_ent, (double)sizeof(T),
                                    (double)(uintptr_t)h->d_mvcoef, (double)(uintptr_t)h->d_csr_off,
                                    (double)dft_use<T>(h), (double)(uintptr_t)h->d_dftG, (double)(uintptr_t)h->d_dftW,
                                    (double)fused, (double)sched.every};
+        // a fused step reads the CSR, its tensors and the stencil cache, not the positions and rows they came from:
+        // atoms that move, and with them the number of pairs, leave its graph as it is
+        if (!fused)
+            for (double x : {(double)(uintptr_t)pos, (double)(uintptr_t)pairs, (double)npairs}) key.push_back(x);
         for (int k = 0; k < 9; ++k) key.push_back(bx.h[k]);
         const bool repeat = key == h->cg_seen_key;
         h->cg_seen_key = key;

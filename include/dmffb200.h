@@ -217,7 +217,7 @@ int dmffb_set_timing(dmffb_engine* h, int32_t enabled);
  * 2 pair FIELD, 3 pair MATVEC, 4 spread, 5 FFT (cuFFT), 6 convolution, 7 gather FULL,
  * 8 gather FIELD, 9 self+frame forces, 10 vector/CG ops, 11 neighbour build, 12 CG matvec
  * pair-tensor set-up, 13 pair FULL over the topologically scaled rows (FP64), 14 pair FIELD over
- * the scaled rows (FP64), 15 parameter-adjoint pair kernels, 16 bonded terms, 17 the engine-FFT
+ * the scaled rows (FP64), 15 parameter-adjoint pair kernels, 16 bonded terms, 17 the
  * direct-DFT mesh convolution (dmffb_set_fused_fft), 18 the persistent CG solve
  * (dmffb_set_persistent_cg).  Classes 1 and 2
  * hold only the launches over the unscaled rows (kernel precision). */
