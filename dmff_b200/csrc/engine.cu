@@ -114,7 +114,7 @@ struct dmffb_engine {
     int64_t pair_cap = 0, npairs = 0;
     bool have_pairs = false;
     int32_t *d_atom_cell = nullptr, *d_rank = nullptr, *d_cell_count = nullptr, *d_cell_start = nullptr,
-            *d_pcount = nullptr, *d_pcount_s = nullptr, *d_poff_s = nullptr;
+            *d_pcount = nullptr, *d_pcount_s = nullptr, *d_poff_s = nullptr, *d_cell_atoms = nullptr;
     unsigned* d_bin_done = nullptr;
     int64_t* d_poff = nullptr;
     int ncell_cap = 0;
@@ -1953,7 +1953,7 @@ bool half_cells(const Box& bx, double rc, int nc[3]) {
 // Counting sort of the atoms into the cells nc: cell_start and the cell-ordered float4 positions.
 // With zero, nzero words are cleared on the way.
 int bin_cells(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx, const int nc[3], int32_t* zero = nullptr,
-              int nzero = 0) {
+              int nzero = 0, int32_t* cell_atoms = nullptr) {
     const int n = h->n;
     int st;
     if (!h->d_posc) {
@@ -1989,6 +1989,7 @@ int bin_cells(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx,
     a.zero = zero;
     a.nzero = nzero;
     a.posc = h->d_posc;
+    a.cell_atoms = cell_atoms;
     LAUNCH(h, s, KC_NBLIST, k_bin_count<<<nblk(n, kBinThreads), kBinThreads, 0, s>>>(a));
     LAUNCH(h, s, KC_NBLIST, k_bin_fill<<<nblk(n, 256), 256, 0, s>>>(a));
     CK(cudaGetLastError());
@@ -2171,9 +2172,11 @@ int nb_single_pass(dmffb_engine* h, cudaStream_t s, const NbPlan& p, const doubl
 int nb_count(dmffb_engine* h, cudaStream_t s, const NbPlan& p, const double* pos, const Box& bx, Nb2Args& b) {
     const int n = h->n;
     int st;
-    if ((st = bin_cells(h, s, pos, bx, p.nc, h->d_nbsum, nb_sum_words(n)))) return st;
+    if (!h->d_cell_atoms && (st = dalloc(h, &h->d_cell_atoms, (size_t)h->n_cap * sizeof(int32_t)))) return st;
+    if ((st = bin_cells(h, s, pos, bx, p.nc, h->d_nbsum, nb_sum_words(n), h->d_cell_atoms))) return st;
     b.posc = h->d_posc;
     b.a.cell_start = h->d_cell_start;
+    b.a.cell_atoms = h->d_cell_atoms;
     // keep masks for the fill pass: room for 1.5x the mean candidate count (125 cells of the
     // stencil) per atom, at most 1 GiB; atoms with more candidates repeat the distance tests
     const double mean_cand = 125.0 * (double)n / (double)p.ncell;
@@ -2736,7 +2739,7 @@ void dmffb_destroy(dmffb_engine* h) {
                     h->d_thole, h->d_polsix, h->d_pos, h->d_U, h->d_forces, h->d_posT, h->d_Qg, h->d_QgT,
                     h->d_rec, h->d_gpair, h->d_torque, h->d_fieldT, h->d_grad, h->d_scal, h->d_b, h->d_r, h->d_z, h->d_p,
                     h->d_Ap, h->d_s, h->d_fr, h->d_gQ, h->d_fmv, h->d_pcount_f, h->d_pcount_s, h->d_poff_s, h->d_rank, h->d_bin_done, h->d_nbsum, h->d_mvcoef, h->d_p4, h->d_csr_off, h->d_csr_ent, h->d_csr_deg, h->d_cub2, h->d_grid, h->d_grid2, h->d_cgrid, h->d_bmod, h->d_pairs, h->d_atom_cell,
-                    h->d_cell_count, h->d_cell_start, h->d_pcount, h->d_poff,
+                    h->d_cell_count, h->d_cell_start, h->d_cell_atoms, h->d_pcount, h->d_poff,
                     h->d_c, h->d_tta, h->d_ttb, h->d_ttq, h->d_glr, h->d_gsr, h->d_dc,
                     h->d_q, h->d_qT, h->d_type, h->d_sigtt, h->d_epstt, h->d_dq, h->d_dsig, h->d_deps,
                     h->d_tidx[0], h->d_tidx[1], h->d_tidx[2], h->d_tprm[0], h->d_tprm[1], h->d_tprm[2],

@@ -222,6 +222,7 @@ struct BinArgs {
     int32_t* zero;        // words to clear, or null
     int nzero;
     float4* posc;         // [n]
+    int32_t* cell_atoms;  // [n] the atom indices of posc by themselves, or null
 };
 
 static __global__ void __launch_bounds__(kBinThreads) k_bin_count(BinArgs a) {
@@ -302,7 +303,9 @@ static __global__ void k_bin_fill(BinArgs a) {
     float w[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) w[c] = (float)(s[0] * a.box.h[c] + s[1] * a.box.h[3 + c] + s[2] * a.box.h[6 + c]);
-    a.posc[a.cell_start[a.atom_cell[i]] + a.rank[i]] = make_float4(w[0], w[1], w[2], __int_as_float(i));
+    const int k = a.cell_start[a.atom_cell[i]] + a.rank[i];
+    a.posc[k] = make_float4(w[0], w[1], w[2], __int_as_float(i));
+    if (a.cell_atoms) a.cell_atoms[k] = i;
 }
 
 // Totals of a build (read back by the host) and, behind them in the same array, the sums of the
@@ -411,6 +414,20 @@ __device__ __forceinline__ int nb_bond(const NbArgs& a, int i, int j, int plo, i
     return (j < plo || j > phi) ? 0 : (j > i ? lookup_nbond(a, i, j) : lookup_nbond(a, j, i));
 }
 
+// The lane's part of an atom's pairs j > i within rc with nbond != 0, from the few rows of its covalent map: the
+// count pass then looks up no candidate (30000 atoms at rc 12 A: 623 us with a lookup of each kept one, 475 without).
+__device__ __forceinline__ int nb_scaled(const NbArgs& a, int i, int lane) {
+    int cnt = 0;
+    const int beg = a.cov_ptr[i], end = a.cov_ptr[i + 1];
+    for (int k = beg + lane; k < end; k += 32) {
+        const int j = a.cov_j[k];
+        int first = beg;  // a partner given twice counts once, with its first nbond (lookup_nbond)
+        while (a.cov_j[first] != j) ++first;
+        if (first == k && a.cov_nb[k] != 0 && within_rc(a.box, a.pos + 3 * i, a.pos + 3 * j, a.rc)) ++cnt;
+    }
+    return cnt;
+}
+
 // the counts of one atom (lane 0 of its warp)
 __device__ __forceinline__ void nb_counts(const Nb2Args& b, int i, int nh, int nf, int ns) {
     const int runs = nb_runs(b.a.n), run = i / kNbRun;
@@ -509,7 +526,10 @@ __global__ void __launch_bounds__(128) k_pairs_flat(Nb2Args b) {
 // lays the stencil's cells out as one concatenated candidate list (cell starts and a prefix sum of
 // their counts in shared memory, in the dx, dy, dz order of the 27-cell scan), then walks it in
 // full 32-lane batches; each lane finds its candidate's cell by advancing a cursor (lanes move
-// forward monotonically).  Count pass and fill pass: it serves neighbourhoods too large to stage.
+// forward monotonically), seen from the image that the cell wraps to, as in k_pairs_cell.  Count pass and fill
+// pass: it serves neighbourhoods too large to stage.  30000 atoms at rc 12 A, a whole build: 642 us (683 in a
+// triclinic box); with a minimum image per candidate and its covalent partners looked up in the count pass
+// too 1090 (1173).
 constexpr int kNbWarps = 8;  // warps per block of k_pairs_warp3
 constexpr size_t kNbStageBytes = 44u << 10;  // largest candidate stage of k_pairs_cell: with its static
                                               // shared arrays it stays under the 48 KB default
@@ -519,6 +539,7 @@ __global__ void __launch_bounds__(32 * kNbWarps) k_pairs_warp3(Nb2Args b) {
     constexpr int W = 2 * S + 1, NQ = W * W * W;
     __shared__ int s_beg[kNbWarps][NQ];
     __shared__ int s_off[kNbWarps][NQ + 1];
+    __shared__ float s_sh[kNbWarps][NQ][3];  // lattice vectors that the cell wraps by
     const NbArgs& a = b.a;
     const int wl = threadIdx.x >> 5;
     const int ks = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -536,14 +557,19 @@ __global__ void __launch_bounds__(32 * kNbWarps) k_pairs_warp3(Nb2Args b) {
         const int q = q0 + lane;
         int cnt = 0;
         if (q < NQ) {
-            const int dx = q / (W * W) - S, dy = (q / W) % W - S, dz = q % W - S;
-            const int cx = (c3[0] + dx + a.nc[0]) % a.nc[0];
-            const int cy = (c3[1] + dy + a.nc[1]) % a.nc[1];
-            const int cz = (c3[2] + dz + a.nc[2]) % a.nc[2];
-            const int cc = (cx * a.nc[1] + cy) * a.nc[2] + cz;
+            int c[3] = {c3[0] + q / (W * W) - S, c3[1] + (q / W) % W - S, c3[2] + q % W - S}, wrap[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                wrap[k] = c[k] < 0 ? -1 : (c[k] >= a.nc[k] ? 1 : 0);
+                c[k] -= wrap[k] * a.nc[k];
+            }
+            const int cc = (c[0] * a.nc[1] + c[1]) * a.nc[2] + c[2];
             const int cs = a.cell_start[cc];
             cnt = a.cell_start[cc + 1] - cs;
             s_beg[wl][q] = cs;
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                s_sh[wl][q][k] = (float)(wrap[0] * a.box.h[k] + wrap[1] * a.box.h[3 + k] + wrap[2] * a.box.h[6 + k]);
         }
         int incl = cnt;
 #pragma unroll
@@ -558,7 +584,7 @@ __global__ void __launch_bounds__(32 * kNbWarps) k_pairs_warp3(Nb2Args b) {
     const int total = carry;
     int64_t out_h = (PASS == 1) ? a.offset[i] : 0, out_f = (PASS == 1 && b.off_f) ? b.off_f[i] : 0;
     int64_t out_s = (PASS == 1 && b.srows) ? b.off_s[i] : 0;
-    int cnt_h = 0, cnt_f = 0, cnt_s = 0;
+    int cnt_h = 0, cnt_f = 0;
     const int plo = a.cov_lo ? a.cov_lo[i] : 0, phi = a.cov_hi ? a.cov_hi[i] : a.n;
     const unsigned lt = (1u << lane) - 1u;
     int qc = 0;
@@ -574,22 +600,26 @@ __global__ void __launch_bounds__(32 * kNbWarps) k_pairs_warp3(Nb2Args b) {
             if (mk == 0u) continue;  // warp-uniform: no candidate of this batch is kept
             if ((mk >> lane) & 1u) {
                 while (t >= s_off[wl][qc + 1]) ++qc;
-                j = __float_as_int(b.posc[s_beg[wl][qc] + (t - s_off[wl][qc])].w);
+                j = a.cell_atoms[s_beg[wl][qc] + (t - s_off[wl][qc])];
                 keep = true;
             }
         } else if (t < total) {
             while (t >= s_off[wl][qc + 1]) ++qc;
             const float4 pj = b.posc[s_beg[wl][qc] + (t - s_off[wl][qc])];
             j = __float_as_int(pj.w);
-            if (j != i) keep = nb_keep<false>(a, f, i, j, pj.x - p4.x, pj.y - p4.y, pj.z - p4.z);
+            const float dx = pj.x + s_sh[wl][qc][0] - p4.x, dy = pj.y + s_sh[wl][qc][1] - p4.y, dz = pj.z + s_sh[wl][qc][2] - p4.z;
+            const float r2 = dx * dx + dy * dy + dz * dz;
+            if (r2 < f.rlo2) keep = j != i;
+            else if (r2 <= f.rhi2 && j != i) keep = j > i ? within_rc(a.box, a.pos + 3 * i, a.pos + 3 * j, a.rc)
+                                                          : within_rc(a.box, a.pos + 3 * j, a.pos + 3 * i, a.rc);
         }
         const bool up = keep && j > i;
         const unsigned mf = __ballot_sync(0xffffffffu, keep);
         const unsigned mh = __ballot_sync(0xffffffffu, up);
         if (PASS == 0 && use_mask && lane == 0) mrow[base >> 5] = mf;
-        const int nbd = keep ? nb_bond(a, i, j, plo, phi) : 0;
-        const unsigned ms = __ballot_sync(0xffffffffu, up && nbd != 0);
         if (PASS == 1) {
+            const int nbd = keep ? nb_bond(a, i, j, plo, phi) : 0;
+            const unsigned ms = __ballot_sync(0xffffffffu, up && nbd != 0);
             if (keep) {
                 int sidx = nbd - 1;
                 if (sidx < 0) sidx += 6;
@@ -612,10 +642,12 @@ __global__ void __launch_bounds__(32 * kNbWarps) k_pairs_warp3(Nb2Args b) {
         } else {
             cnt_f += __popc(mf);
             cnt_h += __popc(mh);
-            cnt_s += __popc(ms);
         }
     }
-    if (PASS == 0 && lane == 0) nb_counts(b, i, cnt_h, cnt_f, cnt_s);
+    if (PASS == 0) {
+        const int cnt_s = __reduce_add_sync(0xffffffffu, nb_scaled(a, i, lane));
+        if (lane == 0) nb_counts(b, i, cnt_h, cnt_f, cnt_s);
+    }
 }
 
 // Block-per-cell single pass over the (2S + 1)^3 stencil: one CTA takes every atom of one cell.  Cells of
