@@ -116,6 +116,7 @@ struct dmffb_engine {
     int32_t *d_atom_cell = nullptr, *d_rank = nullptr, *d_cell_count = nullptr, *d_cell_start = nullptr,
             *d_pcount = nullptr, *d_pcount_s = nullptr, *d_poff_s = nullptr, *d_cell_atoms = nullptr;
     unsigned* d_bin_done = nullptr;
+    int32_t* d_bin_tiles = nullptr;
     int64_t* d_poff = nullptr;
     int ncell_cap = 0;
     double* h_scal = nullptr;  // pinned
@@ -1960,6 +1961,7 @@ int bin_cells(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx,
         const int cap = h->n_cap;
         if ((st = dalloc(h, &h->d_atom_cell, cap * sizeof(int32_t))) || (st = dalloc(h, &h->d_rank, cap * sizeof(int32_t))) ||
             (st = dalloc(h, &h->d_bin_done, sizeof(unsigned))) ||
+            (st = dalloc(h, &h->d_bin_tiles, kBinTiles * sizeof(int32_t))) ||
             (st = dalloc(h, &h->d_posc, (size_t)cap * sizeof(float4))))
             return st;
         CK(cudaMemsetAsync(h->d_bin_done, 0, sizeof(unsigned), s));
@@ -1986,11 +1988,13 @@ int bin_cells(dmffb_engine* h, cudaStream_t s, const double* pos, const Box& bx,
     a.cell_count = h->d_cell_count;
     a.cell_start = h->d_cell_start;
     a.done = h->d_bin_done;
+    a.tiles = ncell > 2 * kBinTile ? h->d_bin_tiles : nullptr;
     a.zero = zero;
     a.nzero = nzero;
     a.posc = h->d_posc;
     a.cell_atoms = cell_atoms;
     LAUNCH(h, s, KC_NBLIST, k_bin_count<<<nblk(n, kBinThreads), kBinThreads, 0, s>>>(a));
+    if (a.tiles) LAUNCH(h, s, KC_NBLIST, k_bin_scan<<<nblk(ncell, kBinTile), kBinThreads, 0, s>>>(a));
     LAUNCH(h, s, KC_NBLIST, k_bin_fill<<<nblk(n, 256), 256, 0, s>>>(a));
     CK(cudaGetLastError());
     return DMFFB_OK;
@@ -2738,7 +2742,7 @@ void dmffb_destroy(dmffb_engine* h) {
     void* ptrs[] = {h->d_axis_type, h->d_axis_idx, h->d_cov_ptr, h->d_cov_j, h->d_cov_nb, h->d_Qloc, h->d_pol,
                     h->d_thole, h->d_polsix, h->d_pos, h->d_U, h->d_forces, h->d_posT, h->d_Qg, h->d_QgT,
                     h->d_rec, h->d_gpair, h->d_torque, h->d_fieldT, h->d_grad, h->d_scal, h->d_b, h->d_r, h->d_z, h->d_p,
-                    h->d_Ap, h->d_s, h->d_fr, h->d_gQ, h->d_fmv, h->d_pcount_f, h->d_pcount_s, h->d_poff_s, h->d_rank, h->d_bin_done, h->d_nbsum, h->d_mvcoef, h->d_p4, h->d_csr_off, h->d_csr_ent, h->d_csr_deg, h->d_cub2, h->d_grid, h->d_grid2, h->d_cgrid, h->d_bmod, h->d_pairs, h->d_atom_cell,
+                    h->d_Ap, h->d_s, h->d_fr, h->d_gQ, h->d_fmv, h->d_pcount_f, h->d_pcount_s, h->d_poff_s, h->d_rank, h->d_bin_done, h->d_bin_tiles, h->d_nbsum, h->d_mvcoef, h->d_p4, h->d_csr_off, h->d_csr_ent, h->d_csr_deg, h->d_cub2, h->d_grid, h->d_grid2, h->d_cgrid, h->d_bmod, h->d_pairs, h->d_atom_cell,
                     h->d_cell_count, h->d_cell_start, h->d_cell_atoms, h->d_pcount, h->d_poff,
                     h->d_c, h->d_tta, h->d_ttb, h->d_ttq, h->d_glr, h->d_gsr, h->d_dc,
                     h->d_q, h->d_qT, h->d_type, h->d_sigtt, h->d_epstt, h->d_dq, h->d_dsig, h->d_deps,

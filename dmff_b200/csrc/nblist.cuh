@@ -205,9 +205,12 @@ __global__ void __launch_bounds__(256) k_pairs_warp(NbArgs a) {
 // cursor array.  k_bin_fill writes the cell-ordered float4 positions (x, y, z, atom index as int
 // bits), all that the pair passes read.  `zero` is cleared on the way (the build's sums and totals).
 // Launch-bound at liquid sizes: the seven launches this replaces (FP32 copy, two memsets, count,
-// two-kernel scan, fill) took 13.5 us of device time at 12288 atoms, these two 7.
+// two-kernel scan, fill) took 13.5 us of device time at 12288 atoms, these two 7.  The last CTA takes 3 us for
+// a tile of 4096 cells: boxes of more than two (atoms in a vacuum) leave the scan to k_bin_scan, a CTA per
+// tile, which starts from sums that k_bin_count left per tile (125000 cells: 4 + 5.5 us against 96).
 constexpr int kBinThreads = 512;
-constexpr int kBinItems = 8;  // counts per thread and tile of the last CTA's scan
+constexpr int kBinItems = 8;  // counts per thread and tile of a scan
+constexpr int kBinTile = kBinThreads * kBinItems, kBinTiles = 64 * 64 * 64 / kBinTile;  // at most 64 cells an axis
 
 struct BinArgs {
     int n;
@@ -219,23 +222,75 @@ struct BinArgs {
     int32_t* cell_count;  // [ncell rounded up to kBinItems], zero between calls
     int32_t* cell_start;  // [ncell + 1]
     unsigned* done;       // CTAs that have finished, zero between calls
+    int32_t* tiles;       // [kBinTiles] atoms per tile of cells, zero between calls; null: the last CTA scans
     int32_t* zero;        // words to clear, or null
     int nzero;
     float4* posc;         // [n]
     int32_t* cell_atoms;  // [n] the atom indices of posc by themselves, or null
 };
 
+// cell_start of the tile of counts from cell t0 on, whose atoms come after `before` others, and the counts cleared;
+// returns the tile's atoms (whole CTA)
+__device__ __forceinline__ int bin_tile(const BinArgs& a, int ncell, int t0, int before, int* s_warp) {
+    const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
+    const int c0 = t0 + kBinItems * threadIdx.x;
+    int v[kBinItems];
+#pragma unroll
+    for (int k = 0; k < kBinItems; ++k) v[k] = 0;
+    if (c0 < ncell) {
+        int4* src = (int4*)(a.cell_count + c0);
+        *(int4*)v = __ldcg(src);
+        *(int4*)(v + 4) = __ldcg(src + 1);
+        src[0] = make_int4(0, 0, 0, 0);
+        src[1] = make_int4(0, 0, 0, 0);
+    }
+    int sum = 0;
+#pragma unroll
+    for (int k = 0; k < kBinItems; ++k) sum += v[k];
+    int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += u;
+    }
+    if (lane == 31) s_warp[wl] = incl;
+    __syncthreads();
+    int total = 0;
+    for (int w = 0; w < kBinThreads / 32; ++w) {
+        if (w < wl) before += s_warp[w];
+        total += s_warp[w];
+    }
+    int at = before + incl - sum;
+#pragma unroll
+    for (int k = 0; k < kBinItems; ++k) {
+        if (c0 + k < ncell) a.cell_start[c0 + k] = at;
+        at += v[k];
+    }
+    __syncthreads();
+    return total;
+}
+
 static __global__ void __launch_bounds__(kBinThreads) k_bin_count(BinArgs a) {
     __shared__ bool s_last;
-    __shared__ int s_warp[kBinThreads / 32];
+    __shared__ int s_warp[kBinThreads / 32], s_tile[kBinTiles];
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (a.tiles) {
+        if (threadIdx.x < kBinTiles) s_tile[threadIdx.x] = 0;
+        __syncthreads();
+    }
     if (i < a.n) {
         int c3[3];
         const int c = cell_of(a.box, a.nc, a.pos + 3 * i, c3);
         a.atom_cell[i] = c;
         a.rank[i] = atomicAdd(a.cell_count + c, 1);
+        if (a.tiles) atomicAdd(s_tile + c / kBinTile, 1);
     }
     for (int k = i; k < a.nzero; k += gridDim.x * blockDim.x) a.zero[k] = 0;
+    if (a.tiles) {
+        __syncthreads();
+        if (threadIdx.x < kBinTiles && s_tile[threadIdx.x]) atomicAdd(a.tiles + threadIdx.x, s_tile[threadIdx.x]);
+        return;
+    }
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) s_last = atomicAdd(a.done, 1u) == gridDim.x - 1;
@@ -243,53 +298,26 @@ static __global__ void __launch_bounds__(kBinThreads) k_bin_count(BinArgs a) {
     if (!s_last) return;
     __threadfence();
     const int ncell = a.nc[0] * a.nc[1] * a.nc[2];
-    const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
-    int carry = 0;
-    for (int t0 = 0; t0 < ncell; t0 += kBinThreads * kBinItems) {
-        const int c0 = t0 + kBinItems * threadIdx.x;
-        int v[kBinItems];
-#pragma unroll
-        for (int k = 0; k < kBinItems; ++k) v[k] = 0;
-        if (c0 < ncell) {
-            int4* src = (int4*)(a.cell_count + c0);
-            *(int4*)v = __ldcg(src);
-            *(int4*)(v + 4) = __ldcg(src + 1);
-            src[0] = make_int4(0, 0, 0, 0);
-            src[1] = make_int4(0, 0, 0, 0);
-        }
-        int sum = 0;
-#pragma unroll
-        for (int k = 0; k < kBinItems; ++k) sum += v[k];
-        int incl = sum;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int u = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += u;
-        }
-        if (lane == 31) s_warp[wl] = incl;
-        __syncthreads();
-        int before = carry, total = 0;
-        for (int w = 0; w < kBinThreads / 32; ++w) {
-            if (w < wl) before += s_warp[w];
-            total += s_warp[w];
-        }
-        int at = before + incl - sum;
-#pragma unroll
-        for (int k = 0; k < kBinItems; ++k) {
-            if (c0 + k < ncell) a.cell_start[c0 + k] = at;
-            at += v[k];
-        }
-        carry += total;
-        __syncthreads();
-    }
+    int before = 0;
+    for (int t0 = 0; t0 < ncell; t0 += kBinTile) before += bin_tile(a, ncell, t0, before, s_warp);
     if (threadIdx.x == 0) {
         a.cell_start[ncell] = a.n;
         *a.done = 0u;
     }
 }
 
+static __global__ void __launch_bounds__(kBinThreads) k_bin_scan(BinArgs a) {
+    __shared__ int s_warp[kBinThreads / 32];
+    static_assert(kBinTiles <= 64, "two tiles a lane");
+    const int ncell = a.nc[0] * a.nc[1] * a.nc[2], t = blockIdx.x, lane = threadIdx.x & 31;
+    const int before = __reduce_add_sync(0xffffffffu, (lane < t ? a.tiles[lane] : 0) + (lane + 32 < t ? a.tiles[lane + 32] : 0));
+    bin_tile(a, ncell, t * kBinTile, before, s_warp);
+    if (t == 0 && threadIdx.x == 0) a.cell_start[ncell] = a.n;
+}
+
 static __global__ void k_bin_fill(BinArgs a) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (a.tiles && i < kBinTiles) a.tiles[i] = 0;
     if (i >= a.n) return;
     // the image inside the box: FP32 then resolves a distance to about 1e-7 of the box, however far
     // the caller's coordinates have drifted
