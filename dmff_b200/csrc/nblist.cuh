@@ -7,7 +7,7 @@
 // runs in FP64 with every product and sum rounded separately in a fixed order, so the pair set
 // is reproducible bit for bit by an elementwise float64 computation on the host.
 //
-// The engine's builds: k_bin_count + k_bin_fill sort the atoms into half-width cells, one pass of
+// The engine's builds: k_bin_count (+ k_bin_scan) + k_bin_fill sort the atoms into half-width cells, one pass of
 // k_pairs_cell (k_pairs_flat in boxes below five such cells) runs the distance tests and leaves each
 // atom's rows in its slots, and k_nb_place scans the counts and copies the slots to their final
 // places.  The kernels before those (k_cell_count .. k_pairs_warp: cells at least rc wide, 27-cell
@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(256) k_pairs_warp(NbArgs a) {
 
 // ------------------------------------------------------------------ the engine's builds
 //
-// Counting sort of the atoms into the cells, in two launches.  k_bin_count takes each atom's cell
+// Counting sort of the atoms into the cells, in two launches (three for many cells).  k_bin_count takes each atom's cell
 // and its arrival rank there; the last CTA to finish scans the counts into cell_start and clears
 // them for the next call (they are zero between calls), so no memset, no library scan and no
 // cursor array.  k_bin_fill writes the cell-ordered float4 positions (x, y, z, atom index as int
