@@ -5,6 +5,7 @@
 #include <cufft.h>
 #include <cub/cub.cuh>
 
+#include <climits>
 #include <cmath>
 #include <cstdlib>
 #include <cstdio>
@@ -1460,6 +1461,8 @@ int solve_dipoles(dmffb_engine* h, cudaStream_t s, const double* pos, const Box&
         done = fused && h->h_scal[CGS_DONE] != 0.0;
         return DMFFB_OK;
     };
+    // the persistent solve takes max_iter steps at most, this one up to the first read past them
+    const int limit = small ? h->max_iter : INT_MAX;
     int last = 0;  // the read before this one and its residual
     double last_rms = 0.0;
     if (fused && u0 && !rhs && h->cg_hint > 0) {
@@ -1467,7 +1470,7 @@ int solve_dipoles(dmffb_engine* h, cudaStream_t s, const double* pos, const Box&
         if ((st = run_steps(it)) || (st = read_residual())) return st;
         last = (int)h->h_scal[CGS_LAST];
         last_rms = h->h_scal[CGS_LAST_RMS];
-        const int next = (int)h->h_scal[CGS_NEXT];
+        const int next = std::min((int)h->h_scal[CGS_NEXT], limit);
         if (!done && next > it) {
             if ((st = run_steps(next - it)) || (st = read_residual())) return st;
             it = next;
@@ -1484,7 +1487,8 @@ int solve_dipoles(dmffb_engine* h, cudaStream_t s, const double* pos, const Box&
             break;
         }
         if (it >= h->max_iter) break;
-        const int k = fused ? cg_segment(it, rms, last, last_rms, h->cg_tol * rms_b) : kCgCheckEvery;
+        const int seg = fused ? cg_segment(it, rms, last, last_rms, h->cg_tol * rms_b) : kCgCheckEvery;
+        const int k = std::min(seg, limit - it);
         last = it;
         last_rms = rms;
         if ((st = run_steps(k))) return st;

@@ -55,3 +55,24 @@ def test_persistent_and_replayed_solves_take_the_same_steps(tol):
     eng = _engine(s, precision="fp32", cg_tol=tol)
     n = [_solve(eng, pos, s["box"])[0] for _ in range(4)]  # persistent, then captured and replayed
     assert len(set(n)) == 1, n
+
+
+@pytest.mark.parametrize("max_iter", [1, 4, 6, 7, 8])
+def test_step_limit_of_small_systems(max_iter):
+    """Direct, replayed and persistent solves that run into max_iter stop there."""
+    s = serving_system(200, 12)
+    pos = torch.tensor(s["pos"], dtype=torch.float64, device="cuda")
+    from dmff_b200.engine import AdmpEngine
+    sc = [0.0, 0.0, 1.0, 1.0, 1.0, 1.0]
+    eng = AdmpEngine(len(s["pos"]), 2, True, True, s["rc"], s["kappa"], s["K"], s["axis_types"], s["axis_indices"],
+                     s["cov_rows"], sc, sc, [1.0] * 6, precision="fp32", cg_tol=1e-9, max_iter=max_iter)
+    eng.set_params(s["Q_local"], s["pol"], s["thole"])
+    eng.set_zero_guess(True)
+    out = []
+    for _ in range(4):
+        eng.rebuild_internal_pairs(pos, s["box"])
+        r, _, U = eng.compute(pos, s["box"])
+        out.append((r.n_iter, r.converged, U.cpu().numpy().copy()))
+    assert [(n, c) for n, c, _ in out] == [(max_iter, 0)] * 4
+    for _, _, U in out[1:]:
+        assert np.abs(U - out[0][2]).max() <= 1e-5 * np.abs(out[0][2]).max()
