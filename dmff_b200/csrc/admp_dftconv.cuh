@@ -17,12 +17,6 @@
 //
 // Transforms are unnormalised in both directions (the convention the gather expects).  The DFT
 // matrices hold cos and sin of 2 pi a b / K, a, b = 0 .. K/2, rounded from FP64; G is multiplied in FP64.
-//
-// An FP32 spline value is multiplied by the FP32 reciprocals of 3 and 5, 3.0e-8 and 1.5e-8 too large: a site's
-// charge arrives on the mesh 1.34e-7 too large, and every reciprocal energy comes out 2.7e-7 too large.  cuFFT's
-// own error, of -2.5e-7 to +2e-7 by the extent, adds to that or hides it; the direct sums here have none to speak
-// of (below 3e-8), so G carries the factor's inverse (dft_norm).  Reciprocal energies of 1500 and 6000 atoms, RMS
-// error of 40 boxes (kJ/mol): 36^3 2.3e-3 without it, 7e-4 with it, cuFFT 1.6e-3; 45^3 5.6e-3, 1.3e-3, 1.1e-3.
 #pragma once
 #include "admp_recip.cuh"
 #include "common.cuh"
@@ -60,12 +54,6 @@ struct DftConvArgs {
     double* scal;         // [0] energy, [1..6] k-space tensor
     T* zero_real;         // mesh of K0*K1*K2 elements the column pass sets to 0 (may be null)
 };
-
-// what G is multiplied by for the splines' common factor: two sites' charges, three axes
-template <typename T> __host__ __device__ inline double dft_norm() {
-    const double f = 15.0 * (double)T(1.0 / 3.0) * (double)T(0.2), f3 = f * f * f;
-    return sizeof(T) == 4 ? 1.0 / (f3 * f3) : 1.0;
-}
 
 // work items of each pass
 template <typename T> __host__ __device__ inline int dft_fwd_items(const DftConvArgs<T>& a) {
@@ -313,7 +301,7 @@ __device__ __forceinline__ double dft_influence(const DftConvArgs<T>& a, int kx,
     if (m1 == 0 && m2 == 0 && m3 == 0 && a.kind == CK_COUL) return 0.0;
     double Cv, dlnC;
     influence(a.kind, ksq, a.kappa, a.V, Cv, dlnC);
-    const double G = Cv / (th * th) * dft_norm<T>();
+    const double G = Cv / (th * th);
     if (a.want_energy) {
         const double w = (kz == 0 || 2 * kz == a.K[2]) ? 1.0 : 2.0;
         const double Ek = a.escale * w * G * ((double)re * re + (double)im * im);
@@ -578,8 +566,7 @@ template <typename T> __host__ inline size_t dft_inv_smem(const DftConvArgs<T>& 
 }
 
 // influence function of the half spectrum (k = 0: 0), for the passes of a dipole solve
-static __global__ void k_dft_gtable(int K0, int K1, int K2, Box b, const double* bmod, double kappa, double V, double norm,
-                                    double* G) {
+static __global__ void k_dft_gtable(int K0, int K1, int K2, Box b, const double* bmod, double kappa, double V, double* G) {
     const int hz = K2 / 2 + 1;
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (int64_t)K0 * K1 * hz) return;
@@ -597,7 +584,7 @@ static __global__ void k_dft_gtable(int K0, int K1, int K2, Box b, const double*
         double C, dln;
         influence(CK_COUL, ksq, kappa, V, C, dln);
         const double th = bmod[k1] * bmod[K0 + k2] * bmod[K0 + K1 + k3];
-        g = C / (th * th) * norm;
+        g = C / (th * th);
     }
     G[idx] = g;
 }

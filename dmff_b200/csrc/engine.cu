@@ -751,9 +751,7 @@ int dft_gtable(dmffb_engine* h, cudaStream_t s, const Box& bx) {
         h->dftG_cap = m;
     }
     LAUNCH(h, s, KC_VEC, k_dft_gtable<<<nblk(m, 256), 256, 0, s>>>(h->K[0], h->K[1], h->K[2], bx, h->d_bmod, h->kappa,
-                                                                  fabs(det3(bx.h)),
-                                                                  h->prec == DMFFB_FP32 ? dft_norm<float>() : dft_norm<double>(),
-                                                                  h->d_dftG));
+                                                                  fabs(det3(bx.h)), h->d_dftG));
     CK(cudaGetLastError());
     return DMFFB_OK;
 }
